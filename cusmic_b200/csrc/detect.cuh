@@ -608,21 +608,42 @@ __device__ __forceinline__ void candidate_eval(const FrameDesc &fd, uint2 t, lon
 	}
 }
 
-// The first pass's evaluation of a noise-model candidate at least two pixels
-// from every edge by one thread: its 25 window values from the sig_raw map
-// (region_sig_kernel), their median by a sorting network (NaN-free windows:
-// any network gives the median's value, a zero's sign aside, which no
-// threshold sees), the S1 / S2 bits and the seed slot, as candidate_eval.
-// Returns false for a window holding a NaN (the warp's NaN rule decides it).
+// The first pass's evaluation of a noise-model candidate by one thread: its 25
+// window values from the sig_raw map (region_sig_kernel), their median by a
+// sorting network (NaN-free windows: any network gives the median's value, a
+// zero's sign aside, which no threshold sees), the S1 / S2 bits and the seed
+// slot, as candidate_eval.  A window cell past an edge reads its border-mapped
+// pixel (zero in constant mode), which mirror, reflect and nearest keep within
+// two pixels of the candidate, so the map holds it; wrap maps it to the far
+// side of the frame.  (A warp evaluating each edge candidate on its own, 25
+// border-mapped noise medians per lane, held the launch for 121 us on a
+// 1531 x 1023 frame with maps, 154 us on five of 1018 x 1001 and 122 us on 256
+// cutouts of 40 to 200 pixels; those calls went from 853 to 770, 1193 to 1058
+// and 736 to 593 us.)  Returns false for a candidate within two pixels of an
+// edge under wrap and for a window holding a NaN: the warp evaluates those.
 __device__ __forceinline__ bool map_candidate(const FrameDesc &fd, uint2 t, long long e, int x, int y,
 	const DetectParams &prm, Seed *seeds)
 {
-	const int w = fd.w;
+	const int w = fd.w, h = fd.h;
+	const bool inside = x >= 2 && y >= 2 && x + 2 < w && y + 2 < h;
+	if (!inside && prm.mode == WRAP)
+		return false;
+	int mx[5], my[5];
+#pragma unroll
+	for (int i = 0; i < 5; ++i) {
+		mx[i] = x + i - 2;
+		my[i] = y + i - 2;
+		if (!inside) {
+			mx[i] = border_index(mx[i], w, prm.mode);
+			my[i] = border_index(my[i], h, prm.mode);
+		}
+	}
 	double v[25];
 	bool nan = false;
 #pragma unroll
 	for (int c = 0; c < 25; ++c) {
-		v[c] = fd.sig_raw[(long long)(y + c / 5 - 2) * w + x + c % 5 - 2];
+		const int cx = mx[c % 5], cy = my[c / 5];
+		v[c] = (cx | cy) < 0 ? 0.0 : fd.sig_raw[(long long)cy * w + cx];
 		nan |= isnan(v[c]);
 	}
 	if (nan)
@@ -675,7 +696,7 @@ candidate_high_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restr
 
 // B, high list, first pass on noise-model frames: a thread per candidate
 // whose window the sig_raw map holds (map_candidate); the warp evaluates the
-// others (frame edges, windows with a NaN) one after another with
+// others (wrap's frame edges, windows with a NaN) one after another with
 // candidate_eval.  Its own launch bounds: the thread path holds 25 window
 // values, the warp path (candidate_high_kernel) runs at four blocks per SM.
 __global__ void __launch_bounds__(256, 2)
@@ -699,8 +720,7 @@ candidate_map_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restri
 			const FrameDesc &fd = frames[t.x];
 			if (serves<PATH>(fd)) {
 				const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
-				defer = !(fd.sig_raw && x >= 2 && y >= 2 && x + 2 < fd.w && y + 2 < fd.h &&
-					map_candidate(fd, t, e, x, y, prm, seeds));
+				defer = !(fd.sig_raw && map_candidate(fd, t, e, x, y, prm, seeds));
 			}
 		}
 		for (unsigned m = __ballot_sync(0xffffffffu, defer); m; m &= m - 1) {
