@@ -776,8 +776,8 @@ __device__ __forceinline__ void classify_flush(ClassifyStage &H, ClassifyStage &
 	__syncthreads();
 	const int nh = min(H.n, H.fail), nl = min(L.n, L.fail);
 	if (threadIdx.x == 0) {
-		bases[0] = nh ? atomicAdd(&ctl->n_cand, (unsigned long long)nh) : 0ull;
-		bases[1] = nl ? atomicAdd(&ctl->n_low, (unsigned long long)nl) : 0ull;
+		bases[0] = nh ? atomicAdd(&ctl->pass[0].n_cand, (unsigned long long)nh) : 0ull;
+		bases[1] = nl ? atomicAdd(&ctl->pass[0].n_low, (unsigned long long)nl) : 0ull;
 	}
 	__syncthreads();
 	const unsigned long long cap = ctl->cand_cap;
@@ -867,8 +867,8 @@ classify_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restri
 					}
 				}
 				const uint2 entry = make_uint2((unsigned)f, pix);
-				classify_stage(H, cls == 1, entry, &ctl->n_cand, cands, false, cap);
-				classify_stage(L, cls == 2, entry, &ctl->n_low, cands, true, cap);
+				classify_stage(H, cls == 1, entry, &ctl->pass[0].n_cand, cands, false, cap);
+				classify_stage(L, cls == 2, entry, &ctl->pass[0].n_low, cands, true, cap);
 			}
 		}
 		__syncthreads();

@@ -40,15 +40,16 @@ enum Plane {
 	P_S1,     // significance > cr_threshold
 	P_S2,     // significance > neighbor_threshold
 	P_CAND,   // seed: S1, not excluded, contrast test passed
-	P_FRESH,  // pixels the last growth step added to the mask
-	P_CHG,    // pixels whose value the last replacement changed
+	P_FRESH,  // pixels that the last late pass added to the mask
+	P_EVAL,   // late passes: pixels claimed for re-evaluation (zero between passes)
+	P_LISTED, // late passes: pixels claimed for the work lists (zero between passes)
 	P_ROWMIN, // noise-model frames: per row and bit word, the smallest high word of
 	          // the ordered keys of its finite input pixels (all ones: none)
 	N_PLANES
 };
 
-static_assert(P_S2 == P_S1 + 1 && P_CAND == P_S1 + 2 && P_FRESH == P_S1 + 3,
-	"S1, S2, CAND and FRESH are zeroed as one range before a full pass");
+static_assert(P_S2 == P_S1 + 1 && P_CAND == P_S1 + 2,
+	"S1, S2 and CAND are zeroed as one range (clear_detect_words)");
 
 constexpr double FINE_FLOOR = 0.01;   // reference src/filters.cuh:21
 constexpr double SIGNAL_FLOOR = 1e-5; // reference src/filters.cuh:22
@@ -65,6 +66,12 @@ CB_HD int border_index(int x, int n, int mode)
 		return x < 0 ? 0 : n - 1;
 	if (n == 1)
 		return 0;
+	// One reflection or turn (the windows' offsets are a few pixels) without
+	// the divisions of the general case.
+	const int once = mode == REFLECT ? (x < 0 ? -x - 1 : 2 * n - 1 - x)
+		: mode == MIRROR ? (x < 0 ? -x : 2 * (n - 1) - x) : (x < 0 ? x + n : x - n);
+	if (once >= 0 && once < n)
+		return once;
 	int period = mode == REFLECT ? 2 * n : mode == MIRROR ? 2 * (n - 1) : n;
 	x %= period;
 	if (x < 0)
@@ -104,8 +111,6 @@ struct FrameDesc {
 	uint8_t *mask_out; // uint8 output mask
 	uint32_t *bits;    // N_PLANES planes of `plane` words
 	BlockFloor *floors; // the frame's block floors, row-major by block (null: none)
-	uint32_t *rowcand;  // per row: nonzero when growth must visit the row this pass (null: all)
-	uint32_t *rowchg;   // per row: nonzero when the row has a CHG pixel (null: no tracking)
 	// Noise-model frames, first pass: sig_raw and the noise at every pixel
 	// within two of a HIGH pixel (region_sig_kernel), which the high-list
 	// candidates read instead of recomputing their windows (null: none).
@@ -117,36 +122,43 @@ struct FrameDesc {
 	int w, h, words, has_bg;
 };
 
-// Device-side control state of a frame.
+// Device-side control state of a frame.  Passes are numbered from 0; what a
+// pass appends or flags is kept by the pass's parity, so the next pass can
+// start from it while its own is still empty.
 struct FrameState {
 	unsigned int active;  // the next detection pass runs for this frame
-	unsigned int replace; // this pass flagged new pixels: re-replace targets
 	unsigned int error;   // a target had no finite donor
 	unsigned int passes;  // detection passes run
 	unsigned int fault;   // a bounded wait inside a kernel ran out (the frame stopped)
-	// Nonzero-only facts (set to 1 by many warps, never counted):
-	unsigned long long todo;                  // this pass: any new pixel
-	long long donors_left;                    // static donors not in the mask (counted)
-	unsigned long long holes, allowed, finite; // any hole, any allowed pixel, any finite donor
+	unsigned int todo[2]; // by parity: the pass flagged a new pixel (set by many warps)
+	long long donors_left; // static donors not in the mask (counted)
+	// Nonzero-only facts (set to 1 by many warps, never counted): any hole,
+	// any allowed pixel, any finite donor.
+	unsigned long long holes, allowed, finite;
+};
+
+// Lengths of one pass's work lists.
+struct PassLists {
+	unsigned long long n_cand; // high list: pixels whose significance is evaluated
+	unsigned long long n_low;  // low list: pixels whose sig_raw can only exceed neighbor
+	unsigned long long n_eval; // late passes: pixels whose sig_raw is evaluated again
+	unsigned long long n_chg;  // targets whose value the replacement before changed
 };
 
 // Loop control shared by the per-pass kernels.
 struct Control {
 	unsigned long long n_targets; // length of the target list
 	unsigned long long n_holes;   // length of the hole list prepare_kernel writes
-	unsigned long long n_cand;    // this pass: pixels whose sig_raw can exceed cr_threshold
-	unsigned long long n_low;     // this pass: pixels whose sig_raw can only exceed neighbor
-	unsigned long long cand_cap;  // capacity of the candidate buffer (high from the front,
-	                              // low from the back)
-	int iter;                     // detection passes issued so far
-	int maxiter;
-	int any_active;
-	int ticket;                   // next item of the bulk detection kernel (reset every pass)
-	int fault;                    // a bounded wait ran out in this pass
-	int n_dirty;                  // this pass: length of the dirty-row list
-	unsigned n_sel;               // this pass: targets the replacement visits
-	unsigned pad;
+	unsigned long long cand_cap;  // capacity of the candidate buffer (first pass: high from
+	                              // the front, low from the back)
+	PassLists pass[2];            // by parity
 	unsigned long long n_region;  // first pass: pixels of the noise-model sig_raw map (listed)
+	unsigned long long fresh0;    // late passes: targets listed before the last growth
+	int any[2];                   // by parity: a frame goes on after the pass
+	int ticket;                   // next item of the bulk detection kernel
+	int fault;                    // a bounded wait ran out
+	unsigned barrier;             // arrivals at the late passes' grid barriers
+	unsigned pad;
 	// Injected failures (0: none): the bound, in SM cycles, of one extra wait
 	// on a barrier that nothing completes, made by one warp of the first block
 	// of the bulk-staged prepare ([0]) and of the dense detection kernel ([1]).

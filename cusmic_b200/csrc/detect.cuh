@@ -141,10 +141,10 @@ __device__ __forceinline__ void clear_detect_words(const FrameDesc &fd, long lon
 // row y0 + k) with a single atomic per item; the high list grows from the
 // front of the buffer, the low list from its back.
 __device__ __forceinline__ void stream_flush(int f, int w, int x, int y0, uint32_t hi, uint32_t lo,
-	Control *ctl, uint2 *cands)
+	Control *ctl, int par, uint2 *cands)
 {
 	if (__any_sync(0xffffffffu, hi != 0)) {
-		unsigned long long slot = warp_append(&ctl->n_cand, __popc(hi));
+		unsigned long long slot = warp_append(&ctl->pass[par].n_cand, __popc(hi));
 		while (hi) {
 			const int k = __ffs(hi) - 1;
 			hi &= hi - 1;
@@ -152,7 +152,7 @@ __device__ __forceinline__ void stream_flush(int f, int w, int x, int y0, uint32
 		}
 	}
 	if (__any_sync(0xffffffffu, lo != 0)) {
-		unsigned long long slot = warp_append(&ctl->n_low, __popc(lo));
+		unsigned long long slot = warp_append(&ctl->pass[par].n_low, __popc(lo));
 		while (lo) {
 			const int k = __ffs(lo) - 1;
 			lo &= lo - 1;
@@ -238,7 +238,7 @@ __device__ __forceinline__ void stream_issue(StreamRing &R, const FrameDesc &fd,
 
 __global__ void __launch_bounds__(256)
 sig_stream_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
-	const int4 *__restrict__ items, int nitems, DetectParams prm, Control *ctl, uint2 *cands)
+	const int4 *__restrict__ items, int nitems, DetectParams prm, Control *ctl, int par, uint2 *cands)
 {
 	__shared__ StreamRing rings[8];
 	const int lane = threadIdx.x & 31;
@@ -285,15 +285,15 @@ sig_stream_kernel(const FrameDesc *__restrict__ frames, const FrameState *__rest
 		}
 		cp_async_wait<0>();
 		__syncwarp();
-		stream_flush(item.x, w, x, y0, hi, lo, ctl, cands);
+		stream_flush(item.x, w, x, y0, hi, lo, ctl, par, cands);
 	}
 }
 
 __device__ __forceinline__ void tile_flush(int f, int w, int x, int ybase, uint32_t hi, uint32_t lo,
-	Control *ctl, uint2 *cands)
+	Control *ctl, int par, uint2 *cands)
 {
 	if (__any_sync(0xffffffffu, hi != 0)) {
-		unsigned long long slot = warp_append(&ctl->n_cand, __popc(hi));
+		unsigned long long slot = warp_append(&ctl->pass[par].n_cand, __popc(hi));
 		while (hi) {
 			const int j = __ffs(hi) - 1;
 			hi &= hi - 1;
@@ -301,7 +301,7 @@ __device__ __forceinline__ void tile_flush(int f, int w, int x, int ybase, uint3
 		}
 	}
 	if (__any_sync(0xffffffffu, lo != 0)) {
-		unsigned long long slot = warp_append(&ctl->n_low, __popc(lo));
+		unsigned long long slot = warp_append(&ctl->pass[par].n_low, __popc(lo));
 		while (lo) {
 			const int j = __ffs(lo) - 1;
 			lo &= lo - 1;
@@ -322,7 +322,7 @@ __device__ __forceinline__ void tile_flush(int f, int w, int x, int ybase, uint3
 // noise make noise(m_lo) one value per tile; maps evaluate it per pixel.
 __global__ void __launch_bounds__(256)
 sig_model_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
-	const int4 *__restrict__ tiles, int ntiles, DetectParams prm, Control *ctl, uint2 *cands)
+	const int4 *__restrict__ tiles, int ntiles, DetectParams prm, Control *ctl, int par, uint2 *cands)
 {
 	__shared__ double C[MHALO * MHALO];
 	__shared__ double wmin[8];
@@ -386,7 +386,7 @@ sig_model_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restr
 		}
 		// Bits j of this lane are rows y0 + warp + 8 j: append as rows of a
 		// strip starting at y0 + warp with stride 8.
-		tile_flush(tile.x, w, x0 + lane, y0 + warp, hi, lo, ctl, cands);
+		tile_flush(tile.x, w, x0 + lane, y0 + warp, hi, lo, ctl, par, cands);
 		__syncthreads();
 	}
 }
@@ -395,12 +395,18 @@ sig_model_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restr
 // under the border mode).
 __device__ __noinline__ double noise_model_at(const FrameDesc &fd, int x, int y, int mode)
 {
+	int mx[5], my[5];
+#pragma unroll
+	for (int i = 0; i < 5; ++i) {
+		mx[i] = border_index(x + i - 2, fd.w, mode);
+		my[i] = border_index(y + i - 2, fd.h, mode);
+	}
 	double v[25];
 #pragma unroll
-	for (int dy = 0; dy < 5; ++dy)
-#pragma unroll
-		for (int dx = 0; dx < 5; ++dx)
-			v[dy * 5 + dx] = clean_at(fd, x + dx - 2, y + dy - 2, mode);
+	for (int c = 0; c < 25; ++c) {
+		const int cx = mx[c % 5], cy = my[c / 5];
+		v[c] = (cx | cy) < 0 ? 0.0 : fd.clean[(long long)cy * fd.w + cx];
+	}
 	return noise_from_median(fd, (long long)y * fd.w + x, median_network(v));
 }
 
@@ -672,14 +678,14 @@ __device__ __forceinline__ bool map_candidate(const FrameDesc &fd, uint2 t, long
 template <int PATH>
 __global__ void __launch_bounds__(256, 4)
 candidate_high_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restrict__ cands,
-	DetectParams prm, Control *ctl, Seed *seeds, int fresh)
+	DetectParams prm, Control *ctl, int par, Seed *seeds)
 {
 	__shared__ double patches[8][81];
 	__shared__ double scratch[8][CS_RUNS];
 	double *P = patches[threadIdx.x >> 5], *S = scratch[threadIdx.x >> 5];
 	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
 	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	const long long n = (long long)ctl->n_cand;
+	const long long n = (long long)ctl->pass[par].n_cand;
 	uint2 next = gw < n ? cands[gw] : make_uint2(0u, 0u);
 	for (long long e = gw; e < n; e += nw) {
 		const uint2 t = next;
@@ -690,7 +696,7 @@ candidate_high_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restr
 			continue; // warp-uniform
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 		const bool hole = test_bit(plane_ptr(fd, P_HOLE), fd.words, x, y);
-		candidate_eval<false, PATH>(fd, t, e, x, y, P, S, prm, seeds, fresh != 0, hole);
+		candidate_eval<false, PATH>(fd, t, e, x, y, P, S, prm, seeds, true, hole);
 	}
 }
 
@@ -707,7 +713,7 @@ candidate_map_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restri
 	__shared__ double patches[8][81];
 	__shared__ double scratch[8][CS_RUNS];
 	double *P = patches[threadIdx.x >> 5], *S = scratch[threadIdx.x >> 5];
-	const long long n = (long long)ctl->n_cand;
+	const long long n = (long long)ctl->pass[0].n_cand;
 	const int lane = threadIdx.x & 31;
 	const long long stride = (long long)gridDim.x * blockDim.x;
 	for (long long base = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); base < n;
@@ -735,49 +741,242 @@ candidate_map_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restri
 	}
 }
 
-// B, low list (run after the seed kernel): a lane per candidate first tests
-// its clipped 5 x 5 neighbourhood of the CAND plane with five 36-bit row
-// windows (S2 is read only by the second growth step, within distance 2 of a
-// CAND pixel) and its hole bit; the warp then evaluates the survivors.
+// Growth (reference src/filters.cuh:177-193 twice, src/cleaner.cuh:123-125):
+// grown = dilate3x3(dilate3x3(CAND) & S1) & S2, clipped to the frame; fresh =
+// grown & ~CRMASK joins the mask and the target list (src/cleaner.cuh:22-37).
+//
+// It is driven by the work lists, a thread per listed pixel, because what can
+// grow lies within two pixels of one: 58,520 of 67 million pixels are CAND on
+// 16 frames of 2048 x 2048.  (The row sweeps over the bit planes that this
+// replaced took 126 us in the four passes of those frames, bound by their
+// chains of dependent word loads, most of which found nothing.)
+//
+// first: the pass's planes were zeroed, so everything that grows grows from a
+// CAND pixel's own 5 x 5 neighbourhood.  Otherwise pixels may also grow
+// because an S1 or S2 bit near an old CAND pixel was set; every bit set in the
+// pass belongs to a listed pixel, and the S1 cells within one pixel of it that
+// touch a CAND pixel dilate into its 5 x 5 neighbourhood.  There a
+// LOW pixel's S2 bit may date from an earlier pass (it is evaluated again, on
+// its own, wherever its CAND neighbourhood changed), so only HIGH pixels count.
+
+// What the growth around a pixel reads: five columns around x (bits5) of the
+// rows around y, all loaded before any is used (one memory round trip).
+struct GrowthRows {
+	uint32_t c[5], s1[3], s2[5], in[5], donor[5]; // CAND, S1, S2, CRMASK, DONOR
+};
+
+// own: the pixel is CAND, which alone decides (CAND is not read).  first: any
+// S2 pixel may grow, else only HIGH ones.
+__device__ __forceinline__ void growth_load(const FrameDesc &fd, int x, int y, bool own, bool first,
+	GrowthRows &G)
+{
+	const uint32_t *cand = plane_ptr(fd, P_CAND), *s1 = plane_ptr(fd, P_S1), *s2 = plane_ptr(fd, P_S2);
+	const uint32_t *high = plane_ptr(fd, P_HIGH), *crm = plane_ptr(fd, P_CRMASK), *don = plane_ptr(fd, P_DONOR);
+	const int words = fd.words, h = fd.h;
+	uint32_t hi[5];
+#pragma unroll
+	for (int j = 0; j < 5; ++j) {
+		const int yy = y - 2 + j;
+		const bool in = yy >= 0 && yy < h;
+		G.c[j] = own ? 4u : in ? bits5(cand, words, x, yy) : 0u;
+		G.s2[j] = in ? bits5(s2, words, x, yy) : 0u;
+		hi[j] = first ? 0x1fu : in ? bits5(high, words, x, yy) : 0u;
+		G.in[j] = in ? bits5(crm, words, x, yy) : 0u;
+		G.donor[j] = in ? bits5(don, words, x, yy) : 0u;
+		if (j >= 1 && j <= 3)
+			G.s1[j - 1] = in ? bits5(s1, words, x, yy) : 0u;
+	}
+#pragma unroll
+	for (int j = 0; j < 5; ++j)
+		G.s2[j] &= hi[j];
+}
+
+// The pixels to flag around the pixel, per row (bit i: column x - 2 + i): the
+// S1 cells of the 3 x 3 neighbourhood that touch a CAND pixel, dilated, with
+// S2 set and not in the mask yet.  Returns whether there is any.
+__device__ __forceinline__ bool growth_new(const GrowthRows &G, bool own, uint32_t (&g)[5])
+{
+	uint32_t d[3];
+#pragma unroll
+	for (int i = 0; i < 3; ++i) {
+		uint32_t v = own ? 4u : G.c[i] | G.c[i + 1] | G.c[i + 2];
+		v = (v | (v << 1) | (v >> 1)) & G.s1[i] & 0xeu; // columns x - 1 .. x + 1
+		d[i] = (v | (v << 1) | (v >> 1)) & 0x1fu;
+	}
+	g[0] = d[0] & G.s2[0] & ~G.in[0];
+	g[1] = (d[0] | d[1]) & G.s2[1] & ~G.in[1];
+	g[2] = (d[0] | d[1] | d[2]) & G.s2[2] & ~G.in[2];
+	g[3] = (d[1] | d[2]) & G.s2[3] & ~G.in[3];
+	g[4] = d[2] & G.s2[4] & ~G.in[4];
+	return (g[0] | g[1] | g[2] | g[3] | g[4]) != 0;
+}
+
+// Puts the pixels of g (five rows of five bits around (x, y)) into the mask;
+// returns those this call put there, bit 5 j + i for column x - 2 + i of row
+// y - 2 + j, and counts the static donors among them.  The rows' atomics are
+// issued together.
+__device__ __forceinline__ uint32_t flag_pixels(const FrameDesc &fd, int x, int y, const uint32_t (&g)[5],
+	const GrowthRows &G, bool track, int &lost)
+{
+	uint32_t *crm = plane_ptr(fd, P_CRMASK), *fr = plane_ptr(fd, P_FRESH);
+	const int k = (x - 2) >> 5, s = (x - 2) & 31; // k >= -1: bits left of the frame are zero
+	const long long o = (long long)(y - 2) * fd.words + k;
+	unsigned long long old[5];
+#pragma unroll
+	for (int j = 0; j < 5; ++j) {
+		const unsigned long long wide = (unsigned long long)g[j] << s;
+		const uint32_t lo = (uint32_t)wide, hi = (uint32_t)(wide >> 32);
+		old[j] = lo ? atomicOr(crm + o + (long long)j * fd.words, lo) : 0u;
+		if (hi)
+			old[j] |= (unsigned long long)atomicOr(crm + o + (long long)j * fd.words + 1, hi) << 32;
+	}
+	uint32_t out = 0;
+#pragma unroll
+	for (int j = 0; j < 5; ++j) {
+		const uint32_t now = g[j] & ~(uint32_t)(old[j] >> s);
+		lost += __popc(now & G.donor[j]);
+		out |= now << (5 * j);
+		if (track && now) {
+			const unsigned long long wide = (unsigned long long)now << s;
+			if ((uint32_t)wide)
+				atomicOr(fr + o + (long long)j * fd.words, (uint32_t)wide);
+			if (wide >> 32)
+				atomicOr(fr + o + (long long)j * fd.words + 1, (uint32_t)(wide >> 32));
+		}
+	}
+	return out;
+}
+
+// The fresh pixels of a warp's lanes (flag_pixels masks around (x, y) of frame
+// f) into the target list and their frames' state; called by the whole warp.
+__device__ __forceinline__ void append_fresh(FrameState *state, Control *ctl, int par, uint2 *targets,
+	int f, int w, int x, int y, uint32_t fresh, int lost)
+{
+	if (!__any_sync(0xffffffffu, fresh != 0))
+		return;
+	const int lane = threadIdx.x & 31;
+	unsigned long long slot = warp_append(&ctl->n_targets, __popc(fresh));
+	// The frame's state: once for the warp when the lanes share a frame.
+	const unsigned some = __ballot_sync(0xffffffffu, fresh != 0);
+	const int lead = __ffs(some) - 1, f0 = __shfl_sync(0xffffffffu, f, lead);
+	const bool same = __all_sync(0xffffffffu, !fresh || f == f0);
+	const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)lost);
+	if (fresh) {
+		if (!same || lane == lead) {
+			const int gone = same ? sum : lost;
+			set_flag(&state[f].todo[par]);
+			if (gone)
+				atomicAdd((unsigned long long *)&state[f].donors_left,
+					(unsigned long long)(-(long long)gone));
+		}
+		for (; fresh; fresh &= fresh - 1) {
+			const int b = __ffs(fresh) - 1;
+			targets[slot++] = make_uint2((unsigned)f,
+				(unsigned)((long long)(y - 2 + b / 5) * w + (x - 2 + b % 5)));
+		}
+	}
+}
+
+// The growth around a listed pixel (see above); returns its new pixels as
+// flag_pixels.
+__device__ __forceinline__ uint32_t grow_around(const FrameDesc &fd, int x, int y, bool own, bool first,
+	int &lost)
+{
+	GrowthRows G;
+	growth_load(fd, x, y, own, first, G);
+	uint32_t g[5];
+	return growth_new(G, own, g) ? flag_pixels(fd, x, y, g, G, !first, lost) : 0u;
+}
+
+// The growth of a pixel whose own S2 bit was just found set.
+__device__ __forceinline__ uint32_t grow_self(const FrameDesc &fd, int x, int y, bool first, int &lost)
+{
+	GrowthRows G;
+	growth_load(fd, x, y, false, true, G);
+	G.s2[0] = G.s2[1] = G.s2[3] = G.s2[4] = 0u;
+	G.s2[2] = 4u;
+	uint32_t g[5];
+	return growth_new(G, false, g) ? flag_pixels(fd, x, y, g, G, !first, lost) : 0u;
+}
+
+// Any CAND pixel within two pixels of (x, y) (S2 is read only by the second
+// growth step, within that distance of a CAND pixel), and no hole there.
+__device__ __forceinline__ bool low_near(const FrameDesc &fd, int x, int y)
+{
+	const uint32_t *cand = plane_ptr(fd, P_CAND);
+	const bool hole = test_bit(plane_ptr(fd, P_HOLE), fd.words, x, y);
+	uint32_t any = 0;
+#pragma unroll
+	for (int d = -2; d <= 2; ++d)
+		any |= y + d >= 0 && y + d < fd.h ? bits5(cand, fd.words, x, y + d) : 0u;
+	return any && !hole;
+}
+
+// The warp's evaluation of a low-list pixel near a CAND pixel: its S2 bit,
+// which, when set, may grow the pixel itself.
+template <int PATH>
+__device__ __forceinline__ void low_eval(const FrameDesc *__restrict__ frames, FrameState *state, uint2 t,
+	const DetectParams &prm, Control *ctl, int par, uint2 *targets, double *P, double *S, bool fresh)
+{
+	const FrameDesc &fd = frames[t.x];
+	const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
+	double nz;
+	const double sig = candidate_sig<true, PATH>(fd, x, y, P, S, prm, nz, fresh);
+	uint32_t got = 0;
+	int lost = 0;
+	if ((threadIdx.x & 31) == 0 && sig > prm.nb)
+		got = grow_self(fd, x, y, fresh, lost);
+	append_fresh(state, ctl, par, targets, (int)t.x, fd.w, x, y, got, lost);
+}
+
+// Low list and growth of a full pass (run after the seeds): a lane per low
+// entry tests its neighbourhood, the warp evaluates the survivors one after
+// another.  `grow`: this launch grows the high list (a mixed batch launches
+// the low list once per kind of frame, and grows once).
 template <int PATH>
 __global__ void __launch_bounds__(256, PATH == PATH_ERROR ? 4 : 3)
-candidate_low_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restrict__ cands,
-	DetectParams prm, Control *ctl, int fresh)
+low_grow_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const uint2 *__restrict__ cands,
+	DetectParams prm, Control *ctl, int par, uint2 *targets, int grow)
 {
 	__shared__ double patches[8][81];
 	__shared__ double scratch[8][PATH == PATH_ERROR ? 25 : CS_RUNS];
-	const int lane = threadIdx.x & 31;
-	double *P = patches[threadIdx.x >> 5], *S = scratch[threadIdx.x >> 5];
-	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	const long long n = (long long)ctl->n_low;
-	const unsigned long long cap = ctl->cand_cap;
-	// Entries per warp and sweep: 32 for a long list; a short list (the late
-	// passes) is spread thinner so that its survivors, which a warp
-	// evaluates one after another, land on different warps.
-	const int chunk = n >= nw * 32 ? 32 : n > nw ? (int)((n + nw - 1) / nw) : 1;
-	for (long long base = gw * chunk; base < n; base += nw * chunk) {
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const long long stride = (long long)gridDim.x * blockDim.x;
+	const long long nc = grow ? (long long)ctl->pass[par].n_cand : 0, nl = (long long)ctl->pass[par].n_low;
+	const long long start = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31);
+	for (long long base = start; base < nc; base += stride) { // warp-uniform
 		const long long e = base + lane;
+		uint2 t = make_uint2(0u, 0u);
+		int w = 1, x = 0, y = 0, lost = 0;
+		uint32_t got = 0;
+		if (e < nc) {
+			t = cands[e];
+			const FrameDesc &fd = frames[t.x];
+			w = fd.w;
+			x = (int)(t.y % (unsigned)w);
+			y = (int)(t.y / (unsigned)w);
+			if (test_bit(plane_ptr(fd, P_CAND), fd.words, x, y))
+				got = grow_around(fd, x, y, true, true, lost);
+		}
+		append_fresh(state, ctl, par, targets, (int)t.x, w, x, y, got, lost);
+	}
+	const unsigned long long cap = ctl->cand_cap;
+	const long long gw = start >> 5, nw = stride >> 5;
+	// The entries are dealt to the warps one by one: neighbouring entries,
+	// whose survivors come in clusters, land on different warps.
+	for (long long base = gw; base < nl; base += nw * 32) { // warp-uniform
+		const long long e = base + lane * nw;
 		uint2 t = make_uint2(0, 0);
 		bool near = false;
-		if (lane < chunk && e < n) {
+		if (e < nl) {
 			t = cands[cap - 1 - e];
 			const FrameDesc &fd = frames[t.x];
-			const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
-			const uint32_t *cand = plane_ptr(fd, P_CAND);
-			unsigned long long any = 0;
-#pragma unroll
-			for (int d = -2; d <= 2; ++d)
-				any |= bit_window(cand, fd.words, fd.h, y + d, x >> 5);
-			near = serves<PATH>(fd) && ((any >> (x & 31)) & 0x1full) &&
-				!test_bit(plane_ptr(fd, P_HOLE), fd.words, x, y);
+			near = serves<PATH>(fd) && low_near(fd, (int)(t.y % (unsigned)fd.w), (int)(t.y / (unsigned)fd.w));
 		}
 		for (unsigned m = __ballot_sync(0xffffffffu, near); m; m &= m - 1) {
 			const int j = __ffs(m) - 1;
 			const uint2 tj = make_uint2(__shfl_sync(0xffffffffu, t.x, j), __shfl_sync(0xffffffffu, t.y, j));
-			const FrameDesc &fd = frames[tj.x];
-			candidate_eval<true, PATH>(fd, tj, base + j, (int)(tj.y % (unsigned)fd.w),
-				(int)(tj.y / (unsigned)fd.w), P, S, prm, nullptr, fresh != 0);
+			low_eval<PATH>(frames, state, tj, prm, ctl, par, targets, patches[warp], scratch[warp], true);
 		}
 	}
 }
@@ -865,11 +1064,18 @@ __device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, dou
 						qx = clampi(qx, 0, w - 1);
 						qy = clampi(qy, 0, h - 1);
 					}
-					m = median9(clean_at(fd, qx - 1, qy - 1, mode), clean_at(fd, qx, qy - 1, mode),
-						clean_at(fd, qx + 1, qy - 1, mode), clean_at(fd, qx - 1, qy, mode),
-						clean_at(fd, qx, qy, mode), clean_at(fd, qx + 1, qy, mode),
-						clean_at(fd, qx - 1, qy + 1, mode), clean_at(fd, qx, qy + 1, mode),
-						clean_at(fd, qx + 1, qy + 1, mode));
+					int mx[3], my[3];
+#pragma unroll
+					for (int i = 0; i < 3; ++i) {
+						mx[i] = border_index(qx + i - 1, w, mode);
+						my[i] = border_index(qy + i - 1, h, mode);
+					}
+					double v[9];
+#pragma unroll
+					for (int c = 0; c < 9; ++c)
+						v[c] = (mx[c % 3] | my[c / 3]) < 0 ? 0.0
+							: fd.clean[(long long)my[c / 3] * w + mx[c % 3]];
+					m = median9(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]);
 				}
 				m3[s] = m;
 			}
@@ -883,22 +1089,19 @@ __device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, dou
 	if (lane == 0)
 		write_bit(plane_ptr(fd, P_CAND) + (long long)y * fd.words + (x >> 5), 1u << (x & 31), cand,
 			fresh);
-	// Growth can flag pixels within two rows of a CAND pixel.
-	if (cand && fd.rowcand && lane < 5 && y + lane - 2 >= 0 && y + lane - 2 < h)
-		fd.rowcand[y + lane - 2] = 1u;
 }
 
 // C (list-based): one warp per seed slot.
 __global__ void __launch_bounds__(256)
 seed_kernel(const FrameDesc *__restrict__ frames, const Seed *__restrict__ seeds, DetectParams prm,
-	const Control *ctl, int fresh)
+	const Control *ctl, int par)
 {
 	__shared__ double patches[8][81];
 	__shared__ double triples[8][3][63];
 	const int warp = threadIdx.x >> 5;
 	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
 	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	const long long n = (long long)ctl->n_cand;
+	const long long n = (long long)ctl->pass[par].n_cand;
 	Seed next = gw < n ? seeds[gw] : Seed{NO_SEED, 0, 0.0, 0.0};
 	for (long long e = gw; e < n; e += nw) {
 		const Seed sd = next;
@@ -908,7 +1111,7 @@ seed_kernel(const FrameDesc *__restrict__ frames, const Seed *__restrict__ seeds
 			continue; // warp-uniform
 		const FrameDesc &fd = frames[sd.frame];
 		seed_eval(fd, (int)(sd.pixel % (unsigned)fd.w), (int)(sd.pixel / (unsigned)fd.w), sd.sig,
-			sd.noise, prm, patches[warp], triples[warp], fresh != 0);
+			sd.noise, prm, patches[warp], triples[warp], true);
 	}
 }
 
@@ -922,7 +1125,7 @@ seed_kernel(const FrameDesc *__restrict__ frames, const Seed *__restrict__ seeds
 template <int PATH>
 __global__ void __launch_bounds__(256, PATH == PATH_ERROR ? 4 : 3)
 candidate_seed_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restrict__ cands,
-	DetectParams prm, Control *ctl, Seed *seeds, int fresh)
+	DetectParams prm, Control *ctl, Seed *seeds)
 {
 	// Error-map frames only: the scratch of candidate_sig holds just the 25
 	// values of the NaN rule, and the triples of the seed test serve as it.
@@ -933,7 +1136,7 @@ candidate_seed_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restr
 	double *P = patches[warp];
 	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
 	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	const long long n = (long long)ctl->n_cand;
+	const long long n = (long long)ctl->pass[0].n_cand;
 	uint2 next = gw < n ? cands[gw] : make_uint2(0u, 0u);
 	for (long long e = gw; e < n; e += nw) {
 		const uint2 t = next;
@@ -951,12 +1154,10 @@ candidate_seed_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restr
 			seeds[e] = Seed{NO_SEED, 0, 0.0, 0.0};
 		double nz;
 		const double sig = candidate_sig<false, PATH>(fd, x, y, P, &triples[warp][0][0], prm, nz,
-			fresh != 0, hole);
+			true, hole);
 		// Every lane holds the same sig, so the branch is warp-uniform.
 		if (!hole && sig > prm.cr && !(excl & bit))
-			seed_eval(fd, x, y, sig, nz, prm, P, triples[warp], fresh != 0, true);
-		else if (lane == 0)
-			write_bit(plane_ptr(fd, P_CAND) + word, bit, false, fresh != 0);
+			seed_eval(fd, x, y, sig, nz, prm, P, triples[warp], true, true);
 	}
 }
 

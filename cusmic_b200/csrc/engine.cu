@@ -1,12 +1,13 @@
 // Host side of cusmic_b200: batch layout, workspace pool, launch sequence and
 // the C ABI of include/cusmic.h and include/cusmic_b200.h.
 //
-// One call = init -> prepare -> hole fill -> maxiter x (detect -> grow/update
-// -> control -> replace) -> restore, all on the caller's stream, with no host
-// synchronisation inside the loop: per-frame activity lives on the device and
-// kernels skip frames that stopped (the reference instead copies counts to the
-// host after every pass, src/cleaner.cuh:69-76,128-142).  Plans capture the
-// same sequence into a CUDA graph whose loop is a device-driven while node.
+// One call = init -> prepare -> hole fill -> first pass (detect -> grow/update
+// -> replace) -> the later passes in one cooperative launch -> restore, all on
+// the caller's stream, with no host synchronisation in between: per-frame
+// activity lives on the device and frames that stopped are skipped (the
+// reference instead copies counts to the host after every pass,
+// src/cleaner.cuh:69-76,128-142).  Plans capture the same sequence into a CUDA
+// graph.
 #include "../../include/cusmic.h"
 #include "../../include/cusmic_b200.h"
 #include "common.cuh"
@@ -15,7 +16,7 @@
 #include "kernels.cuh"
 #include "prepare_bulk.cuh"
 #include "prep_detect.cuh"
-#include "incremental.cuh"
+#include "late.cuh"
 #include "backward.cuh"
 #include "sigmap.cuh"
 
@@ -367,10 +368,8 @@ static cusmic_tuning tuning_for(size_t total_px)
 struct Layout {
 	std::vector<FrameDesc> frames;
 	std::vector<long long> bit_off; // word offset of each frame within a plane
-	std::vector<long long> row_off; // first row of each frame in the row marks
-	long long row_words = 0;        // row marks of all frames, padded to 4
 	std::vector<int4> bulk;   // sig_bulk_kernel items {frame, x0, y0, first threshold of the frame}
-	std::vector<int4> grow;   // grow_kernel items {frame, y0, first word, y1}
+	std::vector<int4> grow;   // region_list_kernel items {frame, y0, first word, y1}
 	std::vector<FloorJob> jobs; // floor blocks of each distinct error map and noise-model frame
 	std::vector<long long> thr_base; // per frame: first floor of its blocks
 	long long nthr = 0;
@@ -409,6 +408,8 @@ static DeviceInfo device_info(int dev)
 			     (const void *)prepare_bulk_kernel<false, true>,
 			     (const void *)prepare_bulk_kernel<true, true>})
 			check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
+		check(cudaFuncSetAttribute((const void *)late_passes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			(int)sizeof(LateShared)));
 	}
 	return d;
 }
@@ -419,11 +420,9 @@ struct Workspace {
 	DevBuf<FrameState> state;
 	DevBuf<int2> rows;
 	DevBuf<uint32_t> bits;
-	DevBuf<uint32_t> rowmarks; // growth row marks, then CHG row marks (row_words each)
 	DevBuf<uint2> targets;
 	DevBuf<uint8_t> radius; // per target: window radius of its last replacement
-	DevBuf<int2> dirty;     // dirty-row list of an incremental pass
-	DevBuf<unsigned> sel;   // targets the replacement after a pass visits
+	DevBuf<unsigned> chg;   // targets whose value the last replacement changed
 	DevBuf<Seed> seeds;     // seed slots of the noise-model candidates
 	DevBuf<double> work;    // working pixels of the frames with a background
 	DevBuf<double> sigmap;  // first-pass sig_raw, then noise, of noise-model frames (2 x pixels)
@@ -635,8 +634,6 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 		d.has_bg = im.background != nullptr || !std::isnan(s.bg);
 		d.bits = nullptr;
 		L.bit_off[f] = words;
-		L.row_off.push_back(L.row_words);
-		L.row_words += d.h;
 		L.offsets.push_back((long long)px);
 		words += d.plane;
 		px += (size_t)d.w * d.h;
@@ -670,7 +667,6 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 	}
 	L.total_px = px;
 	choose_kernels(L);
-	L.row_words = (L.row_words + 3) & ~3ll;
 	// Planes padded to 4 words, so every plane starts on a 16-byte boundary.
 	L.plane_words = (words + 3) & ~3ll;
 	L.total_words = (long long)N_PLANES * L.plane_words;
@@ -713,11 +709,9 @@ static void upload(Workspace &ws, Layout &L, cudaStream_t s, bool mapped = false
 	ws.offsets.ensure(nf);
 	if (L.maxiter) {
 		ws.bits.ensure((size_t)L.total_words);
-		ws.rowmarks.ensure(2 * (size_t)L.row_words);
 		ws.targets.ensure(L.total_px);
 		ws.radius.ensure(L.total_px);
-		ws.dirty.ensure(L.rows.size());
-		ws.sel.ensure(L.total_px);
+		ws.chg.ensure(L.total_px);
 		if (L.error_frames < (int)nf)
 			ws.seeds.ensure(L.total_px);
 		ws.cands.ensure(L.total_px);
@@ -738,8 +732,6 @@ static void upload(Workspace &ws, Layout &L, cudaStream_t s, bool mapped = false
 	for (size_t f = 0; f < nf; ++f) {
 		L.frames[f].bits = L.maxiter ? ws.bits.p + L.bit_off[f] : nullptr;
 		L.frames[f].floors = L.maxiter ? ws.floors.p + L.thr_base[f] : nullptr;
-		L.frames[f].rowcand = L.maxiter ? ws.rowmarks.p + L.row_off[f] : nullptr;
-		L.frames[f].rowchg = L.maxiter ? ws.rowmarks.p + L.row_words + L.row_off[f] : nullptr;
 		L.frames[f].out = L.frames[f].clean;
 		const bool sm = L.maxiter && !L.frames[f].error;
 		L.frames[f].sig_raw = sm ? ws.sigmap.p + L.offsets[f] : nullptr;
@@ -788,11 +780,6 @@ static void upload(Workspace &ws, Layout &L, cudaStream_t s, bool mapped = false
 		word_copy_kernel<<<32, 256, 0, s>>>(wc);
 }
 
-struct GraphLoop {
-	cudaGraphConditionalHandle handle = 0;
-	bool use = false;
-};
-
 // Kernel kinds reported by cusmic_plan_profile().
 enum KernelKind { K_INIT, K_PREPARE, K_FILL, K_SIGRAW, K_CAND, K_SEED, K_GROW, K_CONTROL,
 	K_REPLACE, K_RESTORE, K_COPY, K_LOW, K_CLASSIFY, K_FLOOR, K_RECLASS, K_DIRTY, K_SIGMAP, K_KINDS };
@@ -835,95 +822,92 @@ static inline void mark(Recorder *r, int kind)
 // no waves of idle blocks.
 constexpr int WINDOW_BLOCKS_PER_SM = 3, MAP_BLOCKS_PER_SM = 2;
 
-// One detection pass.  The first pass of a call is full: the dense kernel
-// lists every candidate and the classification fills the HIGH / LOW planes.
-// Later passes are incremental (incremental.cuh): they start from the pixels
-// that the last replacement changed and keep the other bits.
+// The first detection pass of a call is full: the dense kernel lists every
+// candidate and the classification fills the HIGH / LOW planes.  It ends with
+// the replacement; the later passes start from the pixels that changed and
+// keep the other bits (launch_late).
 static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cudaStream_t s,
-	const GraphLoop &gl, bool incremental, Recorder *rec = nullptr)
+	Recorder *rec = nullptr)
 {
-	const int nf = (int)L.frames.size(), nrows = (int)L.rows.size();
+	const int nf = (int)L.frames.size();
 	const int nbulk = (int)L.bulk.size();
 	const int cap = di.sms * L.tune.dense_blocks_per_sm, sparse = di.sms * L.tune.sparse_blocks_per_sm;
-	const int rowb = L.tune.row_blocks_per_sm;
-	if (incremental) {
-		// The dirty-row scan also zeroes FRESH of every frame (its growth
-		// visits a row list); the full pass finds S1, S2, CAND, FRESH and the
-		// growth row marks zeroed by the prologue.
-		const long long n16 = L.plane_words / 4; // 16-byte words of one plane
-		const long long need = ((n16 > nrows ? n16 : nrows) + 255) / 256;
-		const int tb = (int)(need < di.sms * 4 ? need : di.sms * 4);
-		dirty_rows_kernel<<<tb, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.rows.p, nrows, L.prm.mode,
-			ws.ctl.p, ws.dirty.p, reinterpret_cast<uint4 *>(ws.bits.p + P_FRESH * L.plane_words), n16);
-		mark(rec, K_DIRTY);
-		const int rgrid = grid_for_rows(di, nrows, rowb);
-		if (L.error_frames)
-			incremental_rows_kernel<false><<<rgrid, 256, 0, s>>>(ws.frames.p, ws.dirty.p,
-				&ws.ctl.p->n_dirty, L.prm, ws.ctl.p, ws.cands.p);
-		if (L.error_frames < nf)
-			incremental_rows_kernel<true><<<rgrid, 256, 0, s>>>(ws.frames.p, ws.dirty.p,
-				&ws.ctl.p->n_dirty, L.prm, ws.ctl.p, ws.cands.p);
-		mark(rec, K_RECLASS);
-	} else {
-		// (A fused batch's prologue listed the pixels already.)
-		if (!L.fused) {
-			sig_bulk_kernel<<<nbulk < cap ? nbulk : cap, BK_THREADS, 0, s>>>(ws.frames.p, ws.state.p,
-				ws.bulk.p, nbulk, L.prm, ws.ctl.p, ws.pre.p, ws.pre_counts.p);
-			mark(rec, K_SIGRAW);
-		}
-		const int cgrid = (nbulk * BK_CWARPS + 7) / 8 < sparse ? (nbulk * BK_CWARPS + 7) / 8 : sparse;
-		classify_kernel<<<cgrid, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.bulk.p, nbulk, ws.pre.p,
-			ws.pre_counts.p, L.prm, ws.ctl.p, ws.cands.p);
-		mark(rec, K_CLASSIFY);
-		if (L.error_frames < nf) { // the noise-model candidates' sig_raw map
-			const int ng = (int)L.grow.size(), need = (ng + 7) / 8, gcap = di.sms * 8;
-			region_list_kernel<<<need < gcap ? need : gcap, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.grow.p,
-				ng, ws.ctl.p, ws.targets.p);
-			region_sig_kernel<<<di.sms * 8, 256, 0, s>>>(ws.frames.p, ws.targets.p, ws.ctl.p, L.prm);
-			mark(rec, K_SIGMAP);
-		}
+	// (A fused batch's prologue listed the pixels already.)
+	if (!L.fused) {
+		sig_bulk_kernel<<<nbulk < cap ? nbulk : cap, BK_THREADS, 0, s>>>(ws.frames.p, ws.state.p,
+			ws.bulk.p, nbulk, L.prm, ws.ctl.p, ws.pre.p, ws.pre_counts.p);
+		mark(rec, K_SIGRAW);
 	}
+	const int cgrid = (nbulk * BK_CWARPS + 7) / 8 < sparse ? (nbulk * BK_CWARPS + 7) / 8 : sparse;
+	classify_kernel<<<cgrid, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.bulk.p, nbulk, ws.pre.p,
+		ws.pre_counts.p, L.prm, ws.ctl.p, ws.cands.p);
+	mark(rec, K_CLASSIFY);
 	// One launch per kind of frame in the batch: each variant compiles only
 	// its noise path (error map or noise model).  Error-map seeds are tested
-	// by the candidate's own warp; noise-model seeds by seed_kernel.
+	// by the candidate's own warp; noise-model candidates, a thread each, read
+	// their windows from the sig_raw map, and seed_kernel tests their seeds.
 	const bool model = L.error_frames < nf;
+	if (model) {
+		const int ng = (int)L.grow.size(), need = (ng + 7) / 8, gcap = di.sms * 8;
+		region_list_kernel<<<need < gcap ? need : gcap, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.grow.p,
+			ng, ws.ctl.p, ws.targets.p);
+		region_sig_kernel<<<di.sms * 8, 256, 0, s>>>(ws.frames.p, ws.targets.p, ws.ctl.p, L.prm);
+		mark(rec, K_SIGMAP);
+	}
 	if (L.error_frames)
 		candidate_seed_kernel<PATH_ERROR><<<sparse, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
-			ws.ctl.p, model ? ws.seeds.p : nullptr, !incremental);
-	if (model && incremental)
-		candidate_high_kernel<PATH_MODEL><<<sparse, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
-			ws.ctl.p, ws.seeds.p, 0);
-	else if (model) // the first pass: windows from the sig_raw map, a thread per candidate
+			ws.ctl.p, model ? ws.seeds.p : nullptr);
+	if (model)
 		candidate_map_kernel<<<di.sms * MAP_BLOCKS_PER_SM, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
 			ws.ctl.p, ws.seeds.p);
 	mark(rec, K_CAND);
 	if (model) {
-		seed_kernel<<<sparse, 256, 0, s>>>(ws.frames.p, ws.seeds.p, L.prm, ws.ctl.p, !incremental);
+		seed_kernel<<<sparse, 256, 0, s>>>(ws.frames.p, ws.seeds.p, L.prm, ws.ctl.p, 0);
 		mark(rec, K_SEED);
 	}
 	if (L.error_frames)
-		candidate_low_kernel<PATH_ERROR><<<sparse, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
-			ws.ctl.p, !incremental);
-	if (L.error_frames < nf)
-		candidate_low_kernel<PATH_MODEL><<<sparse, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
-			ws.ctl.p, !incremental);
-	mark(rec, K_LOW);
-	// Growth visits the items holding marked rows.
-	{
-		const int ng = (int)L.grow.size(), need = (ng + 7) / 8, gcap = di.sms * rowb;
-		grow_kernel<<<need < gcap ? need : gcap, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.grow.p, ng,
-			ws.targets.p, ws.ctl.p);
-	}
+		low_grow_kernel<PATH_ERROR><<<sparse, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.cands.p, L.prm,
+			ws.ctl.p, 0, ws.targets.p, 1);
+	if (model)
+		low_grow_kernel<PATH_MODEL><<<sparse, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.cands.p, L.prm,
+			ws.ctl.p, 0, ws.targets.p, L.error_frames == 0);
 	mark(rec, K_GROW);
-	control_kernel<<<1, 1024, 0, s>>>(ws.state.p, nf, ws.ctl.p, gl.handle, gl.use ? 1 : 0);
-	mark(rec, K_CONTROL);
-	const int tb = di.sms * 4;
-	replace_select_kernel<<<tb, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.targets.p,
-		&ws.ctl.p->n_targets, ws.radius.p, ws.ctl.p, ws.sel.p,
-		reinterpret_cast<uint4 *>(ws.rowmarks.p + L.row_words), L.row_words / 4);
-	replace_kernel<<<di.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.targets.p,
-		&ws.ctl.p->n_targets, ws.sel.p, &ws.ctl.p->n_sel, ws.radius.p);
+	replace_kernel<<<di.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(ws.frames.p, ws.state.p, nf, ws.targets.p,
+		ws.ctl.p, 0, ws.radius.p, ws.chg.p);
 	mark(rec, K_REPLACE);
+}
+
+// The passes after the first (late.cuh): the first late pass's lists in two
+// launches, then one cooperative launch, whose blocks all run at once and meet
+// at grid barriers.  Small batches take fewer blocks, which makes the barriers
+// cheaper.
+static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cudaStream_t s,
+	Recorder *rec = nullptr)
+{
+	if (L.maxiter < 2)
+		return;
+	const int grid = (int)std::min<size_t>(std::max<size_t>(8, L.total_px / 16384), (size_t)di.sms);
+	const int wide = (int)std::min<size_t>(std::max<size_t>(8, L.total_px / 4096), (size_t)di.sms * 8);
+	const FrameDesc *frames = ws.frames.p;
+	FrameState *state = ws.state.p;
+	int nf = (int)L.frames.size(), maxiter = L.maxiter;
+	DetectParams prm = L.prm;
+	Control *ctl = ws.ctl.p;
+	uint2 *cands = ws.cands.p, *targets = ws.targets.p;
+	// The pre list (at least 16 bytes per pixel) is done with after the first
+	// pass's classification.
+	uint2 *eval = reinterpret_cast<uint2 *>(ws.pre.p), *low = eval + L.total_px;
+	static_assert(sizeof(PreCand) == 2 * sizeof(uint2), "the pre list holds both lists");
+	uint8_t *radius = ws.radius.p;
+	unsigned *chg = ws.chg.p;
+	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, prm, ctl, cands, low, eval, targets, chg,
+		ws.jobs.p, L.error_frames < nf ? (int)L.jobs.size() : 0);
+	auto classes = L.error_frames < nf ? late_classes_kernel<true> : late_classes_kernel<false>;
+	classes<<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
+	void *args[] = {&frames, &state, &nf, &prm, &ctl, &maxiter, &cands, &low, &eval, &targets, &radius, &chg};
+	check(cudaLaunchCooperativeKernel((const void *)late_passes_kernel, dim3(grid), dim3(LATE_THREADS), args,
+		sizeof(LateShared), s));
+	mark(rec, K_RECLASS);
 }
 
 // prepare: the bulk-staged kernel when every frame suits it; else one
@@ -971,19 +955,16 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		mark(rec, K_COPY);
 		return;
 	}
-	// The same launch zeroes the bit planes from CRMASK to CHG and both
-	// row-mark arrays: nothing else writes them before the first pass, which
-	// therefore clears nothing itself.  prepare writes every word of HOLE,
-	// EXCL and DONOR, and of ROWMIN on noise-model frames (the only frames
-	// whose ROWMIN is read).  Planes and row marks are padded to 16 bytes.
+	// The same launch zeroes the bit planes from CRMASK to LISTED: nothing
+	// else writes them before the first pass, which therefore clears nothing
+	// itself.  prepare writes every word of HOLE, EXCL and DONOR, and of ROWMIN
+	// on noise-model frames (the only frames whose ROWMIN is read).  Planes
+	// are padded to 16 bytes.
 	static_assert(P_HOLE == 0 && P_EXCL == 1 && P_DONOR == 2 && P_CRMASK == 3 &&
 		P_ROWMIN == N_PLANES - 1, "plane order");
 	const long long z16 = (long long)(P_ROWMIN - P_CRMASK) * L.plane_words / 4;
-	const long long r16 = 2 * L.row_words / 4;
-	const long long zb = (std::max(z16, r16) + 255) / 256, fb = (nf + 255) / 256,
-		zcap = (long long)di.sms * 8;
+	const long long zb = (z16 + 255) / 256, fb = (nf + 255) / 256, zcap = (long long)di.sms * 8;
 	uint4 *const zero = reinterpret_cast<uint4 *>(ws.bits.p + P_CRMASK * L.plane_words);
-	uint4 *const zero2 = reinterpret_cast<uint4 *>(ws.rowmarks.p);
 	if (L.fused) {
 		// The error-map floors (they read the maps only) in the same launch
 		// as the state and the zeroing, then prepare with the first pass's
@@ -991,7 +972,7 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		const long long jb = ((long long)L.jobs.size() + 7) / 8;
 		prep_init_kernel<<<(int)std::max({fb, std::min(zb, zcap), std::min(jb, zcap)}), 256, 0, s>>>(
 			ws.state.p, nf, ws.ctl.p, L.maxiter, (unsigned long long)L.total_px, L.poison_wait[0],
-			L.poison_wait[1], zero, z16, zero2, r16, ws.frames.p, ws.jobs.p, (int)L.jobs.size(), L.prm,
+			L.poison_wait[1], zero, z16, ws.frames.p, ws.jobs.p, (int)L.jobs.size(), L.prm,
 			ws.floors.p);
 		mark(rec, K_INIT); // the state, the zeroed planes and the floors
 		const int nbulk = (int)L.bulk.size(), pcap = di.sms * PD_BLOCKS_PER_SM;
@@ -1004,8 +985,7 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		return;
 	}
 	init_kernel<<<(int)std::max(fb, std::min(zb, zcap)), 256, 0, s>>>(ws.state.p, nf, ws.ctl.p,
-		L.maxiter, (unsigned long long)L.total_px, L.poison_wait[0], L.poison_wait[1], zero, z16, zero2,
-		r16);
+		L.maxiter, (unsigned long long)L.total_px, L.poison_wait[0], L.poison_wait[1], zero, z16);
 	mark(rec, K_INIT); // the state and the zeroed planes
 	launch_prepare(ws, L, di, s);
 	mark(rec, K_PREPARE);
@@ -1044,8 +1024,10 @@ static void enqueue_plain(Workspace &ws, const Layout &L, const DeviceInfo &di, 
 	if (rec)
 		rec->begin(s);
 	launch_prologue(ws, L, di, s, rec);
-	for (int it = 0; it < L.maxiter; ++it)
-		launch_pass(ws, L, di, s, GraphLoop{}, it > 0, rec);
+	if (L.maxiter) {
+		launch_pass(ws, L, di, s, rec);
+		launch_late(ws, L, di, s, rec);
+	}
 	launch_epilogue(ws, L, di, s, rec);
 	check(cudaGetLastError());
 }
@@ -1649,10 +1631,9 @@ extern "C" int cusmic_batch_host(const cusmic_image *ims, size_t nf, const cusmi
 
 // ---------------------------------------------------------------------------
 // Plans: a fixed batch with its own workspace, descriptors uploaded once, and
-// optionally the whole cleaning captured as one CUDA graph.  The maxiter loop
-// becomes a conditional WHILE node whose condition control_kernel sets from
-// the device (any frame still active and passes left), so the early exit costs
-// no host round trip.
+// optionally the whole cleaning captured as one CUDA graph.  The passes after
+// the first are one node (late_passes_kernel), which ends as soon as no frame
+// is active, so the early exit costs no host round trip.
 
 struct cusmic_plan {
 	int device = -1;
@@ -1689,38 +1670,8 @@ static void capture_graph(cusmic_plan &p)
 	try {
 		launch_prologue(p.ws, p.L, p.di, cs);
 		if (p.L.maxiter) {
-			cudaStreamCaptureStatus st;
-			cudaGraph_t g;
-			const cudaGraphNode_t *deps = nullptr;
-			size_t nd = 0;
-			check(cudaStreamGetCaptureInfo(cs, &st, nullptr, &g, &deps, &nd));
-			// The full first pass sets the loop condition (its control
-			// kernel runs upstream of the while node); the body repeats the
-			// incremental pass.
-			cudaGraphConditionalHandle handle;
-			check(cudaGraphConditionalHandleCreate(&handle, g, 0, cudaGraphCondAssignDefault));
-			launch_pass(p.ws, p.L, p.di, cs, GraphLoop{handle, true}, false);
-			check(cudaStreamGetCaptureInfo(cs, &st, nullptr, &g, &deps, &nd));
-			cudaGraphNodeParams cp = {};
-			cp.type = cudaGraphNodeTypeConditional;
-			cp.conditional.handle = handle;
-			cp.conditional.type = cudaGraphCondTypeWhile;
-			cp.conditional.size = 1;
-			cudaGraphNode_t node;
-			check(cudaGraphAddNode(&node, g, deps, nd, &cp));
-			cudaGraph_t body = cp.conditional.phGraph_out[0];
-			check(cudaStreamUpdateCaptureDependencies(cs, &node, 1,
-				cudaStreamSetCaptureDependencies));
-			cudaStream_t bs;
-			check(cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking));
-			cudaError_t err = cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0,
-				cudaStreamCaptureModeThreadLocal);
-			if (err == cudaSuccess) {
-				launch_pass(p.ws, p.L, p.di, bs, GraphLoop{handle, true}, true);
-				err = cudaStreamEndCapture(bs, nullptr);
-			}
-			cudaStreamDestroy(bs);
-			check(err);
+			launch_pass(p.ws, p.L, p.di, cs);
+			launch_late(p.ws, p.L, p.di, cs);
 		}
 		launch_epilogue(p.ws, p.L, p.di, cs);
 	} catch (...) {
@@ -1795,8 +1746,6 @@ extern "C" int cusmic_plan_bind(cusmic_plan *p, const cusmic_image *ims, double 
 		for (size_t f = 0; f < nf; ++f) {
 			L.frames[f].bits = p->L.frames[f].bits;
 			L.frames[f].floors = p->L.frames[f].floors;
-			L.frames[f].rowcand = p->L.frames[f].rowcand;
-			L.frames[f].rowchg = p->L.frames[f].rowchg;
 			L.frames[f].sig_raw = p->L.frames[f].sig_raw;
 			L.frames[f].noise = p->L.frames[f].noise;
 			L.frames[f].out = L.frames[f].clean; // the new output buffer
@@ -2159,8 +2108,6 @@ extern "C" int remove_cosmics_device_noalloc(const cusmic_image *im, const cusmi
 		init_kernel<<<1, 256, 0, s>>>(state, 1, ctl, o->maxiter,
 			(unsigned long long)im->width * im->height);
 		const int row_blocks = (h + 7) / 8 < nd.sms * 8 ? (h + 7) / 8 : nd.sms * 8;
-		const int grow_items = (h + GROW_ROWS - 1) / GROW_ROWS * ((fd.words + 31) / 32);
-		const int grow_blocks = (grow_items + 7) / 8 < nd.sms * 8 ? (grow_items + 7) / 8 : nd.sms * 8;
 		if (!o->maxiter) {
 			copy_kernel<<<row_blocks, 256, 0, s>>>(frames, rows, h);
 		} else {
@@ -2170,25 +2117,24 @@ extern "C" int remove_cosmics_device_noalloc(const cusmic_image *im, const cusmi
 			prepare_kernel<PREP_ANY><<<row_blocks, 256, 0, s>>>(frames, state, rows, h);
 			fill_kernel<<<row_blocks, 256, 0, s>>>(frames, state, rows, h);
 			for (int it = 0; it < o->maxiter; ++it) {
+				const int par = it & 1;
 				if (error_map) {
 					const int b = (L.nitems + 7) / 8 < nd.sms * 8 ? (L.nitems + 7) / 8 : nd.sms * 8;
 					sig_stream_kernel<<<b, 256, 0, s>>>(frames, state, items, L.nitems, prm, ctl,
-						cands);
+						par, cands);
 				} else {
 					const int b = L.nitems < nd.sms * 8 ? L.nitems : nd.sms * 8;
 					sig_model_kernel<<<b, 256, 0, s>>>(frames, state, items, L.nitems, prm, ctl,
-						cands);
+						par, cands);
 				}
 				// The dense kernels above zeroed S1, S2 and CAND.
 				candidate_high_kernel<PATH_ANY><<<nd.sms * 8, 256, 0, s>>>(frames, cands, prm, ctl,
-					seeds, 1);
-				seed_kernel<<<nd.sms * 8, 256, 0, s>>>(frames, seeds, prm, ctl, 1);
-				candidate_low_kernel<PATH_ANY><<<nd.sms * 8, 256, 0, s>>>(frames, cands, prm, ctl, 1);
-				grow_kernel<<<grow_blocks, 256, 0, s>>>(frames, state, nullptr, grow_items, targets,
-					ctl);
-				control_kernel<<<1, 1024, 0, s>>>(state, 1, ctl, 0, 0);
-				replace_kernel<<<nd.sms * 8, 256, 0, s>>>(frames, state, targets, &ctl->n_targets, nullptr,
-					nullptr, nullptr);
+					par, seeds);
+				seed_kernel<<<nd.sms * 8, 256, 0, s>>>(frames, seeds, prm, ctl, par);
+				low_grow_kernel<PATH_ANY><<<nd.sms * 3, 256, 0, s>>>(frames, state, cands, prm, ctl, par,
+					targets, 1);
+				replace_kernel<<<nd.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(frames, state, 1, targets,
+					ctl, par, nullptr, nullptr);
 			}
 			restore_kernel<<<row_blocks, 256, 0, s>>>(frames, rows, h);
 		}

@@ -65,10 +65,10 @@ __device__ __forceinline__ unsigned long long warp_append(unsigned long long *co
 // Per-frame facts that the loop control only tests for zero (any hole, any
 // allowed pixel, any new pixel, any donor left): many warps set the same flag
 // with a plain store instead of contending on an atomic counter.
-__device__ __forceinline__ void set_flag(unsigned long long *flag)
+template <class T> __device__ __forceinline__ void set_flag(T *flag)
 {
-	if (!*(volatile unsigned long long *)flag)
-		*(volatile unsigned long long *)flag = 1;
+	if (!*(volatile T *)flag)
+		*(volatile T *)flag = 1;
 }
 
 // Map validation of the host entry point on the device (reference
@@ -89,17 +89,15 @@ validate_kernel(const double *__restrict__ v, long long n, int minimum, unsigned
 }
 
 // Per-frame state and loop control of a call; with `zero`, also zeroes the n16
-// 16-byte words at zero (the bit planes that nothing writes before the first
-// pass, and the row marks) with a grid-stride loop of 16-byte stores.
+// 16-byte words there (the bit planes that nothing writes before the first
+// pass) with a grid-stride loop of 16-byte stores.
 __device__ __forceinline__ void init_state(FrameState *state, int nf, Control *ctl, int maxiter,
 	unsigned long long cand_cap, long long poison_prepare, long long poison_detect, uint4 *zero,
-	long long n16, uint4 *zero2, long long n16b)
+	long long n16)
 {
 	const long long stride = (long long)gridDim.x * blockDim.x;
 	for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n16; j += stride)
 		zero[j] = make_uint4(0u, 0u, 0u, 0u);
-	for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n16b; j += stride)
-		zero2[j] = make_uint4(0u, 0u, 0u, 0u);
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i < nf) {
 		FrameState s = {};
@@ -108,9 +106,7 @@ __device__ __forceinline__ void init_state(FrameState *state, int nf, Control *c
 	}
 	if (i == 0) {
 		Control c = {};
-		c.maxiter = maxiter;
 		c.cand_cap = cand_cap;
-		c.any_active = maxiter > 0;
 		c.poison_wait[0] = poison_prepare;
 		c.poison_wait[1] = poison_detect;
 		*ctl = c;
@@ -119,9 +115,9 @@ __device__ __forceinline__ void init_state(FrameState *state, int nf, Control *c
 
 __global__ void init_kernel(FrameState *state, int nf, Control *ctl, int maxiter,
 	unsigned long long cand_cap, long long poison_prepare = 0, long long poison_detect = 0,
-	uint4 *zero = nullptr, long long n16 = 0, uint4 *zero2 = nullptr, long long n16b = 0)
+	uint4 *zero = nullptr, long long n16 = 0)
 {
-	init_state(state, nf, ctl, maxiter, cand_cap, poison_prepare, poison_detect, zero, n16, zero2, n16b);
+	init_state(state, nf, ctl, maxiter, cand_cap, poison_prepare, poison_detect, zero, n16);
 }
 
 // IEEE bits mapped to an unsigned total order (reference src/replace.cuh:37-48).
@@ -309,204 +305,8 @@ prepare_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const in
 	}
 }
 
-// 36-bit window of a bit-plane row around word k: bits 0..35 are pixels
-// 32k-2 .. 32k+33 (zero outside the frame).
-__device__ __forceinline__ unsigned long long bit_window(const uint32_t *plane, int words, int h,
-	int y, int k)
-{
-	if (y < 0 || y >= h)
-		return 0;
-	const uint32_t *row = plane + (long long)y * words;
-	unsigned long long c = row[k];
-	unsigned long long l = k > 0 ? row[k - 1] : 0u;
-	unsigned long long r = k + 1 < words ? row[k + 1] : 0u;
-	return (l >> 30) | (c << 2) | ((r & 3ull) << 34);
-}
-
-__device__ __forceinline__ unsigned long long dilate_row(unsigned long long e)
-{
-	return e | (e << 1) | (e >> 1);
-}
-
-// Rows of a growth item (grow_kernel).
+// Rows of an item of region_list_kernel.
 constexpr int GROW_ROWS = 16;
-
-// 36-bit window of a bit-plane row (bit_window) for a lane whose word is past
-// the row: zero.
-__device__ __forceinline__ unsigned long long lane_window(const uint32_t *plane, int words, int h,
-	int y, int k)
-{
-	return k < words ? bit_window(plane, words, h, y, k) : 0ull;
-}
-
-// Reference src/filters.cuh:177-193 twice (src/cleaner.cuh:123-125) and
-// src/cleaner.cuh:22-37: grown = dilate3x3(dilate3x3(cand) & S1) & S2 on bit
-// planes (clipped to the frame), fresh = grown & ~crmask, crmask |= grown,
-// the FRESH plane, the per-frame facts (any fresh pixel; the count of static
-// donors left, which the reference recounts in accumulate), and fresh pixels
-// appended to the target list.
-//
-// One warp per item of GROW_ROWS rows x 32 bit words (a lane per word), from
-// `items` {frame, first row, first word, end row}, or with items null from
-// frame 0 in row-major item order.  The warp sweeps down its rows keeping the
-// horizontal dilations of the CAND rows y .. y + 1 and of the S1-masked rows
-// y - 1 .. y in registers, so each row step reads one CAND window, an S1
-// window only where a dilated CAND pixel is near, S2 and CRMASK only where
-// something can grow, and DONOR only where pixels are flagged; the item
-// appends its fresh pixels with one atomic.  (Issuing the loads of four rows
-// together, unconditionally, measured slower.)
-//
-// With row marks (fd.rowcand) an item none of whose rows is marked is
-// skipped: a full pass marks the rows within two of a CAND pixel (nothing
-// grows elsewhere), an incremental pass the rows within six of a pixel whose
-// value the last replacement changed (elsewhere grown repeats the last pass
-// and is already in the mask).  A visited item computes all its rows (an
-// unmarked row adds nothing) and clears the CHG bits of its rows with a CHG
-// mark (every such row is marked; replace_select_kernel then clears the
-// marks).  FRESH is written on every visited row (the pass starts with it
-// zeroed where it skips).
-__global__ void __launch_bounds__(256)
-grow_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const int4 *__restrict__ items,
-	int nitems, uint2 *targets, Control *ctl)
-{
-	const int lane = threadIdx.x & 31;
-	const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-	for (int i = gw; i < nitems; i += nw) {
-		int4 it;
-		if (items) {
-			it = items[i];
-		} else {
-			const int strips = (frames[0].words + 31) / 32, y0 = (i / strips) * GROW_ROWS;
-			it = make_int4(0, y0, (i % strips) * 32, min(y0 + GROW_ROWS, frames[0].h));
-		}
-		const int f = it.x;
-		if (!state[f].active)
-			continue; // warp-uniform
-		const FrameDesc &fd = frames[f];
-		const int w = fd.w, h = fd.h, words = fd.words, y0 = it.y, n = it.w - it.y, k = it.z + lane;
-		const bool row_lane = lane < n;
-		const unsigned visit = __ballot_sync(0xffffffffu,
-			row_lane && (!fd.rowcand || fd.rowcand[y0 + lane]));
-		if (!visit)
-			continue; // warp-uniform
-		const unsigned chg = fd.rowchg
-			? __ballot_sync(0xffffffffu, row_lane && fd.rowchg[y0 + lane]) : 0u;
-		const uint32_t *cand = plane_ptr(fd, P_CAND), *s1 = plane_ptr(fd, P_S1);
-		const uint32_t *s2 = plane_ptr(fd, P_S2), *donor = plane_ptr(fd, P_DONOR);
-		uint32_t *crm = plane_ptr(fd, P_CRMASK), *fr = plane_ptr(fd, P_FRESH);
-		uint32_t *cg = plane_ptr(fd, P_CHG);
-		// Dilated CAND rows y0 - 2 .. y0 + 1, then the dilated S1-masked rows
-		// y0 - 1 and y0 (h0, h1); c0, c1: dilated CAND rows y and y + 1.
-		unsigned long long c0, c1, h0, h1;
-		{
-			const unsigned long long d0 = dilate_row(lane_window(cand, words, h, y0 - 2, k));
-			const unsigned long long d1 = dilate_row(lane_window(cand, words, h, y0 - 1, k));
-			c0 = dilate_row(lane_window(cand, words, h, y0, k));
-			c1 = dilate_row(lane_window(cand, words, h, y0 + 1, k));
-			const unsigned long long a = d0 | d1 | c0, b = d1 | c0 | c1;
-			h0 = a ? dilate_row(a & lane_window(s1, words, h, y0 - 1, k)) : 0ull;
-			h1 = b ? dilate_row(b & lane_window(s1, words, h, y0, k)) : 0ull;
-		}
-		int cnt = 0, lost = 0;
-		unsigned rows_fresh = 0; // bit j: this lane flagged pixels in row y0 + j
-#pragma unroll 4
-		for (int j = 0; j < n; ++j) {
-			const int y = y0 + j;
-			const unsigned long long c2 = dilate_row(lane_window(cand, words, h, y + 2, k));
-			const unsigned long long cc = c0 | c1 | c2;
-			const unsigned long long h2 = cc ? dilate_row(cc & lane_window(s1, words, h, y + 1, k)) : 0ull;
-			const uint32_t near = (uint32_t)((h0 | h1 | h2) >> 2); // bits 2..33: the word's pixels
-			if (k < words) {
-				const long long o = (long long)y * words + k;
-				uint32_t fresh = 0;
-				if (near) {
-					const uint32_t grown = near & s2[o], old = crm[o];
-					fresh = grown & ~old;
-					if (fresh) {
-						crm[o] = old | fresh;
-						cnt += __popc(fresh);
-						lost += __popc(fresh & donor[o]);
-						rows_fresh |= 1u << j;
-					}
-				}
-				fr[o] = fresh;
-				if ((chg >> j) & 1u)
-					cg[o] = 0u;
-			}
-			c0 = c1;
-			c1 = c2;
-			h0 = h1;
-			h1 = h2;
-		}
-		const bool any = __any_sync(0xffffffffu, cnt != 0);
-		if (any) {
-			unsigned long long slot = warp_append(&ctl->n_targets, cnt);
-			for (unsigned m = rows_fresh; m; m &= m - 1) {
-				const int y = y0 + __ffs(m) - 1;
-				uint32_t fresh = fr[(long long)y * words + k]; // this lane's own store
-				const unsigned base = (unsigned)((long long)y * w + 32 * k);
-				while (fresh) {
-					const int b = __ffs(fresh) - 1;
-					fresh &= fresh - 1;
-					targets[slot++] = make_uint2((unsigned)f, base + b);
-				}
-			}
-		}
-		lost = __reduce_add_sync(0xffffffffu, (unsigned)lost);
-		if (lane == 0) {
-			if (any)
-				set_flag(&state[f].todo);
-			if (lost)
-				atomicAdd((unsigned long long *)&state[f].donors_left,
-					(unsigned long long)(-(long long)lost));
-		}
-	}
-}
-
-// Per-frame loop control after a pass (reference src/cleaner.cuh:128-142,
-// 175-181): a frame with new pixels but no donors fails, a frame without new
-// pixels stops (its later passes would repeat this one), the others replace
-// and continue.  With a graph handle, sets the while-node condition.
-__global__ void __launch_bounds__(1024)
-control_kernel(FrameState *state, int nf, Control *ctl, cudaGraphConditionalHandle handle,
-	int use_handle)
-{
-	int any = 0;
-	const int fault = ctl->fault;
-	for (int f = threadIdx.x; f < nf; f += blockDim.x) {
-		FrameState s = state[f];
-		s.replace = 0;
-		if (s.active) {
-			++s.passes;
-			if (fault) { // this pass's detection is incomplete: stop, report
-				s.fault = 1;
-				s.active = 0;
-			} else if (s.todo && s.donors_left <= 0) {
-				s.error = 1;
-				s.active = 0;
-			} else if (s.todo) {
-				s.replace = 1;
-				any = 1;
-			} else {
-				s.active = 0;
-			}
-		}
-		s.todo = 0;
-		state[f] = s;
-	}
-	any = __syncthreads_or(any);
-	if (threadIdx.x == 0) {
-		int it = ++ctl->iter;
-		ctl->any_active = any;
-		ctl->n_cand = 0;
-		ctl->n_low = 0;
-		ctl->ticket = 0;
-		ctl->n_dirty = 0;
-		ctl->n_sel = 0;
-		if (use_handle)
-			cudaGraphSetConditional(handle, (any && it < ctl->maxiter) ? 1u : 0u);
-	}
-}
 
 // Reference src/replace.cuh:50-56.
 __device__ __forceinline__ double midpoint(double lo, double hi)
@@ -763,62 +563,16 @@ __device__ __forceinline__ bool fresh_in_window(const FrameDesc &fd, int x, int 
 	return any != 0;
 }
 
-// Which targets the replacement after a pass must visit, for frames whose
-// pass flagged new pixels: a lane per target; the indices of those to visit
-// are appended to `sel` (count in ctl->n_sel).  The same threads first zero
-// `clear` (n16 16-byte words: the CHG row marks, which this pass has read
-// and the replacement that follows sets).
-//
-// radius keeps, per target, the window radius of its last replacement.  A
-// target whose last window (radius r <= KEEP_RADIUS_MAX) holds no pixel the
-// last growth step flagged keeps its value: donors are never added (the mask
-// only grows) and keep their values, so the smaller windows still hold none,
-// the same window holds the same donors, and the same median would come out.
-// A new target is itself a flagged pixel.
-__global__ void __launch_bounds__(256)
-replace_select_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
-	const uint2 *__restrict__ list, const unsigned long long *count,
-	const uint8_t *__restrict__ radius, Control *ctl, unsigned *sel, uint4 *clear, long long n16)
-{
-	const int lane = threadIdx.x & 31;
-	const long long n = (long long)*count;
-	const long long stride = (long long)gridDim.x * blockDim.x;
-	for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n16; i += stride)
-		clear[i] = make_uint4(0u, 0u, 0u, 0u);
-	for (long long base = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); base < n;
-	     base += stride) {
-		const long long e = base + lane;
-		bool todo = false;
-		if (e < n) {
-			const uint2 t = list[e];
-			if (state[t.x].replace) {
-				todo = true;
-				const int r = radius[e];
-				if (r <= KEEP_RADIUS_MAX) {
-					const FrameDesc &fd = frames[t.x];
-					todo = fresh_in_window(fd, (int)(t.y % (unsigned)fd.w), (int)(t.y / (unsigned)fd.w), r);
-				}
-			}
-		}
-		const unsigned b = __ballot_sync(0xffffffffu, todo);
-		unsigned at = 0;
-		if (lane == 0 && b)
-			at = atomicAdd(&ctl->n_sel, (unsigned)__popc(b));
-		at = __shfl_sync(0xffffffffu, at, 0);
-		if (todo)
-			sel[at + __popc(b & ((1u << lane) - 1u))] = (unsigned)e;
-	}
-}
-
 // Bits of columns x - 2 .. x + 2 of row y of a bit plane (bit i: column
 // x - 2 + i; columns outside the frame read as zero: the words' padding bits
 // are zero, and words before the row's first or after its last read as zero).
+// The second word is read only where the five columns reach into it.
 __device__ __forceinline__ uint32_t bits5(const uint32_t *plane, int words, int x, int y)
 {
-	const int a = x - 2, k = a >> 5; // k >= -1
+	const int a = x - 2, k = a >> 5, s = a & 31; // k >= -1
 	const uint32_t *row = plane + (long long)y * words;
-	const uint32_t lo = k >= 0 ? row[k] : 0u, hi = k + 1 < words ? row[k + 1] : 0u;
-	return (uint32_t)((((unsigned long long)hi << 32) | lo) >> (a - 32 * k)) & 0x1fu;
+	const uint32_t lo = k >= 0 ? row[k] : 0u, hi = s > 27 && k + 1 < words ? row[k + 1] : 0u;
+	return __funnelshift_r(lo, hi, s) & 0x1fu;
 }
 
 // replace_one's first window (radius 2, clipped to the frame: at most 25
@@ -871,85 +625,135 @@ __device__ __forceinline__ bool first_window_value(const FrameDesc &fd, int x, i
 	return true;
 }
 
-// The bookkeeping of a target's replacement: its window radius, and with
-// fd.rowchg, when its value changed (bit for bit), its CHG bit and its row
-// mark (the next incremental pass starts from those pixels).
-__device__ __forceinline__ void replaced(const FrameDesc &fd, int x, int y, long long e, int r, bool changed,
-	uint8_t *radius)
-{
-	if (radius)
-		radius[e] = (uint8_t)(r < 255 ? r : 255);
-	if (changed && fd.rowchg) {
-		atomicOr(plane_ptr(fd, P_CHG) + (long long)y * fd.words + (x >> 5), 1u << (x & 31));
-		fd.rowchg[y] = 1u;
-	}
-}
-
 // Items the thread path of a block leaves, replaced by all of its warps.
 struct WindowQueue {
 	long long e[256];
 	int n;
 };
 
-// Replacement after a pass (src/replace.cuh:111-153): the targets listed in
-// sel (with radius: each replacement's window radius is kept), or with sel
-// null every target of the frames whose pass flagged new pixels.  A thread
-// per target evaluates its first window (first_window_value); the targets it
-// leaves (windows inside a cluster of flagged pixels) are queued in shared
-// memory and the block's warps replace them with replace_one, spread over all
-// eight warps so that a cluster does not hold one warp for many targets.
-// Targets are in the mask, so never donors: no target reads another's value.
-__global__ void __launch_bounds__(256)
-replace_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
-	const uint2 *__restrict__ list, const unsigned long long *count, const unsigned *sel,
-	const unsigned *nsel, uint8_t *radius)
+// Whether the replacement after a pass of parity par runs for a frame: the
+// pass flagged a pixel and a donor is left (reference src/cleaner.cuh:128-142).
+__device__ __forceinline__ bool replaces(const FrameState &s, int par)
 {
-	__shared__ WindowQueue Q;
+	return s.todo[par] && s.donors_left > 0;
+}
+
+// Per-frame loop control after a pass (reference src/cleaner.cuh:128-142,
+// 175-181): a frame with new pixels but no donors fails, a frame without new
+// pixels stops (its later passes would repeat this one), the others replace
+// and continue.  Runs in the replacement's grid (a thread per frame): the
+// replacement reads only todo[par] and donors_left, which this leaves alone.
+__device__ __forceinline__ void pass_control(FrameState *state, int nf, Control *ctl, int par)
+{
+	const int fault = *(volatile int *)&ctl->fault;
+	for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
+		FrameState &s = state[f];
+		s.todo[par ^ 1] = 0;
+		if (!s.active)
+			continue;
+		++s.passes;
+		bool on = false;
+		if (fault) // this pass's detection is incomplete: stop, report
+			s.fault = 1;
+		else if (s.todo[par] && s.donors_left <= 0)
+			s.error = 1;
+		else
+			on = s.todo[par] != 0;
+		s.active = on;
+		if (on)
+			ctl->any[par] = 1;
+	}
+}
+
+// Replacement after a pass of parity par (src/replace.cuh:111-153), for the
+// frames whose pass flagged new pixels.  A thread per target evaluates its
+// first window (first_window_value); the targets it leaves (windows inside a
+// cluster of flagged pixels) are queued in shared memory and the block's warps
+// replace them with replace_one, spread over all eight warps so that a cluster
+// does not hold one warp for many targets.  Targets are in the mask, so never
+// donors: no target reads another's value.
+//
+// With chg, the indices of the targets whose value changed (bit for bit) are
+// appended there (count in n_chg): the next pass starts from those pixels.
+__device__ __forceinline__ void replace_targets(const FrameDesc *__restrict__ frames,
+	const FrameState *state, int par, const uint2 *list, long long n, uint8_t *radius, unsigned *chg,
+	unsigned long long *n_chg, WindowQueue &Q)
+{
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-	const long long n = sel ? (long long)*nsel : (long long)*count;
 	const long long stride = (long long)gridDim.x * blockDim.x;
+	__syncthreads();
 	if (threadIdx.x == 0)
 		Q.n = 0;
 	__syncthreads();
 	for (long long base = blockIdx.x * (long long)blockDim.x; base < n; base += stride) { // block-uniform
-		const long long s = base + threadIdx.x;
-		if (s < n) {
-			const long long e = sel ? (long long)sel[s] : s;
+		const long long e = base + threadIdx.x;
+		bool changed = false;
+		if (e < n) {
 			const uint2 t = list[e];
-			if (sel || state[t.x].replace) {
+			if (replaces(state[t.x], par)) {
 				const FrameDesc &fd = frames[t.x];
 				const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 				double v;
 				if (first_window_value(fd, x, y, v)) {
 					double &dst = fd.clean[(long long)y * fd.w + x];
-					const bool ch = __double_as_longlong(dst) != __double_as_longlong(v);
+					changed = __double_as_longlong(dst) != __double_as_longlong(v);
 					dst = v;
+					if (radius)
+						radius[e] = 2;
 					// Keep the block's floor a lower bound of its clean values.
 					if (fd.floors && !fd.error)
 						atomicMin(&fd.floors[(y >> 5) * ((fd.w + 31) >> 5) + (x >> 5)].key, order_key(v));
-					replaced(fd, x, y, e, 2, ch, radius);
 				} else {
 					Q.e[atomicAdd(&Q.n, 1)] = e;
 				}
 			}
 		}
+		if (chg) {
+			const unsigned b = __ballot_sync(0xffffffffu, changed);
+			unsigned long long at = 0;
+			if (lane == 0 && b)
+				at = atomicAdd(n_chg, (unsigned long long)__popc(b));
+			at = __shfl_sync(0xffffffffu, at, 0);
+			if (changed)
+				chg[at + __popc(b & ((1u << lane) - 1u))] = (unsigned)e;
+		}
 		__syncthreads();
 		const int nq = Q.n;
 		for (int q = warp; q < nq; q += nwarps) {
-			const long long e = Q.e[q];
-			const uint2 t = list[e];
+			const long long eq = Q.e[q];
+			const uint2 t = list[eq];
 			const FrameDesc &fd = frames[t.x];
-			const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 			bool ch = false;
-			const int r = replace_one(fd, x, y, &ch);
-			if (lane == 0)
-				replaced(fd, x, y, e, r, ch, radius);
+			const int r = replace_one(fd, (int)(t.y % (unsigned)fd.w), (int)(t.y / (unsigned)fd.w), &ch);
+			if (lane == 0) {
+				if (radius)
+					radius[eq] = (uint8_t)(r < 255 ? r : 255);
+				if (chg && ch)
+					chg[atomicAdd(n_chg, 1ull)] = (unsigned)eq;
+			}
 		}
 		__syncthreads();
 		if (threadIdx.x == 0)
 			Q.n = 0;
 		__syncthreads();
 	}
+}
+
+// The replacement after a full pass of parity par (every target of the frames
+// that flagged pixels), with the pass's loop control in the same grid.
+// Without chg (no late passes follow) the next full pass's lists are reset.
+__global__ void __launch_bounds__(256, 3)
+replace_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int nf, const uint2 *list,
+	Control *ctl, int par, uint8_t *radius, unsigned *chg)
+{
+	__shared__ WindowQueue Q;
+	pass_control(state, nf, ctl, par);
+	if (!chg && blockIdx.x == 0 && threadIdx.x == 0) {
+		ctl->pass[par ^ 1] = PassLists{};
+		ctl->any[par ^ 1] = 0;
+	}
+	replace_targets(frames, state, par, list, (long long)ctl->n_targets, radius, chg,
+		&ctl->pass[par ^ 1].n_chg, Q);
 }
 
 // Initial fill of non-finite pixels (src/cleaner.cuh:78-100) for frames with

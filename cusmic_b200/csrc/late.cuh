@@ -1,0 +1,661 @@
+// Late detection passes (every pass after the first), all of them in one
+// cooperative launch.
+//
+// A pass of the reference (src/cleaner.cuh:102-142) recomputes the whole
+// detection chain on the current clean pixels, and between two passes only
+// the pixels that the replacement wrote change.  Every quantity of the chain
+// at a pixel p reads clean pixels within a fixed Chebyshev distance of p,
+// measured in the frame (mirror, reflect and nearest map a window position
+// onto an in-frame pixel no farther from p; constant reads a zero) or on the
+// torus (wrap):
+//
+//   sig_raw = lap / (2 noise)       distance 2 (lap 1, noise-model median 2)
+//   sig = sig_raw - med5(sig_raw)   distance 4
+//   fine = med3 -> med7             distance 4
+//   S1, S2, CAND                    distance 4
+//   grown pixel (two dilations)     distance 6 (S2, S1 and CAND within 2)
+//
+// So with D the targets whose value the last replacement changed (the chg
+// list that replace_targets writes), pass k + 1 differs from pass k only near
+// D.  A late pass keeps the bit planes of the previous one and works on lists
+// that start from D, in stages separated by grid barriers:
+//
+//  1. Half a warp per pixel of D (a lane per row of its 13 x 13
+//     neighbourhood): the pixels within 2 are listed for re-evaluation (once
+//     each, claimed in the EVAL plane); the HIGH pixels within 4 go to the high
+//     list and the LOW pixels within 6 to the low list (once each, claimed in
+//     the LISTED plane, by their old classes).
+//  2. A thread per re-evaluated pixel: its exact sig_raw, hence its class
+//     (sig_raw > cr_threshold or NaN: HIGH, else > neighbor_threshold: LOW;
+//     classify_kernel's first-pass classes are supersets, from the Laplacian
+//     upper bound).  A pixel that enters a class joins that list (its old class
+//     listed it in stage 1 already if it keeps it); one that leaves HIGH loses
+//     its S1 and CAND bits (sig <= sig_raw <= cr_threshold), one that leaves
+//     both classes its S2 bit.
+//  3. The high list's pixels that are HIGH now: significance and seed test, as
+//     in a full pass but setting or clearing each bit.
+//  4. The low list and the growth (low_list, growth_rows).
+//  5. The replacement of the targets whose window holds a new pixel, and the
+//     loop control.
+//
+// What stays exact: S1 and CAND everywhere, S2 of every HIGH pixel and of
+// every LOW pixel with a CAND pixel within 2 (the only S2 bits growth reads): a
+// LOW pixel whose CAND neighbourhood changed is within 6 of D.  Outside HIGH
+// sig <= cr_threshold, and a pixel outside both classes has sig <=
+// neighbor_threshold, so its bits are zero.
+//
+// Why one launch and lists: after the first pass little changes (16 frames of
+// 2048 x 2048: 64,998 targets in the first pass, then 799, 688 and 290 changed
+// pixels), so the passes are chains of latencies.  As eight launches each,
+// scanning row marks and bit planes, in a graph's while node, passes 2 to 4
+// took 0.30 ms of that batch's 1.04 ms, and a call without a graph issued 24
+// launches for them whatever was left to do.
+#pragma once
+
+#include "bulk.cuh"
+#include "common.cuh"
+#include "detect.cuh"
+#include "kernels.cuh"
+
+namespace cb {
+
+// One block of 32 warps per SM: the fewest arrivals at a grid barrier for the
+// warps that 64 registers a thread allow.
+constexpr int LATE_THREADS = 1024;
+constexpr int LATE_WARPS = LATE_THREADS / 32;
+
+static_assert(FLOOR_BLOCK == 32, "a bit word of a row lies in one floor block");
+
+// model_threshold of block (bx, by) of a noise-model frame; outside wrap mode
+// only the 3 x 3 neighbouring blocks count, read directly.
+__device__ __forceinline__ double block_threshold(const FrameDesc &fd, int bx, int by, int mode,
+	double tmin2)
+{
+	if (mode == WRAP)
+		return model_threshold(fd, bx, by, mode, tmin2);
+	const BlockFloor *bf = fd.floors;
+	const int bw = (fd.w + FLOOR_BLOCK - 1) / FLOOR_BLOCK, bh = (fd.h + FLOOR_BLOCK - 1) / FLOOR_BLOCK;
+	unsigned long long key = ~0ull;
+#pragma unroll
+	for (int i = -1; i <= 1; ++i)
+#pragma unroll
+		for (int j = -1; j <= 1; ++j) {
+			const int yy = by + i, xx = bx + j;
+			if (yy >= 0 && yy < bh && xx >= 0 && xx < bw)
+				key = min(key, bf[yy * bw + xx].key);
+		}
+	if (mode == CONSTANT && (bx == 0 || by == 0 || (bx + 1) * FLOOR_BLOCK + 2 > fd.w ||
+		(by + 1) * FLOOR_BLOCK + 2 > fd.h))
+		key = min(key, order_key(0.0));
+	double m = order_value(key);
+	m = m < SIGNAL_FLOOR ? SIGNAL_FLOOR : m;
+	const BlockFloor &own = bf[by * bw + bx];
+	const double g = fd.gain_map ? -order_value(own.gkey) : fd.gain;
+	const double rn = fd.rn_map ? order_value(own.rkey) : fd.rn;
+	return tmin2 * (sqrt(rn * rn + g * m) / g);
+}
+
+__device__ __forceinline__ int wrap_index(int i, int n)
+{
+	i %= n;
+	return i < 0 ? i + n : i;
+}
+
+// Grid barrier of a cooperative launch: the `round`-th call (from 1) returns
+// once every block has arrived `round` times, with their earlier writes
+// visible.  Bounded like every wait (about one second of SM clock): a wait that
+// runs out faults every frame and returns false, and so does every later one.
+__device__ __forceinline__ bool grid_barrier(Control *ctl, unsigned round, FrameState *state, int nf)
+{
+	__shared__ int open;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		__threadfence();
+		atomicAdd(&ctl->barrier, 1u);
+		const unsigned want = round * gridDim.x;
+		const long long t0 = clock64();
+		bool ok = true;
+		while ((int)(*(volatile unsigned *)&ctl->barrier - want) < 0) {
+			if (*(volatile int *)&ctl->fault || clock64() - t0 > BK_WAIT_CYCLES) {
+				ok = false;
+				break;
+			}
+		}
+		if (!ok) {
+			atomicOr(&ctl->fault, 1);
+			for (int f = 0; f < nf; ++f)
+				state[f].fault = 1;
+		}
+		__threadfence();
+		open = ok;
+	}
+	__syncthreads();
+	return open != 0;
+}
+
+// A block's entries for the three lists of stage 1: their numbers, then their
+// first slots.
+struct ListSlots {
+	int n[3];
+	unsigned long long at[3];
+};
+
+// Stage 1 (called by every thread of the grid, in blocks of WARPS warps).  A
+// block's warps reserve their list slots together, one atomic per list: an
+// atomic per warp and list on the same three counters (0.8 ns each, one after
+// another) held this stage for 82 us on 64,998 changed targets.
+template <int WARPS>
+__device__ __forceinline__ void late_neighbours(const FrameDesc *__restrict__ frames, const uint2 *targets,
+	const unsigned *chg, PassLists &L, int mode, uint2 *cands, uint2 *low, uint2 *eval, ListSlots &R)
+{
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const long long n = (long long)L.n_chg;
+	const bool wrap = mode == WRAP;
+	const int dy = (lane & 15) - 6, ay = dy < 0 ? -dy : dy;
+	// Entries per block and sweep: fewer for a short list, which spreads it.
+	const long long share = (n + gridDim.x - 1) / gridDim.x;
+	const int chunk = share < 2 * WARPS ? (int)share : 2 * WARPS;
+	for (long long base = (long long)blockIdx.x * chunk; base < n; base += (long long)gridDim.x * chunk) {
+		const int own_entry = 2 * warp + (lane >> 4);
+		const long long i = base + own_entry;
+		bool valid = own_entry < chunk && i < n && dy <= 6;
+		uint2 t = make_uint2(0u, 0u);
+		int x = 0, yy = 0, w = 1, words = 1;
+		uint32_t *high = nullptr, *lowp = nullptr, *ep = nullptr, *lp = nullptr;
+		bool torus = false; // the row's window crosses the frame's edge on the torus
+		if (valid) {
+			t = targets[chg[i]];
+			const FrameDesc &fd = frames[t.x];
+			w = fd.w;
+			words = fd.words;
+			x = (int)(t.y % (unsigned)w);
+			yy = (int)(t.y / (unsigned)w) + dy;
+			if (wrap)
+				yy = wrap_index(yy, fd.h);
+			valid = yy >= 0 && yy < fd.h;
+			torus = wrap && (x < 6 || x + 6 >= w);
+			const long long row = (long long)(valid ? yy : 0) * words;
+			high = plane_ptr(fd, P_HIGH) + row;
+			lowp = plane_ptr(fd, P_LOW) + row;
+			ep = plane_ptr(fd, P_EVAL) + row;
+			lp = plane_ptr(fd, P_LISTED) + row;
+		}
+		// Pieces of the lane's row: its window [x - 6, x + 6] at once (at most
+		// two words), or on the torus across an edge column by column.
+		const int pieces = wrap ? (__syncthreads_or(valid && torus) ? 13 : 1) : 1;
+		for (int p = 0; p < pieces; ++p) { // block-uniform
+			unsigned long long m2 = 0, m4 = 0, m6 = 0; // bits from column 32 k
+			int k = 0;
+			if (valid && torus) {
+				const int dx = p - 6, ax = dx < 0 ? -dx : dx, c = wrap_index(x + dx, w);
+				k = c >> 5;
+				m6 = 1ull << (c & 31);
+				m4 = ax <= 4 && ay <= 4 ? m6 : 0ull;
+				m2 = ax <= 2 && ay <= 2 ? m6 : 0ull;
+			} else if (valid && p == 0) {
+				auto span = [&](int r) { // columns x - r .. x + r in the frame
+					const int a = max(x - r, 0), b = min(x + r, w - 1);
+					return ((1ull << (b - a + 1)) - 1ull) << (a - 32 * k);
+				};
+				k = max(x - 6, 0) >> 5;
+				m6 = span(6);
+				m4 = ay <= 4 ? span(4) : 0ull;
+				m2 = ay <= 2 ? span(2) : 0ull;
+			}
+			unsigned long long ne = 0, nh = 0, nl = 0;
+			if (m6) {
+				const bool two = (m6 >> 32) != 0;
+				const unsigned long long H = high[k] | (unsigned long long)(two ? high[k + 1] : 0u) << 32;
+				const unsigned long long W = lowp[k] | (unsigned long long)(two ? lowp[k + 1] : 0u) << 32;
+				const unsigned long long want = (H & m4) | (W & ~H & m6);
+				auto claim = [&](uint32_t *word, uint32_t bits) { return bits ? atomicOr(word, bits) : 0u; };
+				const uint32_t e0 = claim(ep + k, (uint32_t)m2), e1 = claim(ep + k + 1, (uint32_t)(m2 >> 32));
+				const uint32_t l0 = claim(lp + k, (uint32_t)want), l1 = claim(lp + k + 1, (uint32_t)(want >> 32));
+				ne = m2 & ~(e0 | (unsigned long long)e1 << 32);
+				const unsigned long long got = want & ~(l0 | (unsigned long long)l1 << 32);
+				nh = got & H;
+				nl = got & ~H;
+			}
+			// Positions in the three lists: counts (at most 13 per lane) side
+			// by side in one scan of the warp, then the block's.
+			int sum = __popcll(ne) | __popcll(nh) << 10 | __popcll(nl) << 20;
+			const int own = sum;
+#pragma unroll
+			for (int o = 1; o < 32; o <<= 1) {
+				const int v = __shfl_up_sync(0xffffffffu, sum, o);
+				if (lane >= o)
+					sum += v;
+			}
+			const int total = __shfl_sync(0xffffffffu, sum, 31);
+			if (threadIdx.x < 3)
+				R.n[threadIdx.x] = 0;
+			__syncthreads();
+			int mine = 0; // lanes 0..2: the warp's first entry of the list in the block's
+			if (lane < 3 && total)
+				mine = atomicAdd(&R.n[lane], (total >> (10 * lane)) & 1023);
+			__syncthreads();
+			if (threadIdx.x < 3) {
+				const int c = R.n[threadIdx.x];
+				unsigned long long *counter = threadIdx.x == 0 ? &L.n_eval : threadIdx.x == 1 ? &L.n_cand : &L.n_low;
+				R.at[threadIdx.x] = c ? atomicAdd(counter, (unsigned long long)c) : 0ull;
+			}
+			__syncthreads();
+			const unsigned pix = (unsigned)((long long)yy * w + 32 * k);
+			auto put = [&](uint2 *list, int which, unsigned long long bits) {
+				unsigned long long slot = R.at[which] + __shfl_sync(0xffffffffu, mine, which) +
+					(((sum - own) >> (10 * which)) & 1023);
+				for (; bits; bits &= bits - 1)
+					list[slot++] = make_uint2(t.x, pix + __ffsll((long long)bits) - 1);
+			};
+			put(eval, 0, ne);
+			put(cands, 1, nh);
+			put(low, 2, nl);
+		}
+	}
+}
+
+// The class of lane's re-evaluated pixel t (0: none, 1: HIGH, 2: LOW) into the
+// planes and lists; called by the whole warp, `have`: the lane has one.
+__device__ __forceinline__ void late_class(const FrameDesc *__restrict__ frames, uint2 t, int cls, bool have,
+	PassLists &L, uint2 *cands, uint2 *low)
+{
+	const int lane = threadIdx.x & 31;
+	bool to_high = false, to_low = false;
+	if (have) {
+		const FrameDesc &fd = frames[t.x];
+		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
+		const long long o = (long long)y * fd.words + (x >> 5);
+		const uint32_t bit = 1u << (x & 31);
+		uint32_t *H = plane_ptr(fd, P_HIGH) + o, *W = plane_ptr(fd, P_LOW) + o;
+		uint32_t *s1 = plane_ptr(fd, P_S1) + o, *s2 = plane_ptr(fd, P_S2) + o, *cd = plane_ptr(fd, P_CAND) + o;
+		const bool oh = (*H & bit) != 0, ol = (*W & bit) != 0; // only this thread writes the pixel's bits
+		const bool o1 = (*s1 & bit) != 0, o2 = (*s2 & bit) != 0, oc = (*cd & bit) != 0;
+		to_high = cls == 1 && !oh;
+		to_low = cls == 2 && !ol;
+		if (to_high)
+			atomicOr(H, bit);
+		if (oh && cls != 1)
+			atomicAnd(H, ~bit);
+		if (to_low)
+			atomicOr(W, bit);
+		if (ol && cls != 2)
+			atomicAnd(W, ~bit);
+		if (o1 && cls != 1)
+			atomicAnd(s1, ~bit);
+		if (oc && cls != 1)
+			atomicAnd(cd, ~bit);
+		if (o2 && cls == 0)
+			atomicAnd(s2, ~bit);
+		plane_ptr(fd, P_EVAL)[o] = 0u; // every claim of the plane ends in this stage
+	}
+	const unsigned bh = __ballot_sync(0xffffffffu, to_high), bl = __ballot_sync(0xffffffffu, to_low);
+	if (!(bh | bl))
+		return;
+	unsigned long long at = 0;
+	if (lane == 0 && bh)
+		at = atomicAdd(&L.n_cand, (unsigned long long)__popc(bh));
+	if (lane == 1 && bl)
+		at = atomicAdd(&L.n_low, (unsigned long long)__popc(bl));
+	const unsigned long long ah = __shfl_sync(0xffffffffu, at, 0), al = __shfl_sync(0xffffffffu, at, 1);
+	const unsigned below = (1u << lane) - 1u;
+	if (to_high)
+		cands[ah + __popc(bh & below)] = t;
+	if (to_low)
+		low[al + __popc(bl & below)] = t;
+}
+
+__device__ __forceinline__ int class_of(double v, const DetectParams &prm)
+{
+	return v > prm.cr || v != v ? 1 : v > prm.nb ? 2 : 0;
+}
+
+// Stage 2 (called by every warp of the grid).  On noise-model frames a pixel
+// whose Laplacian is at most its floor block's bound cannot pass either
+// threshold; the others wait in the warp's queue Q (64 entries).  THREADS: 32
+// of them at a time, a thread per median (long lists); else the warp sorts
+// each one's window (short lists, few registers).
+//
+// A list that takes THREADS finds the block thresholds written since the last
+// replacement (late_neighbours_kernel).
+template <bool THREADS, bool MODEL = true>
+__device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frames, const uint2 *eval,
+	const DetectParams &prm, PassLists &L, uint2 *cands, uint2 *low, uint2 *Q)
+{
+	const int lane = threadIdx.x & 31;
+	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+	const long long n = (long long)L.n_eval;
+	const int mode = prm.mode, lm = lap_mode(mode);
+	const double tmin2 = fmin(prm.thi2, prm.tlo2);
+	int nq = 0; // queued (warp-uniform)
+	auto drain = [&](int count) { // the first `count` <= 32 queued pixels
+		__syncwarp();
+		uint2 t = make_uint2(0u, 0u);
+		int cls = 0;
+		if (!THREADS) {
+			t = Q[lane < count ? lane : 0];
+			for (int q = 0; q < count; ++q) {
+				const uint2 u = Q[q];
+				const FrameDesc &fd = frames[u.x];
+				const int w = fd.w, x = (int)(u.y % (unsigned)w), y = (int)(u.y / (unsigned)w);
+				double c = INFINITY;
+				if (lane < 25) {
+					const int cx = x + lane % 5 - 2, cy = y + lane / 5 - 2;
+					c = cx >= 0 && cy >= 0 && cx < w && cy < fd.h ? fd.clean[(long long)cy * w + cx]
+						: clean_at(fd, cx, cy, mode);
+				}
+				const double lap = lap_at(fd, x, y, lm); // every lane: one round trip with the window
+				const double m = __shfl_sync(0xffffffffu, warp_sort32(c), 12);
+				const int k = class_of(lap / (2 * noise_from_median(fd, u.y, m)), prm);
+				if (lane == q)
+					cls = k;
+			}
+		} else if (lane < count) {
+			t = Q[lane];
+			const FrameDesc &fd = frames[t.x];
+			const int w = fd.w, x = (int)(t.y % (unsigned)w), y = (int)(t.y / (unsigned)w);
+			double nz, lap;
+			if (x >= 2 && y >= 2 && x + 2 < w && y + 2 < fd.h) {
+				double v[25];
+				const double *src = fd.clean + t.y - 2 * (long long)w - 2;
+#pragma unroll
+				for (int a = 0; a < 5; ++a)
+#pragma unroll
+					for (int b = 0; b < 5; ++b)
+						v[a * 5 + b] = src[(long long)a * w + b];
+				lap = lap_formula(v[12], v[7], v[17], v[11], v[13]);
+				nz = noise_from_median(fd, t.y, median_network(v));
+			} else {
+				nz = noise_model_at(fd, x, y, mode);
+				lap = lap_at(fd, x, y, lm);
+			}
+			cls = class_of(lap / (2 * nz), prm);
+		}
+		__syncwarp();
+		if (lane + 32 < nq)
+			Q[lane] = Q[lane + 32];
+		nq -= count;
+		__syncwarp();
+		late_class(frames, t, cls, lane < count, L, cands, low);
+	};
+	for (long long base = gw * 32; base < n; base += nw * 32) {
+		const long long e = base + lane;
+		uint2 t = make_uint2(0u, 0u);
+		int cls = 0;
+		bool have = e < n, wait = false;
+		if (have) {
+			t = eval[e];
+			const FrameDesc &fd = frames[t.x];
+			const int w = fd.w, x = (int)(t.y % (unsigned)w), y = (int)(t.y / (unsigned)w);
+			double lap;
+			if (x >= 1 && y >= 1 && x + 1 < w && y + 1 < fd.h) {
+				const double *c = fd.clean + t.y;
+				lap = lap_formula(c[0], c[-w], c[w], c[-1], c[1]);
+			} else {
+				lap = lap_at(fd, x, y, lm);
+			}
+			if (!MODEL || fd.error) {
+				cls = class_of(lap / (2 * fd.error[t.y]), prm);
+			} else {
+				const double T = THREADS ? fd.floors[(y >> 5) * ((w + 31) >> 5) + (x >> 5)].thr
+					: block_threshold(fd, x >> 5, y >> 5, mode, tmin2);
+				wait = !(T >= 0 && lap <= T);
+			}
+		}
+		late_class(frames, t, cls, have && !wait, L, cands, low);
+		if (!MODEL)
+			continue;
+		const unsigned b = __ballot_sync(0xffffffffu, wait);
+		if (b) {
+			if (wait)
+				Q[nq + __popc(b & ((1u << lane) - 1u))] = t;
+			nq += __popc(b);
+			if (nq >= 32)
+				drain(32);
+		}
+	}
+	if (nq)
+		drain(nq);
+}
+
+// Entries 0 .. n - 1 of a list by blocks: a thread per entry tests it (keep),
+// then the block's warps take the survivors (work, by the whole warp) from a
+// queue in shared memory.  A block's share shrinks with the list, so that a
+// short one spreads over the grid.  The entries are dealt to the blocks one by
+// one, so neighbouring entries, whose survivors come in clusters, go to
+// different blocks.
+struct LateQueue {
+	uint16_t e[LATE_THREADS];
+	int n;
+};
+
+template <class Keep, class Work>
+__device__ __forceinline__ void block_sweep(long long n, LateQueue &Q, Keep keep, Work work)
+{
+	const int warp = threadIdx.x >> 5;
+	const long long share = (n + gridDim.x - 1) / gridDim.x;
+	const int chunk = share < LATE_THREADS ? (int)share : LATE_THREADS;
+	const long long step = gridDim.x;
+	for (long long base = blockIdx.x; base < n;
+	     base += (long long)gridDim.x * chunk) {
+		if (threadIdx.x == 0)
+			Q.n = 0;
+		__syncthreads();
+		const long long e = base + step * threadIdx.x;
+		if ((int)threadIdx.x < chunk && e < n && keep(e))
+			Q.e[atomicAdd(&Q.n, 1)] = (uint16_t)threadIdx.x;
+		__syncthreads();
+		const int nq = Q.n;
+		for (int q = warp; q < nq; q += LATE_WARPS)
+			work(base + step * Q.e[q]);
+		__syncthreads();
+	}
+}
+
+// Stage 3: the listed pixels that are HIGH (and no hole) now, a warp each.
+__device__ __forceinline__ void late_candidates(const FrameDesc *__restrict__ frames, const uint2 *cands,
+	const DetectParams &prm, const PassLists &L, LateQueue &Q, double *P, double *S, double (*T)[63])
+{
+	const int lane = threadIdx.x & 31;
+	block_sweep((long long)L.n_cand, Q, [&](long long e) {
+		const uint2 t = cands[e];
+		const FrameDesc &fd = frames[t.x];
+		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
+		return test_bit(plane_ptr(fd, P_HIGH), fd.words, x, y) &
+			!test_bit(plane_ptr(fd, P_HOLE), fd.words, x, y);
+	}, [&](long long e) {
+		const uint2 t = cands[e];
+		const FrameDesc &fd = frames[t.x];
+		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
+		const bool excl = test_bit(plane_ptr(fd, P_EXCL), fd.words, x, y);
+		double nz;
+		const double sig = candidate_sig<false, PATH_ANY>(fd, x, y, P, S, prm, nz, false);
+		// Every lane holds the same sig, so the branch is warp-uniform.
+		if (sig > prm.cr && !excl)
+			seed_eval(fd, x, y, sig, nz, prm, P, T, false, true);
+		else if (lane == 0)
+			write_bit(plane_ptr(fd, P_CAND) + (long long)y * fd.words + (x >> 5), 1u << (x & 31), false);
+	});
+}
+
+// Stage 4, the high list's part: a thread per listed pixel grows around it.
+// The grid's last blocks come first, its first blocks have the low list's
+// survivors when both are short.
+__device__ __forceinline__ void late_grow(const FrameDesc *__restrict__ frames, FrameState *state,
+	const uint2 *cands, const PassLists &L, Control *ctl, int par, uint2 *targets)
+{
+	const int lane = threadIdx.x & 31;
+	const long long stride = (long long)gridDim.x * blockDim.x, n = (long long)L.n_cand;
+	const long long start = (gridDim.x - 1 - blockIdx.x) * (long long)blockDim.x + (threadIdx.x & ~31);
+	for (long long base = start; base < n; base += stride) { // warp-uniform
+		const long long e = base + lane;
+		uint2 t = make_uint2(0u, 0u);
+		int w = 1, x = 0, y = 0, lost = 0;
+		uint32_t got = 0;
+		if (e < n) {
+			t = cands[e];
+			const FrameDesc &fd = frames[t.x];
+			w = fd.w;
+			x = (int)(t.y % (unsigned)w);
+			y = (int)(t.y / (unsigned)w);
+			got = grow_around(fd, x, y, false, false, lost);
+			plane_ptr(fd, P_LISTED)[(long long)y * fd.words + (x >> 5)] = 0u;
+		}
+		append_fresh(state, ctl, par, targets, (int)t.x, w, x, y, got, lost);
+	}
+}
+
+// Stage 4, the low list's part.
+__device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, FrameState *state,
+	const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par, uint2 *targets,
+	LateQueue &Q, double *P, double *S)
+{
+	block_sweep((long long)L.n_low, Q, [&](long long e) {
+		const uint2 t = low[e];
+		const FrameDesc &fd = frames[t.x];
+		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
+		plane_ptr(fd, P_LISTED)[(long long)y * fd.words + (x >> 5)] = 0u;
+		return low_near(fd, x, y);
+	}, [&](long long e) {
+		low_eval<PATH_ANY>(frames, state, low[e], prm, ctl, par, targets, P, S, false);
+	});
+}
+
+// Stage 5: the replacement, by warps (few targets are left to do).  A target
+// whose last replacement used a window of radius r <= KEEP_RADIUS_MAX without
+// a pixel of FRESH (what this pass's growth flagged) keeps its value: donors
+// are never added (the mask only grows) and keep their values, so the smaller
+// windows still hold none, the same window holds the same donors, and the same
+// median would come out.  A new target is itself a FRESH pixel.
+__device__ __forceinline__ void late_replace(const FrameDesc *__restrict__ frames, const FrameState *state,
+	int par, const uint2 *targets, long long n, long long fresh0, uint8_t *radius, unsigned *chg,
+	unsigned long long *n_chg, LateQueue &Q)
+{
+	block_sweep(n, Q, [&](long long e) {
+		const uint2 t = targets[e];
+		const int r = radius[e]; // (a new target's is not set yet)
+		if (!replaces(state[t.x], par))
+			return false;
+		if (e >= fresh0 || r > KEEP_RADIUS_MAX)
+			return true;
+		const FrameDesc &fd = frames[t.x];
+		return fresh_in_window(fd, (int)(t.y % (unsigned)fd.w), (int)(t.y / (unsigned)fd.w), r);
+	}, [&](long long e) {
+		const uint2 t = targets[e];
+		const FrameDesc &fd = frames[t.x];
+		bool changed = false;
+		const int r = replace_one(fd, (int)(t.y % (unsigned)fd.w), (int)(t.y / (unsigned)fd.w), &changed);
+		if ((threadIdx.x & 31) == 0) {
+			radius[e] = (uint8_t)(r < 255 ? r : 255);
+			if (changed)
+				chg[atomicAdd(n_chg, 1ull)] = (unsigned)e;
+		}
+	});
+}
+
+// Stages 1 and 2 of the first late pass, which starts from every target of the
+// full pass: launches of their own, whose registers let 48 and more warps per
+// SM hide the claims' and loads' latency.
+constexpr int LN_THREADS = 512;
+
+__global__ void __launch_bounds__(LN_THREADS, 3)
+late_neighbours_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, Control *ctl,
+	uint2 *cands, uint2 *low, uint2 *eval, const uint2 *targets, const unsigned *chg,
+	const FloorJob *__restrict__ jobs, int njobs)
+{
+	__shared__ ListSlots slots;
+	// The noise-model blocks' thresholds, for late_classes_kernel (a thread per
+	// block; the replacement lowered the floors).
+	const double tmin2 = fmin(prm.thi2, prm.tlo2);
+	for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < njobs; j += gridDim.x * blockDim.x) {
+		const FloorJob jb = jobs[j];
+		const FrameDesc &fd = frames[jb.frame];
+		if (!fd.error)
+			fd.floors[(jb.y0 >> 5) * ((fd.w + 31) >> 5) + (jb.x0 >> 5)].thr =
+				block_threshold(fd, jb.x0 >> 5, jb.y0 >> 5, prm.mode, tmin2);
+	}
+	late_neighbours<LN_THREADS / 32>(frames, targets, chg, ctl->pass[1], prm.mode, cands, low, eval, slots);
+}
+
+// MODEL: the batch has noise-model frames.
+template <bool MODEL>
+__global__ void __launch_bounds__(256, MODEL ? 2 : 6)
+late_classes_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, Control *ctl, uint2 *cands,
+	uint2 *low, const uint2 *eval)
+{
+	__shared__ uint2 queue[MODEL ? 8 : 1][64];
+	late_classes<true, MODEL>(frames, eval, prm, ctl->pass[1], cands, low, queue[MODEL ? threadIdx.x >> 5 : 0]);
+}
+
+struct LateShared {
+	double patches[LATE_WARPS][81];
+	double scratch[LATE_WARPS][CS_RUNS]; // sorted runs or triples of a warp's patch
+	uint2 queue[LATE_WARPS][64];
+	LateQueue Q;
+	ListSlots slots;
+};
+
+// Passes 1 .. maxiter - 1 (the full pass is number 0), the first of them from
+// stage 3.  cands: the high list; low, eval: buffers of as many entries as the
+// batch has pixels (the first pass's pre list, which is done with); chg: the
+// changed targets' indices.
+__global__ void __launch_bounds__(LATE_THREADS, 1)
+late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int nf, DetectParams prm,
+	Control *ctl, int maxiter, uint2 *cands, uint2 *low, uint2 *eval, uint2 *targets, uint8_t *radius,
+	unsigned *chg)
+{
+	extern __shared__ __align__(16) unsigned char late_smem[];
+	LateShared &S = *reinterpret_cast<LateShared *>(late_smem);
+	const int warp = threadIdx.x >> 5;
+	const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+	double (*triples)[63] = reinterpret_cast<double (*)[63]>(&S.scratch[warp][0]);
+	static_assert(3 * 63 <= CS_RUNS, "the triples fit the runs' scratch");
+	unsigned round = 0;
+	for (int it = 1; it < maxiter; ++it) {
+		const int par = it & 1;
+		PassLists &L = ctl->pass[par], &next = ctl->pass[par ^ 1];
+		if (!*(volatile int *)&ctl->any[par ^ 1])
+			return; // every frame stopped after the last pass
+		if (!*(volatile unsigned long long *)&L.n_chg) {
+			// The last replacement changed no value: this pass repeats it, and
+			// finds nothing new.
+			pass_control(state, nf, ctl, par);
+			return;
+		}
+		if (it > 1) {
+			late_neighbours<LATE_WARPS>(frames, targets, chg, L, prm.mode, cands, low, eval, S.slots);
+			// The last growth's FRESH bits: its replacement is done.
+			for (long long i = (long long)ctl->fresh0 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
+			     i < (long long)ctl->n_targets; i += (long long)gridDim.x * blockDim.x) {
+				const uint2 t = targets[i];
+				const FrameDesc &fd = frames[t.x];
+				plane_ptr(fd, P_FRESH)[(long long)(t.y / (unsigned)fd.w) * fd.words +
+					((t.y % (unsigned)fd.w) >> 5)] = 0u;
+			}
+			if (!grid_barrier(ctl, ++round, state, nf))
+				return;
+			late_classes<false>(frames, eval, prm, L, cands, low, S.queue[warp]);
+			if (!grid_barrier(ctl, ++round, state, nf))
+				return;
+		}
+		if (first) { // what the coming stages and the next pass append to
+			ctl->fresh0 = ctl->n_targets;
+			next = PassLists{};
+			ctl->any[par] = 0;
+		}
+		late_candidates(frames, cands, prm, L, S.Q, S.patches[warp], S.scratch[warp], triples);
+		if (!grid_barrier(ctl, ++round, state, nf))
+			return;
+		late_grow(frames, state, cands, L, ctl, par, targets);
+		late_low(frames, state, low, prm, L, ctl, par, targets, S.Q, S.patches[warp], S.scratch[warp]);
+		if (!grid_barrier(ctl, ++round, state, nf))
+			return;
+		pass_control(state, nf, ctl, par);
+		late_replace(frames, state, par, targets, (long long)ctl->n_targets, (long long)ctl->fresh0, radius,
+			chg, &next.n_chg, S.Q);
+		if (it + 1 < maxiter && !grid_barrier(ctl, ++round, state, nf))
+			return;
+	}
+}
+
+} // namespace cb

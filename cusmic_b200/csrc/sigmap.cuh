@@ -24,7 +24,6 @@
 
 #include "common.cuh"
 #include "detect.cuh"
-#include "incremental.cuh"
 #include "kernels.cuh"
 
 namespace cb {

@@ -1,5 +1,6 @@
 """The kernels of a detection pass where their work splits: candidates within
-two pixels of an edge (read from the first pass's sig_raw map).  Masks and
+two pixels of an edge (read from the first pass's sig_raw map) and the late
+passes, which work on lists in one launch.  Masks and
 pixels are those of the CPU oracle bit for bit."""
 
 import numpy as np
@@ -34,3 +35,68 @@ def test_model_candidates_on_edges(cuda, oracle, mode, shape):
     data = edge_scene(shape[0] * 101 + shape[1], *shape)
     frame = dict(data=data, gain=1.5, readnoise=3.0)
     check_against_oracle(oracle, [frame], dict(SETTINGS, border=mode, gain=1.5, readnoise=3.0))
+
+
+def structured(seed, h, w, hits=60):
+    """Clusters of hits and tracks whose growth takes several passes."""
+    rng = np.random.default_rng(seed)
+    data = 200 + rng.normal(0, 12, (h, w))
+    for _ in range(max(1, h * w * hits // 10000)):
+        y, x = rng.integers(0, h), rng.integers(0, w)
+        n = int(rng.integers(1, 9))
+        ang = rng.uniform(0, np.pi)
+        a = rng.uniform(150, 3000)
+        for t in range(n):
+            yy, xx = int(y + t * np.sin(ang)), int(x + t * np.cos(ang))
+            if 0 <= yy < h and 0 <= xx < w:
+                data[yy, xx] += a * rng.uniform(0.15, 1)
+    return data
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("shape", ((1, 1), (4, 6), (12, 13), (13, 45), (40, 32), (64, 97),
+                                   (150, 260)))
+@pytest.mark.parametrize("noise", ("error", "model"))
+def test_late_passes(cuda, oracle, mode, shape, noise):
+    """Eight passes on frames from one pixel to several blocks of the late
+    launch, narrower than the 13 x 13 neighbourhood of a changed pixel too
+    (wrap folds it onto itself), with holes and masked pixels."""
+    h, w = shape
+    data = structured(h * 31 + w, h, w)
+    rng = np.random.default_rng(h + w)
+    mask = rng.random((h, w)) < 0.02
+    if h * w > 100:
+        data[rng.random((h, w)) < 0.005] = np.nan
+    frame = dict(data=data, mask=mask)
+    kw = dict(contrast=1.5, cr_threshold=4.0, neighbor_threshold=1.0, border=mode, maxiter=8)
+    if noise == "error":
+        frame["error"] = np.full((h, w), 12.0)
+    else:
+        frame.update(gain=1.5, readnoise=3.0)
+        kw.update(gain=1.5, readnoise=3.0)
+    check_against_oracle(oracle, [frame], kw)
+
+
+def test_late_passes_everything_listed(cuda, oracle):
+    """Zero thresholds: every pixel is a candidate in every pass, so the work
+    lists fill their buffers."""
+    data = structured(5, 60, 75)
+    for kw, frame in ((dict(), dict(data=data, error=np.full(data.shape, 12.0))),
+                      (dict(gain=1.5, readnoise=3.0), dict(data=data, gain=1.5, readnoise=3.0))):
+        check_against_oracle(oracle, [frame], dict(contrast=0.5, cr_threshold=0.0, maxiter=4,
+                                                   neighbor_threshold=0.0, **kw))
+
+
+def test_late_passes_ragged_mixed(cuda, oracle):
+    """Frames of both noise kinds that stop after different numbers of passes,
+    in one batch."""
+    frames = []
+    for i, (h, w) in enumerate(((40, 50), (7, 200), (130, 90), (64, 64), (3, 3))):
+        data = structured(i, h, w, hits=(5, 60, 120, 0, 40)[i])
+        if i % 2:
+            frames.append(dict(data=data, error=np.full((h, w), 12.0)))
+        else:
+            frames.append(dict(data=data, gain=1.5, readnoise=3.0))
+    check_against_oracle(oracle, frames, dict(contrast=1.5, cr_threshold=4.0, gain=1.5,
+                                              readnoise=3.0, neighbor_threshold=1.0, maxiter=6),
+                         ragged=True)
