@@ -52,6 +52,7 @@ struct DetectParams {
 	double tmin;  // min(cr, nb): sig_raw above it can pass a threshold
 	double thi2;  // 2 cr (1 - 1e-12): division-free superset test for sig_raw > cr
 	double tlo2;  // 2 nb (1 - 1e-12): the same for sig_raw > neighbor
+	double rcontrast; // 1 / contrast
 	int mode;
 };
 
@@ -523,24 +524,78 @@ __device__ __forceinline__ double patch_window_median(const double *P, double *S
 	return med;
 }
 
+// What a warp finds out about a candidate's significance sig = center - med5:
+// the threshold tests, bounds of sig (equal when it was computed), and what
+// exact_sig needs to compute it.
+struct Sig {
+	bool s1, s2;      // sig > cr, sig > neighbor
+	double lo, hi;    // lo <= sig <= hi
+	double noise;     // at the pixel
+	double center, v; // sig_raw at the pixel; the lane's window value (lanes < 25)
+};
+
+// The exact significance (called by the whole warp).
+__device__ __forceinline__ double exact_sig(const Sig &g)
+{
+	if (g.lo == g.hi)
+		return g.lo;
+	const double v = (threadIdx.x & 31) < 25 ? g.v : INFINITY;
+	return g.center - __shfl_sync(0xffffffffu, warp_sort32(v), 12);
+}
+
+// The 9 x 9 patch of clean around an interior pixel, three rows of a column
+// per lane (lane 9 g + c < 27: rows 3 g .. 3 g + 2 of column c).
+__device__ __forceinline__ void load_patch(const FrameDesc &fd, int x, int y, double (&p)[3])
+{
+	const int lane = threadIdx.x & 31;
+	p[0] = p[1] = p[2] = 0;
+	if (lane < 27) {
+		const double *src = fd.clean + (long long)(y - 4 + 3 * (lane / 9)) * fd.w + (x - 4 + lane % 9);
+		p[0] = src[0];
+		p[1] = src[fd.w];
+		p[2] = src[2 * (long long)fd.w];
+	}
+}
+
+__device__ __forceinline__ void store_patch(double *P, const double (&p)[3])
+{
+	const int lane = threadIdx.x & 31;
+	__syncwarp(); // earlier reads of P
+	if (lane < 27) {
+		double *q = P + 27 * (lane / 9) + lane % 9;
+		q[0] = p[0];
+		q[9] = p[1];
+		q[18] = p[2];
+	}
+	__syncwarp();
+}
+
 // S: the warp's scratch of at least CS_RUNS doubles on noise-model frames
 // (25 otherwise).
+//
+// No sort: fl(center - v) falls as v grows, so sig > t, the test at the
+// window's rank 12 value, holds exactly when it holds at 13 or more of the 25
+// values (a ballot per threshold).  The window median lies between 0 (sig_raw
+// is never negative for positive noise) and SIG_MED_HI when 13 values do,
+// which bounds sig for the contrast test; only a seed that these bounds leave
+// undecided has its window sorted (exact_sig).
+constexpr double SIG_MED_HI = 1.5;
+
 template <bool LOW, int PATH = PATH_ANY>
-__device__ __forceinline__ double candidate_sig(const FrameDesc &fd, int x, int y, double *P,
-	double *S, const DetectParams &prm, double &nz_center_out, bool fresh, bool skip = false)
+__device__ __forceinline__ Sig candidate_sig(const FrameDesc &fd, int x, int y, double *P, double *S,
+	const DetectParams &prm, bool fresh, bool skip = false)
 {
 	const int lane = threadIdx.x & 31;
 	const int w = fd.w, h = fd.h, mode = prm.mode, lm = lap_mode(mode);
 	const bool err = has_error_map<PATH>(fd);
+	Sig g;
 	double v = INFINITY, nz = 0;
 	if (x >= 4 && y >= 4 && x + 4 < w && y + 4 < h) { // warp-uniform
-		__syncwarp();
-		const double *src = fd.clean + (long long)(y - 4) * w + (x - 4);
-		for (int k = lane; k < 81; k += 32)
-			P[k] = src[(long long)(k / 9) * w + k % 9];
+		double p[3];
+		load_patch(fd, x, y, p);
 		if (lane < 25 && err) // loads with the patch
 			nz = fd.error[(long long)(y + lane / 5 - 2) * w + x + lane % 5 - 2];
-		__syncwarp();
+		store_patch(P, p);
 		const int dy = lane / 5, dx = lane % 5;
 		if (!err) { // warp-uniform
 			const double m = patch_window_median(P, S);
@@ -565,50 +620,66 @@ __device__ __forceinline__ double candidate_sig(const FrameDesc &fd, int x, int 
 		}
 	}
 	const double center = __shfl_sync(0xffffffffu, v, 12);
-	const double nz_center = __shfl_sync(0xffffffffu, nz, 12);
-	double med;
-	if (__any_sync(0xffffffffu, isnan(v))) {
-		// The reference's NaN rule on the 25 values, in the warp's scratch
-		// (a register array indexed at run time would live in local memory).
-		__syncwarp();
-		if (lane < 25)
-			S[lane] = v;
-		__syncwarp();
-		med = lane == 0 ? window_median_exact(S, 25) : 0.0;
-		med = __shfl_sync(0xffffffffu, med, 0);
-		__syncwarp();
+	g.center = center;
+	g.v = v;
+	g.noise = __shfl_sync(0xffffffffu, nz, 12);
+	const bool cell = lane < 25;
+	if (__any_sync(0xffffffffu, cell && !(v >= 0))) { // a NaN, or a negative noise
+		double med;
+		if (__any_sync(0xffffffffu, isnan(v))) {
+			// The reference's NaN rule on the 25 values, in the warp's scratch
+			// (a register array indexed at run time would live in local memory).
+			__syncwarp();
+			if (cell)
+				S[lane] = v;
+			__syncwarp();
+			med = lane == 0 ? window_median_exact(S, 25) : 0.0;
+			med = __shfl_sync(0xffffffffu, med, 0);
+			__syncwarp();
+		} else {
+			med = __shfl_sync(0xffffffffu, warp_sort32(v), 12);
+		}
+		g.lo = g.hi = center - med;
+		g.s1 = g.lo > prm.cr;
+		g.s2 = g.lo > prm.nb;
 	} else {
-		med = __shfl_sync(0xffffffffu, warp_sort32(v), 12);
+		const double d = center - v;
+		g.s2 = __popc(__ballot_sync(0xffffffffu, cell && d > prm.nb)) >= 13;
+		if (!LOW) {
+			g.s1 = __popc(__ballot_sync(0xffffffffu, cell && d > prm.cr)) >= 13;
+			g.hi = center;
+			g.lo = g.s1 ? prm.cr : -INFINITY; // (read for S1 pixels)
+			if (__popc(__ballot_sync(0xffffffffu, cell && v <= SIG_MED_HI)) >= 13)
+				g.lo = fmax(g.lo, center - SIG_MED_HI);
+		}
 	}
-	const double sig = center - med;
 	if (lane == 0 && !skip) {
-		// Set or clear: an incremental pass keeps the bits of the previous
-		// pass and re-evaluates some pixels.
+		// Set or clear: a late pass keeps the bits of the previous pass and
+		// re-evaluates some pixels.
 		const long long word = (long long)y * fd.words + (x >> 5);
 		const uint32_t bit = 1u << (x & 31);
-		write_bit(plane_ptr(fd, P_S2) + word, bit, sig > prm.nb, fresh);
+		write_bit(plane_ptr(fd, P_S2) + word, bit, g.s2, fresh);
 		if (!LOW)
-			write_bit(plane_ptr(fd, P_S1) + word, bit, sig > prm.cr, fresh);
+			write_bit(plane_ptr(fd, P_S1) + word, bit, g.s1, fresh);
 	}
-	nz_center_out = nz_center;
-	return sig;
+	return g;
 }
 
 // candidate_sig plus the seed slot of candidate e (list-based kernels).  A
 // hole (src/filters.cuh:137-146: sig = 0) gets no bit and no seed; its flag
 // is loaded before the evaluation and only read after it.
-template <bool LOW, int PATH = PATH_ANY>
+template <int PATH = PATH_ANY>
 __device__ __forceinline__ void candidate_eval(const FrameDesc &fd, uint2 t, long long e, int x, int y,
 	double *P, double *S, const DetectParams &prm, Seed *seeds, bool fresh, bool hole = false)
 {
-	double nz;
 	const long long word = (long long)y * fd.words + (x >> 5);
 	const uint32_t bit = 1u << (x & 31);
-	const uint32_t excl = LOW ? 0u : plane_ptr(fd, P_EXCL)[word];
-	const double sig = candidate_sig<LOW, PATH>(fd, x, y, P, S, prm, nz, fresh, hole);
-	if (!LOW && (threadIdx.x & 31) == 0) {
-		const bool seed = !hole && sig > prm.cr && !(excl & bit);
-		seeds[e] = seed ? Seed{t.x, t.y, sig, nz} : Seed{NO_SEED, 0, 0.0, 0.0};
+	const uint32_t excl = plane_ptr(fd, P_EXCL)[word];
+	const Sig g = candidate_sig<false, PATH>(fd, x, y, P, S, prm, fresh, hole);
+	const bool seed = !hole && g.s1 && !(excl & bit); // warp-uniform
+	const double sig = seed ? exact_sig(g) : 0.0;
+	if ((threadIdx.x & 31) == 0) {
+		seeds[e] = seed ? Seed{t.x, t.y, sig, g.noise} : Seed{NO_SEED, 0, 0.0, 0.0};
 		if (!seed) // the seed kernel decides the CAND bit of a seed
 			write_bit(plane_ptr(fd, P_CAND) + word, bit, false, fresh);
 	}
@@ -696,7 +767,7 @@ candidate_high_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restr
 			continue; // warp-uniform
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 		const bool hole = test_bit(plane_ptr(fd, P_HOLE), fd.words, x, y);
-		candidate_eval<false, PATH>(fd, t, e, x, y, P, S, prm, seeds, true, hole);
+		candidate_eval<PATH>(fd, t, e, x, y, P, S, prm, seeds, true, hole);
 	}
 }
 
@@ -736,7 +807,7 @@ candidate_map_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restri
 			const FrameDesc &fd = frames[tj.x];
 			const int x = (int)(tj.y % (unsigned)fd.w), y = (int)(tj.y / (unsigned)fd.w);
 			const bool hole = test_bit(plane_ptr(fd, P_HOLE), fd.words, x, y);
-			candidate_eval<false, PATH>(fd, tj, base + j, x, y, P, S, prm, seeds, true, hole);
+			candidate_eval<PATH>(fd, tj, base + j, x, y, P, S, prm, seeds, true, hole);
 		}
 	}
 }
@@ -920,11 +991,10 @@ __device__ __forceinline__ void low_eval(const FrameDesc *__restrict__ frames, F
 {
 	const FrameDesc &fd = frames[t.x];
 	const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
-	double nz;
-	const double sig = candidate_sig<true, PATH>(fd, x, y, P, S, prm, nz, fresh);
+	const Sig g = candidate_sig<true, PATH>(fd, x, y, P, S, prm, fresh);
 	uint32_t got = 0;
 	int lost = 0;
-	if ((threadIdx.x & 31) == 0 && sig > prm.nb)
+	if ((threadIdx.x & 31) == 0 && g.s2)
 		got = grow_self(fd, x, y, fresh, lost);
 	append_fresh(state, ctl, par, targets, (int)t.x, fd.w, x, y, got, lost);
 }
@@ -1012,80 +1082,170 @@ __device__ __forceinline__ double warp_rank64(double a, double b)
 	return __shfl_sync(0xffffffffu, a, RANK);
 }
 
+// How many of the 49 3 x 3 windows of a 9 x 9 patch hold five or more pixels
+// above t_hi, and how many hold five or more below t_lo (called by the whole
+// warp, the patch as load_patch distributes it).  The patch becomes 81 bits
+// per threshold by ballots; lane 8 k + j (j < 7) sums the three columns, then
+// the three rows, of the seven windows starting in row j, bit-sliced.
+struct WindowCounts {
+	int above, below;
+};
+
+__device__ __forceinline__ WindowCounts count_windows(const double (&p)[3], double t_hi, double t_lo)
+{
+	const int lane = threadIdx.x & 31, j = lane & 7;
+	uint32_t rows[3];
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		const uint32_t up = __ballot_sync(0xffffffffu, lane < 27 && p[k] > t_hi);
+		const uint32_t dn = __ballot_sync(0xffffffffu, lane < 27 && p[k] < t_lo);
+		// The one of rows j .. j + 2 that is k modulo 3.
+		rows[k] = (lane < 8 ? up : dn) >> (9 * ((j + 2 - k) / 3));
+	}
+	uint32_t one[3], two[3]; // a row's sums of three columns: ones and twos
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		const uint32_t a = rows[k], b = a >> 1, c = a >> 2;
+		one[k] = a ^ b ^ c;
+		two[k] = (a & b) | (c & (a ^ b));
+	}
+	const uint32_t z = one[0] ^ one[1] ^ one[2];
+	const uint32_t carry = (one[0] & one[1]) | (one[2] & (one[0] ^ one[1]));
+	const uint32_t x1 = two[0] ^ two[1], c1 = two[0] & two[1], x2 = two[2] ^ carry, c2 = two[2] & carry;
+	const uint32_t odd = x1 ^ x2, c3 = x1 & x2;
+	// z + 2 (odd + 2 (c1 + c2 + c3)) >= 5
+	const uint32_t five = ((c1 & c2) | ((c1 | c2 | c3) & (odd | z))) & 0x7fu;
+	const int n = j < 7 && lane < 16 ? __popc(five) : 0;
+	const unsigned sum = __reduce_add_sync(0xffffffffu, (unsigned)(lane < 8 ? n : n << 8));
+	return WindowCounts{(int)(sum & 0xffu), (int)(sum >> 8)};
+}
+
 // The warp's fine-structure test of a seed at (x, y) (src/filters.cuh:148-175):
-// 49 3 x 3 medians (two per lane), their 7 x 7 median, fine structure and the
-// contrast test, setting the CAND bit.  A seed at least 4 pixels from every
-// edge stages its 9 x 9 patch of clean in the warp's shared memory (P), sorts
-// the 63 vertical triples of the patch once (T) and takes each 3 x 3 median
-// from three sorted triples (median9's rule).
-__device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, double sig, double noise,
-	const DetectParams &prm, double *P, double (*T)[63], bool fresh, bool staged = false)
+// fine = max((med3 - med7) / noise, 0.01) with med7 the median of the 49 3 x 3
+// medians around it, and CAND = sig / fine > contrast.
+//
+// A seed at least 4 pixels from every edge is decided without any 3 x 3 median
+// but its own: the test holds at med7 exactly when it holds with 25 or more of
+// the 49 medians in med7's place (it can only turn true as that value grows),
+// a median m satisfies it when med3 - m < sig noise / contrast (and sig / 0.01
+// > contrast), and m > t exactly when five or more of its nine pixels are.  So
+// the seed is CAND when 25 windows hold five pixels above t_hi = med3 - sig_lo
+// noise / contrast, and not when 25 hold five below t_lo, the same with sig_hi,
+// both with a margin of 1e-12 for the roundings (of two products here, of a
+// difference and two divisions in the test).  sig need not be exact for that:
+// sig_lo and sig_hi bound it.  What these counts leave open, values outside
+// the range where the margin covers the roundings, and seeds near an edge take
+// the medians and the exact sig (from exact(), called by the whole warp).
+//
+// (Sorting the 25 window values, 63 column triples and 49 medians across the
+// warp took about 950 warp instructions per candidate and seed on error maps.
+// The candidates and seeds of 16 frames of 2048 x 2048 took 168 us with it and
+// 95 with the counts, 379 and 213 us where the error map underestimates the
+// noise of most frames; the noise-model seeds of 64 ragged frames 476 and
+// 251 us.)
+template <class Exact>
+__device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, double sig_lo, double sig_hi,
+	double noise, const DetectParams &prm, double *P, double (*T)[63], bool fresh, bool staged,
+	Exact exact)
 {
 	const int lane = threadIdx.x & 31;
 	const int w = fd.w, h = fd.h, mode = prm.mode;
-	double m3[2] = {INFINITY, INFINITY};
-	if (x >= 4 && y >= 4 && x + 4 < w && y + 4 < h) { // warp-uniform
-		__syncwarp();
-		if (!staged) { // else the candidate evaluation left this patch in P
-			const double *src = fd.clean + (long long)(y - 4) * w + (x - 4);
-			for (int k = lane; k < 81; k += 32)
-				P[k] = src[(long long)(k / 9) * w + k % 9];
-			__syncwarp();
+	const bool interior = x >= 4 && y >= 4 && x + 4 < w && y + 4 < h; // warp-uniform
+	int verdict = -1; // undecided
+	if (interior) {
+		double p[3];
+		if (staged) { // the candidate evaluation left this patch in P
+			const double *q = P + (lane < 27 ? 27 * (lane / 9) + lane % 9 : 0);
+			p[0] = q[0];
+			p[1] = q[9];
+			p[2] = q[18];
+		} else {
+			load_patch(fd, x, y, p);
+			store_patch(P, p);
 		}
-		for (int k = lane; k < 63; k += 32) {
-			double a = P[k], b = P[k + 9], c = P[k + 18];
-			cas(a, b);
-			cas(b, c);
-			cas(a, b);
-			T[0][k] = a;
-			T[1][k] = b;
-			T[2][k] = c;
-		}
-		__syncwarp();
+		const double k = prm.contrast, floor_k = k * FINE_FLOOR;
+		const bool sane = noise > 1e-100 && noise < 1e100 && sig_hi < 1e100 && k > 1e-100 && k < 1e100;
+		if (sane && sig_hi < floor_k * (1 - 1e-12)) {
+			verdict = 0;
+		} else if (sane && sig_lo > floor_k * (1 + 1e-12)) {
+			// The seed's own 3 x 3 median: the value of rank 4, by counting.
+			const double own = lane < 9 ? P[30 + 9 * (lane / 3) + lane % 3] : 0.0;
+			int rank = 0;
 #pragma unroll
-		for (int s = 0; s < 2; ++s) {
-			const int j = lane + 32 * s;
-			if (j < 49) {
-				const int k = (j / 7) * 9 + j % 7; // window rows j/7 .. +2, columns j%7 .. +2
-				const double *lo = &T[0][k], *mid = &T[1][k], *hi = &T[2][k];
-				m3[s] = med3(dmax(dmax(lo[0], lo[1]), lo[2]), med3(mid[0], mid[1], mid[2]),
-					dmin(dmin(hi[0], hi[1]), hi[2]));
+			for (int i = 0; i < 9; ++i) {
+				const double o = P[30 + 9 * (i / 3) + i % 3];
+				rank += i < lane ? o <= own : o < own;
 			}
-		}
-	} else {
-#pragma unroll
-		for (int s = 0; s < 2; ++s) {
-			const int j = lane + 32 * s;
-			if (j < 49) {
-				int qx = x + j % 7 - 3, qy = y + j / 7 - 3;
-				double m = 0;
-				if (!(mode == CONSTANT && (qx < 0 || qx >= w || qy < 0 || qy >= h))) {
-					if (mode == NEAREST) {
-						qx = clampi(qx, 0, w - 1);
-						qy = clampi(qy, 0, h - 1);
-					}
-					int mx[3], my[3];
-#pragma unroll
-					for (int i = 0; i < 3; ++i) {
-						mx[i] = border_index(qx + i - 1, w, mode);
-						my[i] = border_index(qy + i - 1, h, mode);
-					}
-					double v[9];
-#pragma unroll
-					for (int c = 0; c < 9; ++c)
-						v[c] = (mx[c % 3] | my[c / 3]) < 0 ? 0.0
-							: fd.clean[(long long)my[c / 3] * w + mx[c % 3]];
-					m = median9(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]);
-				}
-				m3[s] = m;
-			}
+			const unsigned at = __ballot_sync(0xffffffffu, lane < 9 && rank == 4);
+			const double med3 = __shfl_sync(0xffffffffu, own, __ffs(at) - 1);
+			const double ql = sig_lo * noise * prm.rcontrast, qh = sig_hi * noise * prm.rcontrast;
+			const double t_hi = (med3 - ql * (1 - 1e-12)) + 1e-15 * (fabs(med3) + ql);
+			const double t_lo = (med3 - qh * (1 + 1e-12)) - 1e-15 * (fabs(med3) + qh);
+			const WindowCounts n = count_windows(p, t_hi, t_lo);
+			verdict = n.above >= 25 ? 1 : n.below >= 25 ? 0 : -1;
 		}
 	}
-	const double med3c = __shfl_sync(0xffffffffu, m3[0], 24);
-	const double med7 = warp_rank64<24>(m3[0], m3[1]);
-	double fine = (med3c - med7) / noise;
-	fine = fine < FINE_FLOOR ? FINE_FLOOR : fine;
-	const bool cand = sig / fine > prm.contrast;
+	bool cand = verdict > 0;
+	if (verdict < 0) { // warp-uniform
+		const double sig = exact();
+		double m3[2] = {INFINITY, INFINITY};
+		if (interior) {
+			__syncwarp();
+			for (int k = lane; k < 63; k += 32) {
+				double a = P[k], b = P[k + 9], c = P[k + 18];
+				cas(a, b);
+				cas(b, c);
+				cas(a, b);
+				T[0][k] = a;
+				T[1][k] = b;
+				T[2][k] = c;
+			}
+			__syncwarp();
+#pragma unroll
+			for (int s = 0; s < 2; ++s) {
+				const int j = lane + 32 * s;
+				if (j < 49) {
+					const int k = (j / 7) * 9 + j % 7; // window rows j/7 .. +2, columns j%7 .. +2
+					const double *lo = &T[0][k], *mid = &T[1][k], *hi = &T[2][k];
+					m3[s] = med3(dmax(dmax(lo[0], lo[1]), lo[2]), med3(mid[0], mid[1], mid[2]),
+						dmin(dmin(hi[0], hi[1]), hi[2]));
+				}
+			}
+		} else {
+#pragma unroll
+			for (int s = 0; s < 2; ++s) {
+				const int j = lane + 32 * s;
+				if (j < 49) {
+					int qx = x + j % 7 - 3, qy = y + j / 7 - 3;
+					double m = 0;
+					if (!(mode == CONSTANT && (qx < 0 || qx >= w || qy < 0 || qy >= h))) {
+						if (mode == NEAREST) {
+							qx = clampi(qx, 0, w - 1);
+							qy = clampi(qy, 0, h - 1);
+						}
+						int mx[3], my[3];
+#pragma unroll
+						for (int i = 0; i < 3; ++i) {
+							mx[i] = border_index(qx + i - 1, w, mode);
+							my[i] = border_index(qy + i - 1, h, mode);
+						}
+						double v[9];
+#pragma unroll
+						for (int c = 0; c < 9; ++c)
+							v[c] = (mx[c % 3] | my[c / 3]) < 0 ? 0.0
+								: fd.clean[(long long)my[c / 3] * w + mx[c % 3]];
+						m = median9(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]);
+					}
+					m3[s] = m;
+				}
+			}
+		}
+		const double med3c = __shfl_sync(0xffffffffu, m3[0], 24);
+		const double med7 = warp_rank64<24>(m3[0], m3[1]);
+		double fine = (med3c - med7) / noise;
+		fine = fine < FINE_FLOOR ? FINE_FLOOR : fine;
+		cand = sig / fine > prm.contrast;
+	}
 	if (lane == 0)
 		write_bit(plane_ptr(fd, P_CAND) + (long long)y * fd.words + (x >> 5), 1u << (x & 31), cand,
 			fresh);
@@ -1110,8 +1270,8 @@ seed_kernel(const FrameDesc *__restrict__ frames, const Seed *__restrict__ seeds
 		if (sd.frame == NO_SEED)
 			continue; // warp-uniform
 		const FrameDesc &fd = frames[sd.frame];
-		seed_eval(fd, (int)(sd.pixel % (unsigned)fd.w), (int)(sd.pixel / (unsigned)fd.w), sd.sig,
-			sd.noise, prm, patches[warp], triples[warp], true);
+		seed_eval(fd, (int)(sd.pixel % (unsigned)fd.w), (int)(sd.pixel / (unsigned)fd.w), sd.sig, sd.sig,
+			sd.noise, prm, patches[warp], triples[warp], true, false, [&] { return sd.sig; });
 	}
 }
 
@@ -1152,12 +1312,10 @@ candidate_seed_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restr
 		const uint32_t excl = plane_ptr(fd, P_EXCL)[word];
 		if (seeds && lane == 0)
 			seeds[e] = Seed{NO_SEED, 0, 0.0, 0.0};
-		double nz;
-		const double sig = candidate_sig<false, PATH>(fd, x, y, P, &triples[warp][0][0], prm, nz,
-			true, hole);
-		// Every lane holds the same sig, so the branch is warp-uniform.
-		if (!hole && sig > prm.cr && !(excl & bit))
-			seed_eval(fd, x, y, sig, nz, prm, P, triples[warp], true, true);
+		const Sig g = candidate_sig<false, PATH>(fd, x, y, P, &triples[warp][0][0], prm, true, hole);
+		if (!hole && g.s1 && !(excl & bit)) // warp-uniform
+			seed_eval(fd, x, y, g.lo, g.hi, g.noise, prm, P, triples[warp], true, true,
+				[&] { return exact_sig(g); });
 	}
 }
 

@@ -599,6 +599,7 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 	L.poison_wait[1] = inject_wait[1].load();
 	L.maxiter = o.maxiter;
 	L.prm.contrast = o.contrast;
+	L.prm.rcontrast = 1 / o.contrast;
 	L.prm.cr = o.cr_threshold;
 	L.prm.nb = o.neighbor_threshold;
 	L.prm.tmin = std::fmin(o.cr_threshold, o.neighbor_threshold);
@@ -2095,6 +2096,7 @@ extern "C" int remove_cosmics_device_noalloc(const cusmic_image *im, const cusmi
 		fd.has_bg = im->background != nullptr || !std::isnan(o->background);
 		DetectParams prm{};
 		prm.contrast = o->contrast;
+		prm.rcontrast = 1 / o->contrast;
 		prm.cr = o->cr_threshold;
 		prm.nb = o->neighbor_threshold;
 		prm.tmin = std::fmin(o->cr_threshold, o->neighbor_threshold);

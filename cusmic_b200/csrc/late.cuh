@@ -468,11 +468,9 @@ __device__ __forceinline__ void late_candidates(const FrameDesc *__restrict__ fr
 		const FrameDesc &fd = frames[t.x];
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 		const bool excl = test_bit(plane_ptr(fd, P_EXCL), fd.words, x, y);
-		double nz;
-		const double sig = candidate_sig<false, PATH_ANY>(fd, x, y, P, S, prm, nz, false);
-		// Every lane holds the same sig, so the branch is warp-uniform.
-		if (sig > prm.cr && !excl)
-			seed_eval(fd, x, y, sig, nz, prm, P, T, false, true);
+		const Sig g = candidate_sig<false, PATH_ANY>(fd, x, y, P, S, prm, false);
+		if (g.s1 && !excl) // warp-uniform
+			seed_eval(fd, x, y, g.lo, g.hi, g.noise, prm, P, T, false, true, [&] { return exact_sig(g); });
 		else if (lane == 0)
 			write_bit(plane_ptr(fd, P_CAND) + (long long)y * fd.words + (x >> 5), 1u << (x & 31), false);
 	});

@@ -100,3 +100,28 @@ def test_late_passes_ragged_mixed(cuda, oracle):
     check_against_oracle(oracle, frames, dict(contrast=1.5, cr_threshold=4.0, gain=1.5,
                                               readnoise=3.0, neighbor_threshold=1.0, maxiter=6),
                          ragged=True)
+
+
+@pytest.mark.parametrize("contrast", (0.0, 1.0, 2.0, 3.0, 500.0))
+@pytest.mark.parametrize("noise", ("error", "odd_errors", "model"))
+def test_contrast_ties(cuda, oracle, contrast, noise):
+    """Small integers under power-of-two noise: the contrast and significance
+    tests meet their thresholds exactly at many pixels, so decisions by counts
+    have to fall back to the medians; zero, tiny and non-finite error values,
+    and contrasts from zero to one that nothing passes."""
+    rng = np.random.default_rng(int(contrast) + len(noise))
+    h, w = 120, 160
+    data = rng.integers(0, 6, (h, w)) * 4.0 + 64
+    hit = rng.random((h, w)) < 0.05
+    data[hit] += rng.choice([16.0, 32.0, 48.0, 64.0, 256.0], int(hit.sum()))
+    frame = dict(data=data)
+    kw = dict(contrast=contrast, cr_threshold=4.0, neighbor_threshold=2.0, maxiter=3)
+    if noise == "model":
+        frame.update(gain=1.0, readnoise=0.0)
+        kw.update(gain=1.0, readnoise=0.0)
+    else:
+        frame["error"] = np.full((h, w), 2.0)
+        if noise == "odd_errors":
+            odd = rng.random((h, w)) < 0.03
+            frame["error"][odd] = rng.choice([0.0, 1e-200, np.inf, np.nan], int(odd.sum()))
+    check_against_oracle(oracle, [frame], kw)
