@@ -356,10 +356,13 @@ model_floor_kernel(const FrameDesc *__restrict__ frames, const FloorJob *__restr
 			continue;
 		const int n = min(FLOOR_BLOCK, fd.h - jb.y0);
 		const uint32_t *m = plane_ptr(fd, P_ROWMIN) + (long long)jb.y0 * fd.words + jb.x0 / 32;
-		uint32_t hi = 0xffffffffu;
-#pragma unroll 8
-		for (int k = 0; k < n; ++k)
-			hi = min(hi, m[(long long)k * fd.words]);
+		uint32_t v[FLOOR_BLOCK], hi = 0xffffffffu;
+#pragma unroll
+		for (int k = 0; k < FLOOR_BLOCK; ++k) // every load in flight at once
+			v[k] = k < n ? m[(long long)k * fd.words] : 0xffffffffu;
+#pragma unroll
+		for (int k = 0; k < FLOOR_BLOCK; ++k)
+			hi = min(hi, v[k]);
 		floors[jb.out] = BlockFloor{0.0, hi != 0xffffffffu ? (unsigned long long)hi << 32 : ~0ull,
 			~0ull, ~0ull};
 	}

@@ -816,8 +816,7 @@ candidate_map_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restri
 // grown = dilate3x3(dilate3x3(CAND) & S1) & S2, clipped to the frame; fresh =
 // grown & ~CRMASK joins the mask and the target list (src/cleaner.cuh:22-37).
 //
-// It is driven by the work lists, a thread per listed pixel, because what can
-// grow lies within two pixels of one: 58,520 of 67 million pixels are CAND on
+// It is driven by the work lists, because what can grow lies within two pixels of one: 58,520 of 67 million pixels are CAND on
 // 16 frames of 2048 x 2048.  (The row sweeps over the bit planes that this
 // replaced took 126 us in the four passes of those frames, bound by their
 // chains of dependent word loads, most of which found nothing.)
@@ -830,144 +829,79 @@ candidate_map_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restri
 // LOW pixel's S2 bit may date from an earlier pass (it is evaluated again, on
 // its own, wherever its CAND neighbourhood changed), so only HIGH pixels count.
 
-// What the growth around a pixel reads: five columns around x (bits5) of the
-// rows around y, all loaded before any is used (one memory round trip).
-struct GrowthRows {
-	uint32_t c[5], s1[3], s2[5], in[5], donor[5]; // CAND, S1, S2, CRMASK, DONOR
+// Eight lanes work on a listed pixel (x, y), lane r < 5 of them on row
+// y - 2 + r: the S1 cells within one pixel of (x, y) that touch a CAND pixel,
+// dilated, with S2 set (late passes: and HIGH) and not in the mask yet, join
+// the mask and the target list.  A lane loads its row's words together, and
+// the rows meet by shuffles: a few hundred instructions in all, where a thread
+// per pixel unrolls over a thousand, whose fetching took most of the time of
+// a late pass's growth (11 us for 34 pixels).
+enum GrowKind {
+	GROW_FIRST, // the full pass: any S2 pixel
+	GROW_LATE,  // HIGH pixels only, and the new pixels' FRESH bits
+	GROW_SELF   // only (x, y) itself, whose S2 bit was just found set
 };
 
-// own: the pixel is CAND, which alone decides (CAND is not read).  first: any
-// S2 pixel may grow, else only HIGH ones.
-__device__ __forceinline__ void growth_load(const FrameDesc &fd, int x, int y, bool own, bool first,
-	GrowthRows &G)
+// Called by the whole warp (on: the lane's group has a pixel; fd, x, y, f are
+// its group's).  track: set FRESH bits.
+__device__ __forceinline__ void grow_group(const FrameDesc &fd, int f, int x, int y, bool on, GrowKind kind,
+	bool track, FrameState *state, Control *ctl, int par, uint2 *targets)
 {
-	const uint32_t *cand = plane_ptr(fd, P_CAND), *s1 = plane_ptr(fd, P_S1), *s2 = plane_ptr(fd, P_S2);
-	const uint32_t *high = plane_ptr(fd, P_HIGH), *crm = plane_ptr(fd, P_CRMASK), *don = plane_ptr(fd, P_DONOR);
-	const int words = fd.words, h = fd.h;
-	uint32_t hi[5];
-#pragma unroll
-	for (int j = 0; j < 5; ++j) {
-		const int yy = y - 2 + j;
-		const bool in = yy >= 0 && yy < h;
-		G.c[j] = own ? 4u : in ? bits5(cand, words, x, yy) : 0u;
-		G.s2[j] = in ? bits5(s2, words, x, yy) : 0u;
-		hi[j] = first ? 0x1fu : in ? bits5(high, words, x, yy) : 0u;
-		G.in[j] = in ? bits5(crm, words, x, yy) : 0u;
-		G.donor[j] = in ? bits5(don, words, x, yy) : 0u;
-		if (j >= 1 && j <= 3)
-			G.s1[j - 1] = in ? bits5(s1, words, x, yy) : 0u;
+	const int lane = threadIdx.x & 31, r = lane & 7, yy = y - 2 + r;
+	const int words = fd.words, w = fd.w, k = (x - 2) >> 5, s = (x - 2) & 31; // k >= -1
+	const bool in = on && r < 5 && yy >= 0 && yy < fd.h;
+	uint32_t c = 0, s1 = 0, s2 = 0, old = 0, donor = 0;
+	if (in) {
+		c = bits5(plane_ptr(fd, P_CAND), words, x, yy);
+		s1 = bits5(plane_ptr(fd, P_S1), words, x, yy);
+		s2 = kind == GROW_SELF ? (r == 2 ? 4u : 0u) : bits5(plane_ptr(fd, P_S2), words, x, yy);
+		if (kind == GROW_LATE)
+			s2 &= bits5(plane_ptr(fd, P_HIGH), words, x, yy);
+		old = bits5(plane_ptr(fd, P_CRMASK), words, x, yy);
+		donor = bits5(plane_ptr(fd, P_DONOR), words, x, yy);
 	}
-#pragma unroll
-	for (int j = 0; j < 5; ++j)
-		G.s2[j] &= hi[j];
-}
-
-// The pixels to flag around the pixel, per row (bit i: column x - 2 + i): the
-// S1 cells of the 3 x 3 neighbourhood that touch a CAND pixel, dilated, with
-// S2 set and not in the mask yet.  Returns whether there is any.
-__device__ __forceinline__ bool growth_new(const GrowthRows &G, bool own, uint32_t (&g)[5])
-{
-	uint32_t d[3];
-#pragma unroll
-	for (int i = 0; i < 3; ++i) {
-		uint32_t v = own ? 4u : G.c[i] | G.c[i + 1] | G.c[i + 2];
-		v = (v | (v << 1) | (v >> 1)) & G.s1[i] & 0xeu; // columns x - 1 .. x + 1
-		d[i] = (v | (v << 1) | (v >> 1)) & 0x1fu;
-	}
-	g[0] = d[0] & G.s2[0] & ~G.in[0];
-	g[1] = (d[0] | d[1]) & G.s2[1] & ~G.in[1];
-	g[2] = (d[0] | d[1] | d[2]) & G.s2[2] & ~G.in[2];
-	g[3] = (d[1] | d[2]) & G.s2[3] & ~G.in[3];
-	g[4] = d[2] & G.s2[4] & ~G.in[4];
-	return (g[0] | g[1] | g[2] | g[3] | g[4]) != 0;
-}
-
-// Puts the pixels of g (five rows of five bits around (x, y)) into the mask;
-// returns those this call put there, bit 5 j + i for column x - 2 + i of row
-// y - 2 + j, and counts the static donors among them.  The rows' atomics are
-// issued together.
-__device__ __forceinline__ uint32_t flag_pixels(const FrameDesc &fd, int x, int y, const uint32_t (&g)[5],
-	const GrowthRows &G, bool track, int &lost)
-{
-	uint32_t *crm = plane_ptr(fd, P_CRMASK), *fr = plane_ptr(fd, P_FRESH);
-	const int k = (x - 2) >> 5, s = (x - 2) & 31; // k >= -1: bits left of the frame are zero
-	const long long o = (long long)(y - 2) * fd.words + k;
-	unsigned long long old[5];
-#pragma unroll
-	for (int j = 0; j < 5; ++j) {
-		const unsigned long long wide = (unsigned long long)g[j] << s;
-		const uint32_t lo = (uint32_t)wide, hi = (uint32_t)(wide >> 32);
-		old[j] = lo ? atomicOr(crm + o + (long long)j * fd.words, lo) : 0u;
-		if (hi)
-			old[j] |= (unsigned long long)atomicOr(crm + o + (long long)j * fd.words + 1, hi) << 32;
-	}
-	uint32_t out = 0;
-#pragma unroll
-	for (int j = 0; j < 5; ++j) {
-		const uint32_t now = g[j] & ~(uint32_t)(old[j] >> s);
-		lost += __popc(now & G.donor[j]);
-		out |= now << (5 * j);
-		if (track && now) {
-			const unsigned long long wide = (unsigned long long)now << s;
-			if ((uint32_t)wide)
-				atomicOr(fr + o + (long long)j * fd.words, (uint32_t)wide);
-			if (wide >> 32)
-				atomicOr(fr + o + (long long)j * fd.words + 1, (uint32_t)(wide >> 32));
-		}
-	}
-	return out;
-}
-
-// The fresh pixels of a warp's lanes (flag_pixels masks around (x, y) of frame
-// f) into the target list and their frames' state; called by the whole warp.
-__device__ __forceinline__ void append_fresh(FrameState *state, Control *ctl, int par, uint2 *targets,
-	int f, int w, int x, int y, uint32_t fresh, int lost)
-{
-	if (!__any_sync(0xffffffffu, fresh != 0))
+	uint32_t v = c | __shfl_up_sync(0xffffffffu, c, 1, 8) | __shfl_down_sync(0xffffffffu, c, 1, 8);
+	v = r >= 1 && r <= 3 ? (v | (v << 1) | (v >> 1)) & s1 & 0xeu : 0u; // columns x - 1 .. x + 1
+	const uint32_t d = (v | (v << 1) | (v >> 1)) & 0x1fu;
+	uint32_t g = d | __shfl_up_sync(0xffffffffu, d, 1, 8) | __shfl_down_sync(0xffffffffu, d, 1, 8);
+	g &= s2 & ~old;
+	if (!__any_sync(0xffffffffu, g != 0))
 		return;
-	const int lane = threadIdx.x & 31;
-	unsigned long long slot = warp_append(&ctl->n_targets, __popc(fresh));
-	// The frame's state: once for the warp when the lanes share a frame.
-	const unsigned some = __ballot_sync(0xffffffffu, fresh != 0);
-	const int lead = __ffs(some) - 1, f0 = __shfl_sync(0xffffffffu, f, lead);
-	const bool same = __all_sync(0xffffffffu, !fresh || f == f0);
-	const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)lost);
-	if (fresh) {
-		if (!same || lane == lead) {
-			const int gone = same ? sum : lost;
-			set_flag(&state[f].todo[par]);
-			if (gone)
-				atomicAdd((unsigned long long *)&state[f].donors_left,
-					(unsigned long long)(-(long long)gone));
-		}
-		for (; fresh; fresh &= fresh - 1) {
-			const int b = __ffs(fresh) - 1;
-			targets[slot++] = make_uint2((unsigned)f,
-				(unsigned)((long long)(y - 2 + b / 5) * w + (x - 2 + b % 5)));
+	uint32_t now = 0;
+	if (g) { // (columns left of the frame have no S2 bits)
+		uint32_t *crm = plane_ptr(fd, P_CRMASK) + (long long)yy * words + k;
+		const unsigned long long wide = (unsigned long long)g << s;
+		const uint32_t lo = (uint32_t)wide, hi = (uint32_t)(wide >> 32);
+		const uint32_t o0 = lo ? atomicOr(crm, lo) : 0u, o1 = hi ? atomicOr(crm + 1, hi) : 0u;
+		now = g & ~(uint32_t)((o0 | (unsigned long long)o1 << 32) >> s);
+		if (track && now) {
+			uint32_t *fr = plane_ptr(fd, P_FRESH) + (long long)yy * words + k;
+			const unsigned long long n = (unsigned long long)now << s;
+			if ((uint32_t)n)
+				atomicOr(fr, (uint32_t)n);
+			if (n >> 32)
+				atomicOr(fr + 1, (uint32_t)(n >> 32));
 		}
 	}
-}
-
-// The growth around a listed pixel (see above); returns its new pixels as
-// flag_pixels.
-__device__ __forceinline__ uint32_t grow_around(const FrameDesc &fd, int x, int y, bool own, bool first,
-	int &lost)
-{
-	GrowthRows G;
-	growth_load(fd, x, y, own, first, G);
-	uint32_t g[5];
-	return growth_new(G, own, g) ? flag_pixels(fd, x, y, g, G, !first, lost) : 0u;
-}
-
-// The growth of a pixel whose own S2 bit was just found set.
-__device__ __forceinline__ uint32_t grow_self(const FrameDesc &fd, int x, int y, bool first, int &lost)
-{
-	GrowthRows G;
-	growth_load(fd, x, y, false, true, G);
-	G.s2[0] = G.s2[1] = G.s2[3] = G.s2[4] = 0u;
-	G.s2[2] = 4u;
-	uint32_t g[5];
-	return growth_new(G, false, g) ? flag_pixels(fd, x, y, g, G, !first, lost) : 0u;
+	// The new pixels into the target list, and their frames' state: once for
+	// the warp when its groups share a frame.
+	const unsigned some = __ballot_sync(0xffffffffu, now != 0);
+	if (!some)
+		return;
+	unsigned long long slot = warp_append(&ctl->n_targets, __popc(now));
+	const int lost = __popc(now & donor);
+	const int lead = __ffs(some) - 1, f0 = __shfl_sync(0xffffffffu, f, lead);
+	const bool same = __all_sync(0xffffffffu, !now || f == f0);
+	const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)lost);
+	if (now && (!same || lane == lead)) {
+		const int gone = same ? sum : lost;
+		set_flag(&state[f].todo[par]);
+		if (gone)
+			atomicAdd((unsigned long long *)&state[f].donors_left, (unsigned long long)(-(long long)gone));
+	}
+	const unsigned base = (unsigned)((long long)yy * w + x - 2);
+	for (; now; now &= now - 1)
+		targets[slot++] = make_uint2((unsigned)f, base + __ffs(now) - 1);
 }
 
 // Any CAND pixel within two pixels of (x, y) (S2 is read only by the second
@@ -992,11 +926,8 @@ __device__ __forceinline__ void low_eval(const FrameDesc *__restrict__ frames, F
 	const FrameDesc &fd = frames[t.x];
 	const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 	const Sig g = candidate_sig<true, PATH>(fd, x, y, P, S, prm, fresh);
-	uint32_t got = 0;
-	int lost = 0;
-	if ((threadIdx.x & 31) == 0 && g.s2)
-		got = grow_self(fd, x, y, fresh, lost);
-	append_fresh(state, ctl, par, targets, (int)t.x, fd.w, x, y, got, lost);
+	if (g.s2) // warp-uniform
+		grow_group(fd, (int)t.x, x, y, (threadIdx.x & 31) < 8, GROW_SELF, !fresh, state, ctl, par, targets);
 }
 
 // Low list and growth of a full pass (run after the seeds): a lane per low
@@ -1013,32 +944,43 @@ low_grow_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const u
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const long long stride = (long long)gridDim.x * blockDim.x;
 	const long long nc = grow ? (long long)ctl->pass[par].n_cand : 0, nl = (long long)ctl->pass[par].n_low;
-	const long long start = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31);
-	for (long long base = start; base < nc; base += stride) { // warp-uniform
+	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, nw = stride >> 5;
+	// Entries per warp and sweep: 32 for a long list, fewer for a short one,
+	// whose survivors then land on different warps.  (Dealing the entries to the
+	// warps one by one spreads them better, but no two lanes' loads share a line
+	// then: 60 instead of 48 us on 16 frames of 2048 x 2048.)
+	auto chunk_of = [&](long long n) { return n >= nw * 32 ? 32 : n > nw ? (int)((n + nw - 1) / nw) : 1; };
+	const int cc = chunk_of(nc), cl = chunk_of(nl);
+	for (long long base = gw * cc; base < nc; base += nw * cc) { // warp-uniform
 		const long long e = base + lane;
 		uint2 t = make_uint2(0u, 0u);
-		int w = 1, x = 0, y = 0, lost = 0;
-		uint32_t got = 0;
-		if (e < nc) {
+		bool cand = false;
+		if (lane < cc && e < nc) {
 			t = cands[e];
 			const FrameDesc &fd = frames[t.x];
-			w = fd.w;
-			x = (int)(t.y % (unsigned)w);
-			y = (int)(t.y / (unsigned)w);
-			if (test_bit(plane_ptr(fd, P_CAND), fd.words, x, y))
-				got = grow_around(fd, x, y, true, true, lost);
+			cand = test_bit(plane_ptr(fd, P_CAND), fd.words, (int)(t.y % (unsigned)fd.w),
+				(int)(t.y / (unsigned)fd.w));
 		}
-		append_fresh(state, ctl, par, targets, (int)t.x, w, x, y, got, lost);
+		for (unsigned m = __ballot_sync(0xffffffffu, cand); m;) { // four CAND pixels at a time
+			int j = -1;
+#pragma unroll
+			for (int q = 0; q < 4; ++q) {
+				if (q == lane >> 3)
+					j = __ffs(m) - 1;
+				m &= m - 1;
+			}
+			const unsigned f = __shfl_sync(0xffffffffu, t.x, j & 31), pix = __shfl_sync(0xffffffffu, t.y, j & 31);
+			const FrameDesc &fd = frames[f];
+			grow_group(fd, (int)f, (int)(pix % (unsigned)fd.w), (int)(pix / (unsigned)fd.w), j >= 0, GROW_FIRST,
+				false, state, ctl, par, targets);
+		}
 	}
 	const unsigned long long cap = ctl->cand_cap;
-	const long long gw = start >> 5, nw = stride >> 5;
-	// The entries are dealt to the warps one by one: neighbouring entries,
-	// whose survivors come in clusters, land on different warps.
-	for (long long base = gw; base < nl; base += nw * 32) { // warp-uniform
-		const long long e = base + lane * nw;
+	for (long long base = gw * cl; base < nl; base += nw * cl) { // warp-uniform
+		const long long e = base + lane;
 		uint2 t = make_uint2(0, 0);
 		bool near = false;
-		if (e < nl) {
+		if (lane < cl && e < nl) {
 			t = cands[cap - 1 - e];
 			const FrameDesc &fd = frames[t.x];
 			near = serves<PATH>(fd) && low_near(fd, (int)(t.y % (unsigned)fd.w), (int)(t.y / (unsigned)fd.w));

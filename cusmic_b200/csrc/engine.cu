@@ -381,6 +381,7 @@ struct Layout {
 	DetectParams prm{};
 	int maxiter = 0;
 	int error_frames = 0; // frames with an error map (a rebound plan keeps which)
+	bool map_floors = false; // some frame's floors are read from its maps
 	// Kernel choices that depend on the buffers' alignment (a rebound plan
 	// whose choices change is captured again): the bulk-staged prepare, and
 	// prepare with the dense detection in one kernel (prep_detect_kernel).
@@ -619,6 +620,7 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 		d.data = im.data;
 		d.error = im.error;
 		L.error_frames += im.error != nullptr;
+		L.map_floors = L.map_floors || im.error || im.gain || im.readnoise;
 		d.gain_map = im.error ? nullptr : im.gain;
 		d.rn_map = im.error ? nullptr : im.readnoise;
 		d.bg_map = im.background;
@@ -956,7 +958,8 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		mark(rec, K_COPY);
 		return;
 	}
-	// The same launch zeroes the bit planes from CRMASK to LISTED: nothing
+	// The same launch zeroes the output masks and the bit planes from CRMASK to
+	// LISTED: nothing
 	// else writes them before the first pass, which therefore clears nothing
 	// itself.  prepare writes every word of HOLE, EXCL and DONOR, and of ROWMIN
 	// on noise-model frames (the only frames whose ROWMIN is read).  Planes
@@ -964,8 +967,10 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 	static_assert(P_HOLE == 0 && P_EXCL == 1 && P_DONOR == 2 && P_CRMASK == 3 &&
 		P_ROWMIN == N_PLANES - 1, "plane order");
 	const long long z16 = (long long)(P_ROWMIN - P_CRMASK) * L.plane_words / 4;
-	const long long zb = (z16 + 255) / 256, fb = (nf + 255) / 256, zcap = (long long)di.sms * 8;
-	uint4 *const zero = reinterpret_cast<uint4 *>(ws.bits.p + P_CRMASK * L.plane_words);
+	const ZeroRange zero{reinterpret_cast<uint4 *>(ws.bits.p + P_CRMASK * L.plane_words), z16,
+		ws.frames.p, (long long)L.total_px};
+	const long long zb = (std::max(z16, zero.bytes / 16) + 255) / 256, fb = (nf + 255) / 256,
+		zcap = (long long)di.sms * 8;
 	if (L.fused) {
 		// The error-map floors (they read the maps only) in the same launch
 		// as the state and the zeroing, then prepare with the first pass's
@@ -973,7 +978,7 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		const long long jb = ((long long)L.jobs.size() + 7) / 8;
 		prep_init_kernel<<<(int)std::max({fb, std::min(zb, zcap), std::min(jb, zcap)}), 256, 0, s>>>(
 			ws.state.p, nf, ws.ctl.p, L.maxiter, (unsigned long long)L.total_px, L.poison_wait[0],
-			L.poison_wait[1], zero, z16, ws.frames.p, ws.jobs.p, (int)L.jobs.size(), L.prm,
+			L.poison_wait[1], zero, ws.frames.p, ws.jobs.p, (int)L.jobs.size(), L.prm,
 			ws.floors.p);
 		mark(rec, K_INIT); // the state, the zeroed planes and the floors
 		const int nbulk = (int)L.bulk.size(), pcap = di.sms * PD_BLOCKS_PER_SM;
@@ -986,7 +991,7 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		return;
 	}
 	init_kernel<<<(int)std::max(fb, std::min(zb, zcap)), 256, 0, s>>>(ws.state.p, nf, ws.ctl.p,
-		L.maxiter, (unsigned long long)L.total_px, L.poison_wait[0], L.poison_wait[1], zero, z16);
+		L.maxiter, (unsigned long long)L.total_px, L.poison_wait[0], L.poison_wait[1], zero);
 	mark(rec, K_INIT); // the state and the zeroed planes
 	launch_prepare(ws, L, di, s);
 	mark(rec, K_PREPARE);
@@ -995,8 +1000,9 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 	// replacement lower with the values they write.
 	if (!L.jobs.empty()) {
 		const int nj = (int)L.jobs.size(), cap = di.sms * 8;
-		floor_kernel<<<(nj + 7) / 8 < cap ? (nj + 7) / 8 : cap, 256, 0, s>>>(ws.frames.p, ws.jobs.p,
-			nj, L.prm, ws.floors.p);
+		if (L.map_floors) // (a warp per job; the others' jobs are model_floor_kernel's)
+			floor_kernel<<<(nj + 7) / 8 < cap ? (nj + 7) / 8 : cap, 256, 0, s>>>(ws.frames.p, ws.jobs.p,
+				nj, L.prm, ws.floors.p);
 		if (L.error_frames < nf)
 			model_floor_kernel<<<(nj + 255) / 256 < cap ? (nj + 255) / 256 : cap, 256, 0, s>>>(
 				ws.frames.p, ws.jobs.p, nj, ws.floors.p);
@@ -1014,7 +1020,8 @@ static void launch_epilogue(Workspace &ws, const Layout &L, const DeviceInfo &di
 	if (!L.maxiter)
 		return;
 	const int nrows = (int)L.rows.size();
-	restore_kernel<<<grid_for_rows(di, nrows, L.tune.row_blocks_per_sm), 256, 0, s>>>(ws.frames.p, ws.rows.p, nrows);
+	finish_kernel<<<grid_for_rows(di, nrows, L.tune.row_blocks_per_sm), 256, 0, s>>>(ws.frames.p, ws.state.p,
+		ws.rows.p, nrows, ws.targets.p, ws.ctl.p);
 	mark(rec, K_RESTORE);
 }
 

@@ -88,16 +88,39 @@ validate_kernel(const double *__restrict__ v, long long n, int minimum, unsigned
 		atomicOr(flags, bit);
 }
 
-// Per-frame state and loop control of a call; with `zero`, also zeroes the n16
-// 16-byte words there (the bit planes that nothing writes before the first
-// pass) with a grid-stride loop of 16-byte stores.
+// What a call's first launch zeroes: the n16 16-byte words of the bit planes
+// that nothing writes before the first pass, and the output masks (of which
+// finish_kernel sets the flagged pixels): `bytes` bytes, the frames' masks back
+// to back, from the first descriptor's (a plan's buffers change, its launches
+// do not).
+struct ZeroRange {
+	uint4 *planes;
+	long long n16;
+	const FrameDesc *frames;
+	long long bytes;
+};
+
+// Per-frame state and loop control of a call, and the zeroing, with grid-stride
+// loops of 16-byte stores.
 __device__ __forceinline__ void init_state(FrameState *state, int nf, Control *ctl, int maxiter,
-	unsigned long long cand_cap, long long poison_prepare, long long poison_detect, uint4 *zero,
-	long long n16)
+	unsigned long long cand_cap, long long poison_prepare, long long poison_detect, const ZeroRange &z)
 {
 	const long long stride = (long long)gridDim.x * blockDim.x;
-	for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n16; j += stride)
-		zero[j] = make_uint4(0u, 0u, 0u, 0u);
+	const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+	for (long long j = first; j < z.n16; j += stride)
+		z.planes[j] = make_uint4(0u, 0u, 0u, 0u);
+	if (z.bytes) { // the aligned body by 16 bytes, the ends byte by byte
+		uint8_t *mask = z.frames[0].mask_out;
+		const long long head = min(z.bytes, (long long)(-(uintptr_t)mask & 15u));
+		const long long body = (z.bytes - head) / 16, tail = z.bytes - head - 16 * body;
+		uint4 *m16 = reinterpret_cast<uint4 *>(mask + head);
+		for (long long j = first; j < body; j += stride)
+			m16[j] = make_uint4(0u, 0u, 0u, 0u);
+		if (first < head)
+			mask[first] = 0;
+		if (first < tail)
+			mask[head + 16 * body + first] = 0;
+	}
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i < nf) {
 		FrameState s = {};
@@ -115,9 +138,9 @@ __device__ __forceinline__ void init_state(FrameState *state, int nf, Control *c
 
 __global__ void init_kernel(FrameState *state, int nf, Control *ctl, int maxiter,
 	unsigned long long cand_cap, long long poison_prepare = 0, long long poison_detect = 0,
-	uint4 *zero = nullptr, long long n16 = 0)
+	ZeroRange zero = ZeroRange{})
 {
-	init_state(state, nf, ctl, maxiter, cand_cap, poison_prepare, poison_detect, zero, n16);
+	init_state(state, nf, ctl, maxiter, cand_cap, poison_prepare, poison_detect, zero);
 }
 
 // IEEE bits mapped to an unsigned total order (reference src/replace.cuh:37-48).
@@ -829,9 +852,48 @@ fill_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__
 	}
 }
 
-// Reference src/image.cuh:50-70, in place: clean -= bg, non-finite inputs
-// restored bit for bit, uint8 mask from the bit plane.  Without a background
-// the clean pixels are already the output and are not rewritten.
+// The end of a call (reference src/image.cuh:50-70).  prepare wrote every
+// output pixel but the flagged ones, and the masks start zero, so what is left
+// is sparse: the flagged pixels' mask bytes and, for a frame with a background
+// (whose working pixels are a buffer of their own), their values, from the
+// target list; and the non-finite inputs of the frames whose working pixels are
+// the output, bit for bit, from the HOLE words (a warp per row).  Writing every
+// mask byte from the CRMASK words took 24 us on 16 frames of 2048 x 2048 and
+// 108 us on 64 ragged frames, whose rows are not aligned; zeroing the masks in
+// the first launch and this take 10 + 6 and 26 + 9 us.
+__global__ void __launch_bounds__(256)
+finish_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
+	const int2 *__restrict__ rows, int nrows, const uint2 *__restrict__ targets,
+	const Control *__restrict__ ctl)
+{
+	const long long n = (long long)ctl->n_targets, stride = (long long)gridDim.x * blockDim.x;
+	for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += stride) {
+		const uint2 t = targets[e];
+		const FrameDesc &fd = frames[t.x];
+		fd.mask_out[t.y] = 1;
+		if (fd.out != fd.clean)
+			fd.out[t.y] = fd.clean[t.y] + -1 * (fd.bg_map ? fd.bg_map[t.y] : fd.bg);
+	}
+	const int lane = threadIdx.x & 31;
+	const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+	for (int r = gw; r < nrows; r += nw) {
+		const int2 item = rows[r];
+		const FrameDesc &fd = frames[item.x];
+		if (!state[item.x].holes || fd.out != fd.clean)
+			continue; // warp-uniform
+		const uint32_t *hole = plane_ptr(fd, P_HOLE) + (long long)item.y * fd.words;
+		const long long rowpix = (long long)item.y * fd.w;
+		for (int k = lane; k < fd.words; k += 32)
+			for (uint32_t hb = hole[k]; hb; hb &= hb - 1) {
+				const long long i = rowpix + 32 * k + __ffs(hb) - 1;
+				fd.clean[i] = fd.data[i];
+			}
+	}
+}
+
+// The same for a call without the zeroed masks and the separate output
+// buffers (the allocation-free entry point): clean -= bg in place, non-finite
+// inputs restored, every mask byte from the bit plane.
 __global__ void __launch_bounds__(256)
 restore_kernel(const FrameDesc *__restrict__ frames, const int2 *__restrict__ rows, int nrows)
 {
@@ -850,72 +912,6 @@ restore_kernel(const FrameDesc *__restrict__ frames, const int2 *__restrict__ ro
 		uint8_t *mask_out = fd.mask_out + rowpix;
 		const double bgv = fd.bg;
 		const bool has_bg = fd.has_bg;
-		// A separate output buffer: prepare wrote every output pixel but the
-		// flagged ones (and restored the holes).
-		double *out = fd.out && fd.out != fd.clean ? fd.out + rowpix : nullptr;
-		if (!has_bg || out) { // warp-uniform
-			// clean (or out) already holds the output but for the flagged
-			// pixels of a separate output: only the mask, those pixels and
-			// the non-finite inputs are written.  Groups of 32 bit words (1024
-			// pixels), two groups' words loaded before either is used; a
-			// full group of an aligned row goes out as two contiguous
-			// 512-byte warp stores (lane j: the 16 pixels of half (j & 1) of
-			// word 16 q + j / 2), the rest byte by byte.
-			const bool vec = ((uintptr_t)mask_out & 15u) == 0;
-			for (int k0 = 0; k0 < words; k0 += 64) {
-				uint32_t cw[2], hw[2];
-#pragma unroll
-				for (int g = 0; g < 2; ++g) {
-					const int k = k0 + 32 * g + lane;
-					cw[g] = k < words ? crm[k] : 0u;
-					hw[g] = k < words ? hole[k] : 0u;
-				}
-#pragma unroll
-				for (int g = 0; g < 2; ++g) {
-					const int kb = k0 + 32 * g, k = kb + lane;
-					if (kb >= words)
-						break; // warp-uniform
-					if (vec && 32 * (kb + 32) <= w) { // warp-uniform
-#pragma unroll
-						for (int q = 0; q < 2; ++q) {
-							const uint32_t word = __shfl_sync(0xffffffffu, cw[g], 16 * q + (lane >> 1));
-							const uint32_t half = word >> (16 * (lane & 1));
-							uint32_t v[4];
-#pragma unroll
-							for (int b = 0; b < 4; ++b) {
-								const uint32_t nib = half >> (4 * b);
-								v[b] = (nib & 1u) | ((nib >> 1) & 1u) << 8 | ((nib >> 2) & 1u) << 16 |
-								       ((nib >> 3) & 1u) << 24;
-							}
-							*reinterpret_cast<uint4 *>(mask_out + 32 * kb + 512 * q + 16 * lane) =
-								make_uint4(v[0], v[1], v[2], v[3]);
-						}
-					} else {
-						// Unaligned rows: the group's words one after
-						// another, a lane per pixel (coalesced byte stores).
-						const int nk = min(32, words - kb);
-						for (int j = 0; j < nk; ++j) {
-							const uint32_t word = __shfl_sync(0xffffffffu, cw[g], j);
-							const int x = 32 * (kb + j) + lane;
-							if (x < w)
-								mask_out[x] = (word >> lane) & 1u;
-						}
-					}
-					if (out) {
-						for (uint32_t fb = cw[g]; fb; fb &= fb - 1) {
-							const int x = 32 * k + __ffs(fb) - 1;
-							out[x] = clean[x] + -1 * (bgmap ? bgmap[x] : bgv);
-						}
-					} else {
-						for (uint32_t hb = hw[g]; hb; hb &= hb - 1) {
-							const int x = 32 * k + __ffs(hb) - 1;
-							clean[x] = data[x];
-						}
-					}
-				}
-			}
-			continue;
-		}
 		for (int xb = 0; xb < w; xb += 32 * ROW_UNROLL) {
 			double v[ROW_UNROLL], bg[ROW_UNROLL];
 			uint32_t hb[ROW_UNROLL], cb[ROW_UNROLL];

@@ -378,8 +378,11 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 		__syncwarp();
 		late_class(frames, t, cls, lane < count, L, cands, low);
 	};
-	for (long long base = gw * 32; base < n; base += nw * 32) {
-		const long long e = base + lane;
+	// Long lists go to the warps in runs of 32, whose loads share lines; short
+	// ones are dealt one by one, so that few medians wait behind each other.
+	const long long first = THREADS ? gw * 32 : gw, step = THREADS ? 1 : nw;
+	for (long long base = first; base < n; base += nw * 32) {
+		const long long e = base + lane * step;
 		uint2 t = make_uint2(0u, 0u);
 		int cls = 0;
 		bool have = e < n, wait = false;
@@ -423,24 +426,28 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 // queue in shared memory.  A block's share shrinks with the list, so that a
 // short one spreads over the grid.  The entries are dealt to the blocks one by
 // one, so neighbouring entries, whose survivors come in clusters, go to
-// different blocks.
+// different blocks.  aside: other work of every warp, done before the first
+// sweep's barrier, beside other warps' tests.
 struct LateQueue {
 	uint16_t e[LATE_THREADS];
 	int n;
 };
 
-template <class Keep, class Work>
-__device__ __forceinline__ void block_sweep(long long n, LateQueue &Q, Keep keep, Work work)
+template <class Keep, class Work, class Aside>
+__device__ __forceinline__ void block_sweep(long long n, LateQueue &Q, Keep keep, Work work, Aside aside)
 {
 	const int warp = threadIdx.x >> 5;
 	const long long share = (n + gridDim.x - 1) / gridDim.x;
 	const int chunk = share < LATE_THREADS ? (int)share : LATE_THREADS;
 	const long long step = gridDim.x;
-	for (long long base = blockIdx.x; base < n;
-	     base += (long long)gridDim.x * chunk) {
+	bool first = true;
+	for (long long base = blockIdx.x; base < n || first; base += (long long)gridDim.x * chunk) { // block-uniform
 		if (threadIdx.x == 0)
 			Q.n = 0;
 		__syncthreads();
+		if (first)
+			aside();
+		first = false;
 		const long long e = base + step * threadIdx.x;
 		if ((int)threadIdx.x < chunk && e < n && keep(e))
 			Q.e[atomicAdd(&Q.n, 1)] = (uint16_t)threadIdx.x;
@@ -473,39 +480,32 @@ __device__ __forceinline__ void late_candidates(const FrameDesc *__restrict__ fr
 			seed_eval(fd, x, y, g.lo, g.hi, g.noise, prm, P, T, false, true, [&] { return exact_sig(g); });
 		else if (lane == 0)
 			write_bit(plane_ptr(fd, P_CAND) + (long long)y * fd.words + (x >> 5), 1u << (x & 31), false);
-	});
+	}, [] {});
 }
 
-// Stage 4, the high list's part: a thread per listed pixel grows around it.
-// The grid's last blocks come first, its first blocks have the low list's
-// survivors when both are short.
+// Stage 4, the high list's part: eight lanes grow around each listed pixel.
+// The entries are dealt to the blocks in fours, and within a block to its last
+// warps first (its first ones have the low list's entries).
 __device__ __forceinline__ void late_grow(const FrameDesc *__restrict__ frames, FrameState *state,
 	const uint2 *cands, const PassLists &L, Control *ctl, int par, uint2 *targets)
 {
-	const int lane = threadIdx.x & 31;
-	const long long stride = (long long)gridDim.x * blockDim.x, n = (long long)L.n_cand;
-	const long long start = (gridDim.x - 1 - blockIdx.x) * (long long)blockDim.x + (threadIdx.x & ~31);
-	for (long long base = start; base < n; base += stride) { // warp-uniform
-		const long long e = base + lane;
-		uint2 t = make_uint2(0u, 0u);
-		int w = 1, x = 0, y = 0, lost = 0;
-		uint32_t got = 0;
-		if (e < n) {
-			t = cands[e];
-			const FrameDesc &fd = frames[t.x];
-			w = fd.w;
-			x = (int)(t.y % (unsigned)w);
-			y = (int)(t.y / (unsigned)w);
-			got = grow_around(fd, x, y, false, false, lost);
+	const long long n = (long long)L.n_cand;
+	const int back = LATE_WARPS - 1 - (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	for (long long base = 4 * ((long long)back * gridDim.x + blockIdx.x); base < n;
+	     base += 4ll * LATE_WARPS * gridDim.x) { // warp-uniform
+		const long long e = base + (lane >> 3);
+		const uint2 t = e < n ? cands[e] : make_uint2(0u, 0u);
+		const FrameDesc &fd = frames[t.x];
+		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
+		if (e < n && (lane & 7) == 0)
 			plane_ptr(fd, P_LISTED)[(long long)y * fd.words + (x >> 5)] = 0u;
-		}
-		append_fresh(state, ctl, par, targets, (int)t.x, w, x, y, got, lost);
+		grow_group(fd, (int)t.x, x, y, e < n, GROW_LATE, true, state, ctl, par, targets);
 	}
 }
 
-// Stage 4, the low list's part.
+// Stage 4: the growth, and the low list's pixels near a CAND pixel, a warp each.
 __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, FrameState *state,
-	const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par, uint2 *targets,
+	const uint2 *cands, const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par, uint2 *targets,
 	LateQueue &Q, double *P, double *S)
 {
 	block_sweep((long long)L.n_low, Q, [&](long long e) {
@@ -516,7 +516,7 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 		return low_near(fd, x, y);
 	}, [&](long long e) {
 		low_eval<PATH_ANY>(frames, state, low[e], prm, ctl, par, targets, P, S, false);
-	});
+	}, [&] { late_grow(frames, state, cands, L, ctl, par, targets); });
 }
 
 // Stage 5: the replacement, by warps (few targets are left to do).  A target
@@ -548,7 +548,7 @@ __device__ __forceinline__ void late_replace(const FrameDesc *__restrict__ frame
 			if (changed)
 				chg[atomicAdd(n_chg, 1ull)] = (unsigned)e;
 		}
-	});
+	}, [] {});
 }
 
 // Stages 1 and 2 of the first late pass, which starts from every target of the
@@ -644,8 +644,7 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 		late_candidates(frames, cands, prm, L, S.Q, S.patches[warp], S.scratch[warp], triples);
 		if (!grid_barrier(ctl, ++round, state, nf))
 			return;
-		late_grow(frames, state, cands, L, ctl, par, targets);
-		late_low(frames, state, low, prm, L, ctl, par, targets, S.Q, S.patches[warp], S.scratch[warp]);
+		late_low(frames, state, cands, low, prm, L, ctl, par, targets, S.Q, S.patches[warp], S.scratch[warp]);
 		if (!grid_barrier(ctl, ++round, state, nf))
 			return;
 		pass_control(state, nf, ctl, par);

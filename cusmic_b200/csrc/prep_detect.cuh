@@ -410,11 +410,10 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 // need no launch of their own and overlap the zeroing.
 __global__ void __launch_bounds__(256)
 prep_init_kernel(FrameState *state, int nf, Control *ctl, int maxiter, unsigned long long cand_cap,
-	long long poison_prepare, long long poison_detect, uint4 *zero, long long n16,
-	const FrameDesc *__restrict__ frames, const FloorJob *__restrict__ jobs, int njobs,
+	long long poison_prepare, long long poison_detect, ZeroRange zero, const FrameDesc *__restrict__ frames, const FloorJob *__restrict__ jobs, int njobs,
 	DetectParams prm, BlockFloor *floors)
 {
-	init_state(state, nf, ctl, maxiter, cand_cap, poison_prepare, poison_detect, zero, n16);
+	init_state(state, nf, ctl, maxiter, cand_cap, poison_prepare, poison_detect, zero);
 	floor_jobs(frames, jobs, njobs, prm, floors);
 }
 
