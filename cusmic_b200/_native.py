@@ -23,7 +23,7 @@ EXPORTS = (
     "cusmic_plan_create", "cusmic_plan_bind", "cusmic_plan_execute", "cusmic_plan_wait",
     "cusmic_plan_passes", "cusmic_plan_profile", "cusmic_plan_backward", "cusmic_plan_destroy",
     "remove_cosmics_device_noalloc", "cusmic_set_tuning", "cusmic_get_tuning",
-    "cusmic_inject_fault", "cusmic_batch_host",
+    "cusmic_inject_fault", "cusmic_batch_host", "cusmic_check_maps", "cusmic_checked_batch_device",
 )
 TUNING_PATH = Path(__file__).with_name("tuning.json")
 KERNEL_KINDS = ("init", "prepare", "fill", "sigraw", "cand", "seed", "grow", "control",
@@ -50,6 +50,11 @@ class FrameScalars(ctypes.Structure):
     """struct cusmic_frame_scalars."""
     _fields_ = [("gain", ctypes.c_double), ("readnoise", ctypes.c_double),
                 ("background", ctypes.c_double)]
+
+
+class MapCheck(ctypes.Structure):
+    """struct cusmic_map_check."""
+    _fields_ = [("map", ctypes.c_void_p), ("n", ctypes.c_size_t), ("minimum", ctypes.c_int)]
 
 
 class Tuning(ctypes.Structure):
@@ -121,6 +126,11 @@ def lib():
     L.cusmic_get_tuning.argtypes = [sz, ctypes.POINTER(Tuning)]
     L.cusmic_batch_host.restype = ip
     L.cusmic_batch_host.argtypes = [img, sz, opt, sca, vp, vp, cp, sz]
+    chk, up = ctypes.POINTER(MapCheck), ctypes.POINTER(ctypes.c_uint)
+    L.cusmic_check_maps.restype = ip
+    L.cusmic_check_maps.argtypes = [chk, sz, up, vp, cp, sz]
+    L.cusmic_checked_batch_device.restype = ip
+    L.cusmic_checked_batch_device.argtypes = [img, sz, opt, vp, vp, chk, sz, up, vp, cp, sz]
     L.cusmic_inject_fault.restype = ip
     L.cusmic_inject_fault.argtypes = [ip, ctypes.c_longlong]
     _lib = L

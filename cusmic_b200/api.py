@@ -59,47 +59,114 @@ class Image:
     readnoise: Array | float | None = None
 
     def __post_init__(self):
-        data = _as_tensor(self.data)
-        if data.dtype != torch.float64:
-            raise TypeError("data must contain float64 pixels")
-        if data.dim() not in (2, 3) or not data.numel():
-            raise ValueError("data must be a nonempty 2D frame or 3D stack")
-        device = _cuda_device(data)
-        self.data = data if data.is_cuda else data.to(device)
-        shape, frame = tuple(self.data.shape), tuple(self.data.shape[-2:])
-        fields = ("error",) if self.error is not None else ("effective_gain", "readnoise")
-        # The content checks of every map run on the device and are read back
-        # with one copy (one host synchronisation per Image, on the current
-        # stream); the first failing check, in the reference's order, raises.
-        checks = []
+        self.data, device = _checked_data(self.data)
         with torch.cuda.device(device):
-            for name in (*fields, "background"):
-                value = getattr(self, name)
-                if value is None:
-                    continue
-                value = _as_tensor(value, device)
-                if value.dtype.is_complex or value.dtype == torch.bool or \
-                        not (value.dtype.is_floating_point or value.dtype in (
-                            torch.int8, torch.int16, torch.int32, torch.int64, torch.uint8)):
-                    raise TypeError(f"{name} must be real numeric data")
-                if tuple(value.shape) not in (shape, frame) and (name == "error" or value.dim() != 0):
-                    raise ValueError(f"{name} has an incompatible shape")
-                value = value.to(torch.float64)
-                checks.append((~torch.isfinite(value).all(), f"{name} must be finite"))
-                if name in ("error", "effective_gain"):
-                    checks.append(((value <= 0).any(), f"{name} must be positive"))
-                if name == "readnoise":
-                    checks.append(((value < 0).any(), "readnoise must be nonnegative"))
+            fields, checks = _calibration(self.data, device, self.error, self.background,
+                                          self.effective_gain, self.readnoise)
+            checks.run()
+            for name, value in fields.items():
+                if isinstance(value, float):
+                    value = torch.full((), value, dtype=torch.float64, device=device)
                 setattr(self, name, value)
-            if checks:
-                failed = torch.stack([flag for flag, _ in checks]).cpu().tolist()
-                for bad, (_, message) in zip(failed, checks):
-                    if bad:
-                        raise ValueError(message)
-            if self.mask is not None:
-                self.mask = _as_tensor(self.mask, device).to(torch.bool)
-                if tuple(self.mask.shape) not in (shape, frame):
-                    raise ValueError("mask must match the data or one frame")
+            self.mask = _checked_mask(self.mask, self.data, device)
+
+
+def _checked_data(data):
+    data = _as_tensor(data)
+    if data.dtype != torch.float64:
+        raise TypeError("data must contain float64 pixels")
+    if data.dim() not in (2, 3) or not data.numel():
+        raise ValueError("data must be a nonempty 2D frame or 3D stack")
+    device = _cuda_device(data)
+    return data if data.is_cuda else data.to(device), device
+
+
+def _checked_mask(mask, data, device):
+    if mask is None:
+        return None
+    mask = _as_tensor(mask, device).to(torch.bool)
+    if tuple(mask.shape) not in (tuple(data.shape), tuple(data.shape[-2:])):
+        raise ValueError("mask must match the data or one frame")
+    return mask
+
+
+class _Checks:
+    """The content checks of an image's calibration, in the reference's order:
+    scalars are decided here, maps on the device (cusmic_check_maps, or with
+    the cleaning itself); the first that failed raises."""
+
+    RULES = {"error": (1, "positive"), "effective_gain": (1, "positive"),
+             "readnoise": (0, "nonnegative"), "background": (-1, None)}
+
+    def __init__(self):
+        self.items = []   # (name, index of its map or None, failed bits of a scalar)
+        self.tensors = []  # the maps, contiguous
+
+    def add(self, name, value):
+        minimum, _ = self.RULES[name]
+        if isinstance(value, float):
+            low = value <= 0 if minimum == 1 else value < 0 if minimum == 0 else False
+            self.items.append((name, None, (not isfinite(value)) | low << 1))
+        else:
+            self.items.append((name, len(self.tensors), 0))
+            self.tensors.append(value.detach().contiguous())
+
+    def maps(self):
+        """The maps as struct cusmic_map_check."""
+        arr = (_native.MapCheck * max(1, len(self.tensors)))()
+        names = [name for name, index, _ in self.items if index is not None]
+        for i, (name, t) in enumerate(zip(names, self.tensors)):
+            arr[i] = _native.MapCheck(t.data_ptr(), t.numel(), self.RULES[name][0])
+        return arr, len(self.tensors)
+
+    @property
+    def scalar_failed(self):
+        return any(bits for _, _, bits in self.items)
+
+    def report(self, flags):
+        for name, index, bits in self.items:
+            if index is not None:
+                bits = flags >> (2 * index) & 3
+            if bits & 1:
+                raise ValueError(f"{name} must be finite")
+            if bits & 2:
+                raise ValueError(f"{name} must be {self.RULES[name][1]}")
+
+    def run(self):
+        flags = ctypes.c_uint(0)
+        if self.tensors:
+            arr, n = self.maps()
+            msg = ctypes.create_string_buffer(256)
+            stream = torch.cuda.current_stream(self.tensors[0].device).cuda_stream
+            _native.raise_for(_native.lib().cusmic_check_maps(arr, n, ctypes.byref(flags), stream,
+                                                              msg, len(msg)), msg)
+        self.report(flags.value)
+
+
+def _calibration(data, device, error, background, effective_gain, readnoise):
+    """The calibration that applies (an error map replaces gain and read
+    noise) as float64 device maps or floats, and its content checks."""
+    shape, frame = tuple(data.shape), tuple(data.shape[-2:])
+    given = {"error": error} if error is not None else \
+        {"effective_gain": effective_gain, "readnoise": readnoise}
+    given["background"] = background
+    fields, checks = {}, _Checks()
+    for name, value in given.items():
+        if value is None:
+            continue
+        value = _as_tensor(value)
+        if value.dim() or value.is_cuda:
+            value = _as_tensor(value, device)
+        if value.dtype.is_complex or value.dtype == torch.bool or \
+                not (value.dtype.is_floating_point or value.dtype in (
+                    torch.int8, torch.int16, torch.int32, torch.int64, torch.uint8)):
+            raise TypeError(f"{name} must be real numeric data")
+        if tuple(value.shape) not in (shape, frame) and (name == "error" or value.dim() != 0):
+            raise ValueError(f"{name} has an incompatible shape")
+        value = value.to(torch.float64)
+        fields[name] = value if value.dim() else float(value)
+        checks.add(name, fields[name])
+    return fields, checks
 
 
 @dataclass(frozen=True)
@@ -139,52 +206,64 @@ class Cleaner:
         if self.maxiter and image.error is None and (
                 image.effective_gain is None or image.readnoise is None):
             raise ValueError("Provide error, or both effective_gain and readnoise")
-        data = image.data
+        names = ("error",) if image.error is not None else ("effective_gain", "readnoise")
+        fields = {}
+        for name in (*names, "background"):
+            value = getattr(image, name)
+            if value is not None:
+                fields[name] = float(value) if value.dim() == 0 else value
+        return self._clean(image.data, fields, image.mask)
+
+    def _clean(self, data, fields, mask, checks=None):
+        """The cleaning of validated inputs; with ``checks``, their content
+        checks run with it and raise first."""
         device = data.device
         stack = data if data.dim() == 3 else data.unsqueeze(0)
         stack = stack.contiguous()
         nf, h, w = stack.shape
+        step = 8 * h * w
         keep = [stack]
 
-        def maps(value):
-            if value is None or value.dim() == 0:
+        def maps(value, size=8):
+            if value is None or isinstance(value, float):
                 return [None] * nf
             v = value.contiguous()
             keep.append(v)
-            if v.dim() == 3:
-                return [v[i].data_ptr() for i in range(nf)]
-            return [v.data_ptr()] * nf
+            at = v.data_ptr()
+            return [at + i * size * h * w for i in range(nf)] if v.dim() == 3 else [at] * nf
 
-        def scalar(value, default):
-            return float(value) if value is not None and value.dim() == 0 else default
+        def scalar(name, default):
+            value = fields.get(name)
+            return value if isinstance(value, float) else default
 
-        err = maps(image.error)
-        gain = maps(image.effective_gain) if image.error is None else [None] * nf
-        rn = maps(image.readnoise) if image.error is None else [None] * nf
-        bg = maps(image.background)
-        msk = [None] * nf
-        if image.mask is not None:
-            m = image.mask.to(torch.uint8).contiguous()
-            keep.append(m)
-            msk = [m[i].data_ptr() for i in range(nf)] if m.dim() == 3 else [m.data_ptr()] * nf
-        opts = self.options(
-            gain=scalar(image.effective_gain, nan) if image.error is None else nan,
-            readnoise=scalar(image.readnoise, 0.0) if image.error is None else 0.0,
-            background=scalar(image.background, nan))
+        err, gain, rn, bg = (maps(fields.get(name)) for name in
+                             ("error", "effective_gain", "readnoise", "background"))
+        # A bool tensor's bytes are the mask bytes.
+        msk = maps(None if mask is None else mask.contiguous().view(torch.uint8), 1)
+        opts = self.options(gain=scalar("effective_gain", nan), readnoise=scalar("readnoise", 0.0),
+                            background=scalar("background", nan))
         ims = (_native.Image * nf)()
+        at = stack.data_ptr()
         for i in range(nf):
-            ims[i] = _native.Image(stack[i].data_ptr(), err[i], gain[i], rn[i], bg[i], msk[i], w, h)
+            ims[i] = _native.Image(at + i * step, err[i], gain[i], rn[i], bg[i], msk[i], w, h)
         clean = torch.empty((nf, h, w), dtype=torch.float64, device=device)
-        flags = torch.empty((nf, h, w), dtype=torch.uint8, device=device)
+        flags = torch.empty((nf, h, w), dtype=torch.bool, device=device)
         msg = ctypes.create_string_buffer(512)
         with torch.cuda.device(device):
             stream = torch.cuda.current_stream(device).cuda_stream
-            status = _native.lib().remove_cosmics_batch_device(
-                ims, nf, ctypes.byref(opts), clean.data_ptr(), flags.data_ptr(), stream, msg,
-                len(msg))
+            if checks is None:
+                status = _native.lib().remove_cosmics_batch_device(
+                    ims, nf, ctypes.byref(opts), clean.data_ptr(), flags.data_ptr(), stream, msg,
+                    len(msg))
+            else:
+                failed = ctypes.c_uint(0)
+                arr, n = checks.maps()
+                status = _native.lib().cusmic_checked_batch_device(
+                    ims, nf, ctypes.byref(opts), clean.data_ptr(), flags.data_ptr(), arr, n,
+                    ctypes.byref(failed), stream, msg, len(msg))
+                checks.report(failed.value)
         del keep
         _native.raise_for(status, msg)
-        flags = flags.to(torch.bool)
         if data.dim() == 2:
             return clean[0], flags[0]
         return clean, flags
@@ -230,6 +309,21 @@ def remove_cosmics(
     Work runs on the input device's current stream; the call returns after it
     completes.  A replacement with no finite, unmasked donors raises ValueError.
     """
-    image = Image(data, error, mask, background, effective_gain, readnoise)
-    clean = Cleaner(contrast, cr_threshold, neighbor_threshold, maxiter, border_mode)
-    return clean(image)
+    # As Cleaner(...)(Image(...)), with the maps checked on the device by the
+    # call that cleans them: one submission and one synchronisation.  Whatever
+    # else fails, a failing map is reported first, as Image would.
+    data, device = _checked_data(data)
+    with torch.cuda.device(device):
+        fields, checks = _calibration(data, device, error, background, effective_gain, readnoise)
+        if checks.scalar_failed:
+            checks.run()
+        try:
+            mask = _checked_mask(mask, data, device)
+            cleaner = Cleaner(contrast, cr_threshold, neighbor_threshold, maxiter, border_mode)
+            if maxiter and error is None and ("effective_gain" not in fields or
+                                              "readnoise" not in fields):
+                raise ValueError("Provide error, or both effective_gain and readnoise")
+            return cleaner._clean(data, fields, mask, checks)
+        except Exception:
+            checks.run()
+            raise

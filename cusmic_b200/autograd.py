@@ -76,7 +76,8 @@ class _Clean(torch.autograd.Function):
         bg = image.background
         scalar_bg = bg is not None and bg.dim() == 0
         batch = Batch.stack(stack, error=image.error,
-                            mask=None if image.mask is None else image.mask.to(torch.uint8),
+                            mask=None if image.mask is None
+                            else image.mask.contiguous().view(torch.uint8),
                             gain=image.effective_gain if _is_map(image.effective_gain) else None,
                             readnoise=image.readnoise if _is_map(image.readnoise) else None,
                             background=bg if _is_map(bg) else None)
@@ -98,8 +99,11 @@ class _Clean(torch.autograd.Function):
         ctx.shape = data.shape
         ctx.bg_shape = None if bg is None else tuple(bg.shape)
         ctx.nf = nf
-        clean = batch.clean.clone()
-        mask = batch.mask_out.to(torch.bool)
+        # The batch's own output buffers, made for this call: the backward
+        # reads neither (detached, so that the outputs' graph, which holds the
+        # batch, is not held by it).
+        clean = batch.clean.detach()
+        mask = batch.mask_out.view(torch.bool)
         if data.dim() == 2:
             clean, mask = clean[0], mask[0]
         ctx.mark_non_differentiable(mask)

@@ -131,6 +131,7 @@ struct FrameState {
 	unsigned int passes;  // detection passes run
 	unsigned int fault;   // a bounded wait inside a kernel ran out (the frame stopped)
 	unsigned int todo[2]; // by parity: the pass flagged a new pixel (set by many warps)
+	unsigned int map_flags, pad; // frame 0: failed map checks of the call (check_maps_kernel)
 	long long donors_left; // static donors not in the mask (counted)
 	// Nonzero-only facts (set to 1 by many warps, never counted): any hole,
 	// any allowed pixel, any finite donor.

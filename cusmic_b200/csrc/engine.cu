@@ -35,6 +35,7 @@
 #include <stdexcept>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #ifndef CUSMIC_B200_VERSION
@@ -415,11 +416,21 @@ static DeviceInfo device_info(int dev)
 	return d;
 }
 
+// A part of a device buffer.
+template <class T> struct DevPart {
+	T *p = nullptr;
+};
+
 struct Workspace {
 	int device = -1;
-	DevBuf<FrameDesc> frames;
+	// Every descriptor array of a call, uploaded with one copy, and its parts.
+	DevBuf<unsigned char> desc;
+	DevPart<FrameDesc> frames;
+	DevPart<int2> rows;
+	DevPart<int4> bulk, grow;
+	DevPart<FloorJob> jobs;
+	DevPart<long long> offsets;
 	DevBuf<FrameState> state;
-	DevBuf<int2> rows;
 	DevBuf<uint32_t> bits;
 	DevBuf<uint2> targets;
 	DevBuf<uint8_t> radius; // per target: window radius of its last replacement
@@ -428,14 +439,10 @@ struct Workspace {
 	DevBuf<double> work;    // working pixels of the frames with a background
 	DevBuf<double> sigmap;  // first-pass sig_raw, then noise, of noise-model frames (2 x pixels)
 	DevBuf<uint2> cands;
-	DevBuf<int4> bulk;
-	DevBuf<int4> grow;
-	DevBuf<FloorJob> jobs;
 	DevBuf<BlockFloor> floors;
 	DevBuf<PreCand> pre;
 	DevBuf<int> pre_counts;
 	DevBuf<Control> ctl;
-	DevBuf<long long> offsets;
 	PinBuf<unsigned char> stage;
 	PinBuf<FrameState> hstate;
 	// Host-API staging of inputs and outputs.
@@ -701,15 +708,9 @@ static const void *host_device_ptr(const void *p)
 static void upload(Workspace &ws, Layout &L, cudaStream_t s, bool mapped = false)
 {
 	const size_t nf = L.frames.size();
-	ws.frames.ensure(nf);
 	ws.state.ensure(nf);
-	ws.bulk.ensure(L.bulk.size() ? L.bulk.size() : 1);
-	ws.grow.ensure(L.grow.size() ? L.grow.size() : 1);
-	ws.jobs.ensure(L.jobs.size() ? L.jobs.size() : 1);
 	ws.floors.ensure(L.nthr ? (size_t)L.nthr : 1);
-	ws.rows.ensure(L.rows.size());
 	ws.ctl.ensure(1);
-	ws.offsets.ensure(nf);
 	if (L.maxiter) {
 		ws.bits.ensure((size_t)L.total_words);
 		ws.targets.ensure(L.total_px);
@@ -742,45 +743,39 @@ static void upload(Workspace &ws, Layout &L, cudaStream_t s, bool mapped = false
 		if (L.maxiter && L.frames[f].has_bg)
 			L.frames[f].clean = ws.work.p + L.offsets[f];
 	}
-	// Every descriptor array goes through one pinned staging buffer.  The
-	// previous call using this workspace synchronised before returning, so
-	// the buffer is free.
-	struct Part {
-		void *dst;
-		const void *src;
-		size_t bytes;
-	};
-	const Part parts[] = {
-		{ws.frames.p, L.frames.data(), nf * sizeof(FrameDesc)},
-		{ws.rows.p, L.rows.data(), L.rows.size() * sizeof(int2)},
-		{ws.bulk.p, L.bulk.data(), L.bulk.size() * sizeof(int4)},
-		{ws.grow.p, L.grow.data(), L.grow.size() * sizeof(int4)},
-		{ws.jobs.p, L.jobs.data(), L.jobs.size() * sizeof(FloorJob)},
-		{ws.offsets.p, L.offsets.data(), nf * sizeof(long long)},
-	};
+	// Every descriptor array goes through one pinned staging buffer and one
+	// copy (a copy per array cost a small call 3 us of stream time each).  The
+	// previous call using this workspace synchronised before returning, so the
+	// buffer is free.
 	size_t total = 0;
-	for (const Part &q : parts)
-		total += (q.bytes + 15) & ~size_t(15);
+	auto place = [&](size_t bytes) {
+		const size_t at = total;
+		total = (total + bytes + 255) & ~size_t(255);
+		return at;
+	};
+	const size_t at_frames = place(nf * sizeof(FrameDesc)), at_rows = place(L.rows.size() * sizeof(int2)),
+		at_bulk = place(L.bulk.size() * sizeof(int4)), at_grow = place(L.grow.size() * sizeof(int4)),
+		at_jobs = place(L.jobs.size() * sizeof(FloorJob)), at_offsets = place(nf * sizeof(long long));
+	ws.desc.ensure(total);
 	ws.stage.ensure(total);
-	WordCopies wc{};
-	const unsigned char *dstage = mapped
-		? static_cast<const unsigned char *>(host_device_ptr(ws.stage.p)) : nullptr;
-	size_t at = 0;
-	for (const Part &q : parts) {
-		if (q.bytes) {
-			std::memcpy(ws.stage.p + at, q.src, q.bytes);
-			if (mapped) {
-				static_assert(sizeof(FrameDesc) % 8 == 0 && sizeof(FloorJob) % 8 == 0, "8-byte parts");
-				wc.part[wc.n++] = WordCopy{reinterpret_cast<const unsigned long long *>(dstage + at),
-					static_cast<unsigned long long *>(q.dst), (long long)(q.bytes / 8)};
-			} else {
-				check(cudaMemcpyAsync(q.dst, ws.stage.p + at, q.bytes, cudaMemcpyHostToDevice, s));
-			}
-		}
-		at += (q.bytes + 15) & ~size_t(15);
+	auto put = [&](auto &part, size_t at, const auto &v) {
+		std::memcpy(ws.stage.p + at, v.data(), v.size() * sizeof(v[0]));
+		part.p = reinterpret_cast<std::remove_reference_t<decltype(part.p)>>(ws.desc.p + at);
+	};
+	put(ws.frames, at_frames, L.frames);
+	put(ws.rows, at_rows, L.rows);
+	put(ws.bulk, at_bulk, L.bulk);
+	put(ws.grow, at_grow, L.grow);
+	put(ws.jobs, at_jobs, L.jobs);
+	put(ws.offsets, at_offsets, L.offsets);
+	if (!mapped) {
+		check(cudaMemcpyAsync(ws.desc.p, ws.stage.p, total, cudaMemcpyHostToDevice, s));
+		return;
 	}
-	if (mapped && wc.n)
-		word_copy_kernel<<<32, 256, 0, s>>>(wc);
+	WordCopies wc{};
+	wc.part[wc.n++] = WordCopy{static_cast<const unsigned long long *>(host_device_ptr(ws.stage.p)),
+		reinterpret_cast<unsigned long long *>(ws.desc.p), (long long)(total / 8)};
+	word_copy_kernel<<<32, 256, 0, s>>>(wc);
 }
 
 // Kernel kinds reported by cusmic_plan_profile().
@@ -1053,20 +1048,37 @@ static void check_state(const FrameState &st)
 
 // Copy per-frame state back and turn it into a status (stream must be idle
 // after this returns).
-static void finish(Workspace &ws, size_t nf, cudaStream_t s, std::vector<int> *passes = nullptr)
+// With map_flags, the failed map checks of the call go there first.
+static void finish(Workspace &ws, size_t nf, cudaStream_t s, unsigned *map_flags = nullptr)
 {
 	ws.hstate.ensure(nf);
 	check(cudaMemcpyAsync(ws.hstate.p, ws.state.p, nf * sizeof(FrameState), cudaMemcpyDeviceToHost, s));
 	check(cudaStreamSynchronize(s));
 	check(cudaGetLastError());
-	if (passes)
-		passes->assign(nf, 0);
-	for (size_t f = 0; f < nf; ++f) {
-		const FrameState &st = ws.hstate.p[f];
-		if (passes)
-			(*passes)[f] = (int)st.passes;
-		check_state(st);
+	if (map_flags)
+		*map_flags = ws.hstate.p[0].map_flags;
+	for (size_t f = 0; f < nf; ++f)
+		check_state(ws.hstate.p[f]);
+}
+
+// The caller's map checks as the kernel takes them (at most four).
+static MapChecks map_checks(const cusmic_map_check *maps, size_t n, int *blocks, const DeviceInfo &di)
+{
+	if (n > 4 || (n && !maps))
+		throw InvalidArgument("at most four maps are checked at once");
+	MapChecks c{};
+	size_t most = 1;
+	for (size_t i = 0; i < n; ++i) {
+		if (!maps[i].map || ((uintptr_t)maps[i].map & 7))
+			throw InvalidArgument("float64 buffers must be 8-byte aligned");
+		c.map[i].v = maps[i].map;
+		c.map[i].n = (long long)maps[i].n;
+		c.map[i].minimum = maps[i].minimum;
+		most = std::max(most, maps[i].n);
 	}
+	c.count = (int)n;
+	*blocks = (int)std::min<size_t>((most + 511) / 512, (size_t)di.sms * 8);
+	return c;
 }
 
 template <class F> static int guarded(F run, char *msg, size_t len)
@@ -1097,17 +1109,21 @@ template <class F> static int guarded(F run, char *msg, size_t len)
 
 static void run_device(const cusmic_image *ims, size_t nf, const cusmic_options &o,
 	const cusmic_frame_scalars *sc, double *clean, uint8_t *mask, cudaStream_t s,
-	std::vector<int> *passes = nullptr)
+	const cusmic_map_check *maps = nullptr, size_t nmaps = 0, unsigned *map_flags = nullptr)
 {
 	check_device_alignment(ims, nf, clean);
 	int dev;
 	check(cudaGetDevice(&dev));
 	DeviceInfo di = device_info(dev);
+	int check_blocks = 0;
+	const MapChecks checks = map_checks(maps, nmaps, &check_blocks, di);
 	Layout L = make_layout(ims, nf, o, sc, clean, mask, di);
 	Lease ws(dev);
 	upload(*ws, L, s);
 	enqueue_plain(*ws, L, di, s);
-	finish(*ws, nf, s, passes);
+	if (nmaps) // after the call's kernels, whose first one cleared the flags
+		check_maps_kernel<<<check_blocks, 256, 0, s>>>(checks, &ws->state.p[0].map_flags);
+	finish(*ws, nf, s, map_flags);
 }
 
 } // namespace cb
@@ -1217,6 +1233,44 @@ extern "C" int remove_cosmics_device(const cusmic_image *im, const cusmic_option
 	uint8_t *mask, void *stream, char *msg, size_t len)
 {
 	return remove_cosmics_batch_device(im, 1, o, clean, mask, stream, msg, len);
+}
+
+extern "C" int cusmic_checked_batch_device(const cusmic_image *ims, size_t nf,
+	const cusmic_options *o, double *clean, uint8_t *mask, const cusmic_map_check *maps, size_t nmaps,
+	unsigned *map_flags, void *stream, char *msg, size_t len)
+{
+	if (map_flags)
+		*map_flags = 0;
+	return guarded([&] {
+		check_arguments(ims, nf, o, nullptr, clean, mask, true);
+		run_device(ims, nf, *o, nullptr, clean, mask, (cudaStream_t)stream, maps, nmaps, map_flags);
+	}, msg, len);
+}
+
+extern "C" int cusmic_check_maps(const cusmic_map_check *maps, size_t nmaps, unsigned *map_flags,
+	void *stream, char *msg, size_t len)
+{
+	return guarded([&] {
+		if (!map_flags)
+			throw InvalidArgument("no place for the flags");
+		*map_flags = 0;
+		if (!nmaps)
+			return;
+		int dev, blocks = 0;
+		check(cudaGetDevice(&dev));
+		const DeviceInfo di = device_info(dev);
+		const MapChecks checks = map_checks(maps, nmaps, &blocks, di);
+		const cudaStream_t s = (cudaStream_t)stream;
+		Lease ws(dev);
+		ws->hflags.ensure(2);
+		ws->hflags_host.ensure(2);
+		check(cudaMemsetAsync(ws->hflags.p, 0, sizeof(unsigned), s));
+		check_maps_kernel<<<blocks, 256, 0, s>>>(checks, ws->hflags.p);
+		check(cudaMemcpyAsync(ws->hflags_host.p, ws->hflags.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+		check(cudaStreamSynchronize(s));
+		check(cudaGetLastError());
+		*map_flags = ws->hflags_host.p[0];
+	}, msg, len);
 }
 
 extern "C" int cusmic_ragged_batch_device(const cusmic_image *ims, size_t nf,

@@ -43,6 +43,32 @@ cusmic_ragged_batch_device(const struct cusmic_image *ims, size_t nf,
 	const struct cusmic_options *options, const struct cusmic_frame_scalars *scalars,
 	double *clean, uint8_t *mask, void *stream, char *msg, size_t message_size);
 
+/* A device float64 map whose contents are checked: every value finite, and
+ * positive (minimum 1), nonnegative (minimum 0) or either (minimum -1). */
+struct cusmic_map_check {
+	const double *map;
+	size_t n;
+	int minimum;
+};
+
+/* Check up to four maps on the current device; bit 2 i of *flags reports a
+ * value of map i that is not finite, bit 2 i + 1 one below its minimum.
+ * Synchronises.  No counterpart in the reference, whose host entry point checks
+ * its maps on the host (src/api.cu:107-114). */
+int
+cusmic_check_maps(const struct cusmic_map_check *maps, size_t nmaps, unsigned *flags, void *stream,
+	char *msg, size_t message_size);
+
+/* remove_cosmics_batch_device with the map checks in the same submission (one
+ * synchronisation for both): *flags as cusmic_check_maps; when it is nonzero
+ * the outputs and the status mean nothing.  *flags is zero when the arguments
+ * were rejected before anything ran. */
+int
+cusmic_checked_batch_device(const struct cusmic_image *ims, size_t nf,
+	const struct cusmic_options *options, double *clean, uint8_t *mask,
+	const struct cusmic_map_check *maps, size_t nmaps, unsigned *flags, void *stream, char *msg,
+	size_t message_size);
+
 /* Ragged batch of 1..65535 frames in HOST memory, results into host memory
  * (frame f's outputs at offset sum_{g<f} width_g * height_g of clean and
  * mask).  Frames are cleaned on the current device in chunks of whole frames;

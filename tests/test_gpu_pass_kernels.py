@@ -125,3 +125,44 @@ def test_contrast_ties(cuda, oracle, contrast, noise):
             odd = rng.random((h, w)) < 0.03
             frame["error"][odd] = rng.choice([0.0, 1e-200, np.inf, np.nan], int(odd.sum()))
     check_against_oracle(oracle, [frame], kw)
+
+
+@pytest.mark.parametrize("kw,message", [
+    (dict(error="zero"), "error must be positive"),
+    (dict(error="nan"), "error must be finite"),
+    (dict(error="nan", contrast=-1.0), "error must be finite"),
+    (dict(error="zero", mask="shape"), "error must be positive"),
+    (dict(error="zero", background="nan"), "error must be positive"),
+    (dict(error="ones", background="nan"), "background must be finite"),
+    (dict(effective_gain="zero", readnoise=-1.0), "effective_gain must be positive"),
+    (dict(effective_gain="nan"), "effective_gain must be finite"),
+    (dict(effective_gain="ones", readnoise="minus"), "readnoise must be nonnegative"),
+    (dict(effective_gain=2.0, readnoise=-1.0, background="nan"), "readnoise must be nonnegative"),
+    (dict(error="ones", contrast=-1.0), "contrast must be finite"),
+    (dict(error="ones", mask="shape"), "mask must match"),
+    (dict(effective_gain=2.0), "Provide error"),
+])
+@pytest.mark.parametrize("at", (0, 1, -1))
+def test_map_checks_with_the_call(cuda, kw, message, at):
+    """remove_cosmics checks its maps in the call that cleans them: the first
+    failing one is reported first, before other faults of the call, as Image
+    does; failing values at a map's ends, in a map of odd length."""
+    from cusmic_b200 import remove_cosmics
+    h, w = 7, 33
+    bad = {"zero": 0.0, "nan": np.nan, "minus": -1.0, "ones": 1.0}
+
+    def make(name, v):
+        if name == "mask":
+            return np.zeros((h, w + 1), bool)
+        if not isinstance(v, str):
+            return v
+        # One value past the buffer's start: 8 but not 16-byte aligned.
+        flat = cuda.ones(h * w + 1, dtype=cuda.float64, device="cuda")[1:]
+        flat[at] = bad[v]
+        return flat.view(h, w)
+    args = dict(contrast=3.0, cr_threshold=5.0, neighbor_threshold=3.0)
+    args.update({k: make(k, v) for k, v in kw.items()})
+    with pytest.raises(ValueError, match=message):
+        remove_cosmics(np.full((h, w), 10.0), **args)
+    clean, mask = remove_cosmics(np.full((h, w), 10.0), 3, 5, 3, error=make("error", "ones"))
+    assert mask.dtype == cuda.bool and not bool(mask.any()) and bool((clean == 10).all())
