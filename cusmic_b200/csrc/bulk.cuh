@@ -733,154 +733,131 @@ sig_bulk_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restri
 		}
 }
 
-// Candidates staged in shared memory by classify_kernel before one global
-// append per block and list.
-constexpr int CL_CAP = 1024;
+// Entries a warp of classify_kernel stages per list before it appends them.
+constexpr int CL_CAP = 128;
 
 struct ClassifyStage {
-	uint2 buf[CL_CAP];
-	int n;    // slots reserved
-	int fail; // first reservation that did not fit (entries from there went straight out)
+	uint2 buf[8][2][CL_CAP]; // per warp: high, low
+	int n[8][2];             // left at the end
+	unsigned long long at[2];
 };
 
-// Stage the lanes whose `pred` holds (entry e); a reservation that does not
-// fit appends those entries to the global list directly.
-__device__ __forceinline__ void classify_stage(ClassifyStage &S, bool pred, uint2 e,
-	unsigned long long *counter, uint2 *cands, bool from_back, unsigned long long cap)
-{
-	const int lane = threadIdx.x & 31;
-	const unsigned b = __ballot_sync(0xffffffffu, pred);
-	if (!b)
-		return;
-	const int k = __popc(b), rank = __popc(b & ((1u << lane) - 1u));
-	int old = 0;
-	if (lane == 0)
-		old = atomicAdd(&S.n, k);
-	old = __shfl_sync(0xffffffffu, old, 0);
-	if (old + k <= CL_CAP) {
-		if (pred)
-			S.buf[old + rank] = e;
-		return;
-	}
-	unsigned long long base = 0;
-	if (lane == 0) {
-		atomicMin(&S.fail, old);
-		base = atomicAdd(counter, (unsigned long long)k);
-	}
-	base = __shfl_sync(0xffffffffu, base, 0);
-	if (pred)
-		cands[from_back ? cap - 1 - (base + rank) : base + rank] = e;
-}
-
-// Write a stage out with one atomic per list (block-uniform call).
-__device__ __forceinline__ void classify_flush(ClassifyStage &H, ClassifyStage &L, Control *ctl,
-	uint2 *cands, unsigned long long *bases)
-{
-	__syncthreads();
-	const int nh = min(H.n, H.fail), nl = min(L.n, L.fail);
-	if (threadIdx.x == 0) {
-		bases[0] = nh ? atomicAdd(&ctl->pass[0].n_cand, (unsigned long long)nh) : 0ull;
-		bases[1] = nl ? atomicAdd(&ctl->pass[0].n_low, (unsigned long long)nl) : 0ull;
-	}
-	__syncthreads();
-	const unsigned long long cap = ctl->cand_cap;
-	for (int i = threadIdx.x; i < nh; i += blockDim.x)
-		cands[bases[0] + i] = H.buf[i];
-	for (int i = threadIdx.x; i < nl; i += blockDim.x)
-		cands[cap - 1 - (bases[1] + i)] = L.buf[i];
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		H.n = L.n = 0;
-		H.fail = L.fail = CL_CAP;
-	}
-	__syncthreads();
-}
-
 // sig_raw of the listed pixels, lap / (2 noise) (src/filters.cuh:125-135),
-// with the error map or the exact noise model at the pixel: one warp per
-// consumer-warp region of an item, one lane per entry.  The high list grows
-// from the front of the candidate buffer, the low list from its back; a NaN
-// goes to the high list (the candidate kernel decides).  Error-map entries
-// listed with a bound of +inf get their exact Laplacian first.
-__global__ void __launch_bounds__(256, 4)
+// with the error map or the exact noise model at the pixel: a warp per item,
+// whose four regions it reads as one list, a lane per entry, the next 32
+// entries loading meanwhile.  The high list grows from the front of the
+// candidate buffer, the low list from its back; a NaN goes to the high list
+// (the candidate kernel decides).  Error-map entries listed with a bound of
+// +inf get their exact Laplacian first.  A warp appends 128 entries at a time,
+// the block's warps together what is left.  (A warp per region, with 20 of 32
+// lanes busy and two block barriers for each eight regions, took 66 us on 16
+// frames of 2048 x 2048.)  MODEL: the batch has noise-model frames.
+template <bool MODEL>
+__global__ void __launch_bounds__(256, MODEL ? 3 : 6)
 classify_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
 	const int4 *__restrict__ items, int nitems, const PreCand *__restrict__ pre,
 	const int *__restrict__ pre_counts, DetectParams prm, Control *ctl, uint2 *cands)
 {
-	__shared__ ClassifyStage H, L;
-	__shared__ unsigned long long bases[2];
+	static_assert(BK_CWARPS == 4, "an item's counts are one int4");
+	__shared__ ClassifyStage S;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	// After a bounded wait of the dense kernel ran out, the counts of the
 	// items it left are stale: list nothing (the loop control then stops
 	// every frame and the call reports the fault).
 	if (*(const volatile int *)&ctl->fault)
 		return;
-	if (threadIdx.x == 0) {
-		H.n = L.n = 0;
-		H.fail = L.fail = CL_CAP;
+	const unsigned long long cap = ctl->cand_cap;
+	const unsigned below = (1u << lane) - 1u;
+	int nst[2] = {0, 0};
+	auto put = [&](int li, bool take, uint2 e) { // called by the whole warp
+		const unsigned b = __ballot_sync(0xffffffffu, take);
+		const int k = __popc(b);
+		if (nst[li] + k > CL_CAP) {
+			__syncwarp();
+			unsigned long long at = 0;
+			if (lane == 0)
+				at = atomicAdd(li ? &ctl->pass[0].n_low : &ctl->pass[0].n_cand, (unsigned long long)nst[li]);
+			at = __shfl_sync(0xffffffffu, at, 0);
+			for (int i = lane; i < nst[li]; i += 32)
+				cands[li ? cap - 1 - (at + i) : at + i] = S.buf[warp][li][i];
+			nst[li] = 0;
+			__syncwarp();
+		}
+		if (take)
+			S.buf[warp][li][nst[li] + __popc(b & below)] = e;
+		nst[li] += k;
+	};
+	const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+	for (int i = gw; i < nitems; i += nw) {
+		const int f = items[i].x;
+		if (!state[f].active)
+			continue; // warp-uniform
+		const FrameDesc &fd = frames[f];
+		const int4 c = reinterpret_cast<const int4 *>(pre_counts)[i];
+		const int c1 = c.x + c.y, c2 = c1 + c.z, n = c2 + c.w;
+		const PreCand *e = pre + (long long)i * BK_CWARPS * BK_REGION;
+		auto entry = [&](int j) { // of the item's four regions as one list
+			const int part = (j >= c.x) + (j >= c1) + (j >= c2);
+			const int start = part == 0 ? 0 : part == 1 ? c.x : part == 2 ? c1 : c2;
+			return j < n ? e[(long long)part * BK_REGION + j - start] : PreCand{0u, 0u, 0.0};
+		};
+		PreCand next = entry(lane);
+		for (int k0 = 0; k0 < n; k0 += 32) {
+			const PreCand pc = next;
+			if (k0 + 32 < n)
+				next = entry(k0 + 32 + lane);
+			int cls = 0;
+			if (k0 + lane < n) {
+				const unsigned pix = pc.pixel, px = pix % (unsigned)fd.w, py = pix / (unsigned)fd.w;
+				double lap = pc.lap, nz;
+				if (!MODEL || fd.error) {
+					nz = fd.error[pix];
+					// A bound of +inf marks a pixel whose Laplacian reads a hole
+					// (prep_detect_kernel) or overflowed: the exact Laplacian of
+					// the filled working pixels.
+					if (lap == INFINITY)
+						lap = lap_at(fd, (int)px, (int)py, lap_mode(prm.mode));
+				} else if (px >= 2 && py >= 2 && (int)px + 2 < fd.w && (int)py + 2 < fd.h) {
+					double win[25];
+					const double *src = fd.clean + pix - 2 * (long long)fd.w - 2;
+#pragma unroll
+					for (int a = 0; a < 5; ++a)
+#pragma unroll
+						for (int b = 0; b < 5; ++b)
+							win[a * 5 + b] = src[(long long)a * fd.w + b];
+					nz = noise_from_median(fd, pix, median_network(win));
+				} else {
+					nz = noise_model_at(fd, (int)px, (int)py, prm.mode);
+				}
+				const double v = lap / (2 * nz);
+				cls = v > prm.cr || v != v ? 1 : v > prm.nb ? 2 : 0;
+				if (cls) // the class planes that late passes keep up to date
+					atomicOr(plane_ptr(fd, cls == 1 ? P_HIGH : P_LOW) + (long long)py * fd.words + (px >> 5),
+						1u << (px & 31));
+			}
+			put(0, cls == 1, make_uint2((unsigned)f, pc.pixel));
+			put(1, cls == 2, make_uint2((unsigned)f, pc.pixel));
+		}
+	}
+	if (lane < 2)
+		S.n[warp][lane] = lane ? nst[1] : nst[0];
+	__syncthreads();
+	if (threadIdx.x < 2) {
+		int sum = 0;
+		for (int v = 0; v < 8; ++v)
+			sum += S.n[v][threadIdx.x];
+		S.at[threadIdx.x] = sum ? atomicAdd(threadIdx.x ? &ctl->pass[0].n_low : &ctl->pass[0].n_cand,
+			(unsigned long long)sum) : 0ull;
 	}
 	__syncthreads();
-	const unsigned long long cap = ctl->cand_cap;
-	const int nreg = nitems * BK_CWARPS;
-	for (int base = blockIdx.x * 8; base < nreg; base += gridDim.x * 8) { // block-uniform
-		const int rg = base + warp;
-		const int f = rg < nreg ? items[rg / BK_CWARPS].x : 0;
-		if (rg < nreg && state[f].active) { // warp-uniform
-			const int n = pre_counts[rg];
-			const FrameDesc &fd = frames[f];
-			const PreCand *e = pre + (long long)rg * BK_REGION;
-			for (int k0 = 0; k0 < n; k0 += 32) {
-				int cls = 0;
-				unsigned pix = 0;
-				if (k0 + lane < n) {
-					const PreCand pc = e[k0 + lane];
-					pix = pc.pixel;
-					if (fd.error) {
-						// A bound of +inf marks a pixel whose Laplacian reads a hole
-						// (prep_detect_kernel) or overflowed: the exact Laplacian of
-						// the filled working pixels.
-						const double lap = pc.lap != INFINITY ? pc.lap
-							: lap_at(fd, (int)(pix % (unsigned)fd.w), (int)(pix / (unsigned)fd.w),
-								lap_mode(prm.mode));
-						const double v = lap / (2 * fd.error[pix]);
-						cls = v > prm.cr || v != v ? 1 : v > prm.nb ? 2 : 0;
-					} else {
-						const int px = (int)(pix % (unsigned)fd.w), py = (int)(pix / (unsigned)fd.w);
-						double nz;
-						if (px >= 2 && py >= 2 && px + 2 < fd.w && py + 2 < fd.h) {
-							double win[25];
-							const double *src = fd.clean + pix - 2 * (long long)fd.w - 2;
 #pragma unroll
-							for (int a = 0; a < 5; ++a)
-#pragma unroll
-								for (int b = 0; b < 5; ++b)
-									win[a * 5 + b] = src[(long long)a * fd.w + b];
-							nz = noise_from_median(fd, pix, median_network(win));
-						} else {
-							nz = noise_model_at(fd, px, py, prm.mode);
-						}
-						const double v = pc.lap / (2 * nz);
-						cls = v > prm.cr || v != v ? 1 : v > prm.nb ? 2 : 0;
-					}
-					// The class planes that incremental passes keep up to date.
-					if (cls) {
-						const unsigned px = pix % (unsigned)fd.w, py = pix / (unsigned)fd.w;
-						atomicOr(plane_ptr(fd, cls == 1 ? P_HIGH : P_LOW) +
-							(long long)py * fd.words + (px >> 5), 1u << (px & 31));
-					}
-				}
-				const uint2 entry = make_uint2((unsigned)f, pix);
-				classify_stage(H, cls == 1, entry, &ctl->pass[0].n_cand, cands, false, cap);
-				classify_stage(L, cls == 2, entry, &ctl->pass[0].n_low, cands, true, cap);
-			}
-		}
-		__syncthreads();
-		const bool full = H.n >= CL_CAP / 2 || L.n >= CL_CAP / 2;
-		__syncthreads(); // every thread has read the counts before any stages again
-		if (full)
-			classify_flush(H, L, ctl, cands, bases);
+	for (int li = 0; li < 2; ++li) {
+		unsigned long long at = S.at[li];
+		for (int v = 0; v < warp; ++v)
+			at += S.n[v][li];
+		for (int i = lane; i < nst[li]; i += 32)
+			cands[li ? cap - 1 - (at + i) : at + i] = S.buf[warp][li][i];
 	}
-	classify_flush(H, L, ctl, cands, bases);
 }
 
 } // namespace cb

@@ -836,9 +836,9 @@ static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 			ws.bulk.p, nbulk, L.prm, ws.ctl.p, ws.pre.p, ws.pre_counts.p);
 		mark(rec, K_SIGRAW);
 	}
-	const int cgrid = (nbulk * BK_CWARPS + 7) / 8 < sparse ? (nbulk * BK_CWARPS + 7) / 8 : sparse;
-	classify_kernel<<<cgrid, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.bulk.p, nbulk, ws.pre.p,
-		ws.pre_counts.p, L.prm, ws.ctl.p, ws.cands.p);
+	auto classify = L.error_frames < nf ? classify_kernel<true> : classify_kernel<false>;
+	classify<<<std::min((nbulk + 7) / 8, sparse), 256, 0, s>>>(ws.frames.p, ws.state.p, ws.bulk.p, nbulk,
+		ws.pre.p, ws.pre_counts.p, L.prm, ws.ctl.p, ws.cands.p);
 	mark(rec, K_CLASSIFY);
 	// One launch per kind of frame in the batch: each variant compiles only
 	// its noise path (error map or noise model).  Error-map seeds are tested
