@@ -34,8 +34,8 @@
 // Borders: the chained filters read intermediates at border-mapped positions
 // (med7 reads med3 at border_index(x), med5 reads sig_raw there).  B and C
 // fold each window position with the median's border map before evaluating
-// the intermediate, except that a 3 x 3 median under mirror, reflect or wrap
-// is evaluated directly on border-extended clean pixels: those border maps
+// the intermediate, except that the medians of clean under mirror, reflect or
+// wrap are taken directly on border-extended clean pixels: those border maps
 // are invariant under a group of isometries that folds any coordinate onto
 // its image, so both give the same multiset.  The Laplacian itself reads its
 // neighbours with nearest semantics for mirror and reflect
@@ -440,16 +440,14 @@ __device__ __forceinline__ double warp_sort32(double v)
 // the second growth step, i.e. within distance 2 of a CAND pixel; candidates
 // with no CAND bit in their clipped 5 x 5 neighbourhood are skipped.
 //
-// A candidate at least 4 pixels from every edge stages the 9 x 9 patch of
-// clean around it in the warp's shared memory (every position it touches is
-// in the frame, so no border mapping is needed) and takes its Laplacians and,
-// on noise-model frames, its 25 noise windows from it; the others read
-// border-mapped values from global memory.  The patch stays for a seed test
-// of the same pixel.
-// The warp's evaluation of the candidate at (x, y): sig over its 5 x 5
-// window, the S2 bit (and S1 unless LOW) unless `skip`; `fresh`: the bit
-// planes were zeroed for this pass; returns sig (every lane) and the
-// noise at the pixel (nz_center).  P is the warp's 9 x 9 patch buffer.
+// A candidate whose patch serves (patch_serves: every one under mirror, reflect
+// and wrap, else those at least 4 pixels from every edge) stages the 9 x 9 patch
+// of border-extended clean pixels around it in the warp's shared memory and
+// takes, on noise-model frames, its 25 noise windows from it, and away from the
+// edges its Laplacians; the others read border-mapped values from global
+// memory.  The patch stays for a seed test of the same pixel.  (With every
+// candidate near an edge on the border-mapped path, 25 gathered medians per
+// lane, the late passes of 256 cutouts took 163 us, 130 with the patch.)
 // Which frames a kernel variant serves: any (decided per frame), error-map
 // frames only, or noise-model frames only (a variant compiles one path and
 // needs fewer registers).
@@ -543,17 +541,42 @@ __device__ __forceinline__ double exact_sig(const Sig &g)
 	return g.center - __shfl_sync(0xffffffffu, warp_sort32(v), 12);
 }
 
-// The 9 x 9 patch of clean around an interior pixel, three rows of a column
-// per lane (lane 9 g + c < 27: rows 3 g .. 3 g + 2 of column c).
-__device__ __forceinline__ void load_patch(const FrameDesc &fd, int x, int y, double (&p)[3])
+__device__ __forceinline__ bool interior4(const FrameDesc &fd, int x, int y)
+{
+	return x >= 4 && y >= 4 && x + 4 < fd.w && y + 4 < fd.h;
+}
+
+// Whether the 9 x 9 patch around (x, y), border-extended, holds the windows of
+// the pixel's medians: away from the edges, and under mirror, reflect and wrap
+// everywhere.  Those border maps are invariant under a group of isometries
+// that folds any coordinate onto its image, so the median at a folded position
+// and the one at the position itself on the extended pixels have the same
+// multiset.  (nearest and constant fold medians, not pixels.)
+__device__ __forceinline__ bool patch_serves(const FrameDesc &fd, int x, int y, int mode)
+{
+	return interior4(fd, x, y) || (mode != NEAREST && mode != CONSTANT);
+}
+
+// That patch, three rows of a column per lane (lane 9 g + c < 27: rows 3 g ..
+// 3 g + 2 of column c).
+__device__ __forceinline__ void load_patch(const FrameDesc &fd, int x, int y, int mode, double (&p)[3])
 {
 	const int lane = threadIdx.x & 31;
 	p[0] = p[1] = p[2] = 0;
 	if (lane < 27) {
-		const double *src = fd.clean + (long long)(y - 4 + 3 * (lane / 9)) * fd.w + (x - 4 + lane % 9);
-		p[0] = src[0];
-		p[1] = src[fd.w];
-		p[2] = src[2 * (long long)fd.w];
+		int cx = x - 4 + lane % 9, cy[3];
+#pragma unroll
+		for (int i = 0; i < 3; ++i)
+			cy[i] = y - 4 + 3 * (lane / 9) + i;
+		if (!interior4(fd, x, y)) { // warp-uniform
+			cx = border_index(cx, fd.w, mode);
+#pragma unroll
+			for (int i = 0; i < 3; ++i)
+				cy[i] = border_index(cy[i], fd.h, mode);
+		}
+#pragma unroll
+		for (int i = 0; i < 3; ++i)
+			p[i] = fd.clean[(long long)cy[i] * fd.w + cx];
 	}
 }
 
@@ -588,42 +611,45 @@ __device__ __forceinline__ Sig candidate_sig(const FrameDesc &fd, int x, int y, 
 	const int lane = threadIdx.x & 31;
 	const int w = fd.w, h = fd.h, mode = prm.mode, lm = lap_mode(mode);
 	const bool err = has_error_map<PATH>(fd);
+	const bool inside = interior4(fd, x, y), staged = patch_serves(fd, x, y, mode); // warp-uniform
 	Sig g;
 	double v = INFINITY, nz = 0;
-	if (x >= 4 && y >= 4 && x + 4 < w && y + 4 < h) { // warp-uniform
+	// The lane's window cell, folded into the frame (negative: a zero).
+	int mx = x + lane % 5 - 2, my = y + lane / 5 - 2;
+	if (!inside) {
+		mx = border_index(mx, w, mode);
+		my = border_index(my, h, mode);
+	}
+	const bool cell = lane < 25, real = cell && (mx | my) >= 0;
+	const long long at = (long long)my * w + mx;
+	if (staged) {
 		double p[3];
-		load_patch(fd, x, y, p);
-		if (lane < 25 && err) // loads with the patch
-			nz = fd.error[(long long)(y + lane / 5 - 2) * w + x + lane % 5 - 2];
+		load_patch(fd, x, y, mode, p);
+		if (cell && err) // loads with the patch
+			nz = fd.error[at];
 		store_patch(P, p);
-		const int dy = lane / 5, dx = lane % 5;
 		if (!err) { // warp-uniform
 			const double m = patch_window_median(P, S);
-			if (lane < 25)
-				nz = noise_from_median(fd, (long long)(y + dy - 2) * w + x + dx - 2, m);
+			if (cell)
+				nz = noise_from_median(fd, at, m);
 		}
-		if (lane < 25) {
-			const double *q = P + (dy + 2) * 9 + dx + 2; // the window cell
-			v = lap_formula(q[0], q[-9], q[9], q[-1], q[1]) / (2 * nz);
+	} else if (real) {
+		nz = err ? fd.error[at] : noise_model_at(fd, mx, my, mode);
+	}
+	if (cell) {
+		double lap = 0;
+		if (inside) {
+			const double *q = P + (lane / 5 + 2) * 9 + lane % 5 + 2; // the window cell
+			lap = lap_formula(q[0], q[-9], q[9], q[-1], q[1]);
+		} else if (real) {
+			lap = lap_at(fd, mx, my, lm);
 		}
-	} else if (lane < 25) {
-		const int mx = border_index(x + lane % 5 - 2, w, mode);
-		const int my = border_index(y + lane / 5 - 2, h, mode);
-		v = 0;
-		if (mx >= 0 && my >= 0) {
-			const long long i = (long long)my * w + mx;
-			nz = err ? fd.error[i] : noise_model_at(fd, mx, my, mode);
-			const double lap = lap_formula(fd.clean[i], clean_at(fd, mx, my - 1, lm),
-				clean_at(fd, mx, my + 1, lm), clean_at(fd, mx - 1, my, lm),
-				clean_at(fd, mx + 1, my, lm));
-			v = lap / (2 * nz);
-		}
+		v = real ? lap / (2 * nz) : 0.0;
 	}
 	const double center = __shfl_sync(0xffffffffu, v, 12);
 	g.center = center;
 	g.v = v;
 	g.noise = __shfl_sync(0xffffffffu, nz, 12);
-	const bool cell = lane < 25;
 	if (__any_sync(0xffffffffu, cell && !(v >= 0))) { // a NaN, or a negative noise
 		double med;
 		if (__any_sync(0xffffffffu, isnan(v))) {
@@ -1066,7 +1092,7 @@ __device__ __forceinline__ WindowCounts count_windows(const double (&p)[3], doub
 // fine = max((med3 - med7) / noise, 0.01) with med7 the median of the 49 3 x 3
 // medians around it, and CAND = sig / fine > contrast.
 //
-// A seed at least 4 pixels from every edge is decided without any 3 x 3 median
+// A seed whose patch serves (patch_serves) is decided without any 3 x 3 median
 // but its own: the test holds at med7 exactly when it holds with 25 or more of
 // the 49 medians in med7's place (it can only turn true as that value grows),
 // a median m satisfies it when med3 - m < sig noise / contrast (and sig / 0.01
@@ -1076,7 +1102,7 @@ __device__ __forceinline__ WindowCounts count_windows(const double (&p)[3], doub
 // both with a margin of 1e-12 for the roundings (of two products here, of a
 // difference and two divisions in the test).  sig need not be exact for that:
 // sig_lo and sig_hi bound it.  What these counts leave open, values outside
-// the range where the margin covers the roundings, and seeds near an edge take
+// the range where the margin covers the roundings, and the other seeds take
 // the medians and the exact sig (from exact(), called by the whole warp).
 //
 // (Sorting the 25 window values, 63 column triples and 49 medians across the
@@ -1092,9 +1118,9 @@ __device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, dou
 {
 	const int lane = threadIdx.x & 31;
 	const int w = fd.w, h = fd.h, mode = prm.mode;
-	const bool interior = x >= 4 && y >= 4 && x + 4 < w && y + 4 < h; // warp-uniform
+	const bool patch = patch_serves(fd, x, y, mode); // warp-uniform
 	int verdict = -1; // undecided
-	if (interior) {
+	if (patch) {
 		double p[3];
 		if (staged) { // the candidate evaluation left this patch in P
 			const double *q = P + (lane < 27 ? 27 * (lane / 9) + lane % 9 : 0);
@@ -1102,7 +1128,7 @@ __device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, dou
 			p[1] = q[9];
 			p[2] = q[18];
 		} else {
-			load_patch(fd, x, y, p);
+			load_patch(fd, x, y, mode, p);
 			store_patch(P, p);
 		}
 		const double k = prm.contrast, floor_k = k * FINE_FLOOR;
@@ -1131,7 +1157,7 @@ __device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, dou
 	if (verdict < 0) { // warp-uniform
 		const double sig = exact();
 		double m3[2] = {INFINITY, INFINITY};
-		if (interior) {
+		if (patch) {
 			__syncwarp();
 			for (int k = lane; k < 63; k += 32) {
 				double a = P[k], b = P[k + 9], c = P[k + 18];
@@ -1161,10 +1187,8 @@ __device__ __forceinline__ void seed_eval(const FrameDesc &fd, int x, int y, dou
 					int qx = x + j % 7 - 3, qy = y + j / 7 - 3;
 					double m = 0;
 					if (!(mode == CONSTANT && (qx < 0 || qx >= w || qy < 0 || qy >= h))) {
-						if (mode == NEAREST) {
-							qx = clampi(qx, 0, w - 1);
-							qy = clampi(qy, 0, h - 1);
-						}
+						qx = clampi(qx, 0, w - 1); // nearest folds the medians
+						qy = clampi(qy, 0, h - 1);
 						int mx[3], my[3];
 #pragma unroll
 						for (int i = 0; i < 3; ++i) {
