@@ -12,7 +12,7 @@ import threading
 
 import torch
 
-from .api import Cleaner, Image
+from .api import Cleaner, _calibration, _checked_data, _checked_mask
 from .plan import Batch, Plan
 
 # Idle plans per batch signature (device, shapes, which maps are present and
@@ -69,27 +69,28 @@ def _plan_for(batch, options):
 
 class _Clean(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, data, background, image, cleaner):
+    def forward(ctx, data, background, fields, mask, cleaner):
         stack = data if data.dim() == 3 else data.unsqueeze(0)
         stack = stack.detach().contiguous()
         nf = stack.shape[0]
-        bg = image.background
-        scalar_bg = bg is not None and bg.dim() == 0
-        batch = Batch.stack(stack, error=image.error,
-                            mask=None if image.mask is None
-                            else image.mask.contiguous().view(torch.uint8),
-                            gain=image.effective_gain if _is_map(image.effective_gain) else None,
-                            readnoise=image.readnoise if _is_map(image.readnoise) else None,
-                            background=bg if _is_map(bg) else None)
-        gain = float(image.effective_gain) if _is_scalar(image.effective_gain) else math.nan
-        rn = float(image.readnoise) if _is_scalar(image.readnoise) else 0.0
+
+        def field(name, scalar, default):
+            """The named calibration if it is a number (scalar) or a map."""
+            value = fields.get(name)
+            return value if value is not None and isinstance(value, float) == scalar else default
+
+        gain_map, rn_map, bg_map = (field(name, False, None) for name in
+                                    ("effective_gain", "readnoise", "background"))
+        batch = Batch.stack(stack, error=fields.get("error"),
+                            mask=None if mask is None else mask.contiguous().view(torch.uint8),
+                            gain=gain_map, readnoise=rn_map, background=bg_map)
         options = dict(contrast=float(cleaner.contrast),
                        cr_threshold=float(cleaner.cr_threshold),
                        neighbor_threshold=float(cleaner.neighbor_threshold),
                        maxiter=int(cleaner.maxiter), border=cleaner.border_mode,
-                       gain=gain if image.error is None else math.nan,
-                       readnoise=rn if image.error is None else 0.0,
-                       background=float(bg) if scalar_bg else math.nan)
+                       gain=field("effective_gain", True, math.nan),
+                       readnoise=field("readnoise", True, 0.0),
+                       background=field("background", True, math.nan))
         lease = _plan_for(batch, options)
         plan = lease.plan
         plan.execute()
@@ -97,17 +98,18 @@ class _Clean(torch.autograd.Function):
         ctx.lease = lease
         ctx.plan = plan
         ctx.shape = data.shape
-        ctx.bg_shape = None if bg is None else tuple(bg.shape)
+        ctx.bg_shape = None if "background" not in fields else \
+            () if bg_map is None else tuple(bg_map.shape)
         ctx.nf = nf
         # The batch's own output buffers, made for this call: the backward
         # reads neither (detached, so that the outputs' graph, which holds the
         # batch, is not held by it).
         clean = batch.clean.detach()
-        mask = batch.mask_out.view(torch.bool)
+        flags = batch.mask_out.view(torch.bool)
         if data.dim() == 2:
-            clean, mask = clean[0], mask[0]
-        ctx.mark_non_differentiable(mask)
-        return clean, mask
+            clean, flags = clean[0], flags[0]
+        ctx.mark_non_differentiable(flags)
+        return clean, flags
 
     @staticmethod
     def backward(ctx, grad_clean, grad_mask):
@@ -121,15 +123,7 @@ class _Clean(torch.autograd.Function):
             else:
                 per_frame = gbg.reshape(ctx.nf, *ctx.shape[-2:])
                 g_background = per_frame.sum(0) if len(ctx.bg_shape) == 2 else per_frame
-        return gx, g_background, None, None
-
-
-def _is_map(v):
-    return v is not None and isinstance(v, torch.Tensor) and v.dim() > 0
-
-
-def _is_scalar(v):
-    return v is not None and (not isinstance(v, torch.Tensor) or v.dim() == 0)
+        return gx, g_background, None, None, None
 
 
 def remove_cosmics_differentiable(data, contrast=3, cr_threshold=5, neighbor_threshold=3,
@@ -138,8 +132,12 @@ def remove_cosmics_differentiable(data, contrast=3, cr_threshold=5, neighbor_thr
     """``remove_cosmics`` whose cleaned output is differentiable in ``data``
     and ``background`` (a tensor scalar or map), with the mask frozen."""
     bg_t = background if isinstance(background, torch.Tensor) else None
-    image = Image(data.detach(), error, mask,
-                  background.detach() if bg_t is not None else background,
-                  effective_gain, readnoise)
+    checked, device = _checked_data(data.detach())
+    with torch.cuda.device(device):
+        fields, checks = _calibration(checked, device, error,
+                                      background.detach() if bg_t is not None else background,
+                                      effective_gain, readnoise)
+        checks.run()
+        mask = _checked_mask(mask, checked, device)
     cleaner = Cleaner(contrast, cr_threshold, neighbor_threshold, maxiter, border_mode)
-    return _Clean.apply(data, bg_t, image, cleaner)
+    return _Clean.apply(data, bg_t, fields, mask, cleaner)
