@@ -64,37 +64,6 @@ namespace cb {
 constexpr int LATE_THREADS = 1024;
 constexpr int LATE_WARPS = LATE_THREADS / 32;
 
-static_assert(FLOOR_BLOCK == 32, "a bit word of a row lies in one floor block");
-
-// model_threshold of block (bx, by) of a noise-model frame; outside wrap mode
-// only the 3 x 3 neighbouring blocks count, read directly.
-__device__ __forceinline__ double block_threshold(const FrameDesc &fd, int bx, int by, int mode,
-	double tmin2)
-{
-	if (mode == WRAP)
-		return model_threshold(fd, bx, by, mode, tmin2);
-	const BlockFloor *bf = fd.floors;
-	const int bw = (fd.w + FLOOR_BLOCK - 1) / FLOOR_BLOCK, bh = (fd.h + FLOOR_BLOCK - 1) / FLOOR_BLOCK;
-	unsigned long long key = ~0ull;
-#pragma unroll
-	for (int i = -1; i <= 1; ++i)
-#pragma unroll
-		for (int j = -1; j <= 1; ++j) {
-			const int yy = by + i, xx = bx + j;
-			if (yy >= 0 && yy < bh && xx >= 0 && xx < bw)
-				key = min(key, bf[yy * bw + xx].key);
-		}
-	if (mode == CONSTANT && (bx == 0 || by == 0 || (bx + 1) * FLOOR_BLOCK + 2 > fd.w ||
-		(by + 1) * FLOOR_BLOCK + 2 > fd.h))
-		key = min(key, order_key(0.0));
-	double m = order_value(key);
-	m = m < SIGNAL_FLOOR ? SIGNAL_FLOOR : m;
-	const BlockFloor &own = bf[by * bw + bx];
-	const double g = fd.gain_map ? -order_value(own.gkey) : fd.gain;
-	const double rn = fd.rn_map ? order_value(own.rkey) : fd.rn;
-	return tmin2 * (sqrt(rn * rn + g * m) / g);
-}
-
 __device__ __forceinline__ int wrap_index(int i, int n)
 {
 	i %= n;
