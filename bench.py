@@ -60,10 +60,10 @@ METRIC = "Mpix/s (f64, maxiter=4, identical masks) batched vs plain; bwd/fwd tim
 SETTINGS = dict(contrast=3.0, cr_threshold=5.0, neighbor_threshold=3.0, maxiter=4)
 # ncu, sig_bulk_kernel, 4-frame stack launch: 144.6 MB over 16.78 Mpix.
 SIG_BULK_DRAM_BYTES_PER_PX = 8.62
-# ncu, prepare_bulk_kernel, one 16-frame stack launch (this workload):
-# 565.2 MB read + 514.2 MB written over 67.1 Mpix (written pixels still in
-# L2 at the end of the launch are not counted).
-PREPARE_DRAM_BYTES_PER_PX = 16.08
+# ncu, prepare_kernel, one launch over 8 frames of 2047 x 2048 pixels of this
+# workload's kind: 306.3 MB read + 246.4 MB written over 33.5 Mpix (written
+# pixels still in L2 at the end of the launch are not counted).
+PREPARE_DRAM_BYTES_PER_PX = 16.48
 # ncu, prep_detect_kernel (prepare with the dense detection), one 16-frame
 # stack launch (this workload): 601.2 MB read + 525.2 MB written over
 # 67.1 Mpix.
@@ -356,7 +356,7 @@ def main():
     # prep_detect_kernel, which also runs the first pass's dense detection on
     # the input rows (no separate dense-detection launch, no re-read of the
     # clean pixels; its pre-list writes, 16 B per listed pixel, about 1% of
-    # the pixels, are not counted); other batches the bulk-staged prepare.
+    # the pixels, are not counted); other batches prepare_kernel.
     fused = klaunch["sigraw"] == 0
     prep_px = nf * h * w * klaunch["prepare"]
     prep_bytes = prep_px * (8 + 1 + 8 + 3 / 8)
@@ -364,7 +364,7 @@ def main():
     prep_achieved = prep_bytes / (prep_ms / 1e3) / 1e9
     prep_launch_px = prep_px / max(1, klaunch["prepare"])
     dram_px = PREP_DETECT_DRAM_BYTES_PER_PX if fused else PREPARE_DRAM_BYTES_PER_PX
-    roofline = {"bound": "hbm", "kernel": "prep_detect_kernel" if fused else "prepare_bulk_kernel",
+    roofline = {"bound": "hbm", "kernel": "prep_detect_kernel" if fused else "prepare_kernel",
                 "achieved": round(prep_achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(prep_achieved / peak, 4),
                 "traffic": round(prep_launch_px * dram_px) if dram_px else None,

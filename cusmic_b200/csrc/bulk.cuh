@@ -740,13 +740,17 @@ sig_bulk_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restri
 		asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 	}
 	__syncthreads();
+	// An injected failure of either step (prepare or detection; prepare_kernel
+	// has no wait of its own).
+	const long long poison = ctl->poison_wait[0] > ctl->poison_wait[1] ? ctl->poison_wait[0]
+		: ctl->poison_wait[1];
 	bool ok;
 	int issued = 0; // ring rows issued (producer warp)
 	if (warp == BK_CWARPS)
 		ok = lane || bulk_producer(R, frames, state, items, nitems, lap_mode(prm.mode), ctl, issued,
 			base);
-	else if (warp == 0 && blockIdx.x == 0 && ctl->poison_wait[1] > 0)
-		ok = __all_sync(0xffffffffu, poisoned_wait(&R.poison, &R.abort, ctl->poison_wait[1]));
+	else if (warp == 0 && blockIdx.x == 0 && poison > 0)
+		ok = __all_sync(0xffffffffu, poisoned_wait(&R.poison, &R.abort, poison));
 	else
 		ok = bulk_consumer(R, frames, items, prm, pre, pre_counts);
 	if (!ok && lane == 0) {

@@ -161,8 +161,8 @@ struct Control {
 	unsigned barrier;             // arrivals at the late passes' grid barriers
 	unsigned pad;
 	// Injected failures (0: none): the bound, in SM cycles, of one extra wait
-	// on a barrier that nothing completes, made by one warp of the first block
-	// of the bulk-staged prepare ([0]) and of the dense detection kernel ([1]).
+	// on a barrier that nothing completes, for prepare ([0]) and for the dense
+	// detection ([1]); one warp of the dense detection's first block makes it.
 	long long poison_wait[2];
 };
 

@@ -14,7 +14,6 @@
 #include "detect.cuh"
 #include "bulk.cuh"
 #include "kernels.cuh"
-#include "prepare_bulk.cuh"
 #include "prep_detect.cuh"
 #include "late.cuh"
 #include "backward.cuh"
@@ -383,10 +382,10 @@ struct Layout {
 	int maxiter = 0;
 	int error_frames = 0; // frames with an error map (a rebound plan keeps which)
 	bool map_floors = false; // some frame's floors are read from its maps
-	// Kernel choices that depend on the buffers' alignment (a rebound plan
-	// whose choices change is captured again): the bulk-staged prepare, and
-	// prepare with the dense detection in one kernel (prep_detect_kernel).
-	bool prep_bulk = false, fused = false;
+	// Prepare with the dense detection in one kernel (prep_detect_kernel): it
+	// depends on the buffers' alignment (a rebound plan whose choice changes
+	// is captured again).
+	bool fused = false;
 	cusmic_tuning tune{};
 	long long poison_wait[2] = {0, 0}; // injected failures in force when the batch was laid out
 };
@@ -405,11 +404,6 @@ static DeviceInfo device_info(int dev)
 	DeviceInfo &d = cache[dev];
 	if (!d.sms) { // first use on this (the current) device
 		check(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
-		for (const void *k : {(const void *)prepare_bulk_kernel<false, false>,
-			     (const void *)prepare_bulk_kernel<true, false>,
-			     (const void *)prepare_bulk_kernel<false, true>,
-			     (const void *)prepare_bulk_kernel<true, true>})
-			check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
 		check(cudaFuncSetAttribute((const void *)late_passes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			(int)sizeof(LateShared)));
 	}
@@ -581,15 +575,12 @@ static int item_rows(const cusmic_image *ims, size_t nf, int target_items)
 	return rows;
 }
 
-// The prepare kernels that suit every frame of a batch (see Layout).
+// Whether prep_detect_kernel suits every frame of a batch (see Layout).
 static void choose_kernels(Layout &L)
 {
-	L.prep_bulk = true;
 	L.fused = L.maxiter > 0;
-	for (const FrameDesc &fd : L.frames) {
-		L.prep_bulk = L.prep_bulk && prep_bulk_ok(fd);
+	for (const FrameDesc &fd : L.frames)
 		L.fused = L.fused && prep_detect_ok(fd);
-	}
 }
 
 static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_options &o,
@@ -908,37 +899,41 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	mark(rec, K_RECLASS);
 }
 
-// prepare: the bulk-staged kernel when every frame suits it; else one
-// compiled for noise-model frames without maps, with twice the unroll, when
-// every frame is of that kind; otherwise the kernel that decides per row
-// (faster for error-map frames than any specialisation that was timed).
+// prepare: a variant of prepare_kernel by what the batch has and how wide its
+// rows are.  Reads wait for DRAM behind the kernel's own writes, so a warp's
+// bytes in flight decide, up to the row's length: noise-model frames without
+// maps take 16 words of a row at once from 1024 pixels a row (64 ragged frames
+// of 256 to 4096 pixels a side: 705 us, 8 words 759, 4 words 752; eight frames
+// of 1024 x 1024: 33, 32 and 38 us), 4 below 256 (256 frames of 40 to 200: 29,
+// 22 and 18 us), else 8.  Frames with maps or a mask take 8 words in the kernel
+// that decides per row, with two blocks per SM if some frame has a background
+// map or the noise model with a mask (a value or mask byte more per pixel in
+// registers: 36 us for 5 x 1018 x 1001 frames against 41 with three blocks, 43
+// with 4 words and four), else three (16 x 2048 x 2047 error-map frames with
+// masks: 223 us, two blocks 267, 4 words 242).  Variants for one such kind each
+// were no faster.  Blocks come in several waves, which evens out rows of unequal
+// lengths (ragged frames, 16 words: 763 us with four blocks per SM in all, 713
+// with 8, 688 with 16).
 static void launch_prepare(Workspace &ws, const Layout &L, const DeviceInfo &di, cudaStream_t s)
 {
-	bool model = true, rowmin = false, out = false;
-	const bool bulk = L.prep_bulk;
+	bool model = true, maps = false, out = false;
 	for (const FrameDesc &fd : L.frames) {
 		const int kind = prep_kind(fd);
 		model = model && kind == PREP_MODEL;
-		rowmin = rowmin || kind == PREP_MODEL || kind == PREP_MODEL_MAPS;
+		maps = maps || kind == PREP_MAPS || kind == PREP_MODEL_MAPS;
 		out = out || (fd.out && fd.out != fd.clean);
 	}
-	const int nrows = (int)L.rows.size();
-	// Each variant is compiled for what the batch has (row minima, separate
-	// outputs): the kernels are issue-bound, and an unused branch costs.
-	if (bulk) {
-		const int need = (nrows + PB_WARPS - 1) / PB_WARPS, cap = di.sms * PB_BLOCKS;
-		const int grid = need < cap ? need : cap;
-		auto k = rowmin ? (out ? prepare_bulk_kernel<true, true> : prepare_bulk_kernel<true, false>)
-				: (out ? prepare_bulk_kernel<false, true> : prepare_bulk_kernel<false, false>);
-		k<<<grid, 32 * PB_WARPS, PB_SMEM, s>>>(ws.frames.p, ws.state.p, ws.rows.p, nrows, ws.ctl.p,
-			ws.cands.p);
-		return;
-	}
-	const int grid = grid_for_rows(di, nrows, L.tune.row_blocks_per_sm);
-	auto k = model ? (out ? prepare_kernel<PREP_MODEL, 2 * ROW_UNROLL, true>
-			       : prepare_kernel<PREP_MODEL, 2 * ROW_UNROLL, false>)
-		       : (out ? prepare_kernel<PREP_ANY, ROW_UNROLL, true> : prepare_kernel<PREP_ANY, ROW_UNROLL, false>);
-	k<<<grid, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.rows.p, nrows, ws.ctl.p, ws.cands.p);
+	const size_t nrows = L.rows.size(), width = L.total_px / nrows; // of a mean row
+	const int grid = grid_for_rows(di, nrows, 2 * L.tune.row_blocks_per_sm);
+	auto pick = [&](auto with_out) {
+		constexpr bool O = decltype(with_out)::value;
+		if (model)
+			return width >= 1024 ? prepare_kernel<PREP_MODEL, 16, O, 2>
+				: width < 256 ? prepare_kernel<PREP_MODEL, 4, O, 4> : prepare_kernel<PREP_MODEL, 8, O, 3>;
+		return maps ? prepare_kernel<PREP_ANY, 8, O, 2> : prepare_kernel<PREP_ANY, 8, O, 3>;
+	};
+	auto k = out ? pick(std::true_type{}) : pick(std::false_type{});
+	k<<<grid, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.rows.p, (int)nrows, ws.ctl.p, ws.cands.p);
 }
 
 static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di, cudaStream_t s,
@@ -1816,10 +1811,9 @@ extern "C" int cusmic_plan_bind(cusmic_plan *p, const cusmic_image *ims, double 
 		}
 		p->ims.assign(ims, ims + nf);
 		p->L.frames = L.frames;
-		// New buffers can change which prepare kernels suit the batch: the
-		// graph is captured again with the new choice.
-		const bool recapture = L.prep_bulk != p->L.prep_bulk || L.fused != p->L.fused;
-		p->L.prep_bulk = L.prep_bulk;
+		// New buffers can change whether prep_detect_kernel suits the batch:
+		// the graph is captured again with the new choice.
+		const bool recapture = L.fused != p->L.fused;
 		p->L.fused = L.fused;
 		const size_t bytes = nf * sizeof(FrameDesc);
 		std::memcpy(p->ws.stage.p, p->L.frames.data(), bytes);
@@ -2177,7 +2171,7 @@ extern "C" int remove_cosmics_device_noalloc(const cusmic_image *im, const cusmi
 			// Bit planes start at zero (prepare_kernel writes HOLE, EXCL and
 			// DONOR); the scratch keeps the previous call's contents.
 			check(cudaMemsetAsync(fd.bits, 0, (size_t)N_PLANES * L.plane * sizeof(uint32_t), s));
-			prepare_kernel<PREP_ANY><<<row_blocks, 256, 0, s>>>(frames, state, rows, h);
+			prepare_kernel<PREP_ANY, 8, false, 3><<<row_blocks, 256, 0, s>>>(frames, state, rows, h);
 			fill_kernel<<<row_blocks, 256, 0, s>>>(frames, state, rows, h);
 			for (int it = 0; it < o->maxiter; ++it) {
 				const int par = it & 1;

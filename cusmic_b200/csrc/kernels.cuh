@@ -206,13 +206,11 @@ __device__ __forceinline__ double order_value(unsigned long long k)
 // Reference src/image.cuh:24-48: holes, exclusions, clean = data (+ bg), the
 // static donor plane (the reference's is_donor with an empty mask) and the
 // per-frame facts the initial fill needs (src/cleaner.cuh:78-100).  A warp
-// loads ROW_UNROLL chunks of 32 pixels before using them, so enough bytes are
-// in flight per SM to approach the HBM bandwidth.
-constexpr int ROW_UNROLL = 4;
+// loads several chunks of 32 pixels before using them, so enough bytes are in
+// flight per SM to approach the HBM bandwidth (launch_prepare).
 
 // Frame kinds of prepare_row: the input maps it reads and whether it writes
-// noise-model row minima.  A batch whose frames are all of one kind gets a
-// prepare_kernel compiled for that kind (PREP_ANY decides per row).
+// noise-model row minima (PREP_ANY decides per row).
 enum PrepKind { PREP_ANY, PREP_PLAIN, PREP_MASK, PREP_MAPS, PREP_MODEL, PREP_MODEL_MAPS };
 
 CB_HD int prep_kind(const FrameDesc &fd)
@@ -228,9 +226,16 @@ CB_HD int prep_kind(const FrameDesc &fd)
 // mask, BGMAP = background map.  Descriptor fields are held in registers (the
 // stores below go through pointers the compiler cannot prove distinct from
 // them).
-template <bool MASK, bool BGMAP, bool ROWMIN, int U = ROW_UNROLL, bool OUT = false>
-__device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st, int f, int y,
-	Control *ctl, uint2 *holes)
+//
+// W words of the row at once, the rest in groups of 4.  Memory bounds it (64
+// ragged noise-model frames of 256 to 4096 pixels a side, 178 Mpix of 24 bytes:
+// 858 us with 8 words in flight and a tail group of 8, 705 us).  On small frames
+// it was bound by its last lines, where lane 0 tested each frame flag before
+// setting it, three waits in a row (256 frames of 40 to 200 pixels: 68 us, 27
+// with stores alone, 18 with the groups as they are now).
+template <bool MASK, bool BGMAP, bool ROWMIN, int W, bool OUT>
+__device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st, int f, int y, Control *ctl,
+	uint2 *holes)
 {
 	const int lane = threadIdx.x & 31;
 	const int w = fd.w, words = fd.words;
@@ -242,33 +247,34 @@ __device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st,
 	double *__restrict__ clean = fd.clean + rowpix;
 	// A separate output buffer (a frame with a background): its pixels now,
 	// (x + bg) - bg as the reference's restore computes them, the input at a
-	// hole; restore writes only the flagged ones.
+	// hole; finish_kernel writes only the flagged ones.
 	double *__restrict__ out = OUT && fd.out && fd.out != fd.clean ? fd.out + rowpix : nullptr;
 	const double bgv = fd.bg;
 	const bool has_bg = fd.has_bg;
 	uint32_t *hole_plane = plane_ptr(fd, P_HOLE) + roww, *excl_plane = plane_ptr(fd, P_EXCL) + roww;
 	uint32_t *donor_plane = plane_ptr(fd, P_DONOR) + roww;
-	uint32_t any_hole = 0, any_allowed = 0, any_finite = 0;
-	int ndonor = 0;
 	// Noise-model frames with floors: per bit word the smallest high word of
 	// the ordered keys of the non-hole clean values (a lower bound for the
 	// block floors, which the hole fill then lowers with the values it writes).
 	uint32_t *rowmin = ROWMIN ? plane_ptr(fd, P_ROWMIN) + roww : nullptr;
-	for (int seg = 0; seg * 1024 < w; ++seg) {
+	uint32_t any_hole = 0, any_allowed = 0; // of this lane's words
+	int ndonor = 0;
+	for (int seg = 0; seg < words; seg += 32) {
 		uint32_t my_h = 0, my_e = 0, my_d = 0, my_m = 0xffffffffu;
-		for (int c0 = 0; c0 < 32; c0 += U) {
-			const int xb = seg * 1024 + c0 * 32;
-			if (xb >= w)
-				break; // warp-uniform
+		// Words k = seg + c and on, `count` of them; FULL: all inside the row.
+		auto group = [&](int c, auto count, auto full) {
+			constexpr int U = decltype(count)::value;
+			constexpr bool FULL = decltype(full)::value;
+			const int xl = 32 * (seg + c) + lane;
 			double d[U], bg[U];
 			bool m[U];
 #pragma unroll
 			for (int u = 0; u < U; ++u) {
-				const int x = xb + 32 * u + lane;
+				const int x = xl + 32 * u;
 				d[u] = 0;
 				bg[u] = bgv;
 				m[u] = false;
-				if (x < w) {
+				if (FULL || x < w) {
 					d[u] = data[x];
 					if (MASK && mask)
 						m[u] = mask[x] != 0;
@@ -276,50 +282,75 @@ __device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st,
 						bg[u] = bgmap[x];
 				}
 			}
+			// Without a mask most groups are all donors, which one ballot
+			// shows: the value is finite only where the pixel is.
+			if (FULL && !MASK) {
+				bool good = true;
+#pragma unroll
+				for (int u = 0; u < U; ++u)
+					good = good && isfinite(has_bg ? d[u] + 1 * bg[u] : d[u]);
+				if (__all_sync(0xffffffffu, good)) {
+#pragma unroll
+					for (int u = 0; u < U; ++u) {
+						const double v = has_bg ? d[u] + 1 * bg[u] : d[u];
+						clean[xl + 32 * u] = v;
+						if (OUT && out)
+							out[xl + 32 * u] = v + -1 * bg[u];
+						const uint32_t mw = ROWMIN
+							? __reduce_min_sync(0xffffffffu, (uint32_t)(order_key(v) >> 32)) : 0u;
+						if (lane == c + u) {
+							my_d = 0xffffffffu;
+							my_m = mw;
+						}
+					}
+					return;
+				}
+			}
 #pragma unroll
 			for (int u = 0; u < U; ++u) {
-				const int x0 = xb + 32 * u;
-				const int x = x0 + lane;
-				const bool valid = x < w;
-				bool hole = false, ok = false, donor = false;
-				double c = 0;
+				const int x = xl + 32 * u;
+				const bool valid = FULL || x < w, hole = valid && !isfinite(d[u]);
+				double v = hole ? 0 : d[u];
+				if (has_bg)
+					v += 1 * bg[u];
 				if (valid) {
-					hole = !isfinite(d[u]);
-					ok = !hole && !m[u];
-					c = hole ? 0 : d[u];
-					if (has_bg)
-						c += 1 * bg[u];
-					clean[x] = c;
-					if (out)
-						out[x] = hole ? d[u] : c + -1 * bg[u];
-					donor = ok && isfinite(c);
+					clean[x] = v;
+					if (OUT && out)
+						out[x] = hole ? d[u] : v + -1 * bg[u];
 				}
 				const uint32_t hw = __ballot_sync(0xffffffffu, hole);
-				uint32_t mw = 0xffffffffu;
-				if (ROWMIN)
-					mw = __reduce_min_sync(0xffffffffu,
-						valid && !hole ? (uint32_t)(order_key(c) >> 32) : 0xffffffffu);
-				const uint32_t ew = __ballot_sync(0xffffffffu, valid && !ok);
-				const uint32_t dw = __ballot_sync(0xffffffffu, donor);
-				any_allowed |= __ballot_sync(0xffffffffu, ok);
-				any_finite |= dw;
-				any_hole |= hw;
-				ndonor += __popc(dw);
-				if (lane == c0 + u) {
+				const uint32_t ew = MASK ? __ballot_sync(0xffffffffu, valid && (hole || m[u])) : hw;
+				const uint32_t dw = __ballot_sync(0xffffffffu, valid && !hole && !m[u] && isfinite(v));
+				const uint32_t mw = ROWMIN ? __reduce_min_sync(0xffffffffu,
+					valid && !hole ? (uint32_t)(order_key(v) >> 32) : 0xffffffffu) : 0u;
+				if (lane == c + u) {
 					my_h = hw;
 					my_e = ew;
 					my_d = dw;
 					my_m = mw;
 				}
 			}
+		};
+		const int n = min(32, words - seg);
+		int c = 0;
+		for (; c + W <= n && 32 * (seg + c + W) <= w; c += W)
+			group(c, std::integral_constant<int, W>{}, std::true_type{});
+		for (; c < n; c += 4) {
+			if (W > 4 && 32 * (seg + c + 4) <= w)
+				group(c, std::integral_constant<int, 4>{}, std::true_type{});
+			else
+				group(c, std::integral_constant<int, 4>{}, std::false_type{});
 		}
-		const int k = seg * 32 + lane;
+		const int k = seg + lane;
 		if (k < words) {
 			hole_plane[k] = my_h;
 			excl_plane[k] = my_e;
 			donor_plane[k] = my_d;
 			if (ROWMIN)
 				rowmin[k] = my_m;
+			any_hole |= my_h;
+			any_allowed |= ~my_e & (w - 32 * k >= 32 ? 0xffffffffu : (1u << (w - 32 * k)) - 1u);
+			ndonor += __popc(my_d);
 		}
 		if (holes && __any_sync(0xffffffffu, my_h != 0)) { // list the segment's holes for the fill
 			unsigned long long slot = warp_append(&ctl->n_holes, __popc(my_h));
@@ -327,15 +358,18 @@ __device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st,
 				holes[slot++] = make_uint2((unsigned)f, (unsigned)(rowpix + 32 * k + __ffs(b) - 1));
 		}
 	}
-	if (lane == 0) {
+	any_hole = __ballot_sync(0xffffffffu, any_hole != 0);
+	any_allowed = __ballot_sync(0xffffffffu, any_allowed != 0);
+	ndonor = __reduce_add_sync(0xffffffffu, ndonor);
+	if (lane == 0) { // stores only: a test of the flag would wait for it
 		if (any_hole)
-			set_flag(&st.holes);
+			st.holes = 1;
 		if (any_allowed)
-			set_flag(&st.allowed);
-		if (any_finite)
-			set_flag(&st.finite);
-		if (ndonor)
+			st.allowed = 1;
+		if (ndonor) {
+			st.finite = 1;
 			atomicAdd((unsigned long long *)&st.donors_left, (unsigned long long)ndonor);
+		}
 	}
 }
 
@@ -344,34 +378,37 @@ __device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st,
 // segment's word j, so each plane gets one coalesced store per segment.  The
 // other planes were zeroed before the kernel.  With `holes`, each segment's
 // holes are appended to that list (count in ctl->n_holes) for the hole fill.
-// KIND: the frame kind every row has (PREP_ANY: decided per row); UL: the
-// unroll of the kinds without maps.
-// OUT: some frame of the batch has a separate output buffer.
-template <int KIND = PREP_ANY, int UL = ROW_UNROLL, bool OUT = false>
-__global__ void __launch_bounds__(256, 4)
+// KIND: the frame kind every row has (PREP_ANY: decided per row); W: the words
+// of a row in flight; OUT: some frame of the batch has a separate output buffer;
+// MINB: blocks per SM, which leaves the registers for W.
+template <int KIND, int W, bool OUT, int MINB>
+__global__ void __launch_bounds__(256, MINB)
 prepare_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const int2 *__restrict__ rows,
 	int nrows, Control *ctl = nullptr, uint2 *holes = nullptr)
 {
 	const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+	int2 next = gw < nrows ? rows[gw] : make_int2(0, 0);
 	for (int r = gw; r < nrows; r += nw) {
-		const int2 item = rows[r];
+		const int2 item = next;
+		if (r + nw < nrows) // the next row's entry loads during this row
+			next = rows[r + nw];
 		const FrameDesc &fd = frames[item.x];
 		FrameState &st = state[item.x];
 		switch (KIND == PREP_ANY ? prep_kind(fd) : KIND) {
 		case PREP_MODEL:
-			prepare_row<false, false, true, UL, OUT>(fd, st, item.x, item.y, ctl, holes);
+			prepare_row<false, false, true, W, OUT>(fd, st, item.x, item.y, ctl, holes);
 			break;
 		case PREP_MODEL_MAPS:
-			prepare_row<true, true, true, ROW_UNROLL, OUT>(fd, st, item.x, item.y, ctl, holes);
+			prepare_row<true, true, true, W, OUT>(fd, st, item.x, item.y, ctl, holes);
 			break;
 		case PREP_MASK:
-			prepare_row<true, false, false, UL, OUT>(fd, st, item.x, item.y, ctl, holes);
+			prepare_row<true, false, false, W, OUT>(fd, st, item.x, item.y, ctl, holes);
 			break;
 		case PREP_PLAIN:
-			prepare_row<false, false, false, UL, OUT>(fd, st, item.x, item.y, ctl, holes);
+			prepare_row<false, false, false, W, OUT>(fd, st, item.x, item.y, ctl, holes);
 			break;
 		default:
-			prepare_row<true, true, false, ROW_UNROLL, OUT>(fd, st, item.x, item.y, ctl, holes);
+			prepare_row<true, true, false, W, OUT>(fd, st, item.x, item.y, ctl, holes);
 		}
 	}
 }
@@ -960,6 +997,7 @@ restore_kernel(const FrameDesc *__restrict__ frames, const int2 *__restrict__ ro
 		uint8_t *mask_out = fd.mask_out + rowpix;
 		const double bgv = fd.bg;
 		const bool has_bg = fd.has_bg;
+		constexpr int ROW_UNROLL = 4; // words whose loads are issued before their use
 		for (int xb = 0; xb < w; xb += 32 * ROW_UNROLL) {
 			double v[ROW_UNROLL], bg[ROW_UNROLL];
 			uint32_t hb[ROW_UNROLL], cb[ROW_UNROLL];

@@ -211,8 +211,8 @@ remove_cosmics_device_noalloc(const struct cusmic_image *image, const struct cus
  * caller sets it.  No counterpart in the reference, whose tests inject none.
  *
  *   CUSMIC_FAULT_PREPARE_WAIT, CUSMIC_FAULT_DETECT_WAIT: value > 0 makes one
- *     warp of the bulk-staged prepare kernel, or of the dense detection
- *     kernel, wait up to `value` SM cycles on a barrier that nothing
+ *     warp of the dense detection kernel (which prepares the frames too, or
+ *     follows a prepare kernel that waits for nothing) wait up to `value` SM cycles on a barrier that nothing
  *     completes, in calls (and plans) laid out after this call.  The wait
  *     runs out like a wait whose copies never land: the kernel drains its
  *     copies in flight, the loop control stops every frame and the call

@@ -166,3 +166,36 @@ def test_map_checks_with_the_call(cuda, kw, message, at):
         remove_cosmics(np.full((h, w), 10.0), **args)
     clean, mask = remove_cosmics(np.full((h, w), 10.0), 3, 5, 3, error=make("error", "ones"))
     assert mask.dtype == cuda.bool and not bool(mask.any()) and bool((clean == 10).all())
+
+
+@pytest.mark.parametrize("kind", ("model", "model_background", "mask", "maps"))
+@pytest.mark.parametrize("width", (1, 31, 33, 127, 128, 129, 255, 256, 511, 513, 1023, 1024, 1025,
+                                   1151, 1536, 2177))
+def test_prepare_rows(cuda, oracle, kind, width):
+    """Rows around the sizes of a warp's groups and segments, per kind of
+    frame: whole groups of donors, and groups with non-finite or masked pixels
+    at their first and last columns.  Odd widths also put each row at another
+    alignment."""
+    h = 9
+    rng = np.random.default_rng(width)
+    data = structured(width, h, width)
+    frame, kw = dict(data=data), {}
+    edges = [x for x in (0, 31, 32, 127, 128, 255, 256, 511, 512, 1023, 1024, width - 1) if x < width]
+    for y, bad in ((1, np.nan), (3, np.inf), (5, -np.inf)):
+        data[y, edges[:: y + 1]] = bad
+    if kind in ("mask", "maps"):
+        frame["mask"] = np.zeros((h, width), dtype=bool)
+        frame["mask"][[2, 3, 7], :] = rng.random((3, width)) < 0.03
+        frame["mask"][4, edges] = True
+        frame["mask"][8, :] = True
+    if kind == "mask":
+        frame["error"] = np.full((h, width), 12.0)
+    else:
+        frame.update(gain=1.5, readnoise=3.0)
+        kw.update(gain=1.5, readnoise=3.0)
+    if kind == "maps":
+        frame["background"] = rng.normal(20, 2, (h, width))
+    elif kind == "model_background":
+        frame["background"] = 12.25
+        kw["background"] = 12.25
+    check_against_oracle(oracle, [frame], dict(SETTINGS, **kw))
