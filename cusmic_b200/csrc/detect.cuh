@@ -921,9 +921,9 @@ __device__ __forceinline__ void grow_group(const FrameDesc &fd, int f, int x, in
 	const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)lost);
 	if (now && (!same || lane == lead)) {
 		const int gone = same ? sum : lost;
-		set_flag(&state[f].todo[par]);
+		atomicOr(&state[f].todo[par], 1u);
 		if (gone)
-			atomicAdd((unsigned long long *)&state[f].donors_left, (unsigned long long)(-(long long)gone));
+			atomicAdd(&state[f].masked, (unsigned long long)gone);
 	}
 	const unsigned base = (unsigned)((long long)yy * w + x - 2);
 	for (; now; now &= now - 1)

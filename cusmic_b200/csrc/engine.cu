@@ -1037,7 +1037,7 @@ static void check_state(const FrameState &st)
 {
 	if (st.fault)
 		throw std::runtime_error("a detection kernel gave up waiting for its copies");
-	if (st.error || (st.holes && st.allowed && !st.finite))
+	if (st.error || (st.holes && st.allowed && !st.donors))
 		throw InvalidArgument("no finite replacement donors");
 }
 

@@ -62,15 +62,6 @@ __device__ __forceinline__ unsigned long long warp_append(unsigned long long *co
 	return base + (unsigned long long)(incl - cnt);
 }
 
-// Per-frame facts that the loop control only tests for zero (any hole, any
-// allowed pixel, any new pixel, any donor left): many warps set the same flag
-// with a plain store instead of contending on an atomic counter.
-template <class T> __device__ __forceinline__ void set_flag(T *flag)
-{
-	if (!*(volatile T *)flag)
-		*(volatile T *)flag = 1;
-}
-
 // Map validation of the host entry point on the device (reference
 // src/api.cu:107-114 runs it on the host): sets `bit` in *flags if any of the
 // n values is not finite, or (minimum 1) not positive, or (minimum 0)
@@ -231,8 +222,8 @@ CB_HD int prep_kind(const FrameDesc &fd)
 // ragged noise-model frames of 256 to 4096 pixels a side, 178 Mpix of 24 bytes:
 // 858 us with 8 words in flight and a tail group of 8, 705 us).  On small frames
 // it was bound by its last lines, where lane 0 tested each frame flag before
-// setting it, three waits in a row (256 frames of 40 to 200 pixels: 68 us, 27
-// with stores alone, 18 with the groups as they are now).
+// setting it, three waits in a row behind the other rows' additions to the
+// sector (256 frames of 40 to 200 pixels: 68 us, 17 without).
 template <bool MASK, bool BGMAP, bool ROWMIN, int W, bool OUT>
 __device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st, int f, int y, Control *ctl,
 	uint2 *holes)
@@ -361,15 +352,13 @@ __device__ __forceinline__ void prepare_row(const FrameDesc &fd, FrameState &st,
 	any_hole = __ballot_sync(0xffffffffu, any_hole != 0);
 	any_allowed = __ballot_sync(0xffffffffu, any_allowed != 0);
 	ndonor = __reduce_add_sync(0xffffffffu, ndonor);
-	if (lane == 0) { // stores only: a test of the flag would wait for it
+	if (lane == 0) {
 		if (any_hole)
-			st.holes = 1;
-		if (any_allowed)
-			st.allowed = 1;
-		if (ndonor) {
-			st.finite = 1;
-			atomicAdd((unsigned long long *)&st.donors_left, (unsigned long long)ndonor);
-		}
+			atomicAdd(&st.holes, 1ull);
+		if (ndonor)
+			atomicAdd(&st.donors, (unsigned long long)ndonor);
+		else if (any_allowed)
+			atomicAdd(&st.allowed, 1ull);
 	}
 }
 
@@ -743,14 +732,14 @@ struct WindowQueue {
 // pass flagged a pixel and a donor is left (reference src/cleaner.cuh:128-142).
 __device__ __forceinline__ bool replaces(const FrameState &s, int par)
 {
-	return s.todo[par] && s.donors_left > 0;
+	return s.todo[par] && s.donors > s.masked;
 }
 
 // Per-frame loop control after a pass (reference src/cleaner.cuh:128-142,
 // 175-181): a frame with new pixels but no donors fails, a frame without new
 // pixels stops (its later passes would repeat this one), the others replace
 // and continue.  Runs in the replacement's grid (a thread per frame): the
-// replacement reads only todo[par] and donors_left, which this leaves alone.
+// replacement reads only todo[par] and the donor counts, which this leaves alone.
 __device__ __forceinline__ void pass_control(FrameState *state, int nf, Control *ctl, int par)
 {
 	const int fault = *(volatile int *)&ctl->fault;
@@ -763,7 +752,7 @@ __device__ __forceinline__ void pass_control(FrameState *state, int nf, Control 
 		bool on = false;
 		if (fault) // this pass's detection is incomplete: stop, report
 			s.fault = 1;
-		else if (s.todo[par] && s.donors_left <= 0)
+		else if (s.todo[par] && s.donors <= s.masked)
 			s.error = 1;
 		else
 			on = s.todo[par] != 0;
@@ -883,7 +872,7 @@ fill_list_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restr
 		const long long e = base + threadIdx.x;
 		if (e < n) {
 			const uint2 t = holes[e];
-			if (state[t.x].finite) {
+			if (state[t.x].donors) {
 				const FrameDesc &fd = frames[t.x];
 				const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 				double r;
@@ -922,7 +911,7 @@ fill_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__
 	for (int ri = gw; ri < nrows; ri += nw) {
 		const int2 item = rows[ri];
 		const FrameState &st = state[item.x];
-		if (!st.holes || !st.finite)
+		if (!st.holes || !st.donors)
 			continue; // warp-uniform
 		const FrameDesc &fd = frames[item.x];
 		const uint32_t *hp = plane_ptr(fd, P_HOLE) + (long long)item.y * fd.words;

@@ -179,18 +179,28 @@ __device__ __forceinline__ uint32_t mask_nibble(uint32_t m)
 
 // What a consumer warp gathers over an item for the frame's state.
 struct PdFacts {
-	uint32_t hole, allowed; // any hole, any allowed (without a background: any donor)
-	int donors;             // donors among the words this lane stored
+	uint32_t hole; // any hole
+	int donors;    // donors among the words of this lane
+};
+
+// Where a lane's part of the next own row goes.
+struct PdOwn {
+	double *clean;  // the lane's four working pixels
+	uint32_t *word; // lane 8j: HOLE's word j of the warp's columns, 8j + 1: EXCL's, else DONOR's
+	int w, words;   // steps of the two to the next row
+	uint32_t full;  // the word's columns in the frame
+	bool put;       // the lane stores its word
+	bool wide;      // 32-byte stores (the working pixels' alignment)
 };
 
 // The prepare step of one own row for a lane's four columns x .. x + 3 (all
-// in the frame or none: w is a multiple of 16): the working pixels, the bit
-// words (lane 8j stores word j of the warp's 128 columns, from the lanes'
-// 4-bit groups OR-ed across the eight lanes by shuffles; DONOR is the
+// in the frame or none: w is a multiple of 16; the first is pixel `pix`): the
+// working pixels, the bit words (three lanes store a word of each plane, from
+// the lanes' 4-bit groups OR-ed across eight lanes by shuffles; DONOR is the
 // complement of EXCL within the frame) and the hole list.  Returns the lane's
 // hole bits (bit i = column x + i); `any_hole`: some lane has one; `bad`:
 // some value the warp reads from the row, halo columns included, is a hole.
-__device__ __forceinline__ uint32_t pd_prepare_row(const FrameDesc &fd, int f, int y, int x, bool valid,
+__device__ __forceinline__ uint32_t pd_prepare_row(PdOwn &own, int f, unsigned pix, bool valid,
 	bool has_mask, const double (&v)[6], uint32_t mbytes, Control *ctl, uint2 *holes, PdFacts &acc,
 	bool &any_hole, bool &bad)
 {
@@ -203,7 +213,6 @@ __device__ __forceinline__ uint32_t pd_prepare_row(const FrameDesc &fd, int f, i
 		hn = 0;
 	any_hole = __any_sync(0xffffffffu, hn != 0);
 	bad = any_hole || __any_sync(0xffffffffu, valid && (!isfinite(v[0]) || !isfinite(v[5])));
-	const long long rowpix = (long long)y * fd.w;
 	if (valid) {
 		double c[4] = {v[1], v[2], v[3], v[4]};
 		if (hn) {
@@ -211,9 +220,14 @@ __device__ __forceinline__ uint32_t pd_prepare_row(const FrameDesc &fd, int f, i
 			for (int i = 0; i < 4; ++i)
 				c[i] = (hn >> i) & 1u ? 0.0 : c[i];
 		}
-		double2 *dst = reinterpret_cast<double2 *>(fd.clean + rowpix + x);
-		dst[0] = make_double2(c[0], c[1]);
-		dst[1] = make_double2(c[2], c[3]);
+		if (own.wide) { // warp-uniform
+			asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(own.clean), "d"(c[0]), "d"(c[1]),
+				"d"(c[2]), "d"(c[3]) : "memory");
+		} else {
+			double2 *dst = reinterpret_cast<double2 *>(own.clean);
+			dst[0] = make_double2(c[0], c[1]);
+			dst[1] = make_double2(c[2], c[3]);
+		}
 	}
 	const int sh = 4 * (lane & 7);
 	uint32_t ew = 0, hw = 0;
@@ -229,21 +243,19 @@ __device__ __forceinline__ uint32_t pd_prepare_row(const FrameDesc &fd, int f, i
 		for (int o = 1; o < 8; o <<= 1)
 			hw |= __shfl_xor_sync(0xffffffffu, hw, o);
 	}
-	if ((lane & 7) == 0 && valid) {
-		const uint32_t dw = ~ew & (fd.w - x >= 32 ? 0xffffffffu : 0x0000ffffu);
-		const long long at = (long long)y * fd.words + (x >> 5);
-		plane_ptr(fd, P_HOLE)[at] = hw;
-		plane_ptr(fd, P_EXCL)[at] = ew;
-		plane_ptr(fd, P_DONOR)[at] = dw;
-		acc.donors += __popc(dw);
-		acc.allowed |= dw;
-	}
+	const int which = lane & 7;
+	const uint32_t word = which == 0 ? hw : which == 1 ? ew : ~ew & own.full;
+	if (own.put)
+		*own.word = word;
+	acc.donors += __popc(word); // counts on the lanes of DONOR
 	acc.hole |= hn;
 	if (any_hole) { // the row's holes for the fill
 		unsigned long long slot = warp_append(&ctl->n_holes, __popc(hn));
 		for (uint32_t b = hn; b; b &= b - 1)
-			holes[slot++] = make_uint2((unsigned)f, (unsigned)(rowpix + x + __ffs(b) - 1));
+			holes[slot++] = make_uint2((unsigned)f, pix + __ffs(b) - 1);
 	}
+	own.clean += own.w;
+	own.word += own.words;
 	return hn;
 }
 
@@ -280,7 +292,20 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 				x / FLOOR_BLOCK].thr;
 			thr = hi_word(T >= 0 ? T : 0.0); // NaN lists everything
 		}
-		PdFacts acc{0u, 0u, 0};
+		PdFacts acc{0u, 0};
+		PdOwn own;
+		{
+			const int which = lane & 7, xg = x - 4 * which;
+			own.w = w;
+			own.words = fd.words;
+			own.clean = fd.clean + (long long)y0 * w + x;
+			own.word = plane_ptr(fd, which == 0 ? P_HOLE : which == 1 ? P_EXCL : P_DONOR) +
+				(long long)y0 * fd.words + (xg >> 5);
+			own.full = w - xg >= 32 ? 0xffffffffu : 0x0000ffffu;
+			own.put = which < 3 && xg < w;
+			own.wide = ((uintptr_t)fd.clean & 31u) == 0;
+		}
+		unsigned pix = (unsigned)((long long)y0 * w + x); // of the lane's first column, row y
 		ok = __all_sync(0xffffffffu,
 			mbar_wait(&R.full[(g + 1) & (BK_SLOTS - 1)], ((g + 1) / BK_SLOTS) & 1, &R.abort));
 		if (!ok)
@@ -302,7 +327,7 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 				mbar_arrive(&R.empty[s1]);
 			}
 			bool bad_c;
-			hcur = pd_prepare_row(fd, f, y0, x, valid, has_mask, c, mb, ctl, holes, acc, hrow, bad_c);
+			hcur = pd_prepare_row(own, f, pix, valid, has_mask, c, mb, ctl, holes, acc, hrow, bad_c);
 			double su[6], sc[6];
 			pd_quarters(u, pd_row_bad(u, valid), su);
 			pd_quarters(c, bad_c, sc);
@@ -325,16 +350,16 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 				break;
 			double n[6];
 			load_six(R.c[sd], c0, R.shift[sd], n);
-			const bool own = y + 1 < y1;
-			const uint32_t mb = own && has_mask && valid ? *reinterpret_cast<const uint32_t *>(&M[sd][4 * ct])
+			const bool mine = y + 1 < y1;
+			const uint32_t mb = mine && has_mask && valid ? *reinterpret_cast<const uint32_t *>(&M[sd][4 * ct])
 				: 0u;
 			__syncwarp();
 			if (lane == 0)
 				mbar_arrive(&R.empty[sd]); // row y + 1 is in registers
 			uint32_t hnext = 0;
 			bool hrow_next = false, bad_n;
-			if (own) // warp-uniform
-				hnext = pd_prepare_row(fd, f, y + 1, x, valid, has_mask, n, mb, ctl, holes, acc,
+			if (mine) // warp-uniform
+				hnext = pd_prepare_row(own, f, pix + (unsigned)w, valid, has_mask, n, mb, ctl, holes, acc,
 					hrow_next, bad_n);
 			else
 				bad_n = pd_row_bad(n, valid);
@@ -347,7 +372,6 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 			for (int i = 0; i < 3; ++i)
 				hd[i + 1] = q[i] - q[i + 1];
 			hd[4] = q[3] - qr;
-			const long long pix0 = (long long)y * w + x;
 			double lap[4];
 #pragma unroll
 			for (int i = 0; i < 4; ++i) {
@@ -376,28 +400,25 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 				for (int i = 0; i < 4; ++i) {
 					const unsigned bal = __ballot_sync(0xffffffffu, pass[i]);
 					if (pass[i])
-						region[cnt + __popc(bal & below)] = PreCand{(unsigned)(pix0 + i), (unsigned)f, lap[i]};
+						region[cnt + __popc(bal & below)] = PreCand{pix + i, (unsigned)f, lap[i]};
 					cnt += __popc(bal);
 				}
 			}
+			pix += (unsigned)w;
 		}
 		if (!ok)
 			break;
 		// The item's facts for the frame's state.
+		const bool donor_lane = own.put && (lane & 7) == 2;
 		const bool any_hole = __any_sync(0xffffffffu, acc.hole != 0);
-		const bool any_allowed = __any_sync(0xffffffffu, acc.allowed != 0);
-		const int donors = __reduce_add_sync(0xffffffffu, acc.donors);
+		const int donors = __reduce_add_sync(0xffffffffu, donor_lane ? acc.donors : 0);
 		if (lane == 0) {
 			pre_counts[t * BK_CWARPS + warp] = cnt;
 			FrameState &st = state[f];
 			if (any_hole)
-				set_flag(&st.holes);
-			if (any_allowed) {
-				set_flag(&st.allowed);
-				set_flag(&st.finite);
-			}
-			if (donors)
-				atomicAdd((unsigned long long *)&st.donors_left, (unsigned long long)donors);
+				atomicAdd(&st.holes, 1ull);
+			if (donors) // without a background every allowed pixel is one
+				atomicAdd(&st.donors, (unsigned long long)donors);
 		}
 		g += y1 - y0 + 2;
 	}
