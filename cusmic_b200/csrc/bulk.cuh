@@ -149,6 +149,14 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long *b)
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(b)) : "memory");
 }
 
+// As mbar_arrive, by the lanes with `mine` set, without a branch.
+__device__ __forceinline__ void mbar_arrive_if(unsigned long long *b, bool mine)
+{
+	asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %1, 0;\n"
+		     " @p mbarrier.arrive.shared::cta.b64 _, [%0];\n}\n" ::"r"(smem_u32(b)), "r"((int)mine)
+		: "memory");
+}
+
 // Arrive on b once every cp.async this thread issued so far has landed.
 __device__ __forceinline__ void mbar_arrive_cp_async(unsigned long long *b)
 {
@@ -178,6 +186,22 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity
 		if (mbar_test(b, parity))
 			return true;
 		if ((i & 15) == 0 && (*(const volatile int *)abort || clock64() - t0 > limit))
+			return false;
+	}
+}
+
+// mbar_wait for a whole warp (every lane calls it and gets the same answer): one
+// vote when the phase has completed already, no divergent branch.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long *b, unsigned parity, const int *abort)
+{
+	if (__all_sync(0xffffffffu, mbar_test(b, parity)))
+		return true;
+	const long long t0 = clock64();
+	for (unsigned i = 1;; ++i) {
+		if (__all_sync(0xffffffffu, mbar_test(b, parity)))
+			return true;
+		if ((i & 15) == 0 && __any_sync(0xffffffffu, *(const volatile int *)abort ||
+			clock64() - t0 > BK_WAIT_CYCLES))
 			return false;
 	}
 }
@@ -613,7 +637,7 @@ __device__ __forceinline__ bool bulk_consumer(BulkRing &R, const FrameDesc *__re
 	int g = 0;
 	bool ok = true;
 	for (;;) {
-		ok = __all_sync(0xffffffffu, mbar_wait(&R.full[g & (BK_SLOTS - 1)], (g / BK_SLOTS) & 1, &R.abort));
+		ok = mbar_wait_warp(&R.full[g & (BK_SLOTS - 1)], (g / BK_SLOTS) & 1, &R.abort);
 		if (!ok)
 			break;
 		const int2 meta = R.meta[g & (BK_SLOTS - 1)];
@@ -638,8 +662,7 @@ __device__ __forceinline__ bool bulk_consumer(BulkRing &R, const FrameDesc *__re
 			for (int i = 0; i < 4; ++i)
 				thr[i] = x + i < w ? tv : 0xffffffffu;
 		}
-		ok = __all_sync(0xffffffffu,
-			mbar_wait(&R.full[(g + 1) & (BK_SLOTS - 1)], ((g + 1) / BK_SLOTS) & 1, &R.abort));
+		ok = mbar_wait_warp(&R.full[(g + 1) & (BK_SLOTS - 1)], ((g + 1) / BK_SLOTS) & 1, &R.abort);
 		if (!ok)
 			break;
 		// Row y0 - 1 (values) and row y0 (values and neighbours), as quarters.
@@ -667,7 +690,7 @@ __device__ __forceinline__ bool bulk_consumer(BulkRing &R, const FrameDesc *__re
 		for (int y = y0; y < y1; ++y) {
 			const int gd = g + 2 + (y - y0); // ring row of y + 1
 			const int sd = gd & (BK_SLOTS - 1);
-			ok = __all_sync(0xffffffffu, mbar_wait(&R.full[sd], (gd / BK_SLOTS) & 1, &R.abort));
+			ok = mbar_wait_warp(&R.full[sd], (gd / BK_SLOTS) & 1, &R.abort);
 			if (!ok)
 				break;
 			double n[6];

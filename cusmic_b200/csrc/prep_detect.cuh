@@ -27,9 +27,15 @@
 // for the item's own rows the mask bytes of its columns into a second ring;
 // four consumer warps evaluate four columns per lane.  A consumer lane handles
 // the prepare step of each own row (holes, exclusions, donors, the working
-// pixels as two 16-byte stores) when the row arrives in the ring; the bit
+// pixels as one 32-byte store) when the row arrives in the ring; the bit
 // words of the warp's 128 columns are assembled from the lanes' 4-bit groups
-// by shuffles.  Per-frame facts are set once per item and warp.
+// by shuffles.  Per-frame facts are added once per item and warp.
+//
+// Issue slots bound it (410 warp instructions per 128 pixels, a fifth of them
+// branches and their joins; DRAM at a third of its rate).  One test per row for
+// a value that is not finite, by the largest of the six high words, votes
+// instead of divergent waits, and predicated stores and arrivals left 366: 16
+// frames of 2048 x 2048 290 -> 268 us, two of 8192 x 8192 488 -> 436.
 //
 // The block floors of error maps depend on the maps only, so they are computed
 // before this kernel (prep_init_kernel, with the call's state and zeroing);
@@ -190,8 +196,20 @@ struct PdOwn {
 	int w, words;   // steps of the two to the next row
 	uint32_t full;  // the word's columns in the frame
 	bool put;       // the lane stores its word
-	bool wide;      // 32-byte stores (the working pixels' alignment)
+	int store;      // its pixels: 2 as 32 bytes, 1 as 16 and 16 (by their alignment), 0 not at all
 };
+
+// A lane's four working pixels: one 32-byte store or two of 16 bytes, predicated
+// (no branch).
+__device__ __forceinline__ void store4(const PdOwn &own, const double (&c)[4])
+{
+	asm volatile("{\n .reg .pred w, n;\n setp.eq.s32 w, %0, 2;\n setp.eq.s32 n, %0, 1;\n"
+		     " @w st.global.v4.f64 [%1], {%2, %3, %4, %5};\n"
+		     " @n st.global.v2.f64 [%1], {%2, %3};\n"
+		     " @n st.global.v2.f64 [%1 + 16], {%4, %5};\n}\n"
+		::"r"(own.store), "l"(own.clean), "d"(c[0]), "d"(c[1]), "d"(c[2]), "d"(c[3])
+		: "memory");
+}
 
 // The prepare step of one own row for a lane's four columns x .. x + 3 (all
 // in the frame or none: w is a multiple of 16; the first is pixel `pix`): the
@@ -205,30 +223,27 @@ __device__ __forceinline__ uint32_t pd_prepare_row(PdOwn &own, int f, unsigned p
 	bool &any_hole, bool &bad)
 {
 	const int lane = threadIdx.x & 31;
+	// Twice the high words without their signs: the largest tells whether some
+	// value is not finite.
+	unsigned top = 0;
+#pragma unroll
+	for (int i = 0; i < 6; ++i)
+		top = max(top, (unsigned)__double2hiint(v[i]) << 1);
+	bad = __any_sync(0xffffffffu, valid && top >= 0xffe00000u);
+	any_hole = false;
 	uint32_t hn = 0;
+	double c[4] = {v[1], v[2], v[3], v[4]};
+	if (bad) { // warp-uniform
 #pragma unroll
-	for (int i = 0; i < 4; ++i)
-		hn |= (uint32_t)!isfinite(v[i + 1]) << i;
-	if (!valid)
-		hn = 0;
-	any_hole = __any_sync(0xffffffffu, hn != 0);
-	bad = any_hole || __any_sync(0xffffffffu, valid && (!isfinite(v[0]) || !isfinite(v[5])));
-	if (valid) {
-		double c[4] = {v[1], v[2], v[3], v[4]};
-		if (hn) {
-#pragma unroll
-			for (int i = 0; i < 4; ++i)
-				c[i] = (hn >> i) & 1u ? 0.0 : c[i];
+		for (int i = 0; i < 4; ++i) {
+			hn |= (uint32_t)!isfinite(v[i + 1]) << i;
+			c[i] = isfinite(v[i + 1]) ? v[i + 1] : 0.0;
 		}
-		if (own.wide) { // warp-uniform
-			asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(own.clean), "d"(c[0]), "d"(c[1]),
-				"d"(c[2]), "d"(c[3]) : "memory");
-		} else {
-			double2 *dst = reinterpret_cast<double2 *>(own.clean);
-			dst[0] = make_double2(c[0], c[1]);
-			dst[1] = make_double2(c[2], c[3]);
-		}
+		if (!valid)
+			hn = 0;
+		any_hole = __any_sync(0xffffffffu, hn != 0);
 	}
+	store4(own, c);
 	const int sh = 4 * (lane & 7);
 	uint32_t ew = 0, hw = 0;
 	if (has_mask || any_hole) { // warp-uniform
@@ -272,7 +287,7 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 	int g = 0;
 	bool ok = true;
 	for (;;) {
-		ok = __all_sync(0xffffffffu, mbar_wait(&R.full[g & (BK_SLOTS - 1)], (g / BK_SLOTS) & 1, &R.abort));
+		ok = mbar_wait_warp(&R.full[g & (BK_SLOTS - 1)], (g / BK_SLOTS) & 1, &R.abort);
 		if (!ok)
 			break;
 		const int2 meta = R.meta[g & (BK_SLOTS - 1)];
@@ -303,11 +318,10 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 				(long long)y0 * fd.words + (xg >> 5);
 			own.full = w - xg >= 32 ? 0xffffffffu : 0x0000ffffu;
 			own.put = which < 3 && xg < w;
-			own.wide = ((uintptr_t)fd.clean & 31u) == 0;
+			own.store = !valid ? 0 : ((uintptr_t)fd.clean & 31u) == 0 ? 2 : 1;
 		}
 		unsigned pix = (unsigned)((long long)y0 * w + x); // of the lane's first column, row y
-		ok = __all_sync(0xffffffffu,
-			mbar_wait(&R.full[(g + 1) & (BK_SLOTS - 1)], ((g + 1) / BK_SLOTS) & 1, &R.abort));
+		ok = mbar_wait_warp(&R.full[(g + 1) & (BK_SLOTS - 1)], ((g + 1) / BK_SLOTS) & 1, &R.abort);
 		if (!ok)
 			break;
 		// Row y0 - 1 (values) and row y0 (values and neighbours), as quarters;
@@ -320,7 +334,7 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 			double u[6], c[6];
 			load_six(R.c[s0], c0, R.shift[s0], u);
 			load_six(R.c[s1], c0, R.shift[s1], c);
-			const uint32_t mb = has_mask && valid ? *reinterpret_cast<const uint32_t *>(&M[s1][4 * ct]) : 0u;
+			const uint32_t mb = has_mask ? *reinterpret_cast<const uint32_t *>(&M[s1][4 * ct]) : 0u;
 			__syncwarp();
 			if (lane == 0) { // both rows are in registers now
 				mbar_arrive(&R.empty[s0]);
@@ -345,17 +359,15 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 		for (int y = y0; y < y1; ++y) {
 			const int gd = g + 2 + (y - y0); // ring row of y + 1
 			const int sd = gd & (BK_SLOTS - 1);
-			ok = __all_sync(0xffffffffu, mbar_wait(&R.full[sd], (gd / BK_SLOTS) & 1, &R.abort));
+			ok = mbar_wait_warp(&R.full[sd], (gd / BK_SLOTS) & 1, &R.abort);
 			if (!ok)
 				break;
 			double n[6];
 			load_six(R.c[sd], c0, R.shift[sd], n);
 			const bool mine = y + 1 < y1;
-			const uint32_t mb = mine && has_mask && valid ? *reinterpret_cast<const uint32_t *>(&M[sd][4 * ct])
-				: 0u;
+			const uint32_t mb = mine && has_mask ? *reinterpret_cast<const uint32_t *>(&M[sd][4 * ct]) : 0u;
 			__syncwarp();
-			if (lane == 0)
-				mbar_arrive(&R.empty[sd]); // row y + 1 is in registers
+			mbar_arrive_if(&R.empty[sd], lane == 0); // row y + 1 is in registers
 			uint32_t hnext = 0;
 			bool hrow_next = false, bad_n;
 			if (mine) // warp-uniform
