@@ -889,10 +889,23 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	static_assert(sizeof(PreCand) == 2 * sizeof(uint2), "the pre list holds both lists");
 	uint8_t *radius = ws.radius.p;
 	unsigned *chg = ws.chg.p;
-	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, prm, ctl, cands, low, eval, targets, chg,
-		ws.jobs.p, L.error_frames < nf ? (int)L.jobs.size() : 0);
-	auto classes = L.error_frames < nf ? late_classes_kernel<true> : late_classes_kernel<false>;
-	classes<<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
+	// The class of the noise-model frames' pixels near the first pass's
+	// targets: in parts with a thread per median from about 8 Mpixel (64 ragged
+	// frames, 178 Mpixel: 140 us against 301 with a warp per median; eight
+	// frames of 1024 x 1024: 19 and 18; five of 1018 x 1001: 20 and 15; 256 of
+	// 40 to 200 a side: 18 and 11).
+	const bool model = L.error_frames < nf, thresholds = model && L.total_px > 8u << 20;
+	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, prm, ctl, cands, low, eval,
+		targets, chg, ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
+	if (!model)
+		late_classes_kernel<LATE_TESTS, false><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
+	else if (!thresholds)
+		late_classes_kernel<LATE_SHORT, true><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
+	else {
+		late_classes_kernel<LATE_TESTS, true><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
+		late_classes_kernel<LATE_MEDIANS, true><<<std::min(wide, di.sms * 2), 256, 0, s>>>(frames, prm, ctl,
+			cands, low, eval);
+	}
 	void *args[] = {&frames, &state, &nf, &prm, &ctl, &maxiter, &cands, &low, &eval, &targets, &radius, &chg};
 	check(cudaLaunchCooperativeKernel((const void *)late_passes_kernel, dim3(grid), dim3(LATE_THREADS), args,
 		sizeof(LateShared), s));

@@ -224,7 +224,10 @@ __device__ __forceinline__ void late_neighbours(const FrameDesc *__restrict__ fr
 }
 
 // The class of lane's re-evaluated pixel t (0: none, 1: HIGH, 2: LOW) into the
-// planes and lists; called by the whole warp, `have`: the lane has one.
+// planes and lists; called by the whole warp, `have`: the lane has one.  GATED:
+// the S1, S2 and CAND words are read where a bit can be set and has to go (they
+// are set in the classes only), which saves loads but adds a round trip.
+template <bool GATED>
 __device__ __forceinline__ void late_class(const FrameDesc *__restrict__ frames, uint2 t, int cls, bool have,
 	PassLists &L, uint2 *cands, uint2 *low)
 {
@@ -238,7 +241,8 @@ __device__ __forceinline__ void late_class(const FrameDesc *__restrict__ frames,
 		uint32_t *H = plane_ptr(fd, P_HIGH) + o, *W = plane_ptr(fd, P_LOW) + o;
 		uint32_t *s1 = plane_ptr(fd, P_S1) + o, *s2 = plane_ptr(fd, P_S2) + o, *cd = plane_ptr(fd, P_CAND) + o;
 		const bool oh = (*H & bit) != 0, ol = (*W & bit) != 0; // only this thread writes the pixel's bits
-		const bool o1 = (*s1 & bit) != 0, o2 = (*s2 & bit) != 0, oc = (*cd & bit) != 0;
+		const bool out_high = !GATED || (oh && cls != 1), out = !GATED || ((oh || ol) && cls == 0);
+		const bool o1 = out_high && (*s1 & bit), oc = out_high && (*cd & bit), o2 = out && (*s2 & bit);
 		to_high = cls == 1 && !oh;
 		to_low = cls == 2 && !ol;
 		if (to_high)
@@ -280,14 +284,21 @@ __device__ __forceinline__ int class_of(double v, const DetectParams &prm)
 
 // Stage 2 (called by every warp of the grid).  On noise-model frames a pixel
 // whose Laplacian is at most its floor block's bound cannot pass either
-// threshold; the others wait in the warp's queue Q (64 entries).  THREADS: 32
-// of them at a time, a thread per median (long lists); else the warp sorts
-// each one's window (short lists, few registers).
+// threshold; the others wait in the warp's queue Q (64 entries) for the
+// median of their window.  Short lists (LATE_SHORT) do both at once, a warp per
+// median.  Long ones take two launches, since a thread per median takes 25
+// values in registers: LATE_TESTS at full occupancy, which marks the entries it
+// settles, then LATE_MEDIANS, 32 of the others at a time (in one launch with
+// the medians' registers they took 190 us on 64 ragged noise-model frames of 256
+// to 4096 pixels a side, as two 103 and 37).
 //
-// A list that takes THREADS finds the block thresholds written since the last
-// replacement (late_neighbours_kernel).
-template <bool THREADS, bool MODEL = true>
-__device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frames, const uint2 *eval,
+// A long list finds the block thresholds written since the last replacement
+// (late_neighbours_kernel).
+enum LatePart { LATE_SHORT, LATE_TESTS, LATE_MEDIANS };
+constexpr unsigned EVAL_DONE = 0xffffffffu; // the frame of an entry that is settled
+
+template <LatePart PART, bool MODEL = true>
+__device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frames, uint2 *eval,
 	const DetectParams &prm, PassLists &L, uint2 *cands, uint2 *low, uint2 *Q)
 {
 	const int lane = threadIdx.x & 31;
@@ -301,7 +312,7 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 		__syncwarp();
 		uint2 t = make_uint2(0u, 0u);
 		int cls = 0;
-		if (!THREADS) {
+		if (PART == LATE_SHORT) {
 			t = Q[lane < count ? lane : 0];
 			for (int q = 0; q < count; ++q) {
 				const uint2 u = Q[q];
@@ -345,18 +356,21 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 			Q[lane] = Q[lane + 32];
 		nq -= count;
 		__syncwarp();
-		late_class(frames, t, cls, lane < count, L, cands, low);
+		late_class<PART != LATE_SHORT>(frames, t, cls, lane < count, L, cands, low);
 	};
 	// Long lists go to the warps in runs of 32, whose loads share lines; short
 	// ones are dealt one by one, so that few medians wait behind each other.
-	const long long first = THREADS ? gw * 32 : gw, step = THREADS ? 1 : nw;
+	const long long first = PART == LATE_SHORT ? gw : gw * 32, step = PART == LATE_SHORT ? nw : 1;
 	for (long long base = first; base < n; base += nw * 32) {
 		const long long e = base + lane * step;
 		uint2 t = make_uint2(0u, 0u);
 		int cls = 0;
 		bool have = e < n, wait = false;
-		if (have) {
+		if (have)
 			t = eval[e];
+		if (PART == LATE_MEDIANS) {
+			wait = have && t.x != EVAL_DONE;
+		} else if (have) {
 			const FrameDesc &fd = frames[t.x];
 			const int w = fd.w, x = (int)(t.y % (unsigned)w), y = (int)(t.y / (unsigned)w);
 			double lap;
@@ -369,14 +383,18 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 			if (!MODEL || fd.error) {
 				cls = class_of(lap / (2 * fd.error[t.y]), prm);
 			} else {
-				const double T = THREADS ? fd.floors[(y >> 5) * ((w + 31) >> 5) + (x >> 5)].thr
-					: block_threshold(fd, x >> 5, y >> 5, mode, tmin2);
+				const double T = PART == LATE_SHORT ? block_threshold(fd, x >> 5, y >> 5, mode, tmin2)
+					: fd.floors[(y >> 5) * ((w + 31) >> 5) + (x >> 5)].thr;
 				wait = !(T >= 0 && lap <= T);
 			}
 		}
-		late_class(frames, t, cls, have && !wait, L, cands, low);
-		if (!MODEL)
+		if (PART != LATE_MEDIANS)
+			late_class<PART != LATE_SHORT>(frames, t, cls, have && !wait, L, cands, low);
+		if (PART == LATE_TESTS) {
+			if (MODEL && have && !wait)
+				eval[e].x = EVAL_DONE;
 			continue;
+		}
 		const unsigned b = __ballot_sync(0xffffffffu, wait);
 		if (b) {
 			if (wait)
@@ -531,8 +549,8 @@ late_neighbours_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, C
 	const FloorJob *__restrict__ jobs, int njobs)
 {
 	__shared__ ListSlots slots;
-	// The noise-model blocks' thresholds, for late_classes_kernel (a thread per
-	// block; the replacement lowered the floors).
+	// The noise-model blocks' thresholds, for the long lists' LATE_TESTS (a
+	// thread per block; the replacement lowered the floors).
 	const double tmin2 = fmin(prm.thi2, prm.tlo2);
 	for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < njobs; j += gridDim.x * blockDim.x) {
 		const FloorJob jb = jobs[j];
@@ -544,14 +562,15 @@ late_neighbours_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, C
 	late_neighbours<LN_THREADS / 32>(frames, targets, chg, ctl->pass[1], prm.mode, cands, low, eval, slots);
 }
 
-// MODEL: the batch has noise-model frames.
-template <bool MODEL>
-__global__ void __launch_bounds__(256, MODEL ? 2 : 6)
+// MODEL: the batch has noise-model frames (launch_late has the choice of parts).
+template <LatePart PART, bool MODEL>
+__global__ void __launch_bounds__(256, PART == LATE_MEDIANS ? 2 : 6)
 late_classes_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, Control *ctl, uint2 *cands,
-	uint2 *low, const uint2 *eval)
+	uint2 *low, uint2 *eval)
 {
-	__shared__ uint2 queue[MODEL ? 8 : 1][64];
-	late_classes<true, MODEL>(frames, eval, prm, ctl->pass[1], cands, low, queue[MODEL ? threadIdx.x >> 5 : 0]);
+	constexpr bool QUEUED = PART != LATE_TESTS;
+	__shared__ uint2 queue[QUEUED ? 8 : 1][64];
+	late_classes<PART, MODEL>(frames, eval, prm, ctl->pass[1], cands, low, queue[QUEUED ? threadIdx.x >> 5 : 0]);
 }
 
 struct LateShared {
@@ -601,7 +620,7 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 			}
 			if (!grid_barrier(ctl, ++round, state, nf))
 				return;
-			late_classes<false>(frames, eval, prm, L, cands, low, S.queue[warp]);
+			late_classes<LATE_SHORT>(frames, eval, prm, L, cands, low, S.queue[warp]);
 			if (!grid_barrier(ctl, ++round, state, nf))
 				return;
 		}

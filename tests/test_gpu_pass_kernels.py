@@ -6,7 +6,9 @@ pixels are those of the CPU oracle bit for bit."""
 import numpy as np
 import pytest
 
-from tests.test_gpu_parity import MODES, SETTINGS, check_against_oracle, small_scene
+from tests import cabi
+from tests.test_gpu_parity import (MODES, SETTINGS, assert_bits_equal, check_against_oracle,
+                                   small_scene)
 
 pytestmark = pytest.mark.gpu
 
@@ -199,3 +201,34 @@ def test_prepare_rows(cuda, oracle, kind, width):
         frame["background"] = 12.25
         kw["background"] = 12.25
     check_against_oracle(oracle, [frame], dict(SETTINGS, **kw))
+
+
+@pytest.mark.parametrize("mode", ("reflect", "wrap"))
+def test_long_late_lists(cuda, mode):
+    """A batch above 8 Mpixel, whose first late pass classifies in parts,
+    against the same frames one at a time (which the tests above compare with
+    the oracle): noise models with and without maps, an error map and a frame
+    with every pixel alike."""
+    frames = []
+    for i in range(10):
+        h, w = 900 + 13 * i, 1000 - 7 * i
+        data = structured(i, h, w, hits=40) if i != 4 else np.full((h, w), 50.0)
+        frame = dict(data=data, gain=1.5, readnoise=3.0)
+        if i % 3 == 1:
+            frame["gain"] = np.random.default_rng(i).uniform(1.2, 1.8, (h, w))
+        elif i % 3 == 2:
+            frame = dict(data=data, error=np.full((h, w), 12.0))
+        frames.append(frame)
+    assert sum(f["data"].size for f in frames) > 8 << 20
+    kw = dict(contrast=1.5, cr_threshold=4.0, neighbor_threshold=1.0, maxiter=4, gain=1.5,
+              readnoise=3.0, border=mode)
+    fr = cabi.Frames(frames)
+    st, msg = cabi.run_ragged(fr, cabi.options(**kw))
+    assert st == 0, msg
+    for frame, (clean, mask) in zip(frames, fr.outputs()):
+        one = cabi.Frames([frame])
+        st, msg = cabi.run_ragged(one, cabi.options(**kw))
+        assert st == 0, msg
+        want_clean, want_mask = one.outputs()[0]
+        np.testing.assert_array_equal(mask, want_mask)
+        assert_bits_equal(clean, want_clean)
