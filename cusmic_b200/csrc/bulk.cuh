@@ -518,23 +518,92 @@ __device__ __forceinline__ void bulk_issue(BulkRing &R, int slot, const BulkRow 
 	mbar_arrive_cp_async(&R.full[slot]);
 }
 
-// Producer of sig_bulk_kernel: one thread (lane 0 of the producer warp); g
-// counts the ring rows issued.  Returns false after a fault.  The copies of
-// an item's in-frame rows differ only by their row offsets, in two classes
+// Rows the producer warp issues at a time, one per lane.  A row's copies take a
+// lane a chain of instructions, which the consumers' share of the issue slots
+// stretches: one row at a time, sig_bulk_kernel took 354 us on 64 ragged frames of
+// 256 to 4096 pixels a side and 47 on 256 of 40 to 200, with four 331 and 38
+// (two: 341 and 39; eight leave too few slots for the next group, 358 and 38, and
+// prep_detect_kernel 300 us for 268).  A lane's slot held the row BK_SLOTS
+// back, which an earlier group issued.
+constexpr int BK_ISSUE = 4;
+static_assert(BK_ISSUE <= BK_SLOTS && BK_ISSUE <= 32, "a lane per row, rows of earlier groups ahead");
+
+// Take the next items' indices from ctl->ticket (whole warp).
+__device__ __forceinline__ int next_ticket(Control *ctl)
+{
+	int t = 0;
+	if ((threadIdx.x & 31) == 0)
+		t = atomicAdd(&ctl->ticket, 1);
+	return __shfl_sync(0xffffffffu, t, 0);
+}
+
+// End of the items: an end marker in ring row g (whole warp).
+__device__ __forceinline__ bool bulk_end(BulkRing &R, int &g)
+{
+	const int slot = g & (BK_SLOTS - 1);
+	if (g >= BK_SLOTS && !mbar_wait_warp(&R.empty[slot], ((g / BK_SLOTS) - 1) & 1, &R.abort))
+		return false;
+	if ((threadIdx.x & 31) == 0) {
+		R.meta[slot] = make_int2(-1, 0);
+		mbar_arrive(&R.full[slot]);
+		mbar_arrive(&R.full[slot]);
+	}
+	++g;
+	return true;
+}
+
+// The producer warp's rows of one item: rows y0 - 1 .. y1 from ring row g on,
+// issue(lane's slot, lane's row, its copies) once the slot is free.  The copies
+// of an item's in-frame rows differ only by their row offsets, in two classes
 // by row parity (the 16-byte phase of a row start alternates when w is odd),
 // so they are computed once per item (kept in `base`, shared memory); rows
 // outside the frame (border-mapped or zero) are computed on their own.
+template <class Issue>
+__device__ __forceinline__ bool bulk_rows(BulkRing &R, int &g, BulkRow (&base)[2], int t, int w, int h, int lm,
+	int mis, int x0, int y0, int y1, Issue issue)
+{
+	const int lane = threadIdx.x & 31;
+	const int ra = y0 - 1 < 0 ? 0 : y0 - 1; // first in-frame row of the item
+	if (lane < 2)
+		base[lane] = bulk_row(w, h, lm, mis, x0, lane && ra + 1 < h ? ra + 1 : ra);
+	__syncwarp();
+	for (int r0 = y0 - 1; r0 <= y1; r0 += BK_ISSUE) {
+		const int r = r0 + lane, d = r - ra;
+		const bool mine = lane < BK_ISSUE && r <= y1;
+		const int q = g + lane, slot = q & (BK_SLOTS - 1);
+		BulkRow b;
+		bool ok = true;
+		if (mine) {
+			b = r < 0 || r >= h ? bulk_row(w, h, lm, mis, x0, r)
+				: shift_row(base[d & 1], (long long)(d & ~1) * w);
+			ok = q < BK_SLOTS || mbar_wait(&R.empty[slot], ((q / BK_SLOTS) - 1) & 1, &R.abort);
+		}
+		if (!__all_sync(0xffffffffu, ok))
+			return false;
+		if (mine) {
+			if (r == y0 - 1)
+				R.meta[slot] = make_int2(t, y1);
+			issue(slot, r, b);
+		}
+		g += min(BK_ISSUE, y1 - r0 + 1);
+	}
+	__syncwarp(); // before the next item's base
+	return true;
+}
+
+// Producer of sig_bulk_kernel (the whole producer warp); g counts the ring rows
+// issued.  Returns false after a fault.
 __device__ __forceinline__ bool bulk_producer(BulkRing &R, const FrameDesc *__restrict__ frames,
 	const FrameState *__restrict__ state, const int4 *__restrict__ items, int nitems, int lm,
 	Control *ctl, int &g, BulkRow (&base)[2])
 {
-	int next = atomicAdd(&ctl->ticket, 1);
+	int next = next_ticket(ctl);
 	for (;;) {
 		// Next active item.
 		int t = -1;
 		while (next < nitems) {
 			const int cand = next;
-			next = atomicAdd(&ctl->ticket, 1);
+			next = next_ticket(ctl);
 			const int4 it = items[cand];
 			if (!state[it.x].active)
 				continue;
@@ -543,37 +612,15 @@ __device__ __forceinline__ bool bulk_producer(BulkRing &R, const FrameDesc *__re
 			t = cand;
 			break;
 		}
-		if (t < 0) { // end of the list: an end marker in the next ring row
-			const int slot = g & (BK_SLOTS - 1);
-			if (g >= BK_SLOTS && !mbar_wait(&R.empty[slot], ((g / BK_SLOTS) - 1) & 1, &R.abort))
-				return false;
-			R.meta[slot] = make_int2(-1, 0);
-			mbar_arrive(&R.full[slot]);
-			mbar_arrive(&R.full[slot]);
-			++g;
-			return true;
-		}
-		const int4 it = items[t];
+		if (t < 0)
+			return bulk_end(R, g);
+		const int4 it = items[t]; // items never cross a 32-row floor block
 		const FrameDesc &fd = frames[it.x];
-		const int w = fd.w, h = fd.h, x0 = it.y, y0 = it.z;
-		const int y1 = it.w; // items never cross a 32-row floor block
 		const double *clean = fd.clean;
 		const int mis = (int)(((uintptr_t)clean >> 3) & 1);
-		const int ra = y0 - 1 < 0 ? 0 : y0 - 1; // first in-frame row of the item
-		base[0] = bulk_row(w, h, lm, mis, x0, ra);
-		base[1] = bulk_row(w, h, lm, mis, x0, ra + 1 < h ? ra + 1 : ra);
-		for (int r = y0 - 1; r <= y1; ++r) {
-			const int slot = g & (BK_SLOTS - 1);
-			const int d = r - ra;
-			const BulkRow b = r < 0 || r >= h ? bulk_row(w, h, lm, mis, x0, r)
-				: shift_row(base[d & 1], (long long)(d & ~1) * w);
-			if (g >= BK_SLOTS && !mbar_wait(&R.empty[slot], ((g / BK_SLOTS) - 1) & 1, &R.abort))
-				return false;
-			if (r == y0 - 1)
-				R.meta[slot] = make_int2(t, y1);
-			bulk_issue(R, slot, b, clean);
-			++g;
-		}
+		if (!bulk_rows(R, g, base, t, fd.w, fd.h, lm, mis, it.y, it.z, it.w,
+			[&](int slot, int, const BulkRow &b) { bulk_issue(R, slot, b, clean); }))
+			return false;
 	}
 }
 
@@ -624,6 +671,23 @@ __device__ __forceinline__ void load_six(const double *row, int c, int shift, do
 	}
 }
 
+// A consumer warp's part of an item whose columns in the frame (w wide) end
+// before the warp's: it frees the ring rows [g, g + n) as they arrive.  (Working
+// through its masked lanes cost sig_bulk_kernel 52 us instead of 47 on 256 frames
+// of 40 to 200 pixels a side and 372 instead of 354 on 64 of 256 to 4096, whose
+// last columns leave warps without work.)
+__device__ __forceinline__ bool bulk_pass_by(BulkRing &R, int g, int n)
+{
+	for (int i = g; i < g + n; ++i) {
+		const int slot = i & (BK_SLOTS - 1);
+		if (!mbar_wait_warp(&R.full[slot], (i / BK_SLOTS) & 1, &R.abort))
+			return false;
+		if ((threadIdx.x & 31) == 0)
+			mbar_arrive(&R.empty[slot]);
+	}
+	return true;
+}
+
 // Consumer warps of sig_bulk_kernel: lane ct of the four warps evaluates
 // columns x0 + 4 ct .. x0 + 4 ct + 3.  Returns false after a fault.
 __device__ __forceinline__ bool bulk_consumer(BulkRing &R, const FrameDesc *__restrict__ frames,
@@ -648,6 +712,15 @@ __device__ __forceinline__ bool bulk_consumer(BulkRing &R, const FrameDesc *__re
 		const int f = it.x, x0 = it.y, y0 = it.z;
 		const FrameDesc &fd = frames[f];
 		const int w = fd.w, x = x0 + 4 * ct;
+		if (x0 + 128 * warp >= w) { // none of the warp's columns
+			ok = bulk_pass_by(R, g, y1 - y0 + 2);
+			if (!ok)
+				break;
+			if (lane == 0)
+				pre_counts[t * BK_CWARPS + warp] = 0;
+			g += y1 - y0 + 2;
+			continue;
+		}
 		// High word of the block threshold per column (all ones: not a pixel).
 		unsigned thr[4];
 		{
@@ -770,8 +843,7 @@ sig_bulk_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restri
 	bool ok;
 	int issued = 0; // ring rows issued (producer warp)
 	if (warp == BK_CWARPS)
-		ok = lane || bulk_producer(R, frames, state, items, nitems, lap_mode(prm.mode), ctl, issued,
-			base);
+		ok = bulk_producer(R, frames, state, items, nitems, lap_mode(prm.mode), ctl, issued, base);
 	else if (warp == 0 && blockIdx.x == 0 && poison > 0)
 		ok = __all_sync(0xffffffffu, poisoned_wait(&R.poison, &R.abort, poison));
 	else

@@ -87,18 +87,18 @@ __device__ __forceinline__ void pd_issue(BulkRing &R, uint8_t (*M)[BK_COLS], int
 	mbar_arrive_cp_async(&R.full[slot]);
 }
 
-// Producer (one thread): bulk_producer over the input rows, plus the mask
+// Producer (the whole warp): bulk_producer over the input rows, plus the mask
 // rows.  Returns false after a fault.
 __device__ __forceinline__ bool pd_producer(BulkRing &R, uint8_t (*M)[BK_COLS],
 	const FrameDesc *__restrict__ frames, const FrameState *state, const int4 *__restrict__ items,
 	int nitems, int lm, Control *ctl, int &g, BulkRow (&base)[2])
 {
-	int next = atomicAdd(&ctl->ticket, 1);
+	int next = next_ticket(ctl);
 	for (;;) {
 		int t = -1;
 		while (next < nitems) {
 			const int cand = next;
-			next = atomicAdd(&ctl->ticket, 1);
+			next = next_ticket(ctl);
 			const int4 it = items[cand];
 			if (!state[it.x].active)
 				continue;
@@ -107,39 +107,20 @@ __device__ __forceinline__ bool pd_producer(BulkRing &R, uint8_t (*M)[BK_COLS],
 			t = cand;
 			break;
 		}
-		if (t < 0) { // end of the list: an end marker in the next ring row
-			const int slot = g & (BK_SLOTS - 1);
-			if (g >= BK_SLOTS && !mbar_wait(&R.empty[slot], ((g / BK_SLOTS) - 1) & 1, &R.abort))
-				return false;
-			R.meta[slot] = make_int2(-1, 0);
-			mbar_arrive(&R.full[slot]);
-			mbar_arrive(&R.full[slot]);
-			++g;
-			return true;
-		}
+		if (t < 0)
+			return bulk_end(R, g);
 		const int4 it = items[t];
 		const FrameDesc &fd = frames[it.x];
-		const int w = fd.w, h = fd.h, x0 = it.y, y0 = it.z, y1 = it.w;
+		const int w = fd.w, x0 = it.y, y0 = it.z, y1 = it.w;
 		const double *data = fd.data;
 		const uint8_t *mask = fd.mask;
 		// Mask bytes of an own row: the item's columns, a multiple of 16.
 		const unsigned mbytes = (unsigned)(w - x0 < BK_COLS ? w - x0 : BK_COLS);
-		const int ra = y0 - 1 < 0 ? 0 : y0 - 1; // first in-frame row of the item
-		base[0] = bulk_row(w, h, lm, 0, x0, ra);
-		base[1] = bulk_row(w, h, lm, 0, x0, ra + 1 < h ? ra + 1 : ra);
-		for (int r = y0 - 1; r <= y1; ++r) {
-			const int slot = g & (BK_SLOTS - 1);
-			const int d = r - ra;
-			const BulkRow b = r < 0 || r >= h ? bulk_row(w, h, lm, 0, x0, r)
-				: shift_row(base[d & 1], (long long)(d & ~1) * w);
-			if (g >= BK_SLOTS && !mbar_wait(&R.empty[slot], ((g / BK_SLOTS) - 1) & 1, &R.abort))
-				return false;
-			if (r == y0 - 1)
-				R.meta[slot] = make_int2(t, y1);
+		if (!bulk_rows(R, g, base, t, w, fd.h, lm, 0, x0, y0, y1, [&](int slot, int r, const BulkRow &b) {
 			const uint8_t *mrow = mask && r >= y0 && r < y1 ? mask + (long long)r * w + x0 : nullptr;
 			pd_issue(R, M, slot, b, data, mrow, mbytes);
-			++g;
-		}
+		}))
+			return false;
 	}
 }
 
@@ -298,6 +279,15 @@ __device__ __forceinline__ bool pd_consumer(BulkRing &R, const uint8_t (*M)[BK_C
 		const int f = it.x, x0 = it.y, y0 = it.z;
 		const FrameDesc &fd = frames[f];
 		const int w = fd.w, x = x0 + 4 * ct;
+		if (x0 + 128 * warp >= w) { // none of the warp's columns
+			ok = bulk_pass_by(R, g, y1 - y0 + 2);
+			if (!ok)
+				break;
+			if (lane == 0)
+				pre_counts[t * BK_CWARPS + warp] = 0;
+			g += y1 - y0 + 2;
+			continue;
+		}
 		const bool valid = x < w;
 		const bool has_mask = fd.mask != nullptr;
 		// High word of the block threshold (all ones: not a pixel).
@@ -475,7 +465,7 @@ prep_detect_kernel(const FrameDesc *__restrict__ frames, FrameState *state, cons
 	bool ok;
 	int issued = 0; // ring rows issued (producer warp)
 	if (warp == BK_CWARPS)
-		ok = lane || pd_producer(R, M, frames, state, items, nitems, lap_mode(prm.mode), ctl, issued, base);
+		ok = pd_producer(R, M, frames, state, items, nitems, lap_mode(prm.mode), ctl, issued, base);
 	else if (warp == 0 && blockIdx.x == 0 && poison > 0)
 		ok = __all_sync(0xffffffffu, poisoned_wait(&R.poison, &R.abort, poison));
 	else
