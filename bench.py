@@ -9,7 +9,7 @@ neighbor_threshold=3, maxiter=4, mirror borders.  The inputs (512 MiB of
 pixels) are larger than the 126 MB L2, so no flush is needed between steps.
 
 * ``value``: Mpix/s with inputs resident in HBM, through a plan whose whole
-  maxiter loop is one CUDA graph (device-side while node), timed with CUDA
+  maxiter loop is one CUDA graph (its early exit on the device), timed with CUDA
   events on the launching stream, max over ranks.
 * ``e2e``: the same metric from host buffers to host buffers through the
   C ABI's batch host entry point ``cusmic_batch_host`` (pinned buffers; every
@@ -65,9 +65,9 @@ SIG_BULK_DRAM_BYTES_PER_PX = 8.62
 # pixels still in L2 at the end of the launch are not counted).
 PREPARE_DRAM_BYTES_PER_PX = 16.48
 # ncu, prep_detect_kernel (prepare with the dense detection), one 16-frame
-# stack launch (this workload): 601.2 MB read + 525.2 MB written over
+# stack launch (this workload): 600.1 MB read + 525.2 MB written over
 # 67.1 Mpix.
-PREP_DETECT_DRAM_BYTES_PER_PX = 16.79
+PREP_DETECT_DRAM_BYTES_PER_PX = 16.77
 REF_GPU_SO = ROOT / "oracle" / "_ref" / "libcusmic_ref.so"
 
 
@@ -378,9 +378,9 @@ def main():
     # over every frame of batches that prep_detect_kernel does not serve (on
     # this stack it is part of prepare; see roofline_sig_bulk_ragged).  Per
     # pixel it reads clean (8 B); its bit planes were zeroed by the call's
-    # prologue memset, and its writes (the sparse pre list) are a few MB.  The
+    # first launch, and its writes (the sparse pre list) are a few MB.  The
     # error map is not read there: its 32 x 32 block floors are computed once
-    # per call by floor_kernel.  Later passes are incremental and do not run it.
+    # per call by floor_kernel.  Later passes work on lists and do not run it.
     roofline_sig_bulk = None
     if not fused:
         active_px = nf * h * w * klaunch["sigraw"]
@@ -407,7 +407,7 @@ def main():
            "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
            "data": "synthetic (seeded scene generator, inputs resident in HBM)",
            "config": dict(workload_config(args), parallelism=f"frames sharded, {world} GPU(s)",
-                          path="plan + CUDA graph (while node)", passes=passes,
+                          path="plan + CUDA graph", passes=passes,
                           repeatable=identical, warmup_executions=warm),
            "roofline": roofline, "roofline_sig_bulk": roofline_sig_bulk, "clocks": clk,
            "gpu_launches": launches_per_step * args.steps}

@@ -33,10 +33,10 @@
 //    exact noise (error map, or the noise model from the pixel's own 5 x 5
 //    median); above cr_threshold -> high candidate list, else above
 //    neighbor_threshold -> low list (src/filters.cuh:125-135), and the same
-//    classes into the HIGH / LOW planes that incremental passes update.  The
+//    classes into the HIGH / LOW planes that late passes update.  The
 //    candidate kernels recompute every value they threshold exactly.
 //
-// sig_bulk_kernel is warp-specialised.  One producer thread copies clean row
+// sig_bulk_kernel is warp-specialised.  A producer warp copies clean row
 // segments (BK_COLS columns plus halo columns) into a ring of BK_SLOTS rows in
 // shared memory: one `cp.async.bulk` for the 16-byte aligned body of a row
 // and up to four single elements with 8-byte `cp.async` (an unaligned first
@@ -497,7 +497,7 @@ __device__ __forceinline__ BulkRow shift_row(BulkRow b, long long by)
 	return b;
 }
 
-// Issue the copies of one ring row (one thread: the bulk copy completes on
+// Issue the copies of one ring row (one lane: the bulk copy completes on
 // the row's full barrier by its transaction bytes, the single-element copies
 // by the thread's cp.async arrival).
 __device__ __forceinline__ void bulk_issue(BulkRing &R, int slot, const BulkRow &b, const double *clean)

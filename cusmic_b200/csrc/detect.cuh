@@ -1245,7 +1245,7 @@ seed_kernel(const FrameDesc *__restrict__ frames, const Seed *__restrict__ seeds
 // a seed gets its fine-structure test from the same warp at once (it needs
 // only its own sig and noise and the clean pixels within 4), so no seed list
 // is walked.  PATH as for candidate_high_kernel (error-map frames use it;
-// noise-model candidates cost more and balance better as two kernels).  With
+// noise-model candidates read the sig_raw map).  With
 // `seeds` (a batch that also runs seed_kernel) each served entry's slot is
 // marked empty.
 template <int PATH>
@@ -1255,7 +1255,7 @@ candidate_seed_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restr
 {
 	// Error-map frames only: the scratch of candidate_sig holds just the 25
 	// values of the NaN rule, and the triples of the seed test serve as it.
-	static_assert(PATH == PATH_ERROR, "noise-model candidates run candidate_high_kernel");
+	static_assert(PATH == PATH_ERROR, "noise-model candidates run candidate_map_kernel");
 	__shared__ double patches[8][81];
 	__shared__ double triples[8][3][63];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -897,15 +897,18 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	const bool model = L.error_frames < nf, thresholds = model && L.total_px > 8u << 20;
 	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, prm, ctl, cands, low, eval,
 		targets, chg, ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
+	mark(rec, K_RECLASS);
 	if (!model)
 		late_classes_kernel<LATE_TESTS, false><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
 	else if (!thresholds)
 		late_classes_kernel<LATE_SHORT, true><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
 	else {
 		late_classes_kernel<LATE_TESTS, true><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
+		mark(rec, K_RECLASS);
 		late_classes_kernel<LATE_MEDIANS, true><<<std::min(wide, di.sms * 2), 256, 0, s>>>(frames, prm, ctl,
 			cands, low, eval);
 	}
+	mark(rec, K_RECLASS);
 	void *args[] = {&frames, &state, &nf, &prm, &ctl, &maxiter, &cands, &low, &eval, &targets, &radius, &chg};
 	check(cudaLaunchCooperativeKernel((const void *)late_passes_kernel, dim3(grid), dim3(LATE_THREADS), args,
 		sizeof(LateShared), s));

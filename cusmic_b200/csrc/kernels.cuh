@@ -934,7 +934,7 @@ fill_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__
 // the output, bit for bit, from the HOLE words (a warp per row).  Writing every
 // mask byte from the CRMASK words took 24 us on 16 frames of 2048 x 2048 and
 // 108 us on 64 ragged frames, whose rows are not aligned; zeroing the masks in
-// the first launch and this take 10 + 6 and 26 + 9 us.
+// the first launch and this take 6 + 14 and 31 + 26 us.
 __global__ void __launch_bounds__(256)
 finish_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
 	const int2 *__restrict__ rows, int nrows, const uint2 *__restrict__ targets,

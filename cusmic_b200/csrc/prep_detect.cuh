@@ -21,7 +21,7 @@
 // working pixels (the same values, the same operations), so the lists, and
 // everything after them, are those of the two-kernel path.
 //
-// The block layout is sig_bulk_kernel's: one producer thread streams the
+// The block layout is sig_bulk_kernel's: a producer warp streams the
 // item's rows (BK_COLS columns plus halo columns, border-mapped rows and
 // columns for the Laplacian) of the input into the ring by bulk copies, and
 // for the item's own rows the mask bytes of its columns into a second ring;
@@ -31,11 +31,12 @@
 // words of the warp's 128 columns are assembled from the lanes' 4-bit groups
 // by shuffles.  Per-frame facts are added once per item and warp.
 //
-// Issue slots bound it (410 warp instructions per 128 pixels, a fifth of them
-// branches and their joins; DRAM at a third of its rate).  One test per row for
-// a value that is not finite, by the largest of the six high words, votes
-// instead of divergent waits, and predicated stores and arrivals left 366: 16
-// frames of 2048 x 2048 290 -> 268 us, two of 8192 x 8192 488 -> 436.
+// A warp's chain of instructions per row bounds it: 410 for 128 pixels, a fifth
+// of them branches and their joins, at 18 resident warps per SM, half of the
+// issue slots and a third of DRAM's rate used.  One test per row for a value that
+// is not finite, by the largest of the six high words, votes instead of
+// divergent waits, and predicated stores and arrivals left 328: 16 frames of
+// 2048 x 2048 290 -> 268 us, two of 8192 x 8192 488 -> 436.
 //
 // The block floors of error maps depend on the maps only, so they are computed
 // before this kernel (prep_init_kernel, with the call's state and zeroing);

@@ -8,7 +8,7 @@
 // each evaluated separately.  region_sig_kernel therefore evaluates sig_raw
 // and the noise once at every pixel within two of a HIGH pixel (the union of
 // the windows of every high-list candidate, whose classes classify_kernel
-// wrote into the HIGH plane) and stores both; candidate_high_kernel then
+// wrote into the HIGH plane) and stores both; candidate_map_kernel then
 // reads its window from the map.  The values are computed by the same
 // functions the candidate kernel uses on its border path (noise_model_at,
 // lap_at), so they are the same bits.

@@ -4,7 +4,7 @@
 calibration maps, per-frame scalars and the output buffers, and builds the
 ``cusmic_image`` descriptors.  ``Plan`` wraps ``cusmic_plan_*``: one
 workspace, descriptors uploaded once, and (``graph=True``) the whole cleaning
-captured as a CUDA graph whose maxiter loop is a device-driven while node.
+captured as a CUDA graph whose maxiter loop ends early on the device.
 """
 
 import ctypes

@@ -9,8 +9,8 @@
  *   - ragged batches with per-frame scalar gain / read noise / background,
  *     run as one persistent launch over a tile work list;
  *   - plans: a workspace, tile list and captured CUDA graph of the whole
- *     maxiter loop (with its early exit as a device-side while node), reused
- *     across executions;
+ *     maxiter loop (its early exit is taken on the device), reused across
+ *     executions;
  *   - the adjoint of the cleaned pixels with the detection mask frozen.
  *
  * All pointers of a call belong to the caller's current device.  Status codes
@@ -128,12 +128,13 @@ cusmic_plan_passes(cusmic_plan *plan, int *passes);
 /* Execute the plan once without its graph, with a CUDA event recorded on
  * stream after every kernel, then synchronise.  ms[k] and launches[k] receive
  * the summed duration and launch count of kernel kind k for k in 0..15:
- * init (with the zeroing of the bit planes), prepare, hole fill, sig_raw
- * (dense detection), candidates (5 x 5 medians), seeds (fine structure),
- * grow/update, control, replace, restore, zero-iteration copy, low
- * candidates, classification of the dense pass's list, block floors, and of
- * the incremental passes the reclassification with work-list gather and the
- * dirty-row scan.  A batch whose frames all have an error map and no
+ * init (with the zeroing of the bit planes and masks), prepare, hole fill,
+ * sig_raw (dense detection), and of the first pass candidates (5 x 5 medians),
+ * seeds (fine structure), low candidates with the growth (grow) and the
+ * replacement; restore (the finish from lists), zero-iteration copy,
+ * classification of the dense pass's list, block floors, the later passes
+ * (reclass) and the sig_raw map.  Control, low and dirty have no launch of their
+ * own any more.  A batch whose frames all have an error map and no
  * background, widths that are multiples of 16 and 16-byte aligned buffers
  * runs prepare and the first pass's dense detection as one kernel, reported
  * under prepare (no sig_raw launch).  A timing aid; no counterpart in the
