@@ -123,6 +123,68 @@ __device__ long long donor_at_rank_large(const FrameDesc &fd, const uint32_t *do
 	return -1; // unreachable when rank < donor count
 }
 
+// Both central donors of a window of 33 .. 32 S cells: lane l holds the keys of
+// cells l + 32 s, the warp sorts a copy, and a rank's donor is the
+// (rank - less)-th one with the sorted key, in cell (= linear index) order.
+// Returns the number of donors (0: d_lo and d_hi unset).
+//
+// (donor_at_rank_large reads the window 64 times, bit by bit, for each rank: a
+// few clusters of flagged pixels held the launch for 49 us on eight frames of
+// 1024 x 1024, 18 with the sort.)
+template <int S>
+__device__ __noinline__ int sorted_window_donors(const FrameDesc &fd, const uint32_t *don,
+	const uint32_t *crm, Window win, long long &d_lo, long long &d_hi)
+{
+	const int lane = threadIdx.x & 31;
+	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
+	unsigned long long own[S], k[S];
+	int nd = 0;
+#pragma unroll
+	for (int s = 0; s < S; ++s) {
+		const int pos = lane + 32 * s;
+		own[s] = ~0ull;
+		if (pos < area) {
+			const int x = win.x0 + pos % ww, y = win.y0 + pos / ww;
+			if (donor_at(don, crm, fd.words, x, y))
+				own[s] = order_key(donor_value(fd, (long long)y * fd.w + x));
+		}
+		k[s] = own[s];
+		nd += __popc(__ballot_sync(0xffffffffu, own[s] != ~0ull));
+	}
+	if (!nd)
+		return 0;
+	sort_keys(k);
+	auto donor = [&](int rank) {
+		unsigned long long v = 0;
+#pragma unroll
+		for (int s = 0; s < S; ++s)
+			if (s == rank >> 5)
+				v = k[s];
+		v = __shfl_sync(0xffffffffu, v, rank & 31);
+		int skip = rank;
+#pragma unroll
+		for (int s = 0; s < S; ++s)
+			skip -= __popc(__ballot_sync(0xffffffffu, own[s] < v));
+		int pos = -1; // warp-uniform
+#pragma unroll
+		for (int s = 0; s < S; ++s) {
+			unsigned m = __ballot_sync(0xffffffffu, own[s] == v);
+			const int c = __popc(m);
+			if (pos < 0 && skip < c) {
+				for (; skip > 0; --skip)
+					m &= m - 1;
+				pos = 32 * s + __ffs(m) - 1;
+			} else if (pos < 0) {
+				skip -= c;
+			}
+		}
+		return (long long)(win.y0 + pos / ww) * fd.w + win.x0 + pos % ww;
+	};
+	d_lo = donor((nd - 1) / 2);
+	d_hi = nd % 2 ? d_lo : donor(nd / 2);
+	return nd;
+}
+
 // One warp per flagged pixel: recompute its final replacement window and
 // donors, scatter w * g to the selected donor(s).
 __global__ void __launch_bounds__(256)
@@ -164,6 +226,11 @@ bwd_scatter_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restrict
 					continue;
 				d_lo = donor_at_rank32(key, idx, (nd - 1) / 2);
 				d_hi = nd % 2 ? d_lo : donor_at_rank32(key, idx, nd / 2);
+			} else if (area <= 128) {
+				nd = area <= 64 ? sorted_window_donors<2>(fd, don, crm, win, d_lo, d_hi)
+					: sorted_window_donors<4>(fd, don, crm, win, d_lo, d_hi);
+				if (!nd)
+					continue;
 			} else {
 				int cnt = 0;
 				for (int pos = lane; pos < area; pos += 32)

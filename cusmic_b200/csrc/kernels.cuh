@@ -501,6 +501,41 @@ __device__ double select_rank(const FrameDesc &fd, const uint32_t *don, const ui
 	return order_value(prefix);
 }
 
+// The warp's 32 S keys in ascending unsigned order, by a bitonic network:
+// element i = 32 s + lane in slot s of the lane.
+template <int S>
+__device__ __forceinline__ void sort_keys(unsigned long long (&k)[S])
+{
+	const int lane = threadIdx.x & 31;
+	// Ascending where bit `size` of i is clear.
+#pragma unroll
+	for (int size = 2; size <= 32 * S; size <<= 1) {
+#pragma unroll
+		for (int j = size >> 1; j > 0; j >>= 1) {
+			if (j >= 32) { // partner in the same lane, slot s ^ (j / 32)
+#pragma unroll
+				for (int s = 0; s < S; ++s) {
+					const int t = s ^ (j >> 5);
+					if (t < s)
+						continue;
+					const bool asc = ((32 * s + lane) & size) == 0;
+					const unsigned long long a = k[s], b = k[t];
+					const bool swap = asc ? b < a : a < b;
+					k[s] = swap ? b : a;
+					k[t] = swap ? a : b;
+				}
+			} else { // partner lane ^ j, same slot
+#pragma unroll
+				for (int s = 0; s < S; ++s) {
+					const unsigned long long p = __shfl_xor_sync(0xffffffffu, k[s], j);
+					const bool keep_min = ((lane & j) == 0) == (((32 * s + lane) & size) == 0);
+					k[s] = keep_min ? (p < k[s] ? p : k[s]) : (k[s] < p ? p : k[s]);
+				}
+			}
+		}
+	}
+}
+
 // The donors of a window of 33 .. 32 S cells in key order, for the median:
 // lane l holds the keys of cells l + 32 s (all ones for a non-donor or a cell
 // past the window, which sort last), a bitonic network sorts the warp's 32 S
@@ -531,33 +566,7 @@ __device__ __noinline__ int sorted_window_median(const FrameDesc &fd, const uint
 	}
 	if (!nd)
 		return 0;
-	// Element i = 32 s + lane; ascending where bit `size` of i is clear.
-#pragma unroll
-	for (int size = 2; size <= 32 * S; size <<= 1) {
-#pragma unroll
-		for (int j = size >> 1; j > 0; j >>= 1) {
-			if (j >= 32) { // partner in the same lane, slot s ^ (j / 32)
-#pragma unroll
-				for (int s = 0; s < S; ++s) {
-					const int t = s ^ (j >> 5);
-					if (t < s)
-						continue;
-					const bool asc = ((32 * s + lane) & size) == 0;
-					const unsigned long long a = k[s], b = k[t];
-					const bool swap = asc ? b < a : a < b;
-					k[s] = swap ? b : a;
-					k[t] = swap ? a : b;
-				}
-			} else { // partner lane ^ j, same slot
-#pragma unroll
-				for (int s = 0; s < S; ++s) {
-					const unsigned long long p = __shfl_xor_sync(0xffffffffu, k[s], j);
-					const bool keep_min = ((lane & j) == 0) == (((32 * s + lane) & size) == 0);
-					k[s] = keep_min ? (p < k[s] ? p : k[s]) : (k[s] < p ? p : k[s]);
-				}
-			}
-		}
-	}
+	sort_keys(k);
 	const int rl = (nd - 1) / 2, rh = nd / 2;
 	unsigned long long vl = 0, vh = 0;
 #pragma unroll

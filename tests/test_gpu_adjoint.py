@@ -253,3 +253,42 @@ def test_autograd_reuses_plans(cuda):
     x.grad = None
     (w * clean).sum().backward()  # a second backward of the kept graph
     assert torch.allclose(x.grad, g_kept, rtol=1e-13, atol=1e-13)
+
+
+@pytest.mark.parametrize("radius", (1, 2, 3, 4, 5, 6))
+@pytest.mark.parametrize("bg_kind", ("none", "map"))
+def test_backward_windows_by_size(cuda, oracle, bg_kind, radius):
+    """Hits inside excluded squares of every radius whose replacement window
+    grows to the square's rim (49, 81 and 121 cells are sorted by the warp, 25
+    before and 169 after are not), at the frame's edges and corners too; small
+    integers, so many donors tie and the lowest index decides."""
+    torch = cuda
+    from cusmic_b200.plan import Batch, Plan
+    rng = np.random.default_rng(radius)
+    h, w = 75, 90
+    data = 100.0 + rng.integers(0, 4, (h, w))
+    mask = np.zeros((h, w), dtype=bool)
+    step = 2 * radius + 7
+    hits = [(y, x) for y in range(0, h, step) for x in range(0, w, step)] + [(h - 1, w - 1)]
+    for y, x in hits:
+        mask[max(0, y - radius):y + radius + 1, max(0, x - radius):x + radius + 1] = True
+    for y, x in hits:
+        mask[y, x] = False
+        data[y, x] += 5000
+    bg = rng.integers(0, 3, (h, w)).astype(float) if bg_kind == "map" else None
+    error = np.full((h, w), 5.0)
+    up = lambda a: None if a is None else torch.from_numpy(a).cuda()
+    batch = Batch.stack(up(data[None]), error=up(error), mask=up(mask), background=up(bg))
+    plan = Plan(batch, graph=False, keep=True)
+    plan.execute()
+    plan.wait()
+    g = rng.normal(size=(1, h, w))
+    gx, gbg = plan.backward(up(g))
+    _, want_mask, _ = oracle.clean_frame(data, error=error, mask=mask, background=bg)
+    np.testing.assert_array_equal(batch.mask_out[0].cpu().numpy().astype(bool), want_mask)
+    assert want_mask[tuple(np.transpose(hits))].mean() > 0.5
+    rgx, rmap, _ = oracle.backward(data, want_mask, g[0], mask=mask, background=bg)
+    np.testing.assert_allclose(gx[0].cpu().numpy(), rgx, rtol=1e-13, atol=1e-13)
+    if bg is not None:
+        np.testing.assert_allclose(gbg[0].cpu().numpy(), rmap, rtol=1e-13, atol=1e-13)
+    plan.close()
