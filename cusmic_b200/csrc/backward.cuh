@@ -15,6 +15,12 @@
 
 namespace cb {
 
+// Words of 32 pixels whose loads a warp of bwd_dense_kernel issues before their
+// use (memory bounds it; three frames of 777 x 900 with a background map: 24 us
+// one word at a time, 13.5 with 4, 11 with 8, as with 16; eight of 1024 x 1024: 29
+// and 26).
+constexpr int BWD_WORDS = 8;
+
 // Pass-through part: grad_data = g off the mask, 0 on it; with background
 // maps, grad_bg = -g on the mask and 0 elsewhere.
 __global__ void __launch_bounds__(256)
@@ -29,12 +35,28 @@ bwd_dense_kernel(const FrameDesc *__restrict__ frames, const int2 *__restrict__ 
 		const FrameDesc &fd = frames[item.x];
 		const uint32_t *crm = plane_ptr(fd, P_CRMASK) + (long long)item.y * fd.words;
 		const long long base = offsets[item.x] + (long long)item.y * fd.w;
-		for (int x = lane; x < fd.w; x += 32) {
-			const bool flagged = (crm[x >> 5] >> (x & 31)) & 1u;
-			const double gi = g[base + x];
-			gx[base + x] = flagged ? 0.0 : gi;
-			if (gbg_map)
-				gbg_map[base + x] = flagged ? -gi : 0.0;
+		const int w = fd.w;
+		for (int xb = 0; xb < w; xb += 32 * BWD_WORDS) {
+			double gi[BWD_WORDS];
+			uint32_t cw[BWD_WORDS];
+#pragma unroll
+			for (int u = 0; u < BWD_WORDS; ++u) {
+				const int x = xb + 32 * u + lane;
+				if (x < w) {
+					gi[u] = g[base + x];
+					cw[u] = crm[x >> 5];
+				}
+			}
+#pragma unroll
+			for (int u = 0; u < BWD_WORDS; ++u) {
+				const int x = xb + 32 * u + lane;
+				if (x < w) {
+					const bool flagged = (cw[u] >> lane) & 1u;
+					gx[base + x] = flagged ? 0.0 : gi[u];
+					if (gbg_map)
+						gbg_map[base + x] = flagged ? -gi[u] : 0.0;
+				}
+			}
 		}
 	}
 }
