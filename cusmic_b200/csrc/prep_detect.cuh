@@ -189,7 +189,7 @@ __device__ __forceinline__ void store4(const PdOwn &own, const double (&c)[4])
 		     " @w st.global.v4.f64 [%1], {%2, %3, %4, %5};\n"
 		     " @n st.global.v2.f64 [%1], {%2, %3};\n"
 		     " @n st.global.v2.f64 [%1 + 16], {%4, %5};\n}\n"
-		::"r"(own.store), "l"(own.clean), "d"(c[0]), "d"(c[1]), "d"(c[2]), "d"(c[3])
+		::"r"(own.store), "l"(__cvta_generic_to_global(own.clean)), "d"(c[0]), "d"(c[1]), "d"(c[2]), "d"(c[3])
 		: "memory");
 }
 

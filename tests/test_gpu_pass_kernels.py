@@ -232,3 +232,33 @@ def test_long_late_lists(cuda, mode):
         want_clean, want_mask = one.outputs()[0]
         np.testing.assert_array_equal(mask, want_mask)
         assert_bits_equal(clean, want_clean)
+
+
+@pytest.mark.parametrize("offset", (0, 2, 4))
+@pytest.mark.parametrize("width", (16, 112, 128, 144, 272, 528, 656))
+@pytest.mark.parametrize("noise", ("error", "model"))
+def test_dense_columns_and_alignment(cuda, oracle, noise, width, offset):
+    """Widths at which some of the dense kernels' warps have no column of their
+    512-column items, and output buffers at 16- and 32-byte boundaries (one
+    store or two per lane); 37 rows leave items of 32 and 5."""
+    h = 37
+    data = structured(width, h, width, hits=80)
+    rng = np.random.default_rng(width)
+    data[rng.random((h, width)) < 0.01] = np.nan
+    frame = dict(data=data, mask=rng.random((h, width)) < 0.01)
+    kw = dict(SETTINGS)
+    if noise == "error":
+        frame["error"] = np.full((h, width), 12.0)
+    else:
+        frame.update(gain=1.5, readnoise=3.0)
+        kw.update(gain=1.5, readnoise=3.0)
+    fr = cabi.Frames([frame])
+    whole = fr.clean.new_empty(fr.total + offset)
+    fr.clean = whole[offset:]
+    st, msg = cabi.run_ragged(fr, cabi.options(**kw))
+    assert st == 0, msg
+    settings = {k: v for k, v in kw.items() if k not in ("gain", "readnoise")}
+    want_clean, want_mask, _ = cabi.oracle_frame(oracle, frame, **settings)
+    clean, mask = fr.outputs()[0]
+    np.testing.assert_array_equal(mask, want_mask)
+    assert_bits_equal(clean, want_clean)
