@@ -369,7 +369,7 @@ struct Layout {
 	std::vector<FrameDesc> frames;
 	std::vector<long long> bit_off; // word offset of each frame within a plane
 	std::vector<int4> bulk;   // sig_bulk_kernel items {frame, x0, y0, first threshold of the frame}
-	std::vector<int4> grow;   // region_list_kernel items {frame, y0, first word, y1}
+	std::vector<int4> region; // region_list_kernel items {frame, y0, first word, y1}
 	std::vector<FloorJob> jobs; // floor blocks of each distinct error map and noise-model frame
 	std::vector<long long> thr_base; // per frame: first floor of its blocks
 	long long nthr = 0;
@@ -421,7 +421,7 @@ struct Workspace {
 	DevBuf<unsigned char> desc;
 	DevPart<FrameDesc> frames;
 	DevPart<int2> rows;
-	DevPart<int4> bulk, grow;
+	DevPart<int4> bulk, region;
 	DevPart<FloorJob> jobs;
 	DevPart<long long> offsets;
 	DevBuf<FrameState> state;
@@ -590,6 +590,7 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 	for (size_t f = 0; f < nf; ++f)
 		all_px += ims[f].width * ims[f].height;
 	const cusmic_tuning tune = tuning_for(all_px);
+	const int list_rows = region_rows(all_px);
 	const int rows_per_item = tune.dense_rows ? tune.dense_rows
 		: item_rows(ims, nf, di.sms * tune.dense_blocks_per_sm);
 	Layout L;
@@ -662,9 +663,9 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 		for (int ty = 0; ty < d.h; ty += rows_per_item)
 			for (int tx = 0; tx < d.w; tx += BK_COLS)
 				L.bulk.push_back(make_int4((int)f, tx, ty, std::min(ty + rows_per_item, d.h)));
-		for (int ty = 0; ty < d.h; ty += GROW_ROWS)
+		for (int ty = 0; !d.error && ty < d.h; ty += list_rows)
 			for (int k0 = 0; k0 < d.words; k0 += 32)
-				L.grow.push_back(make_int4((int)f, ty, k0, std::min(ty + GROW_ROWS, d.h)));
+				L.region.push_back(make_int4((int)f, ty, k0, std::min(ty + list_rows, d.h)));
 	}
 	L.total_px = px;
 	choose_kernels(L);
@@ -745,7 +746,7 @@ static void upload(Workspace &ws, Layout &L, cudaStream_t s, bool mapped = false
 		return at;
 	};
 	const size_t at_frames = place(nf * sizeof(FrameDesc)), at_rows = place(L.rows.size() * sizeof(int2)),
-		at_bulk = place(L.bulk.size() * sizeof(int4)), at_grow = place(L.grow.size() * sizeof(int4)),
+		at_bulk = place(L.bulk.size() * sizeof(int4)), at_region = place(L.region.size() * sizeof(int4)),
 		at_jobs = place(L.jobs.size() * sizeof(FloorJob)), at_offsets = place(nf * sizeof(long long));
 	ws.desc.ensure(total);
 	ws.stage.ensure(total);
@@ -756,7 +757,7 @@ static void upload(Workspace &ws, Layout &L, cudaStream_t s, bool mapped = false
 	put(ws.frames, at_frames, L.frames);
 	put(ws.rows, at_rows, L.rows);
 	put(ws.bulk, at_bulk, L.bulk);
-	put(ws.grow, at_grow, L.grow);
+	put(ws.region, at_region, L.region);
 	put(ws.jobs, at_jobs, L.jobs);
 	put(ws.offsets, at_offsets, L.offsets);
 	if (!mapped) {
@@ -837,9 +838,10 @@ static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	// their windows from the sig_raw map, and seed_kernel tests their seeds.
 	const bool model = L.error_frames < nf;
 	if (model) {
-		const int ng = (int)L.grow.size(), need = (ng + 7) / 8, gcap = di.sms * 8;
-		region_list_kernel<<<need < gcap ? need : gcap, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.grow.p,
-			ng, ws.ctl.p, ws.targets.p);
+		const int ng = (int)L.region.size(), need = (ng + 7) / 8, gcap = di.sms * 8;
+		auto list = region_rows(L.total_px) == 8 ? region_list_kernel<8> : region_list_kernel<4>;
+		list<<<need < gcap ? need : gcap, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.region.p, ng,
+			ws.ctl.p, ws.targets.p);
 		region_sig_kernel<<<di.sms * 8, 256, 0, s>>>(ws.frames.p, ws.targets.p, ws.ctl.p, L.prm);
 		mark(rec, K_SIGMAP);
 	}

@@ -402,9 +402,6 @@ prepare_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const in
 	}
 }
 
-// Rows of an item of region_list_kernel.
-constexpr int GROW_ROWS = 16;
-
 // Reference src/replace.cuh:50-56.
 __device__ __forceinline__ double midpoint(double lo, double hi)
 {

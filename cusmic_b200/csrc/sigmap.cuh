@@ -14,7 +14,7 @@
 // lap_at), so they are the same bits.
 //
 // Two launches: region_list_kernel lists the map's pixels (one warp per
-// growth item of GROW_ROWS rows x 32 bit words, a lane per word: a 5 x 5
+// item of ROWS rows x 32 bit words, a lane per word: a 5 x 5
 // dilation of the HIGH plane on bit words, one list append per item), then
 // region_sig_kernel evaluates one listed pixel per thread.  Within an item the
 // list runs row by row, so neighbouring threads hold neighbouring pixels and
@@ -49,6 +49,16 @@ __device__ __forceinline__ unsigned long long nc_window(const uint32_t *plane, i
 	return (l >> 30) | (c << 2) | ((r & 3ull) << 34);
 }
 
+// Rows of an item: a warp's chain grows with them (16 rows: 14 us on one 512 x 512
+// frame and 21 on five of 1018 x 1001, 8 rows 9.5 and 13, 4 rows 6.4 and 8); on
+// large batches, where the loads count, 4 rows read twice their rows (64 ragged
+// frames, 178 Mpixel: 79, 66 and 73 us).
+CB_HD int region_rows(size_t total_px)
+{
+	return total_px > (32u << 20) ? 8 : 4;
+}
+
+template <int ROWS>
 __global__ void __launch_bounds__(256)
 region_list_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ state,
 	const int4 *__restrict__ items, int nitems, Control *ctl, uint2 *list)
@@ -67,17 +77,17 @@ region_list_kernel(const FrameDesc *__restrict__ frames, const FrameState *__res
 		const uint32_t *hp = plane_ptr(fd, P_HIGH);
 		// The word's valid pixel bits (the dilation spreads past the row end).
 		const uint32_t clip = k >= words ? 0u : 32 * k + 32 <= w ? 0xffffffffu : (1u << (w - 32 * k)) - 1u;
-		unsigned long long d[GROW_ROWS + 4];
+		unsigned long long d[ROWS + 4];
 #pragma unroll
-		for (int r = 0; r < GROW_ROWS + 4; ++r) // loads only: one round trip
+		for (int r = 0; r < ROWS + 4; ++r) // loads only: one round trip
 			d[r] = r < n + 4 ? nc_window(hp, words, h, y0 - 2 + r, k) : 0ull;
 #pragma unroll
-		for (int r = 0; r < GROW_ROWS + 4; ++r)
+		for (int r = 0; r < ROWS + 4; ++r)
 			d[r] = dilate_row2(d[r]);
-		uint32_t need[GROW_ROWS];
+		uint32_t need[ROWS];
 		int cnt = 0;
 #pragma unroll
-		for (int j = 0; j < GROW_ROWS; ++j) {
+		for (int j = 0; j < ROWS; ++j) {
 			need[j] = j < n ? (uint32_t)((d[j] | d[j + 1] | d[j + 2] | d[j + 3] | d[j + 4]) >> 2) & clip : 0u;
 			cnt += __popc(need[j]);
 		}
@@ -85,9 +95,9 @@ region_list_kernel(const FrameDesc *__restrict__ frames, const FrameState *__res
 			continue;
 		// Row-major order within the item: row j's pixels of every lane, then
 		// row j + 1's.
-		int row_off[GROW_ROWS], total = 0;
+		int row_off[ROWS], total = 0;
 #pragma unroll
-		for (int j = 0; j < GROW_ROWS; ++j) {
+		for (int j = 0; j < ROWS; ++j) {
 			const int c = __popc(need[j]), o = warp_exclusive_count(c);
 			row_off[j] = total + o;
 			total += __shfl_sync(0xffffffffu, o + c, 31);
@@ -97,7 +107,7 @@ region_list_kernel(const FrameDesc *__restrict__ frames, const FrameState *__res
 			base = atomicAdd(&ctl->n_region, (unsigned long long)total);
 		base = __shfl_sync(0xffffffffu, base, 0);
 #pragma unroll
-		for (int j = 0; j < GROW_ROWS; ++j) {
+		for (int j = 0; j < ROWS; ++j) {
 			unsigned long long at = base + row_off[j];
 			const unsigned rowpix = (unsigned)((long long)(y0 + j) * w + 32 * k);
 			for (uint32_t b = need[j]; b; b &= b - 1)

@@ -262,3 +262,29 @@ def test_dense_columns_and_alignment(cuda, oracle, noise, width, offset):
     clean, mask = fr.outputs()[0]
     np.testing.assert_array_equal(mask, want_mask)
     assert_bits_equal(clean, want_clean)
+
+
+def test_large_map_lists(cuda):
+    """A batch above 32 Mpixel lists the sig_raw map's pixels in items of eight
+    rows; the same frames one at a time in items of four."""
+    rng = np.random.default_rng(3)
+    frames = []
+    for i in range(9):
+        h, w = 1999 + i, 2001 - i
+        data = 200 + rng.normal(0, 12, (h, w))
+        hit = rng.random((h, w)) < 2e-3
+        data[hit] += rng.uniform(100, 4000, int(hit.sum()))
+        frames.append(dict(data=data, gain=1.5, readnoise=3.0))
+    assert sum(f["data"].size for f in frames) > 32 << 20
+    opts = cabi.options(**SETTINGS, gain=1.5, readnoise=3.0)
+    fr = cabi.Frames(frames)
+    st, msg = cabi.run_ragged(fr, opts)
+    assert st == 0, msg
+    for frame, (clean, mask) in zip(frames, fr.outputs()):
+        one = cabi.Frames([frame])
+        st, msg = cabi.run_ragged(one, opts)
+        assert st == 0, msg
+        want_clean, want_mask = one.outputs()[0]
+        assert want_mask.any()
+        np.testing.assert_array_equal(mask, want_mask)
+        assert_bits_equal(clean, want_clean)
