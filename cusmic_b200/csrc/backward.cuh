@@ -94,79 +94,28 @@ __device__ __forceinline__ int donor_at_rank32(unsigned long long key, int idx, 
 	return __shfl_sync(0xffffffffu, idx, __ffs(same) - 1);
 }
 
-// Same for windows larger than 32 cells: radix select of the key, then the
-// (rank - less)-th donor with that key in row-major (= linear index) order.
-__device__ long long donor_at_rank_large(const FrameDesc &fd, const uint32_t *don,
-	const uint32_t *crm, Window win, int rank)
-{
-	const int lane = threadIdx.x & 31;
-	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
-	unsigned long long prefix = 0, used = 0;
-	int r = rank;
-	for (int bit = 63; bit >= 0; --bit) {
-		const unsigned long long flag = 1ull << bit;
-		int below = 0;
-		for (int pos = lane; pos < area; pos += 32) {
-			int x = win.x0 + pos % ww, y = win.y0 + pos / ww;
-			if (!donor_at(don, crm, fd.words, x, y))
-				continue;
-			unsigned long long k = order_key(donor_value(fd, (long long)y * fd.w + x));
-			below += (k & used) == prefix && !(k & flag);
-		}
-		below = warp_sum_int(below);
-		used |= flag;
-		if (r >= below) {
-			prefix |= flag;
-			r -= below;
-		}
-	}
-	// r is now the number of equal keys to skip in row-major order.
-	for (int pos0 = 0; pos0 < area; pos0 += 32) {
-		const int pos = pos0 + lane;
-		bool match = false;
-		int x = 0, y = 0;
-		if (pos < area) {
-			x = win.x0 + pos % ww;
-			y = win.y0 + pos / ww;
-			match = donor_at(don, crm, fd.words, x, y) &&
-				order_key(donor_value(fd, (long long)y * fd.w + x)) == prefix;
-		}
-		unsigned m = __ballot_sync(0xffffffffu, match);
-		int c = __popc(m);
-		if (r < c) {
-			for (int t = r; t > 0; --t)
-				m &= m - 1;
-			int src = __ffs(m) - 1;
-			int sx = __shfl_sync(0xffffffffu, x, src), sy = __shfl_sync(0xffffffffu, y, src);
-			return (long long)sy * fd.w + sx;
-		}
-		r -= c;
-	}
-	return -1; // unreachable when rank < donor count
-}
-
-// Both central donors of a window of 33 .. 32 S cells: lane l holds the keys of
-// cells l + 32 s, the warp sorts a copy, and a rank's donor is the
-// (rank - less)-th one with the sorted key, in cell (= linear index) order.
-// Returns the number of donors (0: d_lo and d_hi unset).
+// Both central donors of up to 32 S cells in row-major order (cell(pos, x, y) for
+// pos < n): lane l holds the keys of cells l + 32 s, the warp sorts a copy, and a
+// rank's donor is the (rank - less)-th one with the sorted key, in cell (= linear
+// index) order.  Returns the number of donors (0: d_lo and d_hi unset).
 //
-// (donor_at_rank_large reads the window 64 times, bit by bit, for each rank: a
+// (A radix select reads the window 64 times, bit by bit, for each rank: a
 // few clusters of flagged pixels held the launch for 49 us on eight frames of
 // 1024 x 1024, 18 with the sort.)
-template <int S>
-__device__ __noinline__ int sorted_window_donors(const FrameDesc &fd, const uint32_t *don,
-	const uint32_t *crm, Window win, long long &d_lo, long long &d_hi)
+template <int S, class Cell>
+__device__ __forceinline__ int sorted_donors(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
+	int n, Cell cell, long long &d_lo, long long &d_hi)
 {
 	const int lane = threadIdx.x & 31;
-	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
 	unsigned long long own[S], k[S];
 	int nd = 0;
 #pragma unroll
 	for (int s = 0; s < S; ++s) {
 		const int pos = lane + 32 * s;
 		own[s] = ~0ull;
-		if (pos < area) {
-			const int x = win.x0 + pos % ww, y = win.y0 + pos / ww;
+		if (pos < n) {
+			int x, y;
+			cell(pos, x, y);
 			if (donor_at(don, crm, fd.words, x, y))
 				own[s] = order_key(donor_value(fd, (long long)y * fd.w + x));
 		}
@@ -200,11 +149,101 @@ __device__ __noinline__ int sorted_window_donors(const FrameDesc &fd, const uint
 				skip -= c;
 			}
 		}
-		return (long long)(win.y0 + pos / ww) * fd.w + win.x0 + pos % ww;
+		int x, y;
+		cell(pos, x, y);
+		return (long long)y * fd.w + x;
 	};
 	d_lo = donor((nd - 1) / 2);
 	d_hi = nd % 2 ? d_lo : donor(nd / 2);
 	return nd;
+}
+
+// A window of 33 .. 32 S cells.
+template <int S>
+__device__ __noinline__ int sorted_window_donors(const FrameDesc &fd, const uint32_t *don,
+	const uint32_t *crm, Window win, long long &d_lo, long long &d_hi)
+{
+	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
+	return sorted_donors<S>(fd, don, crm, area, [&](int pos, int &x, int &y) {
+		x = win.x0 + pos % ww;
+		y = win.y0 + pos / ww;
+	}, d_lo, d_hi);
+}
+
+// Linear index of the donor at `rank` in (key, linear index) order among a
+// ring's cells: radix select of the key, then the (rank - less)-th donor with
+// that key in row-major (= linear index) order.
+__device__ long long ring_donor(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
+	const Ring &q, int rank)
+{
+	const int lane = threadIdx.x & 31;
+	unsigned long long prefix = 0, used = 0;
+	int r = rank;
+	for (int bit = 63; bit >= 0; --bit) {
+		const unsigned long long flag = 1ull << bit;
+		int below = 0;
+		for (int pos = lane; pos < q.n; pos += 32) {
+			int x, y;
+			ring_cell(q, pos, x, y);
+			if (!donor_at(don, crm, fd.words, x, y))
+				continue;
+			unsigned long long k = order_key(donor_value(fd, (long long)y * fd.w + x));
+			below += (k & used) == prefix && !(k & flag);
+		}
+		below = warp_sum_int(below);
+		used |= flag;
+		if (r >= below) {
+			prefix |= flag;
+			r -= below;
+		}
+	}
+	// r is now the number of equal keys to skip in row-major order.
+	for (int pos0 = 0; pos0 < q.n; pos0 += 32) {
+		const int pos = pos0 + lane;
+		bool match = false;
+		int x = 0, y = 0;
+		if (pos < q.n) {
+			ring_cell(q, pos, x, y);
+			match = donor_at(don, crm, fd.words, x, y) &&
+				order_key(donor_value(fd, (long long)y * fd.w + x)) == prefix;
+		}
+		unsigned m = __ballot_sync(0xffffffffu, match);
+		int c = __popc(m);
+		if (r < c) {
+			for (int t = r; t > 0; --t)
+				m &= m - 1;
+			int src = __ffs(m) - 1;
+			int sx = __shfl_sync(0xffffffffu, x, src), sy = __shfl_sync(0xffffffffu, y, src);
+			return (long long)sy * fd.w + sx;
+		}
+		r -= c;
+	}
+	return -1; // unreachable when rank < donor count
+}
+
+// far_window_median's two central donors, as linear indices.
+__device__ __noinline__ int far_window_donors(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
+	int x, int y, int &nd, long long &d_lo, long long &d_hi)
+{
+	const int r = nearest_donor(fd, don, crm, x, y);
+	if (!r)
+		return 0;
+	const Ring q = ring_cells(fd.w, fd.h, x, y, r);
+	if (q.n <= 128) {
+		nd = sorted_donors<4>(fd, don, crm, q.n, [&](int pos, int &cx, int &cy) { ring_cell(q, pos, cx, cy); },
+			d_lo, d_hi);
+		return r;
+	}
+	int cnt = 0;
+	for (int pos = threadIdx.x & 31; pos < q.n; pos += 32) {
+		int cx, cy;
+		ring_cell(q, pos, cx, cy);
+		cnt += donor_at(don, crm, fd.words, cx, cy);
+	}
+	nd = warp_sum_int(cnt);
+	d_lo = ring_donor(fd, don, crm, q, (nd - 1) / 2);
+	d_hi = nd % 2 ? d_lo : ring_donor(fd, don, crm, q, nd / 2);
+	return r;
 }
 
 // One warp per flagged pixel: recompute its final replacement window and
@@ -253,15 +292,8 @@ bwd_scatter_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restrict
 					: sorted_window_donors<4>(fd, don, crm, win, d_lo, d_hi);
 				if (!nd)
 					continue;
-			} else {
-				int cnt = 0;
-				for (int pos = lane; pos < area; pos += 32)
-					cnt += donor_at(don, crm, fd.words, win.x0 + pos % ww, win.y0 + pos / ww);
-				nd = warp_sum_int(cnt);
-				if (!nd)
-					continue;
-				d_lo = donor_at_rank_large(fd, don, crm, win, (nd - 1) / 2);
-				d_hi = nd % 2 ? d_lo : donor_at_rank_large(fd, don, crm, win, nd / 2);
+			} else if (!far_window_donors(fd, don, crm, x, y, nd, d_lo, d_hi)) {
+				break;
 			}
 			if (lane == 0) {
 				// Odd count: the middle donor, weight 1.  Even: the two central

@@ -439,53 +439,117 @@ __device__ __forceinline__ bool donor_at(const uint32_t *don, const uint32_t *cr
 	return ((don[o] & ~crm[o]) >> (x & 31)) & 1u;
 }
 
-// The donor of rank `rank` in key order inside a window larger than 32 cells:
-// an MSB-first radix select over ordered 64-bit keys (same ranks as reference
-// src/replace.cuh:85-109).  Up to 8 cells per lane are kept in registers.
-__device__ double select_rank(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm, Window win,
+// The cells at Chebyshev distance r (>= 1) of (x, y) inside a w x h frame, in
+// row-major order: `top` cells of the row above the middle rows, `sides` (0 to 2)
+// of each of the `mid` middle rows, then the row below.
+struct Ring {
+	int x0, y, r, top, mid, sides, n; // n: all cells, at most 2 (w + h)
+	int left, right, ymid;            // columns of the sides, first middle row
+};
+
+CB_HD Ring ring_cells(int w, int h, int x, int y, int r)
+{
+	Ring q;
+	const int x1 = x + r < w ? x + r : w - 1, y1 = y + r < h ? y + r : h - 1;
+	q.x0 = x - r > 0 ? x - r : 0;
+	q.y = y;
+	q.r = r;
+	q.top = y - r >= 0 ? x1 - q.x0 + 1 : 0;
+	q.ymid = y - r >= 0 ? y - r + 1 : 0;
+	q.mid = (y + r < h ? y1 - 1 : y1) - q.ymid + 1;
+	q.sides = (x - r >= 0) + (x + r < w);
+	q.left = x - r >= 0 ? x - r : x + r;
+	q.right = x + r;
+	q.n = q.top + q.mid * q.sides + (y + r < h ? x1 - q.x0 + 1 : 0);
+	return q;
+}
+
+CB_HD void ring_cell(const Ring &q, int pos, int &cx, int &cy)
+{
+	if (pos < q.top) {
+		cx = q.x0 + pos;
+		cy = q.y - q.r;
+		return;
+	}
+	pos -= q.top;
+	if (pos < q.mid * q.sides) {
+		const int row = q.sides == 2 ? pos >> 1 : pos;
+		cx = q.sides == 2 && (pos & 1) ? q.right : q.left;
+		cy = q.ymid + row;
+		return;
+	}
+	cx = q.x0 + pos - q.mid * q.sides;
+	cy = q.y + q.r;
+}
+
+// Distance from bit c (which may lie outside 0 .. 31) to the nearest set bit of
+// the word b (not zero).
+CB_HD int bit_distance(uint32_t b, int c)
+{
+	int best = 1 << 30;
+	const uint32_t low = c < 0 ? 0u : c >= 31 ? b : b & ((2u << c) - 1u), high = c <= 0 ? b : c > 31 ? 0u : b >> c;
+#if defined(__CUDA_ARCH__)
+	if (low)
+		best = c - (31 - __clz((int)low));
+	if (high)
+		best = min(best, __ffs((int)high) - 1 - (c < 0 ? c : 0));
+#else
+	if (low)
+		best = c - (31 - __builtin_clz(low));
+	if (high && __builtin_ctz(high) - (c < 0 ? c : 0) < best)
+		best = __builtin_ctz(high) - (c < 0 ? c : 0);
+#endif
+	return best;
+}
+
+// Chebyshev distance from (x, y) to the frame's nearest donor (0: it has none),
+// by the whole warp: the bit words of boxes of radius 16, 32, 64, ... until one
+// holds a donor within its radius, (2 R + 1)^2 / 32 words for the last.  Bound by
+// the warp's chain of loads.  Counting every window of a growing radius cell by
+// cell reads 4/3 R^3 cells: the replacement of one target 100 pixels from its
+// donors took 6.4 ms, 300 pixels 129 ms, 1000 pixels seconds; with the words and
+// the rim alone (far_window_median) 0.27, 2.2 and 6.7 ms.
+__device__ __noinline__ int nearest_donor(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
+	int x, int y)
+{
+	const int lane = threadIdx.x & 31, limit = max(fd.w, fd.h);
+	for (int R = 16;; R *= 2) {
+		const int ya = max(0, y - R), yb = min(fd.h - 1, y + R);
+		const int k0 = max(0, x - R) >> 5, nk = (min(fd.w - 1, x + R) >> 5) - k0 + 1, n = (yb - ya + 1) * nk;
+		unsigned best = 0xffffffffu;
+#pragma unroll 4
+		for (int i = lane; i < n; i += 32) {
+			const int row = i / nk, k = k0 + i - row * nk;
+			const long long o = (long long)(ya + row) * fd.words + k;
+			const uint32_t b = don[o] & ~crm[o];
+			if (b)
+				best = min(best, (unsigned)max(abs(ya + row - y), bit_distance(b, x - 32 * k)));
+		}
+		best = __reduce_min_sync(0xffffffffu, best);
+		if (best <= (unsigned)R)
+			return (int)best;
+		if (R >= limit)
+			return 0;
+	}
+}
+
+// The donor of rank `rank` in key order among a ring's cells: an MSB-first radix
+// select over ordered 64-bit keys (same ranks as reference
+// src/replace.cuh:85-109).
+__device__ double ring_rank(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm, const Ring &q,
 	int rank)
 {
 	const int lane = threadIdx.x & 31;
-	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
 	unsigned long long prefix = 0, used = 0;
-	if (area <= 256) {
-		unsigned long long keys[8];
-		unsigned valid = 0;
-#pragma unroll
-		for (int s = 0; s < 8; ++s) {
-			int pos = lane + 32 * s;
-			keys[s] = 0;
-			if (pos < area) {
-				int x = win.x0 + pos % ww, y = win.y0 + pos / ww;
-				if (donor_at(don, crm, fd.words, x, y)) {
-					keys[s] = order_key(fd.clean[(long long)y * fd.w + x]);
-					valid |= 1u << s;
-				}
-			}
-		}
-		for (int bit = 63; bit >= 0; --bit) {
-			const unsigned long long flag = 1ull << bit;
-			int below = 0;
-#pragma unroll
-			for (int s = 0; s < 8; ++s)
-				below += ((valid >> s) & 1u) && (keys[s] & used) == prefix && !(keys[s] & flag);
-			below = warp_sum_int(below);
-			used |= flag;
-			if (rank >= below) {
-				prefix |= flag;
-				rank -= below;
-			}
-		}
-		return order_value(prefix);
-	}
 	for (int bit = 63; bit >= 0; --bit) {
 		const unsigned long long flag = 1ull << bit;
 		int below = 0;
-		for (int pos = lane; pos < area; pos += 32) {
-			int x = win.x0 + pos % ww, y = win.y0 + pos / ww;
+		for (int pos = lane; pos < q.n; pos += 32) {
+			int x, y;
+			ring_cell(q, pos, x, y);
 			if (!donor_at(don, crm, fd.words, x, y))
 				continue;
-			unsigned long long k = order_key(fd.clean[(long long)y * fd.w + x]);
+			const unsigned long long k = order_key(fd.clean[(long long)y * fd.w + x]);
 			below += (k & used) == prefix && !(k & flag);
 		}
 		below = warp_sum_int(below);
@@ -533,29 +597,29 @@ __device__ __forceinline__ void sort_keys(unsigned long long (&k)[S])
 	}
 }
 
-// The donors of a window of 33 .. 32 S cells in key order, for the median:
-// lane l holds the keys of cells l + 32 s (all ones for a non-donor or a cell
-// past the window, which sort last), a bitonic network sorts the warp's 32 S
-// keys in unsigned order (the order select_rank's radix select ranks by),
+// The donors of up to 32 S cells (cell(pos, x, y) for pos < n) in key order, for
+// the median: lane l holds the keys of cells l + 32 s (all ones for a non-donor or
+// past the last cell, which sort last), a bitonic network sorts the warp's 32 S
+// keys in unsigned order (the order ring_rank's radix select ranks by),
 // and the keys of ranks (nd - 1) / 2 and nd / 2 come back as lo and hi.
 // Returns nd, the number of donors (0: lo and hi unset).  About 20 to 30
-// dependent exchange steps instead of select_rank's 64 warp reductions per
+// dependent exchange steps instead of a radix select's 64 warp reductions per
 // rank, so a replacement whose window grew past 5 x 5 no longer holds its
 // launch for tens of microseconds.
-template <int S>
-__device__ __noinline__ int sorted_window_median(const FrameDesc &fd, const uint32_t *don,
-	const uint32_t *crm, Window win, double &lo, double &hi)
+template <int S, class Cell>
+__device__ __forceinline__ int sorted_median(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
+	int n, Cell cell, double &lo, double &hi)
 {
 	const int lane = threadIdx.x & 31;
-	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
 	unsigned long long k[S];
 	int nd = 0;
 #pragma unroll
 	for (int s = 0; s < S; ++s) {
 		const int pos = lane + 32 * s;
 		k[s] = ~0ull;
-		if (pos < area) {
-			const int x = win.x0 + pos % ww, y = win.y0 + pos / ww;
+		if (pos < n) {
+			int x, y;
+			cell(pos, x, y);
 			if (donor_at(don, crm, fd.words, x, y))
 				k[s] = order_key(fd.clean[(long long)y * fd.w + x]);
 		}
@@ -576,6 +640,46 @@ __device__ __noinline__ int sorted_window_median(const FrameDesc &fd, const uint
 	lo = order_value(__shfl_sync(0xffffffffu, vl, rl & 31));
 	hi = order_value(__shfl_sync(0xffffffffu, vh, rh & 31));
 	return nd;
+}
+
+// A window of 33 .. 32 S cells.
+template <int S>
+__device__ __noinline__ int sorted_window_median(const FrameDesc &fd, const uint32_t *don,
+	const uint32_t *crm, Window win, double &lo, double &hi)
+{
+	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
+	return sorted_median<S>(fd, don, crm, area, [&](int pos, int &x, int &y) {
+		x = win.x0 + pos % ww;
+		y = win.y0 + pos / ww;
+	}, lo, hi);
+}
+
+// The smallest window around (x, y) that holds a donor, for a pixel whose windows
+// of up to 128 cells hold none: its radius (0: the frame has no donor), its
+// number of donors nd and the two central ones.  No smaller window holds a donor,
+// so all of them lie on the window's rim: only its cells are read.
+__device__ __noinline__ int far_window_median(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
+	int x, int y, int &nd, double &lo, double &hi)
+{
+	const int r = nearest_donor(fd, don, crm, x, y);
+	if (!r)
+		return 0;
+	const Ring q = ring_cells(fd.w, fd.h, x, y, r);
+	if (q.n <= 128) {
+		nd = sorted_median<4>(fd, don, crm, q.n, [&](int pos, int &cx, int &cy) { ring_cell(q, pos, cx, cy); },
+			lo, hi);
+		return r;
+	}
+	int cnt = 0;
+	for (int pos = threadIdx.x & 31; pos < q.n; pos += 32) {
+		int cx, cy;
+		ring_cell(q, pos, cx, cy);
+		cnt += donor_at(don, crm, fd.words, cx, cy);
+	}
+	nd = warp_sum_int(cnt);
+	lo = ring_rank(fd, don, crm, q, (nd - 1) / 2);
+	hi = nd % 2 ? lo : ring_rank(fd, don, crm, q, nd / 2);
+	return r;
 }
 
 // Reference src/replace.cuh:111-153 for one pixel, by the whole warp: the
@@ -619,14 +723,9 @@ __device__ __forceinline__ int replace_one(const FrameDesc &fd, int x, int y, bo
 			if (!nd)
 				continue;
 		} else {
-			int cnt = 0;
-			for (int pos = lane; pos < area; pos += 32)
-				cnt += donor_at(don, crm, words, win.x0 + pos % ww, win.y0 + pos / ww);
-			nd = warp_sum_int(cnt);
-			if (!nd)
-				continue;
-			lo = select_rank(fd, don, crm, win, (nd - 1) / 2);
-			hi = nd % 2 ? lo : select_rank(fd, don, crm, win, nd / 2);
+			r = far_window_median(fd, don, crm, x, y, nd, lo, hi);
+			if (!r)
+				return 0;
 		}
 		if (lane == 0) {
 			const double v = nd % 2 ? 0.0 + lo : midpoint(lo, hi);
