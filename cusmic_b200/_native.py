@@ -14,7 +14,7 @@ LIB_PATH = Path(__file__).with_name("libcusmic_b200.so")
 CUSMIC_OK, CUSMIC_INVALID, CUSMIC_CUDA_ERROR, CUSMIC_NO_MEMORY = range(4)
 BORDERS = {"reflect": 0, "constant": 1, "nearest": 2, "mirror": 3, "wrap": 4}
 PLAN_GRAPH, PLAN_KEEP = 1, 2
-FAULT_PREPARE_WAIT, FAULT_DETECT_WAIT, FAULT_NO_MEMORY = 1, 2, 3
+FAULT_PREPARE_WAIT, FAULT_DETECT_WAIT, FAULT_NO_MEMORY, FAULT_BARRIER_WAIT = 1, 2, 3, 4
 
 # Every symbol declared in include/cusmic.h and include/cusmic_b200.h.
 EXPORTS = (

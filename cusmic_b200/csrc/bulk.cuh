@@ -850,7 +850,7 @@ sig_bulk_kernel(const FrameDesc *__restrict__ frames, const FrameState *__restri
 		ok = bulk_consumer(R, frames, items, prm, pre, pre_counts);
 	if (!ok && lane == 0) {
 		R.abort = 1;
-		atomicOr(&ctl->fault, 1);
+		atomicOr(&ctl->fault, FAULT_COPY);
 	}
 	__syncthreads();
 	// After a fault: wait (bounded) for the copies still in flight into this

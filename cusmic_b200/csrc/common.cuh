@@ -7,6 +7,7 @@
 //              word (y, k) is pixel (y, 32 k + b); padding bits are zero
 //   targets    uint2   {frame, pixel} list of replacement targets
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <cmath>
 #include <cuda_runtime.h>
@@ -129,7 +130,7 @@ struct FrameState {
 	unsigned int active;  // the next detection pass runs for this frame
 	unsigned int error;   // a target had no finite donor
 	unsigned int passes;  // detection passes run
-	unsigned int fault;   // a bounded wait inside a kernel ran out (the frame stopped)
+	unsigned int fault;   // a bounded wait inside a kernel ran out (the frame stopped): FaultBit
 	unsigned int todo[2]; // by parity: the pass flagged a new pixel (set by many warps)
 	unsigned int map_flags, pad; // frame 0: failed map checks of the call (check_maps_kernel)
 	// Static donors, and those of them that are in the mask.
@@ -151,6 +152,9 @@ struct PassLists {
 	unsigned long long n_chg;  // targets whose value the replacement before changed
 };
 
+// What ran out: a copy into the dense kernels' ring, or a grid barrier.
+enum FaultBit { FAULT_COPY = 1, FAULT_BARRIER = 2 };
+
 // Loop control shared by the per-pass kernels.
 struct Control {
 	unsigned long long n_targets; // length of the target list
@@ -162,14 +166,17 @@ struct Control {
 	unsigned long long fresh0;    // late passes: targets listed before the last growth
 	int any[2];                   // by parity: a frame goes on after the pass
 	int ticket;                   // next item of the bulk detection kernel
-	int fault;                    // a bounded wait ran out
-	unsigned barrier;             // arrivals at the late passes' grid barriers
 	unsigned pad;
+	int fault;                    // a bounded wait ran out (FaultBit); read together with
+	unsigned barrier;             // the arrivals at the late passes' grid barriers
 	// Injected failures (0: none): the bound, in SM cycles, of one extra wait
 	// on a barrier that nothing completes, for prepare ([0]) and for the dense
 	// detection ([1]); one warp of the dense detection's first block makes it.
 	long long poison_wait[2];
 };
+
+static_assert(offsetof(Control, fault) % 8 == 0 && offsetof(Control, barrier) == offsetof(Control, fault) + 4,
+	"grid_barrier reads the fault and the arrivals as one word");
 
 CB_HD uint32_t *plane_ptr(const FrameDesc &f, int p)
 {

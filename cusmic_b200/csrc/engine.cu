@@ -58,7 +58,7 @@ static void check(cudaError_t e)
 // Injected failures (cusmic_inject_fault): the bounds of the injected device
 // waits of calls that start later, and the number of workspace reservations
 // still to fail as an exhausted allocator would.
-static std::atomic<long long> inject_wait[2] = {{0}, {0}};
+static std::atomic<long long> inject_wait[3] = {{0}, {0}, {0}}; // prepare, detection, barrier
 static std::atomic<long long> inject_alloc_failures{0};
 
 // True when this reservation is one that an injection makes fail.
@@ -387,7 +387,7 @@ struct Layout {
 	// is captured again).
 	bool fused = false;
 	cusmic_tuning tune{};
-	long long poison_wait[2] = {0, 0}; // injected failures in force when the batch was laid out
+	long long poison_wait[3] = {0, 0, 0}; // injected failures in force when the batch was laid out
 };
 
 struct DeviceInfo {
@@ -595,8 +595,8 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 		: item_rows(ims, nf, di.sms * tune.dense_blocks_per_sm);
 	Layout L;
 	L.tune = tune;
-	L.poison_wait[0] = inject_wait[0].load();
-	L.poison_wait[1] = inject_wait[1].load();
+	for (int i = 0; i < 3; ++i)
+		L.poison_wait[i] = inject_wait[i].load();
 	L.maxiter = o.maxiter;
 	L.prm.contrast = o.contrast;
 	L.prm.rcontrast = 1 / o.contrast;
@@ -911,7 +911,11 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 			cands, low, eval);
 	}
 	mark(rec, K_RECLASS);
-	void *args[] = {&frames, &state, &nf, &prm, &ctl, &maxiter, &cands, &low, &eval, &targets, &radius, &chg};
+	BarrierWait bw{BARRIER_CYCLES, 0};
+	if (L.poison_wait[2])
+		bw = BarrierWait{L.poison_wait[2], 1};
+	void *args[] = {&frames, &state, &nf, &prm, &ctl, &maxiter, &cands, &low, &eval, &targets, &radius, &chg,
+		&bw};
 	check(cudaLaunchCooperativeKernel((const void *)late_passes_kernel, dim3(grid), dim3(LATE_THREADS), args,
 		sizeof(LateShared), s));
 	mark(rec, K_RECLASS);
@@ -1054,7 +1058,8 @@ static void enqueue_plain(Workspace &ws, const Layout &L, const DeviceInfo &di, 
 static void check_state(const FrameState &st)
 {
 	if (st.fault)
-		throw std::runtime_error("a detection kernel gave up waiting for its copies");
+		throw std::runtime_error(st.fault & FAULT_BARRIER ? "a late pass gave up waiting at a grid barrier"
+								  : "a detection kernel gave up waiting for its copies");
 	if (st.error || (st.holes && st.allowed && !st.donors))
 		throw InvalidArgument("no finite replacement donors");
 }
@@ -2102,6 +2107,9 @@ extern "C" int cusmic_inject_fault(int what, long long value)
 	case CUSMIC_FAULT_PREPARE_WAIT:
 	case CUSMIC_FAULT_DETECT_WAIT:
 		inject_wait[what - CUSMIC_FAULT_PREPARE_WAIT].store(value > 0 ? value : 0);
+		return CUSMIC_OK;
+	case CUSMIC_FAULT_BARRIER_WAIT:
+		inject_wait[2].store(value > 0 ? value : 0);
 		return CUSMIC_OK;
 	case CUSMIC_FAULT_NO_MEMORY:
 		inject_alloc_failures.store(value > 0 ? value : 0);

@@ -856,7 +856,7 @@ __device__ __forceinline__ void pass_control(FrameState *state, int nf, Control 
 		++s.passes;
 		bool on = false;
 		if (fault) // this pass's detection is incomplete: stop, report
-			s.fault = 1;
+			s.fault = fault;
 		else if (s.todo[par] && s.donors <= s.masked)
 			s.error = 1;
 		else

@@ -70,30 +70,48 @@ __device__ __forceinline__ int wrap_index(int i, int n)
 	return i < 0 ? i + n : i;
 }
 
+// The bound of a grid barrier's wait, in SM cycles (about 17 s), and the arrivals
+// it waits for beyond the grid's (an injected failure: one that never comes).
+// Every block of a cooperative launch is resident, so a block waits only while
+// others work, and the bound cuts off no stage that ends: the longest single item
+// is a replacement whose nearest donor is thousands of pixels away (1000 pixels: 7 ms).
+struct BarrierWait {
+	long long limit;
+	unsigned missing;
+};
+constexpr long long BARRIER_CYCLES = 1LL << 35;
+
 // Grid barrier of a cooperative launch: the `round`-th call (from 1) returns
 // once every block has arrived `round` times, with their earlier writes
-// visible.  Bounded like every wait (about one second of SM clock): a wait that
-// runs out faults every frame and returns false, and so does every later one.
-__device__ __forceinline__ bool grid_barrier(Control *ctl, unsigned round, FrameState *state, int nf)
+// visible.  A wait that runs out faults every frame and returns false, and so do
+// the barrier's other blocks that see the fault (the last one to arrive, whose
+// own wait is over at once, among them) and every later barrier.
+__device__ __forceinline__ bool grid_barrier(Control *ctl, unsigned round, FrameState *state, int nf,
+	const BarrierWait &bw)
 {
 	__shared__ int open;
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		__threadfence();
 		atomicAdd(&ctl->barrier, 1u);
-		const unsigned want = round * gridDim.x;
+		const unsigned want = round * gridDim.x + bw.missing;
 		const long long t0 = clock64();
-		bool ok = true;
-		while ((int)(*(volatile unsigned *)&ctl->barrier - want) < 0) {
-			if (*(volatile int *)&ctl->fault || clock64() - t0 > BK_WAIT_CYCLES) {
+		bool ok;
+		for (;;) {
+			// The fault in the low half, the arrivals in the high one.
+			const unsigned long long v = *(volatile unsigned long long *)&ctl->fault;
+			ok = (unsigned)v == 0;
+			if (!ok || (int)((unsigned)(v >> 32) - want) >= 0)
+				break;
+			if (clock64() - t0 > bw.limit) {
 				ok = false;
 				break;
 			}
 		}
 		if (!ok) {
-			atomicOr(&ctl->fault, 1);
+			atomicOr(&ctl->fault, FAULT_BARRIER);
 			for (int f = 0; f < nf; ++f)
-				state[f].fault = 1;
+				state[f].fault = FAULT_BARRIER;
 		}
 		__threadfence();
 		open = ok;
@@ -588,7 +606,7 @@ struct LateShared {
 __global__ void __launch_bounds__(LATE_THREADS, 1)
 late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int nf, DetectParams prm,
 	Control *ctl, int maxiter, uint2 *cands, uint2 *low, uint2 *eval, uint2 *targets, uint8_t *radius,
-	unsigned *chg)
+	unsigned *chg, BarrierWait bw)
 {
 	extern __shared__ __align__(16) unsigned char late_smem[];
 	LateShared &S = *reinterpret_cast<LateShared *>(late_smem);
@@ -618,10 +636,10 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 				plane_ptr(fd, P_FRESH)[(long long)(t.y / (unsigned)fd.w) * fd.words +
 					((t.y % (unsigned)fd.w) >> 5)] = 0u;
 			}
-			if (!grid_barrier(ctl, ++round, state, nf))
+			if (!grid_barrier(ctl, ++round, state, nf, bw))
 				return;
 			late_classes<LATE_SHORT>(frames, eval, prm, L, cands, low, S.queue[warp]);
-			if (!grid_barrier(ctl, ++round, state, nf))
+			if (!grid_barrier(ctl, ++round, state, nf, bw))
 				return;
 		}
 		if (first) { // what the coming stages and the next pass append to
@@ -630,15 +648,15 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 			ctl->any[par] = 0;
 		}
 		late_candidates(frames, cands, prm, L, S.Q, S.patches[warp], S.scratch[warp], triples);
-		if (!grid_barrier(ctl, ++round, state, nf))
+		if (!grid_barrier(ctl, ++round, state, nf, bw))
 			return;
 		late_low(frames, state, cands, low, prm, L, ctl, par, targets, S.Q, S.patches[warp], S.scratch[warp]);
-		if (!grid_barrier(ctl, ++round, state, nf))
+		if (!grid_barrier(ctl, ++round, state, nf, bw))
 			return;
 		pass_control(state, nf, ctl, par);
 		late_replace(frames, state, par, targets, (long long)ctl->n_targets, (long long)ctl->fresh0, radius,
 			chg, &next.n_chg, S.Q);
-		if (it + 1 < maxiter && !grid_barrier(ctl, ++round, state, nf))
+		if (it + 1 < maxiter && !grid_barrier(ctl, ++round, state, nf, bw))
 			return;
 	}
 }

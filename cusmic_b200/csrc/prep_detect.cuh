@@ -473,7 +473,7 @@ prep_detect_kernel(const FrameDesc *__restrict__ frames, FrameState *state, cons
 		ok = pd_consumer(R, M, frames, state, items, ctl, holes, pre, pre_counts);
 	if (!ok && lane == 0) {
 		R.abort = 1;
-		atomicOr(&ctl->fault, 1);
+		atomicOr(&ctl->fault, FAULT_COPY);
 	}
 	__syncthreads();
 	// After a fault: wait (bounded) for the copies still in flight into this

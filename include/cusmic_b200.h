@@ -213,11 +213,17 @@ remove_cosmics_device_noalloc(const struct cusmic_image *image, const struct cus
  *
  *   CUSMIC_FAULT_PREPARE_WAIT, CUSMIC_FAULT_DETECT_WAIT: value > 0 makes one
  *     warp of the dense detection kernel (which prepares the frames too, or
- *     follows a prepare kernel that waits for nothing) wait up to `value` SM cycles on a barrier that nothing
- *     completes, in calls (and plans) laid out after this call.  The wait
+ *     follows a prepare kernel that waits for nothing) wait up to `value` SM
+ *     cycles on a barrier that nothing completes, in calls (and plans) laid out
+ *     after this call.  The wait
  *     runs out like a wait whose copies never land: the kernel drains its
  *     copies in flight, the loop control stops every frame and the call
  *     returns CUSMIC_CUDA_ERROR.  value <= 0 removes the injection.
+ *   CUSMIC_FAULT_BARRIER_WAIT: value > 0 makes the first grid barrier of the
+ *     passes after the first wait up to `value` SM cycles for an arrival that
+ *     never comes, in calls (and plans) laid out after this call that get
+ *     there.  Every block leaves, every frame stops and the call returns
+ *     CUSMIC_CUDA_ERROR.  value <= 0 removes the injection.
  *   CUSMIC_FAULT_NO_MEMORY: the next `value` workspace reservations fail as
  *     an exhausted cudaMalloc would (CUSMIC_NO_MEMORY; the host entry point
  *     leaves its outputs unchanged).
@@ -226,7 +232,8 @@ remove_cosmics_device_noalloc(const struct cusmic_image *image, const struct cus
 enum cusmic_fault {
 	CUSMIC_FAULT_PREPARE_WAIT = 1,
 	CUSMIC_FAULT_DETECT_WAIT = 2,
-	CUSMIC_FAULT_NO_MEMORY = 3
+	CUSMIC_FAULT_NO_MEMORY = 3,
+	CUSMIC_FAULT_BARRIER_WAIT = 4
 };
 
 int
