@@ -169,6 +169,8 @@ struct Control {
 	unsigned pad;
 	int fault;                    // a bounded wait ran out (FaultBit); read together with
 	unsigned barrier;             // the arrivals at the late passes' grid barriers
+	unsigned arrived;             // blocks of the late passes that started (join_team)
+	unsigned team;                // how many of them work, once that is closed
 	// Injected failures (0: none): the bound, in SM cycles, of one extra wait
 	// on a barrier that nothing completes, for prepare ([0]) and for the dense
 	// detection ([1]); one warp of the dense detection's first block makes it.
@@ -177,6 +179,21 @@ struct Control {
 
 static_assert(offsetof(Control, fault) % 8 == 0 && offsetof(Control, barrier) == offsetof(Control, fault) + 4,
 	"grid_barrier reads the fault and the arrivals as one word");
+static_assert(offsetof(Control, arrived) % 8 == 0 && offsetof(Control, team) == offsetof(Control, arrived) + 4,
+	"join_team reads both as one word");
+
+// The blocks that share a launch's work: this one's number and how many there are
+// (all of the grid's, except in the late passes).
+struct Team {
+	unsigned block, blocks;
+};
+
+#ifdef __CUDACC__
+__device__ __forceinline__ Team whole_grid()
+{
+	return Team{blockIdx.x, gridDim.x};
+}
+#endif
 
 CB_HD uint32_t *plane_ptr(const FrameDesc &f, int p)
 {

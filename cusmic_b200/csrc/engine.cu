@@ -2,7 +2,7 @@
 // the C ABI of include/cusmic.h and include/cusmic_b200.h.
 //
 // One call = init -> prepare -> hole fill -> first pass (detect -> grow/update
-// -> replace) -> the later passes in one cooperative launch -> restore, all on
+// -> replace) -> the later passes in one launch -> restore, all on
 // the caller's stream, with no host synchronisation in between: per-frame
 // activity lives on the device and frames that stopped are skipped (the
 // reference instead copies counts to the host after every pass,
@@ -868,10 +868,10 @@ static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	mark(rec, K_REPLACE);
 }
 
-// The passes after the first (late.cuh): the first late pass's lists in two
-// launches, then one cooperative launch, whose blocks all run at once and meet
-// at grid barriers.  Small batches take fewer blocks, which makes the barriers
-// cheaper.
+// The passes after the first (late.cuh): the first late pass's lists in two or
+// three launches, then one launch whose blocks meet at barriers, at most one block
+// for each SM (it fills one; those that find no free SM are left out).  Small
+// batches take fewer blocks, which makes the barriers cheaper.
 static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cudaStream_t s,
 	Recorder *rec = nullptr)
 {
@@ -914,10 +914,8 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	BarrierWait bw{BARRIER_CYCLES, 0};
 	if (L.poison_wait[2])
 		bw = BarrierWait{L.poison_wait[2], 1};
-	void *args[] = {&frames, &state, &nf, &prm, &ctl, &maxiter, &cands, &low, &eval, &targets, &radius, &chg,
-		&bw};
-	check(cudaLaunchCooperativeKernel((const void *)late_passes_kernel, dim3(grid), dim3(LATE_THREADS), args,
-		sizeof(LateShared), s));
+	late_passes_kernel<<<grid, LATE_THREADS, sizeof(LateShared), s>>>(frames, state, nf, prm, ctl, maxiter, cands,
+		low, eval, targets, radius, chg, bw);
 	mark(rec, K_RECLASS);
 }
 

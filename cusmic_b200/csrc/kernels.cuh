@@ -601,14 +601,18 @@ __device__ __forceinline__ void sort_keys(unsigned long long (&k)[S])
 // the median: lane l holds the keys of cells l + 32 s (all ones for a non-donor or
 // past the last cell, which sort last), a bitonic network sorts the warp's 32 S
 // keys in unsigned order (the order ring_rank's radix select ranks by),
-// and the keys of ranks (nd - 1) / 2 and nd / 2 come back as lo and hi.
-// Returns nd, the number of donors (0: lo and hi unset).  About 20 to 30
-// dependent exchange steps instead of a radix select's 64 warp reductions per
+// and the keys of ranks (nd - 1) / 2 and nd / 2 come back as lo and hi.  About 20
+// to 30 dependent exchange steps instead of a radix select's 64 warp reductions per
 // rank, so a replacement whose window grew past 5 x 5 no longer holds its
 // launch for tens of microseconds.
+struct DonorMedian {
+	double lo, hi; // the two central donors (unset without a donor)
+	int nd, r;     // donors; radius of the window
+};
+
 template <int S, class Cell>
-__device__ __forceinline__ int sorted_median(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
-	int n, Cell cell, double &lo, double &hi)
+__device__ __forceinline__ DonorMedian sorted_median(const FrameDesc &fd, const uint32_t *don,
+	const uint32_t *crm, int n, Cell cell)
 {
 	const int lane = threadIdx.x & 31;
 	unsigned long long k[S];
@@ -626,7 +630,7 @@ __device__ __forceinline__ int sorted_median(const FrameDesc &fd, const uint32_t
 		nd += __popc(__ballot_sync(0xffffffffu, k[s] != ~0ull));
 	}
 	if (!nd)
-		return 0;
+		return DonorMedian{0, 0, 0, 0};
 	sort_keys(k);
 	const int rl = (nd - 1) / 2, rh = nd / 2;
 	unsigned long long vl = 0, vh = 0;
@@ -637,49 +641,48 @@ __device__ __forceinline__ int sorted_median(const FrameDesc &fd, const uint32_t
 		if (s == rh >> 5)
 			vh = k[s];
 	}
-	lo = order_value(__shfl_sync(0xffffffffu, vl, rl & 31));
-	hi = order_value(__shfl_sync(0xffffffffu, vh, rh & 31));
-	return nd;
+	return DonorMedian{order_value(__shfl_sync(0xffffffffu, vl, rl & 31)),
+		order_value(__shfl_sync(0xffffffffu, vh, rh & 31)), nd, 0};
 }
 
-// A window of 33 .. 32 S cells.
+// A window of 33 .. 32 S cells (r is left zero).
 template <int S>
-__device__ __noinline__ int sorted_window_median(const FrameDesc &fd, const uint32_t *don,
-	const uint32_t *crm, Window win, double &lo, double &hi)
+__device__ __noinline__ DonorMedian sorted_window_median(const FrameDesc &fd, const uint32_t *don,
+	const uint32_t *crm, Window win)
 {
 	const int ww = win.x1 - win.x0 + 1, area = ww * (win.y1 - win.y0 + 1);
 	return sorted_median<S>(fd, don, crm, area, [&](int pos, int &x, int &y) {
 		x = win.x0 + pos % ww;
 		y = win.y0 + pos / ww;
-	}, lo, hi);
+	});
 }
 
 // The smallest window around (x, y) that holds a donor, for a pixel whose windows
-// of up to 128 cells hold none: its radius (0: the frame has no donor), its
-// number of donors nd and the two central ones.  No smaller window holds a donor,
-// so all of them lie on the window's rim: only its cells are read.
-__device__ __noinline__ int far_window_median(const FrameDesc &fd, const uint32_t *don, const uint32_t *crm,
-	int x, int y, int &nd, double &lo, double &hi)
+// of up to 128 cells hold none (r = 0: the frame has no donor).  No smaller window
+// holds a donor, so all of them lie on the window's rim: only its cells are read.
+__device__ __noinline__ DonorMedian far_window_median(const FrameDesc &fd, const uint32_t *don,
+	const uint32_t *crm, int x, int y)
 {
+	DonorMedian m{0, 0, 0, 0};
 	const int r = nearest_donor(fd, don, crm, x, y);
 	if (!r)
-		return 0;
+		return m;
 	const Ring q = ring_cells(fd.w, fd.h, x, y, r);
 	if (q.n <= 128) {
-		nd = sorted_median<4>(fd, don, crm, q.n, [&](int pos, int &cx, int &cy) { ring_cell(q, pos, cx, cy); },
-			lo, hi);
-		return r;
+		m = sorted_median<4>(fd, don, crm, q.n, [&](int pos, int &cx, int &cy) { ring_cell(q, pos, cx, cy); });
+	} else {
+		int cnt = 0;
+		for (int pos = threadIdx.x & 31; pos < q.n; pos += 32) {
+			int cx, cy;
+			ring_cell(q, pos, cx, cy);
+			cnt += donor_at(don, crm, fd.words, cx, cy);
+		}
+		m.nd = warp_sum_int(cnt);
+		m.lo = ring_rank(fd, don, crm, q, (m.nd - 1) / 2);
+		m.hi = m.nd % 2 ? m.lo : ring_rank(fd, don, crm, q, m.nd / 2);
 	}
-	int cnt = 0;
-	for (int pos = threadIdx.x & 31; pos < q.n; pos += 32) {
-		int cx, cy;
-		ring_cell(q, pos, cx, cy);
-		cnt += donor_at(don, crm, fd.words, cx, cy);
-	}
-	nd = warp_sum_int(cnt);
-	lo = ring_rank(fd, don, crm, q, (nd - 1) / 2);
-	hi = nd % 2 ? lo : ring_rank(fd, don, crm, q, nd / 2);
-	return r;
+	m.r = r;
+	return m;
 }
 
 // Reference src/replace.cuh:111-153 for one pixel, by the whole warp: the
@@ -715,17 +718,20 @@ __device__ __forceinline__ int replace_one(const FrameDesc &fd, int x, int y, bo
 			lo = __shfl_sync(0xffffffffu, v, (nd - 1) / 2);
 			hi = __shfl_sync(0xffffffffu, v, nd / 2);
 		} else if (area <= 64) {
-			nd = sorted_window_median<2>(fd, don, crm, win, lo, hi);
-			if (!nd)
+			const DonorMedian m = sorted_window_median<2>(fd, don, crm, win);
+			if (!m.nd)
 				continue;
+			nd = m.nd, lo = m.lo, hi = m.hi;
 		} else if (area <= 128) {
-			nd = sorted_window_median<4>(fd, don, crm, win, lo, hi);
-			if (!nd)
+			const DonorMedian m = sorted_window_median<4>(fd, don, crm, win);
+			if (!m.nd)
 				continue;
+			nd = m.nd, lo = m.lo, hi = m.hi;
 		} else {
-			r = far_window_median(fd, don, crm, x, y, nd, lo, hi);
-			if (!r)
+			const DonorMedian m = far_window_median(fd, don, crm, x, y);
+			if (!m.r)
 				return 0;
+			r = m.r, nd = m.nd, lo = m.lo, hi = m.hi;
 		}
 		if (lane == 0) {
 			const double v = nd % 2 ? 0.0 + lo : midpoint(lo, hi);
@@ -845,10 +851,10 @@ __device__ __forceinline__ bool replaces(const FrameState &s, int par)
 // pixels stops (its later passes would repeat this one), the others replace
 // and continue.  Runs in the replacement's grid (a thread per frame): the
 // replacement reads only todo[par] and the donor counts, which this leaves alone.
-__device__ __forceinline__ void pass_control(FrameState *state, int nf, Control *ctl, int par)
+__device__ __forceinline__ void pass_control(FrameState *state, int nf, Control *ctl, int par, Team team)
 {
 	const int fault = *(volatile int *)&ctl->fault;
-	for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
+	for (int f = team.block * blockDim.x + threadIdx.x; f < nf; f += team.blocks * blockDim.x) {
 		FrameState &s = state[f];
 		s.todo[par ^ 1] = 0;
 		if (!s.active)
@@ -949,7 +955,7 @@ replace_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int nf, 
 	Control *ctl, int par, uint8_t *radius, unsigned *chg)
 {
 	__shared__ WindowQueue Q;
-	pass_control(state, nf, ctl, par);
+	pass_control(state, nf, ctl, par, whole_grid());
 	if (!chg && blockIdx.x == 0 && threadIdx.x == 0) {
 		ctl->pass[par ^ 1] = PassLists{};
 		ctl->any[par ^ 1] = 0;

@@ -1,5 +1,5 @@
-// Late detection passes (every pass after the first), all of them in one
-// cooperative launch.
+// Late detection passes (every pass after the first), all of them in one launch
+// whose blocks meet at barriers.
 //
 // A pass of the reference (src/cleaner.cuh:102-142) recomputes the whole
 // detection chain on the current clean pixels, and between two passes only
@@ -18,7 +18,7 @@
 // So with D the targets whose value the last replacement changed (the chg
 // list that replace_targets writes), pass k + 1 differs from pass k only near
 // D.  A late pass keeps the bit planes of the previous one and works on lists
-// that start from D, in stages separated by grid barriers:
+// that start from D, in stages separated by barriers:
 //
 //  1. Half a warp per pixel of D (a lane per row of its 13 x 13
 //     neighbourhood): the pixels within 2 are listed for re-evaluation (once
@@ -72,29 +72,79 @@ __device__ __forceinline__ int wrap_index(int i, int n)
 
 // The bound of a grid barrier's wait, in SM cycles (about 17 s), and the arrivals
 // it waits for beyond the grid's (an injected failure: one that never comes).
-// Every block of a cooperative launch is resident, so a block waits only while
-// others work, and the bound cuts off no stage that ends: the longest single item
-// is a replacement whose nearest donor is thousands of pixels away (1000 pixels: 7 ms).
+// Every block of the team is running, so a block waits only while others work,
+// and the bound cuts off no stage that ends: the longest single item is a
+// replacement whose nearest donor is thousands of pixels away (1000 pixels: 7 ms).
 struct BarrierWait {
 	long long limit;
 	unsigned missing;
 };
 constexpr long long BARRIER_CYCLES = 1LL << 35;
 
-// Grid barrier of a cooperative launch: the `round`-th call (from 1) returns
-// once every block has arrived `round` times, with their earlier writes
-// visible.  A wait that runs out faults every frame and returns false, and so do
-// the barrier's other blocks that see the fault (the last one to arrive, whose
-// own wait is over at once, among them) and every later barrier.
-__device__ __forceinline__ bool grid_barrier(Control *ctl, unsigned round, FrameState *state, int nf,
-	const BarrierWait &bw)
+// The late launch's team: the blocks that have started when it is closed.  A block
+// joins with its number (the order of the starts) and takes the first stage's share
+// of that number among gridDim.x; close_team, after that, closes the team once the
+// whole grid has started, or JOIN_CYCLES (about 17 us) after the first block is done,
+// and the team's blocks do the missing shares.  So only running blocks meet at
+// the barriers, and the launch needs no more SMs than are free: beside another
+// stream's kernel that stays, or on a context with part of the SMs, a cooperative
+// launch (whose blocks all have to fit at once) waits or is refused.  A block that
+// comes too late leaves at once.  (Closing the team before the first stage cost
+// every call the 2 us between the first block's start and the last one's.)
+constexpr long long JOIN_CYCLES = 1 << 15;
+constexpr unsigned TEAM_CLOSED = 1u << 31; // in Control::arrived
+
+// False: too late.
+__device__ __forceinline__ bool join_team(Control *ctl, Team &team)
 {
-	__shared__ int open;
+	if (threadIdx.x == 0)
+		team.block = atomicAdd(&ctl->arrived, 1u);
+	__syncthreads();
+	return !(team.block & TEAM_CLOSED);
+}
+
+// Sets the closed team's size (called by every block that joined).
+__device__ __forceinline__ void close_team(Control *ctl, Team &team)
+{
+	if (threadIdx.x == 0) {
+		unsigned n = 0;
+		const long long t0 = clock64();
+		do {
+			// The arrivals in the low half, the closed team's size in the high one.
+			const unsigned long long v = *(volatile unsigned long long *)&ctl->arrived;
+			const unsigned here = (unsigned)v;
+			const long long waited = clock64() - t0;
+			n = here & TEAM_CLOSED ? (unsigned)(v >> 32) : here == gridDim.x ? here : 0u;
+			if (!n && team.block == 0 && waited > JOIN_CYCLES) {
+				n = atomicOr(&ctl->arrived, TEAM_CLOSED);
+				*(volatile unsigned *)&ctl->team = n;
+			}
+			if (waited > BARRIER_CYCLES)
+				n = gridDim.x; // (the first block is long done; the barrier will fault)
+		} while (!n);
+		team.blocks = n;
+	}
+	__syncthreads();
+}
+
+// Barrier of the team: the k-th call returns once every block has arrived k times,
+// with their earlier writes visible (B.calls starts zero).  A wait that runs out
+// faults every frame and returns false, and so do the barrier's other blocks that
+// see the fault (the last one to arrive, whose own wait is over at once, among
+// them) and every later barrier.
+struct BarrierState {
+	unsigned calls;
+	int open;
+};
+
+__device__ __forceinline__ bool grid_barrier(Control *ctl, BarrierState &B, FrameState *state, int nf,
+	const BarrierWait &bw, const Team &team)
+{
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		__threadfence();
 		atomicAdd(&ctl->barrier, 1u);
-		const unsigned want = round * gridDim.x + bw.missing;
+		const unsigned want = ++B.calls * team.blocks + bw.missing;
 		const long long t0 = clock64();
 		bool ok;
 		for (;;) {
@@ -114,10 +164,10 @@ __device__ __forceinline__ bool grid_barrier(Control *ctl, unsigned round, Frame
 				state[f].fault = FAULT_BARRIER;
 		}
 		__threadfence();
-		open = ok;
+		B.open = ok;
 	}
 	__syncthreads();
-	return open != 0;
+	return B.open != 0;
 }
 
 // A block's entries for the three lists of stage 1: their numbers, then their
@@ -133,16 +183,16 @@ struct ListSlots {
 // another) held this stage for 82 us on 64,998 changed targets.
 template <int WARPS>
 __device__ __forceinline__ void late_neighbours(const FrameDesc *__restrict__ frames, const uint2 *targets,
-	const unsigned *chg, PassLists &L, int mode, uint2 *cands, uint2 *low, uint2 *eval, ListSlots &R)
+	const unsigned *chg, PassLists &L, int mode, uint2 *cands, uint2 *low, uint2 *eval, ListSlots &R, Team team)
 {
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const long long n = (long long)L.n_chg;
 	const bool wrap = mode == WRAP;
 	const int dy = (lane & 15) - 6, ay = dy < 0 ? -dy : dy;
 	// Entries per block and sweep: fewer for a short list, which spreads it.
-	const long long share = (n + gridDim.x - 1) / gridDim.x;
+	const long long share = (n + team.blocks - 1) / team.blocks;
 	const int chunk = share < 2 * WARPS ? (int)share : 2 * WARPS;
-	for (long long base = (long long)blockIdx.x * chunk; base < n; base += (long long)gridDim.x * chunk) {
+	for (long long base = (long long)team.block * chunk; base < n; base += (long long)team.blocks * chunk) {
 		const int own_entry = 2 * warp + (lane >> 4);
 		const long long i = base + own_entry;
 		bool valid = own_entry < chunk && i < n && dy <= 6;
@@ -317,11 +367,11 @@ constexpr unsigned EVAL_DONE = 0xffffffffu; // the frame of an entry that is set
 
 template <LatePart PART, bool MODEL = true>
 __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frames, uint2 *eval,
-	const DetectParams &prm, PassLists &L, uint2 *cands, uint2 *low, uint2 *Q)
+	const DetectParams &prm, PassLists &L, uint2 *cands, uint2 *low, uint2 *Q, Team team)
 {
 	const int lane = threadIdx.x & 31;
-	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+	const long long gw = (team.block * (long long)blockDim.x + threadIdx.x) >> 5;
+	const long long nw = ((long long)team.blocks * blockDim.x) >> 5;
 	const long long n = (long long)L.n_eval;
 	const int mode = prm.mode, lm = lap_mode(mode);
 	const double tmin2 = fmin(prm.thi2, prm.tlo2);
@@ -426,50 +476,67 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 		drain(nq);
 }
 
-// Entries 0 .. n - 1 of a list by blocks: a thread per entry tests it (keep),
-// then the block's warps take the survivors (work, by the whole warp) from a
-// queue in shared memory.  A block's share shrinks with the list, so that a
-// short one spreads over the grid.  The entries are dealt to the blocks one by
-// one, so neighbouring entries, whose survivors come in clusters, go to
+// The entries of a list (count() many, which thread 0 asks) by blocks: a thread per
+// entry tests it (keep), then the block's warps take the survivors (work, by the
+// whole warp) from a queue in shared memory.  A block's share shrinks with the list,
+// so that a short one spreads over the team.  The entries are dealt to the blocks
+// one by one, so neighbouring entries, whose survivors come in clusters, go to
 // different blocks.  aside: other work of every warp, done before the first
 // sweep's barrier, beside other warps' tests.
+//
+// What is the same for the whole block stays in shared memory: the work holds
+// every register of a thread (64 at this block size), and what lives across it
+// spills.
 struct LateQueue {
 	uint16_t e[LATE_THREADS];
 	int n;
+	int chunk;
+	Team team;
+	long long end;
 };
 
-template <class Keep, class Work, class Aside>
-__device__ __forceinline__ void block_sweep(long long n, LateQueue &Q, Keep keep, Work work, Aside aside)
+template <class Count, class Keep, class Work, class Aside>
+__device__ __forceinline__ void block_sweep(Count count, LateQueue &Q, Team team, Keep keep, Work work, Aside aside)
 {
 	const int warp = threadIdx.x >> 5;
-	const long long share = (n + gridDim.x - 1) / gridDim.x;
-	const int chunk = share < LATE_THREADS ? (int)share : LATE_THREADS;
-	const long long step = gridDim.x;
-	bool first = true;
-	for (long long base = blockIdx.x; base < n || first; base += (long long)gridDim.x * chunk) { // block-uniform
+	__syncthreads(); // an earlier sweep's reads of Q
+	if (threadIdx.x == 0) {
+		const long long n = count(), share = (n + team.blocks - 1) / team.blocks;
+		Q.chunk = share < LATE_THREADS ? (int)share : LATE_THREADS;
+		Q.team = team;
+		Q.end = n;
+	}
+	// Entry of slot j of the block's k-th chunk.
+	auto entry = [&](int k, int j) {
+		return Q.team.block + (long long)Q.team.blocks * ((long long)k * Q.chunk + j);
+	};
+	for (int k = 0;; ++k) { // block-uniform
 		if (threadIdx.x == 0)
 			Q.n = 0;
 		__syncthreads();
-		if (first)
+		if (k == 0)
 			aside();
-		first = false;
-		const long long e = base + step * threadIdx.x;
-		if ((int)threadIdx.x < chunk && e < n && keep(e))
-			Q.e[atomicAdd(&Q.n, 1)] = (uint16_t)threadIdx.x;
+		if ((int)threadIdx.x < Q.chunk) {
+			const long long e = entry(k, threadIdx.x);
+			if (e < Q.end && keep(e))
+				Q.e[atomicAdd(&Q.n, 1)] = (uint16_t)threadIdx.x;
+		}
 		__syncthreads();
-		const int nq = Q.n;
-		for (int q = warp; q < nq; q += LATE_WARPS)
-			work(base + step * Q.e[q]);
+		for (int q = warp; q < Q.n; q += LATE_WARPS)
+			work(entry(k, Q.e[q]));
 		__syncthreads();
+		if (!Q.chunk || entry(k + 1, 0) >= Q.end)
+			return;
 	}
 }
 
 // Stage 3: the listed pixels that are HIGH (and no hole) now, a warp each.
+template <class Count>
 __device__ __forceinline__ void late_candidates(const FrameDesc *__restrict__ frames, const uint2 *cands,
-	const DetectParams &prm, const PassLists &L, LateQueue &Q, double *P, double *S, double (*T)[63])
+	const DetectParams &prm, Count count, LateQueue &Q, Team team, double *P, double *S, double (*T)[63])
 {
 	const int lane = threadIdx.x & 31;
-	block_sweep((long long)L.n_cand, Q, [&](long long e) {
+	block_sweep(count, Q, team, [&](long long e) {
 		const uint2 t = cands[e];
 		const FrameDesc &fd = frames[t.x];
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
@@ -492,12 +559,12 @@ __device__ __forceinline__ void late_candidates(const FrameDesc *__restrict__ fr
 // The entries are dealt to the blocks in fours, and within a block to its last
 // warps first (its first ones have the low list's entries).
 __device__ __forceinline__ void late_grow(const FrameDesc *__restrict__ frames, FrameState *state,
-	const uint2 *cands, const PassLists &L, Control *ctl, int par, uint2 *targets)
+	const uint2 *cands, const PassLists &L, Control *ctl, int par, uint2 *targets, Team team)
 {
 	const long long n = (long long)L.n_cand;
 	const int back = LATE_WARPS - 1 - (threadIdx.x >> 5), lane = threadIdx.x & 31;
-	for (long long base = 4 * ((long long)back * gridDim.x + blockIdx.x); base < n;
-	     base += 4ll * LATE_WARPS * gridDim.x) { // warp-uniform
+	for (long long base = 4 * ((long long)back * team.blocks + team.block); base < n;
+	     base += 4ll * LATE_WARPS * team.blocks) { // warp-uniform
 		const long long e = base + (lane >> 3);
 		const uint2 t = e < n ? cands[e] : make_uint2(0u, 0u);
 		const FrameDesc &fd = frames[t.x];
@@ -510,10 +577,10 @@ __device__ __forceinline__ void late_grow(const FrameDesc *__restrict__ frames, 
 
 // Stage 4: the growth, and the low list's pixels near a CAND pixel, a warp each.
 __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, FrameState *state,
-	const uint2 *cands, const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par, uint2 *targets,
-	LateQueue &Q, double *P, double *S)
+	const uint2 *cands, const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par,
+	uint2 *targets, LateQueue &Q, Team team, double *P, double *S)
 {
-	block_sweep((long long)L.n_low, Q, [&](long long e) {
+	block_sweep([&] { return (long long)L.n_low; }, Q, team, [&](long long e) {
 		const uint2 t = low[e];
 		const FrameDesc &fd = frames[t.x];
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
@@ -521,7 +588,7 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 		return low_near(fd, x, y);
 	}, [&](long long e) {
 		low_eval<PATH_ANY>(frames, state, low[e], prm, ctl, par, targets, P, S, false);
-	}, [&] { late_grow(frames, state, cands, L, ctl, par, targets); });
+	}, [&] { late_grow(frames, state, cands, L, ctl, par, targets, team); });
 }
 
 // Stage 5: the replacement, by warps (few targets are left to do).  A target
@@ -531,10 +598,11 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 // windows still hold none, the same window holds the same donors, and the same
 // median would come out.  A new target is itself a FRESH pixel.
 __device__ __forceinline__ void late_replace(const FrameDesc *__restrict__ frames, const FrameState *state,
-	int par, const uint2 *targets, long long n, long long fresh0, uint8_t *radius, unsigned *chg,
-	unsigned long long *n_chg, LateQueue &Q)
+	int par, const uint2 *targets, const Control *ctl, uint8_t *radius, unsigned *chg, unsigned long long *n_chg,
+	LateQueue &Q, Team team)
 {
-	block_sweep(n, Q, [&](long long e) {
+	const long long fresh0 = (long long)ctl->fresh0;
+	block_sweep([&] { return (long long)ctl->n_targets; }, Q, team, [&](long long e) {
 		const uint2 t = targets[e];
 		const int r = radius[e]; // (a new target's is not set yet)
 		if (!replaces(state[t.x], par))
@@ -577,7 +645,8 @@ late_neighbours_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, C
 			fd.floors[(jb.y0 >> 5) * ((fd.w + 31) >> 5) + (jb.x0 >> 5)].thr =
 				block_threshold(fd, jb.x0 >> 5, jb.y0 >> 5, prm.mode, tmin2);
 	}
-	late_neighbours<LN_THREADS / 32>(frames, targets, chg, ctl->pass[1], prm.mode, cands, low, eval, slots);
+	late_neighbours<LN_THREADS / 32>(frames, targets, chg, ctl->pass[1], prm.mode, cands, low, eval, slots,
+		whole_grid());
 }
 
 // MODEL: the batch has noise-model frames (launch_late has the choice of parts).
@@ -588,7 +657,8 @@ late_classes_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, Cont
 {
 	constexpr bool QUEUED = PART != LATE_TESTS;
 	__shared__ uint2 queue[QUEUED ? 8 : 1][64];
-	late_classes<PART, MODEL>(frames, eval, prm, ctl->pass[1], cands, low, queue[QUEUED ? threadIdx.x >> 5 : 0]);
+	late_classes<PART, MODEL>(frames, eval, prm, ctl->pass[1], cands, low, queue[QUEUED ? threadIdx.x >> 5 : 0],
+		whole_grid());
 }
 
 struct LateShared {
@@ -599,8 +669,8 @@ struct LateShared {
 	ListSlots slots;
 };
 
-// Passes 1 .. maxiter - 1 (the full pass is number 0), the first of them from
-// stage 3.  cands: the high list; low, eval: buffers of as many entries as the
+// Passes 1 .. maxiter - 1 (the full pass is number 0; maxiter >= 2), the first of
+// them from stage 3.  cands: the high list; low, eval: buffers of as many entries as the
 // batch has pixels (the first pass's pre list, which is done with); chg: the
 // changed targets' indices.
 __global__ void __launch_bounds__(LATE_THREADS, 1)
@@ -611,35 +681,52 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 	extern __shared__ __align__(16) unsigned char late_smem[];
 	LateShared &S = *reinterpret_cast<LateShared *>(late_smem);
 	const int warp = threadIdx.x >> 5;
-	const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+	__shared__ Team team;
+	__shared__ struct {
+		int any;
+		unsigned long long n_chg;
+		long long n_cand;
+	} begin;
+	if (threadIdx.x == 32) { // beside the join: these change only after the team's first barrier
+		begin.any = *(volatile int *)&ctl->any[0];
+		begin.n_chg = *(volatile unsigned long long *)&ctl->pass[1].n_chg;
+		begin.n_cand = *(volatile long long *)&ctl->pass[1].n_cand;
+	}
+	__shared__ BarrierState barrier;
+	if (threadIdx.x == 0)
+		barrier.calls = 0;
+	if (!join_team(ctl, team))
+		return;
+	const bool first = team.block == 0 && threadIdx.x == 0;
 	double (*triples)[63] = reinterpret_cast<double (*)[63]>(&S.scratch[warp][0]);
 	static_assert(3 * 63 <= CS_RUNS, "the triples fit the runs' scratch");
-	unsigned round = 0;
-	for (int it = 1; it < maxiter; ++it) {
+	// Whether the loop ends before the pass of parity par: every frame stopped after
+	// the last pass, or its replacement changed no value, so that this pass would
+	// repeat it and find nothing new.
+	auto ends = [&](int any, unsigned long long n_chg, int par, unsigned blocks) {
+		if (any && !n_chg)
+			pass_control(state, nf, ctl, par, Team{team.block, blocks});
+		return !any || !n_chg;
+	};
+	if (ends(begin.any, begin.n_chg, 1, gridDim.x))
+		return; // (nobody closes the team)
+	for (int it = 1;; ++it) {
 		const int par = it & 1;
 		PassLists &L = ctl->pass[par], &next = ctl->pass[par ^ 1];
-		if (!*(volatile int *)&ctl->any[par ^ 1])
-			return; // every frame stopped after the last pass
-		if (!*(volatile unsigned long long *)&L.n_chg) {
-			// The last replacement changed no value: this pass repeats it, and
-			// finds nothing new.
-			pass_control(state, nf, ctl, par);
-			return;
-		}
 		if (it > 1) {
-			late_neighbours<LATE_WARPS>(frames, targets, chg, L, prm.mode, cands, low, eval, S.slots);
+			late_neighbours<LATE_WARPS>(frames, targets, chg, L, prm.mode, cands, low, eval, S.slots, team);
 			// The last growth's FRESH bits: its replacement is done.
-			for (long long i = (long long)ctl->fresh0 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
-			     i < (long long)ctl->n_targets; i += (long long)gridDim.x * blockDim.x) {
+			for (long long i = (long long)ctl->fresh0 + team.block * (long long)blockDim.x + threadIdx.x;
+			     i < (long long)ctl->n_targets; i += (long long)team.blocks * blockDim.x) {
 				const uint2 t = targets[i];
 				const FrameDesc &fd = frames[t.x];
 				plane_ptr(fd, P_FRESH)[(long long)(t.y / (unsigned)fd.w) * fd.words +
 					((t.y % (unsigned)fd.w) >> 5)] = 0u;
 			}
-			if (!grid_barrier(ctl, ++round, state, nf, bw))
+			if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 				return;
-			late_classes<LATE_SHORT>(frames, eval, prm, L, cands, low, S.queue[warp]);
-			if (!grid_barrier(ctl, ++round, state, nf, bw))
+			late_classes<LATE_SHORT>(frames, eval, prm, L, cands, low, S.queue[warp], team);
+			if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 				return;
 		}
 		if (first) { // what the coming stages and the next pass append to
@@ -647,16 +734,27 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 			next = PassLists{};
 			ctl->any[par] = 0;
 		}
-		late_candidates(frames, cands, prm, L, S.Q, S.patches[warp], S.scratch[warp], triples);
-		if (!grid_barrier(ctl, ++round, state, nf, bw))
+		// Its share; in the first pass of the grid's shares, then of those whose
+		// blocks did not come.
+		Team part{team.block, it > 1 ? team.blocks : gridDim.x};
+		do { // block-uniform (the sweep keeps its team, which saves registers across it)
+			late_candidates(frames, cands, prm, [&] { return it > 1 ? (long long)L.n_cand : begin.n_cand; }, S.Q,
+				part, S.patches[warp], S.scratch[warp], triples);
+			if (it == 1 && S.Q.team.block == team.block)
+				close_team(ctl, team);
+			part = Team{S.Q.team.block + team.blocks, S.Q.team.blocks};
+		} while (part.block < part.blocks);
+		if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 			return;
-		late_low(frames, state, cands, low, prm, L, ctl, par, targets, S.Q, S.patches[warp], S.scratch[warp]);
-		if (!grid_barrier(ctl, ++round, state, nf, bw))
+		late_low(frames, state, cands, low, prm, L, ctl, par, targets, S.Q, team, S.patches[warp], S.scratch[warp]);
+		if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 			return;
-		pass_control(state, nf, ctl, par);
-		late_replace(frames, state, par, targets, (long long)ctl->n_targets, (long long)ctl->fresh0, radius,
-			chg, &next.n_chg, S.Q);
-		if (it + 1 < maxiter && !grid_barrier(ctl, ++round, state, nf, bw))
+		pass_control(state, nf, ctl, par, team);
+		late_replace(frames, state, par, targets, ctl, radius, chg, &next.n_chg, S.Q, team);
+		if (it + 1 >= maxiter || !grid_barrier(ctl, barrier, state, nf, bw, team))
+			return;
+		const int any = *(volatile int *)&ctl->any[par];
+		if (ends(any, *(volatile unsigned long long *)&next.n_chg, par ^ 1, team.blocks))
 			return;
 	}
 }
