@@ -49,10 +49,12 @@ struct InvalidArgument : std::invalid_argument {
 
 static void check(cudaError_t e)
 {
+	if (e == cudaSuccess)
+		return;
+	cudaGetLastError(); // the failure is reported here, not by the next call's check of its launches
 	if (e == cudaErrorMemoryAllocation)
 		throw std::bad_alloc();
-	if (e != cudaSuccess)
-		throw std::runtime_error(cudaGetErrorString(e));
+	throw std::runtime_error(cudaGetErrorString(e));
 }
 
 // Injected failures (cusmic_inject_fault): the bounds of the injected device
