@@ -27,6 +27,7 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
+#include <exception>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -487,6 +488,22 @@ struct Lease {
 	}
 	Workspace *operator->() { return ws.get(); }
 	Workspace &operator*() { return *ws; }
+};
+
+// Waits for a stream when an exception leaves its scope: the workspace of a call
+// goes back to the pool, and the caller's buffers to the caller, only when nothing
+// reads or writes them any more.  (Declared after the lease, so destroyed first.)
+struct DrainOnError {
+	cudaStream_t s;
+	int before = std::uncaught_exceptions();
+	explicit DrainOnError(cudaStream_t stream) : s(stream) {}
+	~DrainOnError()
+	{
+		if (std::uncaught_exceptions() > before) {
+			cudaStreamSynchronize(s);
+			cudaGetLastError();
+		}
+	}
 };
 
 // Options and scalars of frame f after per-frame overrides.
@@ -1137,6 +1154,7 @@ static void run_device(const cusmic_image *ims, size_t nf, const cusmic_options 
 	const MapChecks checks = map_checks(maps, nmaps, &check_blocks, di);
 	Layout L = make_layout(ims, nf, o, sc, clean, mask, di);
 	Lease ws(dev);
+	DrainOnError drain(s);
 	upload(*ws, L, s);
 	enqueue_plain(*ws, L, di, s);
 	if (nmaps) // after the call's kernels, whose first one cleared the flags
@@ -1180,6 +1198,7 @@ extern "C" int remove_cosmics(const cusmic_image *im, const cusmic_options *o, d
 		ws->hclean.ensure(n);
 		ws->hout.ensure(n);
 		cudaStream_t s = nullptr;
+		DrainOnError drain(s);
 		ws->stage_io.in(ws->hdata.p, im->data, n * sizeof(double), s);
 		cusmic_image gpu = *im;
 		gpu.data = ws->hdata.p;
@@ -1280,6 +1299,7 @@ extern "C" int cusmic_check_maps(const cusmic_map_check *maps, size_t nmaps, uns
 		const MapChecks checks = map_checks(maps, nmaps, &blocks, di);
 		const cudaStream_t s = (cudaStream_t)stream;
 		Lease ws(dev);
+		DrainOnError drain(s);
 		ws->hflags.ensure(2);
 		ws->hflags_host.ensure(2);
 		check(cudaMemsetAsync(ws->hflags.p, 0, sizeof(unsigned), s));
@@ -1859,15 +1879,18 @@ extern "C" int cusmic_plan_execute(cusmic_plan *p, void *stream, char *msg, size
 		if (!p)
 			throw InvalidArgument("invalid plan");
 		cudaStream_t s = (cudaStream_t)stream;
+		const size_t nf = p->L.frames.size();
+		p->ws.hstate.ensure(nf);
+		// Whatever of the execution was queued when a step failed, the plan's next
+		// call waits for it.
+		p->last = s;
+		p->executed = false;
 		if (p->exec)
 			check(cudaGraphLaunch(p->exec, s));
 		else
 			enqueue_plain(p->ws, p->L, p->di, s);
-		const size_t nf = p->L.frames.size();
-		p->ws.hstate.ensure(nf);
 		check(cudaMemcpyAsync(p->ws.hstate.p, p->ws.state.p, nf * sizeof(FrameState),
 			cudaMemcpyDeviceToHost, s));
-		p->last = s;
 		p->executed = true;
 	}, msg, len);
 }
@@ -1913,12 +1936,13 @@ extern "C" int cusmic_plan_profile(cusmic_plan *p, void *stream, double *ms, int
 			throw InvalidArgument("invalid plan or profile buffers");
 		cudaStream_t s = (cudaStream_t)stream;
 		Recorder rec;
-		enqueue_plain(p->ws, p->L, p->di, s, &rec);
 		const size_t nf = p->L.frames.size();
 		p->ws.hstate.ensure(nf);
+		p->last = s;
+		p->executed = false;
+		enqueue_plain(p->ws, p->L, p->di, s, &rec);
 		check(cudaMemcpyAsync(p->ws.hstate.p, p->ws.state.p, nf * sizeof(FrameState),
 			cudaMemcpyDeviceToHost, s));
-		p->last = s;
 		p->executed = true;
 		check(cudaStreamSynchronize(s));
 		for (int k = 0; k < kinds; ++k) {
@@ -1951,6 +1975,7 @@ extern "C" int cusmic_plan_backward(cusmic_plan *p, const double *grad_clean, do
 		for (const FrameDesc &d : p->L.frames)
 			map_mode |= d.bg_map != nullptr;
 		cudaStream_t s = (cudaStream_t)stream;
+		DrainOnError drain(s);
 		const Layout &L = p->L;
 		const int nrows = (int)L.rows.size();
 		if (grad_background && !map_mode)
