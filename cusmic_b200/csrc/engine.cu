@@ -389,6 +389,9 @@ struct Layout {
 	// depends on the buffers' alignment (a rebound plan whose choice changes
 	// is captured again).
 	bool fused = false;
+	// Some output mask takes an input mask's place: the masks are zeroed after
+	// prepare has read the inputs, not in the first launch (captured again likewise).
+	bool mask_in_place = false;
 	cusmic_tuning tune{};
 	long long poison_wait[3] = {0, 0, 0}; // injected failures in force when the batch was laid out
 };
@@ -594,12 +597,18 @@ static int item_rows(const cusmic_image *ims, size_t nf, int target_items)
 	return rows;
 }
 
-// Whether prep_detect_kernel suits every frame of a batch (see Layout).
+// What depends on the batch's buffers: whether prep_detect_kernel suits every frame,
+// and where the output masks are zeroed (see Layout).
 static void choose_kernels(Layout &L)
 {
 	L.fused = L.maxiter > 0;
-	for (const FrameDesc &fd : L.frames)
+	L.mask_in_place = false;
+	const uintptr_t out = (uintptr_t)L.frames[0].mask_out, out_end = out + L.total_px;
+	for (const FrameDesc &fd : L.frames) {
 		L.fused = L.fused && prep_detect_ok(fd);
+		const uintptr_t in = (uintptr_t)fd.mask;
+		L.mask_in_place = L.mask_in_place || (in && in < out_end && in + (size_t)fd.w * fd.h > out);
+	}
 }
 
 static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_options &o,
@@ -997,7 +1006,12 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		P_ROWMIN == N_PLANES - 1, "plane order");
 	const long long z16 = (long long)(P_ROWMIN - P_CRMASK) * L.plane_words / 4;
 	const ZeroRange zero{reinterpret_cast<uint4 *>(ws.bits.p + P_CRMASK * L.plane_words), z16,
-		ws.frames.p, (long long)L.total_px};
+		ws.frames.p, L.mask_in_place ? 0ll : (long long)L.total_px};
+	auto zero_later = [&] {
+		if (L.mask_in_place)
+			zero_masks_kernel<<<grid_for_rows(di, (L.total_px + 511) / 512), 256, 0, s>>>(
+				ZeroRange{nullptr, 0, ws.frames.p, (long long)L.total_px});
+	};
 	const long long zb = (std::max(z16, zero.bytes / 16) + 255) / 256, fb = (nf + 255) / 256,
 		zcap = (long long)di.sms * 8;
 	if (L.fused) {
@@ -1013,6 +1027,7 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		const int nbulk = (int)L.bulk.size(), pcap = di.sms * PD_BLOCKS_PER_SM;
 		prep_detect_kernel<<<nbulk < pcap ? nbulk : pcap, BK_THREADS, 0, s>>>(ws.frames.p, ws.state.p,
 			ws.bulk.p, nbulk, L.prm, ws.ctl.p, ws.cands.p, ws.pre.p, ws.pre_counts.p);
+		zero_later();
 		mark(rec, K_PREPARE);
 		fill_list_kernel<<<di.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(ws.frames.p, ws.state.p,
 			ws.cands.p, &ws.ctl.p->n_holes);
@@ -1023,6 +1038,7 @@ static void launch_prologue(Workspace &ws, const Layout &L, const DeviceInfo &di
 		L.maxiter, (unsigned long long)L.total_px, L.poison_wait[0], L.poison_wait[1], zero);
 	mark(rec, K_INIT); // the state and the zeroed planes
 	launch_prepare(ws, L, di, s);
+	zero_later();
 	mark(rec, K_PREPARE);
 	// Block floors: error-map thresholds; noise-model keys from prepare's row
 	// minima of the non-hole pixels, which the hole fill and every later
@@ -1854,10 +1870,12 @@ extern "C" int cusmic_plan_bind(cusmic_plan *p, const cusmic_image *ims, double 
 		}
 		p->ims.assign(ims, ims + nf);
 		p->L.frames = L.frames;
-		// New buffers can change whether prep_detect_kernel suits the batch:
-		// the graph is captured again with the new choice.
-		const bool recapture = L.fused != p->L.fused;
+		// New buffers can change whether prep_detect_kernel suits the batch, and
+		// where the masks are zeroed: the graph is captured again with the new
+		// choice.
+		const bool recapture = L.fused != p->L.fused || L.mask_in_place != p->L.mask_in_place;
 		p->L.fused = L.fused;
+		p->L.mask_in_place = L.mask_in_place;
 		const size_t bytes = nf * sizeof(FrameDesc);
 		std::memcpy(p->ws.stage.p, p->L.frames.data(), bytes);
 		check(cudaMemcpyAsync(p->ws.frames.p, p->ws.stage.p, bytes, cudaMemcpyHostToDevice,

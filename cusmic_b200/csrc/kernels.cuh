@@ -139,6 +139,33 @@ struct ZeroRange {
 	long long bytes;
 };
 
+// The masks of that: the aligned body by 16 bytes, the ends byte by byte.
+__device__ __forceinline__ void zero_masks(const ZeroRange &z)
+{
+	if (!z.bytes)
+		return;
+	const long long stride = (long long)gridDim.x * blockDim.x;
+	const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+	uint8_t *mask = z.frames[0].mask_out;
+	const long long head = min(z.bytes, (long long)(-(uintptr_t)mask & 15u));
+	const long long body = (z.bytes - head) / 16, tail = z.bytes - head - 16 * body;
+	uint4 *m16 = reinterpret_cast<uint4 *>(mask + head);
+	for (long long j = first; j < body; j += stride)
+		m16[j] = make_uint4(0u, 0u, 0u, 0u);
+	if (first < head)
+		mask[first] = 0;
+	if (first < tail)
+		mask[head + 16 * body + first] = 0;
+}
+
+// The same in a launch of its own, after prepare: for a batch whose output masks
+// take an input mask's place.
+__global__ void __launch_bounds__(256)
+zero_masks_kernel(ZeroRange z)
+{
+	zero_masks(z);
+}
+
 // Per-frame state and loop control of a call, and the zeroing, with grid-stride
 // loops of 16-byte stores.
 __device__ __forceinline__ void init_state(FrameState *state, int nf, Control *ctl, int maxiter,
@@ -148,18 +175,7 @@ __device__ __forceinline__ void init_state(FrameState *state, int nf, Control *c
 	const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
 	for (long long j = first; j < z.n16; j += stride)
 		z.planes[j] = make_uint4(0u, 0u, 0u, 0u);
-	if (z.bytes) { // the aligned body by 16 bytes, the ends byte by byte
-		uint8_t *mask = z.frames[0].mask_out;
-		const long long head = min(z.bytes, (long long)(-(uintptr_t)mask & 15u));
-		const long long body = (z.bytes - head) / 16, tail = z.bytes - head - 16 * body;
-		uint4 *m16 = reinterpret_cast<uint4 *>(mask + head);
-		for (long long j = first; j < body; j += stride)
-			m16[j] = make_uint4(0u, 0u, 0u, 0u);
-		if (first < head)
-			mask[first] = 0;
-		if (first < tail)
-			mask[head + 16 * body + first] = 0;
-	}
+	zero_masks(z);
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i < nf) {
 		FrameState s = {};
