@@ -101,6 +101,7 @@ class _Checks:
     def __init__(self):
         self.items = []   # (name, index of its map or None, failed bits of a scalar)
         self.tensors = []  # the maps, contiguous
+        self.failed = False  # report() raised
 
     def add(self, name, value):
         minimum, _ = self.RULES[name]
@@ -127,6 +128,7 @@ class _Checks:
         for name, index, bits in self.items:
             if index is not None:
                 bits = flags >> (2 * index) & 3
+            self.failed = bits != 0
             if bits & 1:
                 raise ValueError(f"{name} must be finite")
             if bits & 2:
@@ -325,5 +327,6 @@ def remove_cosmics(
                 raise ValueError("Provide error, or both effective_gain and readnoise")
             return cleaner._clean(data, fields, mask, checks)
         except Exception:
-            checks.run()
+            if not checks.failed:  # the call failed before, or apart from, its checks
+                checks.run()
             raise
