@@ -120,6 +120,12 @@ class _Checks:
             arr[i] = _native.MapCheck(t.data_ptr(), t.numel(), self.RULES[name][0])
         return arr, len(self.tensors)
 
+    def contiguous(self, fields):
+        """The calibration with the maps as the checks read them, so that a map
+        that is not contiguous is copied once."""
+        return {name: fields[name] if index is None else self.tensors[index]
+                for name, index, _ in self.items}
+
     @property
     def scalar_failed(self):
         return any(bits for _, _, bits in self.items)
@@ -325,7 +331,7 @@ def remove_cosmics(
             if maxiter and error is None and ("effective_gain" not in fields or
                                               "readnoise" not in fields):
                 raise ValueError("Provide error, or both effective_gain and readnoise")
-            return cleaner._clean(data, fields, mask, checks)
+            return cleaner._clean(data, checks.contiguous(fields), mask, checks)
         except Exception:
             if not checks.failed:  # the call failed before, or apart from, its checks
                 checks.run()

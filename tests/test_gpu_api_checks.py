@@ -32,3 +32,32 @@ def test_failing_map_is_checked_once(cuda, monkeypatch):
     with pytest.raises(ValueError, match="error must be positive"):
         remove_cosmics(data, -1, 5, 3, error=error)  # rejected before anything runs
     assert lib.calls.get("cusmic_check_maps") == 1
+
+
+@pytest.mark.parametrize("call", ("plain", "differentiable"))
+def test_strided_map_is_copied_once(cuda, call):
+    """The checks and the cleaning share the contiguous copy of a map that is a
+    transposed view; the results are those of the copy itself."""
+    from cusmic_b200 import remove_cosmics
+    from cusmic_b200.autograd import remove_cosmics_differentiable
+    run = remove_cosmics if call == "plain" else remove_cosmics_differentiable
+    gen = cuda.Generator(device="cuda")
+    gen.manual_seed(4)
+    h, w = 1000, 1200
+    data = 200 + 12 * cuda.randn((h, w), generator=gen, dtype=cuda.float64, device="cuda")
+    data[cuda.rand((h, w), generator=gen, device="cuda") < 4e-3] += 900
+    strided = (12 + cuda.rand((w, h), generator=gen, dtype=cuda.float64, device="cuda")).T
+
+    def peak(error):
+        cuda.cuda.synchronize()
+        cuda.cuda.reset_peak_memory_stats()
+        before = cuda.cuda.memory_allocated()
+        out = run(data, 3, 5, 3, error=error)
+        cuda.cuda.synchronize()
+        return cuda.cuda.max_memory_allocated() - before, out
+    peak(strided.contiguous())
+    own, (clean, mask) = peak(strided.contiguous())
+    copied, (clean2, mask2) = peak(strided)
+    assert bool(mask.any()) and cuda.equal(mask, mask2) and cuda.equal(clean, clean2)
+    # (A contiguous argument's own memory is not in its call's count.)
+    assert copied - own <= 8 * h * w + (1 << 20)
