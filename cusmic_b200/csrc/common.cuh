@@ -167,8 +167,9 @@ struct Control {
 	int any[2];                   // by parity: a frame goes on after the pass
 	int ticket;                   // next item of the bulk detection kernel
 	unsigned pad;
-	int fault;                    // a bounded wait ran out (FaultBit); read together with
-	unsigned barrier;             // the arrivals at the late passes' grid barriers
+	// Read as one 16-byte word by grid_barrier:
+	alignas(16) int fault;        // a bounded wait ran out (FaultBit)
+	unsigned barrier;             // arrivals at the late passes' grid barriers
 	unsigned arrived;             // blocks of the late passes that started (join_team)
 	unsigned team;                // how many of them work, once that is closed
 	// Injected failures (0: none): the bound, in SM cycles, of one extra wait
@@ -177,10 +178,8 @@ struct Control {
 	long long poison_wait[2];
 };
 
-static_assert(offsetof(Control, fault) % 8 == 0 && offsetof(Control, barrier) == offsetof(Control, fault) + 4,
-	"grid_barrier reads the fault and the arrivals as one word");
-static_assert(offsetof(Control, arrived) % 8 == 0 && offsetof(Control, team) == offsetof(Control, arrived) + 4,
-	"join_team reads both as one word");
+static_assert(offsetof(Control, fault) % 16 == 0 && offsetof(Control, team) == offsetof(Control, fault) + 12,
+	"grid_barrier reads the four as one word");
 
 // The blocks that share a launch's work: this one's number and how many there are
 // (all of the grid's, except in the late passes).

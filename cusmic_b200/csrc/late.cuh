@@ -60,7 +60,9 @@
 namespace cb {
 
 // One block of 32 warps per SM: the fewest arrivals at a grid barrier for the
-// warps that 64 registers a thread allow.
+// warps that 64 registers a thread allow.  (The candidate evaluation and the
+// replacement want more: a 176-byte stack frame, 176 bytes of spill stores and 348
+// of loads a thread.)
 constexpr int LATE_THREADS = 1024;
 constexpr int LATE_WARPS = LATE_THREADS / 32;
 
@@ -83,14 +85,14 @@ constexpr long long BARRIER_CYCLES = 1LL << 35;
 
 // The late launch's team: the blocks that have started when it is closed.  A block
 // joins with its number (the order of the starts) and takes the first stage's share
-// of that number among gridDim.x; close_team, after that, closes the team once the
-// whole grid has started, or JOIN_CYCLES (about 17 us) after the first block is done,
-// and the team's blocks do the missing shares.  So only running blocks meet at
-// the barriers, and the launch needs no more SMs than are free: beside another
-// stream's kernel that stays, or on a context with part of the SMs, a cooperative
-// launch (whose blocks all have to fit at once) waits or is refused.  A block that
-// comes too late leaves at once.  (Closing the team before the first stage cost
-// every call the 2 us between the first block's start and the last one's.)
+// of that number among gridDim.x; the first barrier closes the team once the whole
+// grid has started, or JOIN_CYCLES (about 17 us) after the first block got there, and
+// the team's blocks do the missing shares.  So only running blocks meet at the
+// barriers, and the launch needs no more SMs than are free: beside another stream's
+// kernel that stays, or on a context with part of the SMs, a cooperative launch
+// (whose blocks all have to fit at once) waits or is refused.  A block that comes
+// too late leaves at once.  (Closing the team before the first stage cost every call
+// the 2 us between the first block's start and the last one's.)
 constexpr long long JOIN_CYCLES = 1 << 15;
 constexpr unsigned TEAM_CLOSED = 1u << 31; // in Control::arrived
 
@@ -98,66 +100,54 @@ constexpr unsigned TEAM_CLOSED = 1u << 31; // in Control::arrived
 __device__ __forceinline__ bool join_team(Control *ctl, Team &team)
 {
 	if (threadIdx.x == 0)
-		team.block = atomicAdd(&ctl->arrived, 1u);
+		team = Team{atomicAdd(&ctl->arrived, 1u), 0u};
 	__syncthreads();
 	return !(team.block & TEAM_CLOSED);
 }
 
-// Sets the closed team's size (called by every block that joined).
-__device__ __forceinline__ void close_team(Control *ctl, Team &team)
-{
-	if (threadIdx.x == 0) {
-		unsigned n = 0;
-		const long long t0 = clock64();
-		do {
-			// The arrivals in the low half, the closed team's size in the high one.
-			const unsigned long long v = *(volatile unsigned long long *)&ctl->arrived;
-			const unsigned here = (unsigned)v;
-			const long long waited = clock64() - t0;
-			n = here & TEAM_CLOSED ? (unsigned)(v >> 32) : here == gridDim.x ? here : 0u;
-			if (!n && team.block == 0 && waited > JOIN_CYCLES) {
-				n = atomicOr(&ctl->arrived, TEAM_CLOSED);
-				*(volatile unsigned *)&ctl->team = n;
-			}
-			if (waited > BARRIER_CYCLES)
-				n = gridDim.x; // (the first block is long done; the barrier will fault)
-		} while (!n);
-		team.blocks = n;
-	}
-	__syncthreads();
-}
-
 // Barrier of the team: the k-th call returns once every block has arrived k times,
-// with their earlier writes visible (B.calls starts zero).  A wait that runs out
-// faults every frame and returns false, and so do the barrier's other blocks that
-// see the fault (the last one to arrive, whose own wait is over at once, among
-// them) and every later barrier.
+// with their earlier writes visible (B.calls starts zero); the first one sets the
+// team's size.  A wait that runs out faults every frame and returns false, and so do
+// the barrier's other blocks that see the fault (the last one to arrive, whose own
+// wait is over at once, among them) and every later barrier.
 struct BarrierState {
 	unsigned calls;
 	int open;
 };
 
 __device__ __forceinline__ bool grid_barrier(Control *ctl, BarrierState &B, FrameState *state, int nf,
-	const BarrierWait &bw, const Team &team)
+	const BarrierWait &bw, Team &team)
 {
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		__threadfence();
 		atomicAdd(&ctl->barrier, 1u);
-		const unsigned want = ++B.calls * team.blocks + bw.missing;
+		const unsigned call = ++B.calls;
+		unsigned n = team.blocks;
 		const long long t0 = clock64();
 		bool ok;
 		for (;;) {
-			// The fault in the low half, the arrivals in the high one.
-			const unsigned long long v = *(volatile unsigned long long *)&ctl->fault;
-			ok = (unsigned)v == 0;
-			if (!ok || (int)((unsigned)(v >> 32) - want) >= 0)
+			unsigned fault, count, here, size; // one round trip
+			asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];\n"
+				: "=r"(fault), "=r"(count), "=r"(here), "=r"(size)
+				: "l"(__cvta_generic_to_global(&ctl->fault))
+				: "memory");
+			const long long waited = clock64() - t0;
+			if (!n)
+				n = here & TEAM_CLOSED ? size : here == gridDim.x ? here : 0u;
+			if (!n && team.block == 0 && waited > JOIN_CYCLES) {
+				n = atomicOr(&ctl->arrived, TEAM_CLOSED);
+				*(volatile unsigned *)&ctl->team = n;
+			}
+			ok = fault == 0;
+			if (!ok || (n && (int)(count - call * n - bw.missing) >= 0))
 				break;
-			if (clock64() - t0 > bw.limit) {
+			if (waited > bw.limit) {
 				ok = false;
 				break;
 			}
 		}
+		team.blocks = n;
 		if (!ok) {
 			atomicOr(&ctl->fault, FAULT_BARRIER);
 			for (int f = 0; f < nf; ++f)
@@ -499,8 +489,7 @@ template <class Count, class Keep, class Work, class Aside>
 __device__ __forceinline__ void block_sweep(Count count, LateQueue &Q, Team team, Keep keep, Work work, Aside aside)
 {
 	const int warp = threadIdx.x >> 5;
-	__syncthreads(); // an earlier sweep's reads of Q
-	if (threadIdx.x == 0) {
+	if (threadIdx.x == 0) { // (a barrier of the team lies between two sweeps)
 		const long long n = count(), share = (n + team.blocks - 1) / team.blocks;
 		Q.chunk = share < LATE_THREADS ? (int)share : LATE_THREADS;
 		Q.team = team;
@@ -734,18 +723,17 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 			next = PassLists{};
 			ctl->any[par] = 0;
 		}
-		// Its share; in the first pass of the grid's shares, then of those whose
-		// blocks did not come.
-		Team part{team.block, it > 1 ? team.blocks : gridDim.x};
-		do { // block-uniform (the sweep keeps its team, which saves registers across it)
-			late_candidates(frames, cands, prm, [&] { return it > 1 ? (long long)L.n_cand : begin.n_cand; }, S.Q,
-				part, S.patches[warp], S.scratch[warp], triples);
-			if (it == 1 && S.Q.team.block == team.block)
-				close_team(ctl, team);
-			part = Team{S.Q.team.block + team.blocks, S.Q.team.blocks};
-		} while (part.block < part.blocks);
-		if (!grid_barrier(ctl, barrier, state, nf, bw, team))
-			return;
+		// The block's share; in the first pass of the grid's shares, then of those
+		// whose blocks did not come, a barrier after each round.
+		do { // block-uniform
+			const unsigned share = (it > 1 ? 0u : barrier.calls * team.blocks) + team.block;
+			const unsigned shares = it > 1 ? team.blocks : gridDim.x;
+			if (share < shares)
+				late_candidates(frames, cands, prm, [&] { return it > 1 ? (long long)L.n_cand : begin.n_cand; },
+					S.Q, Team{share, shares}, S.patches[warp], S.scratch[warp], triples);
+			if (!grid_barrier(ctl, barrier, state, nf, bw, team))
+				return;
+		} while (it == 1 && barrier.calls * team.blocks < gridDim.x);
 		late_low(frames, state, cands, low, prm, L, ctl, par, targets, S.Q, team, S.patches[warp], S.scratch[warp]);
 		if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 			return;
