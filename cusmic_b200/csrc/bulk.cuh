@@ -48,7 +48,7 @@
 // arrives when it is done with the row.  The producer computes the copies of
 // an item's rows once per item (they differ by row offsets only), so its
 // per-row work is a wait on the row's empty barrier and the issue.  (The S1, S2 and
-// CAND planes were zeroed by the call's prologue memset.)  A block takes items
+// CAND planes were zeroed by the call's first launch.)  A block takes items
 // of BK_COLS x BK_ROWS pixels from a ticket counter (items of frames that
 // stopped are skipped there) and the ring runs straight through from one item
 // into the next.
@@ -76,7 +76,7 @@
 // columns (zeros in constant mode), so the evaluation has no border cases.
 //
 // Every wait is bounded (about one second of SM clock).  A wait that runs out
-// sets Control::fault (the loop-control kernel then stops every active frame
+// sets Control::fault (pass_control then stops every active frame
 // and marks it faulted; the host reports CUSMIC_CUDA_ERROR) and the ring's
 // abort word, which ends the block's other waits early; before the block
 // exits, its producer waits (again bounded) for the copies it still has in
@@ -437,9 +437,9 @@ __device__ __forceinline__ double model_threshold(const FrameDesc &fd, int bx, i
 static_assert(FLOOR_BLOCK == 32, "a bit word of a row lies in one floor block");
 
 // model_threshold of block (bx, by) of a noise-model frame; outside wrap mode
-// only the 3 x 3 neighbouring blocks count, read directly (sig_bulk_kernel of
-// 17 x 4096 x 4160 noise-model frames: 386 us with model_threshold's loops over
-// a wrapped range, 370 us).
+// only the 3 x 3 neighbouring blocks count, read directly (sig_bulk_kernel of 64
+// noise-model frames of 256 to 4096 pixels a side: 386 us with model_threshold's
+// loops over a wrapped range, 370 us).
 __device__ __forceinline__ double block_threshold(const FrameDesc &fd, int bx, int by, int mode,
 	double tmin2)
 {
@@ -621,27 +621,6 @@ __device__ __forceinline__ bool bulk_producer(BulkRing &R, const FrameDesc *__re
 		if (!bulk_rows(R, g, base, t, fd.w, fd.h, lm, mis, it.y, it.z, it.w,
 			[&](int slot, int, const BulkRow &b) { bulk_issue(R, slot, b, clean); }))
 			return false;
-	}
-}
-
-// Columns x - 1 .. x + 2 of a ring row (x = the pair's first column, at cell
-// c + shift; c even, so every 16-byte load is aligned).
-__device__ __forceinline__ void load_quad(const double *row, int c, int shift, double &l, double &a,
-	double &b, double &r)
-{
-	if (shift == 0) {
-		const double2 v = *reinterpret_cast<const double2 *>(row + c);
-		l = row[c - 1];
-		a = v.x;
-		b = v.y;
-		r = row[c + 2];
-	} else {
-		const double2 v0 = *reinterpret_cast<const double2 *>(row + c);
-		const double2 v1 = *reinterpret_cast<const double2 *>(row + c + 2);
-		l = v0.x;
-		a = v0.y;
-		b = v1.x;
-		r = v1.y;
 	}
 }
 

@@ -15,19 +15,20 @@
 //  * fine structure (med3 -> med7) is only read by detect behind
 //    `sig > cr_threshold` on a non-excluded pixel (src/filters.cuh:164-175).
 //
-// So a pass is three kernels:
-//   A  dense and HBM-bound: a division-free, median-free test that keeps a
-//      superset of the pixels whose sig_raw exceeds min(cr, neighbor), appended
-//      to a candidate list, and clearing of the S1/S2/CAND bit words.  With an
-//      error map (sig_stream_kernel) each warp walks a strip of 32 columns down
-//      the frame with a rolling 3-row register window; with the noise model
-//      (sig_model_kernel) a tile kernel bounds the noise from below by the
-//      tile's minimum;
-//   B  one warp per candidate: exact sig_raw over the 5 x 5 window (with the
-//      exact noise model where there is no error map), its median, sig, the
-//      S1/S2 bits and the candidate's seed slot;
-//   C  one warp per seed: 49 3 x 3 medians, their 7 x 7 median, the contrast
-//      test and the CAND bit.
+// So a pass has three steps:
+//   A  dense: a division-free, median-free test that keeps a superset of the
+//      pixels whose sig_raw exceeds min(cr, neighbor) in a candidate list.  The
+//      kernels of bulk.cuh and prep_detect.cuh do that; those below
+//      (sig_stream_kernel and sig_model_kernel, which also clear the S1/S2/CAND
+//      words) serve the call without device allocation only: with an error map
+//      each warp walks a strip of 32 columns down the frame with a rolling 3-row
+//      register window, with the noise model a tile kernel bounds the noise from
+//      below by the tile's minimum;
+//   B  a candidate: exact sig_raw over the 5 x 5 window (with the exact noise model
+//      where there is no error map), sig against both thresholds, the S1/S2 bits
+//      and the candidate's seed slot;
+//   C  a seed: the contrast test and the CAND bit, by counts over the 49 3 x 3
+//      windows, or from their medians where those leave it open.
 // Every value that feeds a threshold is computed in the reference's operation
 // order (no FMA), so the bits equal the reference's.
 //
@@ -49,7 +50,6 @@ namespace cb {
 
 struct DetectParams {
 	double contrast, cr, nb;
-	double tmin;  // min(cr, nb): sig_raw above it can pass a threshold
 	double thi2;  // 2 cr (1 - 1e-12): division-free superset test for sig_raw > cr
 	double tlo2;  // 2 nb (1 - 1e-12): the same for sig_raw > neighbor
 	double rcontrast; // 1 / contrast
@@ -1244,18 +1244,16 @@ seed_kernel(const FrameDesc *__restrict__ frames, const Seed *__restrict__ seeds
 // B and C fused, high list: one warp per candidate, and a candidate that is
 // a seed gets its fine-structure test from the same warp at once (it needs
 // only its own sig and noise and the clean pixels within 4), so no seed list
-// is walked.  PATH as for candidate_high_kernel (error-map frames use it;
-// noise-model candidates read the sig_raw map).  With
-// `seeds` (a batch that also runs seed_kernel) each served entry's slot is
-// marked empty.
-template <int PATH>
-__global__ void __launch_bounds__(256, PATH == PATH_ERROR ? 4 : 3)
+// is walked.  Error-map frames only: noise-model candidates run
+// candidate_map_kernel.  With `seeds` (a batch that also runs seed_kernel) each
+// served entry's slot is marked empty.
+__global__ void __launch_bounds__(256, 4)
 candidate_seed_kernel(const FrameDesc *__restrict__ frames, const uint2 *__restrict__ cands,
 	DetectParams prm, Control *ctl, Seed *seeds)
 {
-	// Error-map frames only: the scratch of candidate_sig holds just the 25
-	// values of the NaN rule, and the triples of the seed test serve as it.
-	static_assert(PATH == PATH_ERROR, "noise-model candidates run candidate_map_kernel");
+	// The scratch of candidate_sig holds just the 25 values of the NaN rule, and
+	// the triples of the seed test serve as it.
+	constexpr int PATH = PATH_ERROR;
 	__shared__ double patches[8][81];
 	__shared__ double triples[8][3][63];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -630,7 +630,6 @@ static Layout make_layout(const cusmic_image *ims, size_t nf, const cusmic_optio
 	L.prm.rcontrast = 1 / o.contrast;
 	L.prm.cr = o.cr_threshold;
 	L.prm.nb = o.neighbor_threshold;
-	L.prm.tmin = std::fmin(o.cr_threshold, o.neighbor_threshold);
 	L.prm.thi2 = 2 * o.cr_threshold * (1 - 1e-12);
 	L.prm.tlo2 = 2 * o.neighbor_threshold * (1 - 1e-12);
 	L.prm.mode = o.border;
@@ -874,7 +873,7 @@ static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 		mark(rec, K_SIGMAP);
 	}
 	if (L.error_frames)
-		candidate_seed_kernel<PATH_ERROR><<<sparse, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
+		candidate_seed_kernel<<<sparse, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
 			ws.ctl.p, model ? ws.seeds.p : nullptr);
 	if (model)
 		candidate_map_kernel<<<di.sms * MAP_BLOCKS_PER_SM, 256, 0, s>>>(ws.frames.p, ws.cands.p, L.prm,
@@ -899,7 +898,10 @@ static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 // The passes after the first (late.cuh): the first late pass's lists in two or
 // three launches, then one launch whose blocks meet at barriers, at most one block
 // for each SM (it fills one; those that find no free SM are left out).  Small
-// batches take fewer blocks, which makes the barriers cheaper.
+// batches take fewer blocks, which makes the barriers cheaper: one for 16384 pixels
+// (one for 4096 or 65536: the same within 8% from 128 x 128 to four frames of 2048 x
+// 2048, either side ahead), in the launches before it one for 4096 (1024 and 16384:
+// the same within 10%).
 static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cudaStream_t s,
 	Recorder *rec = nullptr)
 {
@@ -920,10 +922,11 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	uint8_t *radius = ws.radius.p;
 	unsigned *chg = ws.chg.p;
 	// The class of the noise-model frames' pixels near the first pass's
-	// targets: in parts with a thread per median from about 8 Mpixel (64 ragged
-	// frames, 178 Mpixel: 140 us against 301 with a warp per median; eight
-	// frames of 1024 x 1024: 19 and 18; five of 1018 x 1001: 20 and 15; 256 of
-	// 40 to 200 a side: 18 and 11).
+	// targets: in parts with a thread per median above 8 Mpixel, a warp per median
+	// below.  All passes after the first with the parts and with warps, in us, by the
+	// batch's size: 2.3 Mpixel (256 frames of 40 to 200 a side) 188, 176; 4 177, 174; 8
+	// 195, 186; 12 207, 199; 16 214, 215; 24 227, 238; 32 249, 264; 64 336, 389; 128
+	// 524, 647.  Between 8 and 16 Mpixel the two are within 5%.
 	const bool model = L.error_frames < nf, thresholds = model && L.total_px > 8u << 20;
 	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, prm, ctl, cands, low, eval,
 		targets, chg, ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
@@ -959,7 +962,9 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 // registers: 36 us for 5 x 1018 x 1001 frames against 41 with three blocks, 43
 // with 4 words and four), else three (16 x 2048 x 2047 error-map frames with
 // masks: 223 us, two blocks 267, 4 words 242).  Variants for one such kind each
-// were no faster.  Blocks come in several waves, which evens out rows of unequal
+// were no faster.  (The three-block variants of the deciding kernel spill 96 to 180
+// bytes, the 16-word one without outputs of its own 48; the choices above were timed
+// with that.)  Blocks come in several waves, which evens out rows of unequal
 // lengths (ragged frames, 16 words: 763 us with four blocks per SM in all, 713
 // with 8, 688 with 16).
 static void launch_prepare(Workspace &ws, const Layout &L, const DeviceInfo &di, cudaStream_t s)
@@ -2223,7 +2228,6 @@ extern "C" int remove_cosmics_device_noalloc(const cusmic_image *im, const cusmi
 		prm.rcontrast = 1 / o->contrast;
 		prm.cr = o->cr_threshold;
 		prm.nb = o->neighbor_threshold;
-		prm.tmin = std::fmin(o->cr_threshold, o->neighbor_threshold);
 		prm.thi2 = 2 * o->cr_threshold * (1 - 1e-12);
 		prm.tlo2 = 2 * o->neighbor_threshold * (1 - 1e-12);
 		prm.mode = o->border;

@@ -18,14 +18,6 @@ __device__ __forceinline__ int warp_sum_int(int v)
 	return v;
 }
 
-__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
-{
-#pragma unroll
-	for (int o = 16; o; o >>= 1)
-		v += __shfl_xor_sync(0xffffffffu, v, o);
-	return v;
-}
-
 __device__ __forceinline__ int warp_inclusive_count(int cnt)
 {
 	const int lane = threadIdx.x & 31;

@@ -35,8 +35,9 @@
 // of them branches and their joins, at 18 resident warps per SM, half of the
 // issue slots and a third of DRAM's rate used.  One test per row for a value that
 // is not finite, by the largest of the six high words, votes instead of
-// divergent waits, and predicated stores and arrivals left 328: 16 frames of
-// 2048 x 2048 290 -> 268 us, two of 8192 x 8192 488 -> 436.
+// divergent waits, and predicated stores and arrivals left 366 (16 frames of
+// 2048 x 2048 290 -> 268 us, two of 8192 x 8192 488 -> 436); with the producer's
+// four rows at a time it is 328 (437 -> 427 us on the two).
 //
 // The block floors of error maps depend on the maps only, so they are computed
 // before this kernel (prep_init_kernel, with the call's state and zeroing);
