@@ -62,7 +62,7 @@ class Image:
         self.data, device = _checked_data(self.data)
         with torch.cuda.device(device):
             fields, checks = _calibration(self.data, device, self.error, self.background,
-                                          self.effective_gain, self.readnoise)
+                                          self.effective_gain, self.readnoise, views=True)
             checks.run()
             for name, value in fields.items():
                 if isinstance(value, float):
@@ -104,13 +104,16 @@ class _Checks:
         self.failed = False  # report() raised
 
     def add(self, name, value):
+        """Adds a check; returns the value as the check reads it (contiguous)."""
         minimum, _ = self.RULES[name]
         if isinstance(value, float):
             low = value <= 0 if minimum == 1 else value < 0 if minimum == 0 else False
             self.items.append((name, None, (not isfinite(value)) | low << 1))
         else:
             self.items.append((name, len(self.tensors), 0))
-            self.tensors.append(value.detach().contiguous())
+            value = value.detach().contiguous()
+            self.tensors.append(value)
+        return value
 
     def maps(self):
         """The maps as struct cusmic_map_check."""
@@ -119,12 +122,6 @@ class _Checks:
         for i, (name, t) in enumerate(zip(names, self.tensors)):
             arr[i] = _native.MapCheck(t.data_ptr(), t.numel(), self.RULES[name][0])
         return arr, len(self.tensors)
-
-    def contiguous(self, fields):
-        """The calibration with the maps as the checks read them, so that a map
-        that is not contiguous is copied once."""
-        return {name: fields[name] if index is None else self.tensors[index]
-                for name, index, _ in self.items}
 
     @property
     def scalar_failed(self):
@@ -151,9 +148,11 @@ class _Checks:
         self.report(flags.value)
 
 
-def _calibration(data, device, error, background, effective_gain, readnoise):
+def _calibration(data, device, error, background, effective_gain, readnoise, views=False):
     """The calibration that applies (an error map replaces gain and read
-    noise) as float64 device maps or floats, and its content checks."""
+    noise) as float64 device maps or floats, and its content checks.  ``views``:
+    maps as given; else as the checks read them, so that a map that is not
+    contiguous is copied once."""
     shape, frame = tuple(data.shape), tuple(data.shape[-2:])
     given = {"error": error} if error is not None else \
         {"effective_gain": effective_gain, "readnoise": readnoise}
@@ -172,8 +171,9 @@ def _calibration(data, device, error, background, effective_gain, readnoise):
         if tuple(value.shape) not in (shape, frame) and (name == "error" or value.dim() != 0):
             raise ValueError(f"{name} has an incompatible shape")
         value = value.to(torch.float64)
-        fields[name] = value if value.dim() else float(value)
-        checks.add(name, fields[name])
+        value = value if value.dim() else float(value)
+        checked = checks.add(name, value)
+        fields[name] = value if views else checked
     return fields, checks
 
 
@@ -331,7 +331,7 @@ def remove_cosmics(
             if maxiter and error is None and ("effective_gain" not in fields or
                                               "readnoise" not in fields):
                 raise ValueError("Provide error, or both effective_gain and readnoise")
-            return cleaner._clean(data, checks.contiguous(fields), mask, checks)
+            return cleaner._clean(data, fields, mask, checks)
         except Exception:
             if not checks.failed:  # the call failed before, or apart from, its checks
                 checks.run()

@@ -138,7 +138,6 @@ def remove_cosmics_differentiable(data, contrast=3, cr_threshold=5, neighbor_thr
                                       background.detach() if bg_t is not None else background,
                                       effective_gain, readnoise)
         checks.run()
-        fields = checks.contiguous(fields)
         mask = _checked_mask(mask, checked, device)
     cleaner = Cleaner(contrast, cr_threshold, neighbor_threshold, maxiter, border_mode)
     return _Clean.apply(data, bg_t, fields, mask, cleaner)
