@@ -65,8 +65,6 @@ class Image:
                                           self.effective_gain, self.readnoise, views=True)
             checks.run()
             for name, value in fields.items():
-                if isinstance(value, float):
-                    value = torch.full((), value, dtype=torch.float64, device=device)
                 setattr(self, name, value)
             self.mask = _checked_mask(self.mask, self.data, device)
 
@@ -151,8 +149,8 @@ class _Checks:
 def _calibration(data, device, error, background, effective_gain, readnoise, views=False):
     """The calibration that applies (an error map replaces gain and read
     noise) as float64 device maps or floats, and its content checks.  ``views``:
-    maps as given; else as the checks read them, so that a map that is not
-    contiguous is copied once."""
+    everything as float64 device tensors, as given; else maps as the checks read
+    them, so that a map that is not contiguous is copied once."""
     shape, frame = tuple(data.shape), tuple(data.shape[-2:])
     given = {"error": error} if error is not None else \
         {"effective_gain": effective_gain, "readnoise": readnoise}
@@ -171,9 +169,8 @@ def _calibration(data, device, error, background, effective_gain, readnoise, vie
         if tuple(value.shape) not in (shape, frame) and (name == "error" or value.dim() != 0):
             raise ValueError(f"{name} has an incompatible shape")
         value = value.to(torch.float64)
-        value = value if value.dim() else float(value)
-        checked = checks.add(name, value)
-        fields[name] = value if views else checked
+        checked = checks.add(name, value if value.dim() else float(value.detach()))
+        fields[name] = value.to(device) if views else checked
     return fields, checks
 
 

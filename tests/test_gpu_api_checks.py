@@ -61,3 +61,17 @@ def test_strided_map_is_copied_once(cuda, call):
     assert bool(mask.any()) and cuda.equal(mask, mask2) and cuda.equal(clean, clean2)
     # (A contiguous argument's own memory is not in its call's count.)
     assert copied - own <= 8 * h * w + (1 << 20)
+
+
+def test_image_keeps_scalar_tensors(cuda):
+    """A scalar calibration given as a tensor is the Image's, on the data's
+    device, with its autograd graph."""
+    from cusmic_b200.api import Cleaner, Image
+    gain = cuda.tensor(2.0, dtype=cuda.float64, requires_grad=True)
+    image = Image(cuda.full((8, 9), 10.0, dtype=cuda.float64), effective_gain=gain, readnoise=3.0)
+    assert image.effective_gain.requires_grad and image.effective_gain.is_cuda
+    image.effective_gain.backward()
+    assert float(gain.grad) == 1.0
+    assert image.readnoise.is_cuda and image.readnoise.dtype == cuda.float64
+    clean, mask = Cleaner(3, 5, 3)(image)
+    assert bool((clean == 10).all()) and not bool(mask.any())
