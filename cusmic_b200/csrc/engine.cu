@@ -928,8 +928,8 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	// 195, 186; 12 207, 199; 16 214, 215; 24 227, 238; 32 249, 264; 64 336, 389; 128
 	// 524, 647.  Between 8 and 16 Mpixel the two are within 5%.
 	const bool model = L.error_frames < nf, thresholds = model && L.total_px > 8u << 20;
-	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, prm, ctl, cands, low, eval,
-		targets, chg, ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
+	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, state, prm, ctl, cands, low,
+		eval, targets, chg, ws.rows.p, (int)L.rows.size(), ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
 	mark(rec, K_RECLASS);
 	if (!model)
 		late_classes_kernel<LATE_TESTS, false><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
@@ -946,7 +946,7 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	if (L.poison_wait[2])
 		bw = BarrierWait{L.poison_wait[2], 1};
 	late_passes_kernel<<<grid, LATE_THREADS, sizeof(LateShared), s>>>(frames, state, nf, prm, ctl, maxiter, cands,
-		low, eval, targets, radius, chg, bw);
+		low, eval, targets, radius, chg, ws.rows.p, (int)L.rows.size(), bw);
 	mark(rec, K_RECLASS);
 }
 

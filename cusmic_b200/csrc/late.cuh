@@ -281,6 +281,90 @@ __device__ __forceinline__ void late_neighbours(const FrameDesc *__restrict__ fr
 	}
 }
 
+// Stage 1 when much of the frames changed: a warp per row of 32 words, which takes
+// all of CRMASK in place of D.  (Every changed pixel is in the mask, and what is
+// evaluated again for the others comes out as it was.)  No claims: each pixel is
+// listed by its own word.  Claims of 13 rows for each of a million changed targets
+// took a 2048 x 2048 frame 1.2 ms, more than the pass's evaluations; the rows'
+// words take 30 us whatever changed, and then four million pixels are classified.
+// Hence the rule: when the changed targets are over a 64th of the pixels and a
+// quarter of the mask.
+__device__ __forceinline__ bool late_by_rows(const Control *ctl, const PassLists &L)
+{
+	return 64 * L.n_chg > ctl->cand_cap && 4 * L.n_chg > ctl->n_targets;
+}
+
+// Columns 32 k - 6 .. 32 k + 37 of row y of a plane (bit 0: the first); zero
+// outside the frame, or on the torus what the column or row there maps to.
+__device__ __forceinline__ unsigned long long window6(const uint32_t *plane, int w, int h, int words, int y,
+	int k, bool torus)
+{
+	if (torus)
+		y = wrap_index(y, h);
+	if (y < 0 || y >= h)
+		return 0ull;
+	const uint32_t *row = plane + (long long)y * words;
+	const unsigned long long l = k > 0 ? row[k - 1] >> 26 : 0u, c = row[k], r = k + 1 < words ? row[k + 1] & 63u : 0u;
+	unsigned long long m = l | c << 6 | r << 38;
+	if (torus && (k == 0 || 32 * k + 37 >= w))
+		for (int j = 0; j < 44; ++j) {
+			const int x = 32 * k - 6 + j;
+			if (x < 0 || x >= w) {
+				const int t = wrap_index(x, w);
+				m |= (unsigned long long)((row[t >> 5] >> (t & 31)) & 1u) << j;
+			}
+		}
+	return m;
+}
+
+__device__ __forceinline__ void late_rows(const FrameDesc *__restrict__ frames, const FrameState *state,
+	const int2 *__restrict__ rows, int nrows, PassLists &L, int mode, uint2 *cands, uint2 *low, uint2 *eval,
+	Team team)
+{
+	const int lane = threadIdx.x & 31;
+	const int gw = (team.block * blockDim.x + threadIdx.x) >> 5, nw = (team.blocks * blockDim.x) >> 5;
+	auto wide2 = [](unsigned long long m) { return m | m << 1 | m >> 1 | m << 2 | m >> 2; };
+	for (int i = gw; i < nrows; i += nw) {
+		const int2 item = rows[i];
+		if (!state[item.x].active)
+			continue; // warp-uniform
+		const FrameDesc &fd = frames[item.x];
+		const int w = fd.w, words = fd.words, y = item.y;
+		for (int k0 = 0; k0 < words; k0 += 32) {
+			const int k = k0 + lane;
+			uint32_t ne = 0, nh = 0, nl = 0;
+			if (k < words) {
+				unsigned long long m2 = 0, m4 = 0, m6 = 0;
+#pragma unroll 1
+				for (int dy = -6; dy <= 6; ++dy) {
+					const unsigned long long m = window6(plane_ptr(fd, P_CRMASK), w, fd.h, words, y + dy, k,
+						mode == WRAP);
+					m6 |= m;
+					m4 |= dy >= -4 && dy <= 4 ? m : 0ull;
+					m2 |= dy >= -2 && dy <= 2 ? m : 0ull;
+				}
+				const uint32_t clip = w - 32 * k >= 32 ? 0xffffffffu : (1u << (w - 32 * k)) - 1u;
+				const long long o = (long long)y * words + k;
+				const uint32_t H = plane_ptr(fd, P_HIGH)[o], W = plane_ptr(fd, P_LOW)[o];
+				ne = (uint32_t)(wide2(m2) >> 6) & clip;
+				nh = (uint32_t)(wide2(wide2(m4)) >> 6) & H;
+				nl = (uint32_t)(wide2(wide2(wide2(m6))) >> 6) & W & ~H;
+			}
+			const unsigned pix = (unsigned)((long long)y * w + 32 * k);
+			auto put = [&](uint2 *list, unsigned long long *count, uint32_t bits) {
+				if (!__any_sync(0xffffffffu, bits != 0))
+					return;
+				unsigned long long slot = warp_append(count, __popc(bits));
+				for (; bits; bits &= bits - 1)
+					list[slot++] = make_uint2((unsigned)item.x, pix + __ffs((int)bits) - 1);
+			};
+			put(eval, &L.n_eval, ne);
+			put(cands, &L.n_cand, nh);
+			put(low, &L.n_low, nl);
+		}
+	}
+}
+
 // The class of lane's re-evaluated pixel t (0: none, 1: HIGH, 2: LOW) into the
 // planes and lists; called by the whole warp, `have`: the lane has one.  GATED:
 // the S1, S2 and CAND words are read where a bit can be set and has to go (they
@@ -469,10 +553,12 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 // The entries of a list (count() many, which thread 0 asks) by blocks: a thread per
 // entry tests it (keep), then the block's warps take the survivors (work, by the
 // whole warp) from a queue in shared memory.  A block's share shrinks with the list,
-// so that a short one spreads over the team.  The entries are dealt to the blocks
-// one by one, so neighbouring entries, whose survivors come in clusters, go to
-// different blocks.  aside: other work of every warp, done before the first
-// sweep's barrier, beside other warps' tests.
+// so that a short one spreads over the team.  The entries of a short list are dealt
+// to the blocks one by one, so neighbouring entries, whose survivors come in
+// clusters, go to different blocks; those of a long one in runs of 32, whose tests'
+// loads share lines.  aside: other work of every warp, done before the first
+// sweep's barrier, beside other warps' tests.  many: called by the whole block with
+// the survivors of chunk k queued; it may take some.
 //
 // What is the same for the whole block stays in shared memory: the work holds
 // every register of a thread (64 at this block size), and what lives across it
@@ -480,25 +566,30 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 struct LateQueue {
 	uint16_t e[LATE_THREADS];
 	int n;
-	int chunk;
+	int chunk, run; // run: entries dealt at a time, as a power of two
 	Team team;
-	long long end;
+	unsigned end; // (no list has 2^32 entries: a pixel takes more than 50 bytes of lists)
+
+	// Entry of slot j of the block's k-th chunk.
+	__device__ __forceinline__ unsigned entry(unsigned k, unsigned j) const
+	{
+		const unsigned i = k * chunk + j;
+		return ((team.block + team.blocks * (i >> run)) << run) + (i & ((1u << run) - 1u));
+	}
 };
 
-template <class Count, class Keep, class Work, class Aside>
-__device__ __forceinline__ void block_sweep(Count count, LateQueue &Q, Team team, Keep keep, Work work, Aside aside)
+template <class Count, class Keep, class Many, class Work, class Aside>
+__device__ __forceinline__ void block_sweep(Count count, LateQueue &Q, Team team, Keep keep, Many many, Work work,
+	Aside aside)
 {
 	const int warp = threadIdx.x >> 5;
 	if (threadIdx.x == 0) { // (a barrier of the team lies between two sweeps)
 		const long long n = count(), share = (n + team.blocks - 1) / team.blocks;
 		Q.chunk = share < LATE_THREADS ? (int)share : LATE_THREADS;
+		Q.run = share < LATE_THREADS ? 0 : 5;
 		Q.team = team;
-		Q.end = n;
+		Q.end = (unsigned)n;
 	}
-	// Entry of slot j of the block's k-th chunk.
-	auto entry = [&](int k, int j) {
-		return Q.team.block + (long long)Q.team.blocks * ((long long)k * Q.chunk + j);
-	};
 	for (int k = 0;; ++k) { // block-uniform
 		if (threadIdx.x == 0)
 			Q.n = 0;
@@ -506,15 +597,16 @@ __device__ __forceinline__ void block_sweep(Count count, LateQueue &Q, Team team
 		if (k == 0)
 			aside();
 		if ((int)threadIdx.x < Q.chunk) {
-			const long long e = entry(k, threadIdx.x);
+			const unsigned e = Q.entry(k, threadIdx.x);
 			if (e < Q.end && keep(e))
 				Q.e[atomicAdd(&Q.n, 1)] = (uint16_t)threadIdx.x;
 		}
 		__syncthreads();
+		many(k);
 		for (int q = warp; q < Q.n; q += LATE_WARPS)
-			work(entry(k, Q.e[q]));
+			work(Q.entry(k, Q.e[q]));
 		__syncthreads();
-		if (!Q.chunk || entry(k + 1, 0) >= Q.end)
+		if (!Q.chunk || Q.entry(k + 1, 0) >= Q.end)
 			return;
 	}
 }
@@ -525,13 +617,13 @@ __device__ __forceinline__ void late_candidates(const FrameDesc *__restrict__ fr
 	const DetectParams &prm, Count count, LateQueue &Q, Team team, double *P, double *S, double (*T)[63])
 {
 	const int lane = threadIdx.x & 31;
-	block_sweep(count, Q, team, [&](long long e) {
+	block_sweep(count, Q, team, [&](unsigned e) {
 		const uint2 t = cands[e];
 		const FrameDesc &fd = frames[t.x];
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 		return test_bit(plane_ptr(fd, P_HIGH), fd.words, x, y) &
 			!test_bit(plane_ptr(fd, P_HOLE), fd.words, x, y);
-	}, [&](long long e) {
+	}, [](int) {}, [&](unsigned e) {
 		const uint2 t = cands[e];
 		const FrameDesc &fd = frames[t.x];
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
@@ -569,13 +661,13 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 	const uint2 *cands, const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par,
 	uint2 *targets, LateQueue &Q, Team team, double *P, double *S)
 {
-	block_sweep([&] { return (long long)L.n_low; }, Q, team, [&](long long e) {
+	block_sweep([&] { return (long long)L.n_low; }, Q, team, [&](unsigned e) {
 		const uint2 t = low[e];
 		const FrameDesc &fd = frames[t.x];
 		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
 		plane_ptr(fd, P_LISTED)[(long long)y * fd.words + (x >> 5)] = 0u;
 		return low_near(fd, x, y);
-	}, [&](long long e) {
+	}, [](int) {}, [&](unsigned e) {
 		low_eval<PATH_ANY>(frames, state, low[e], prm, ctl, par, targets, P, S, false);
 	}, [&] { late_grow(frames, state, cands, L, ctl, par, targets, team); });
 }
@@ -586,12 +678,61 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 // are never added (the mask only grows) and keep their values, so the smaller
 // windows still hold none, the same window holds the same donors, and the same
 // median would come out.  A new target is itself a FRESH pixel.
+//
+// A block with LATE_BY_THREADS or more of a chunk's 1024 targets left gives them a
+// thread each first, as replace_targets does (at 64 registers a thread the 25 values
+// spill, and are still faster than a warp per target).
+constexpr int LATE_BY_THREADS = 256;
+
+// (Called by the whole block; a function of its own, so that its registers are not
+// the kernel's.)
+__device__ __noinline__ void late_replace_threads(const FrameDesc *__restrict__ frames, const uint2 *targets,
+	uint8_t *radius, unsigned *chg, unsigned long long *n_chg, LateQueue &Q, int k)
+{
+	const int n = Q.n, lane = threadIdx.x & 31;
+	int left = -1; // the thread's slot, if it is left to the warps
+	unsigned e = 0;
+	bool changed = false;
+	if ((int)threadIdx.x < n) {
+		const int slot = Q.e[threadIdx.x];
+		e = Q.entry(k, slot);
+		const uint2 t = targets[e];
+		const FrameDesc &fd = frames[t.x];
+		const int x = (int)(t.y % (unsigned)fd.w), y = (int)(t.y / (unsigned)fd.w);
+		double v;
+		if (first_window_value(fd, x, y, v)) {
+			double &dst = fd.clean[t.y];
+			changed = __double_as_longlong(dst) != __double_as_longlong(v);
+			dst = v;
+			radius[e] = 2;
+			if (!fd.error) // keep the block's floor a lower bound of its clean values
+				atomicMin(&fd.floors[(y >> 5) * ((fd.w + 31) >> 5) + (x >> 5)].key, order_key(v));
+		} else {
+			left = slot;
+		}
+	}
+	const unsigned b = __ballot_sync(0xffffffffu, changed);
+	unsigned long long at = 0;
+	if (lane == 0 && b)
+		at = atomicAdd(n_chg, (unsigned long long)__popc(b));
+	at = __shfl_sync(0xffffffffu, at, 0);
+	if (changed)
+		chg[at + __popc(b & ((1u << lane) - 1u))] = e;
+	__syncthreads();
+	if (threadIdx.x == 0)
+		Q.n = 0;
+	__syncthreads();
+	if (left >= 0)
+		Q.e[atomicAdd(&Q.n, 1)] = (uint16_t)left;
+	__syncthreads();
+}
+
 __device__ __forceinline__ void late_replace(const FrameDesc *__restrict__ frames, const FrameState *state,
 	int par, const uint2 *targets, const Control *ctl, uint8_t *radius, unsigned *chg, unsigned long long *n_chg,
 	LateQueue &Q, Team team)
 {
-	const long long fresh0 = (long long)ctl->fresh0;
-	block_sweep([&] { return (long long)ctl->n_targets; }, Q, team, [&](long long e) {
+	const unsigned fresh0 = (unsigned)ctl->fresh0;
+	block_sweep([&] { return (long long)ctl->n_targets; }, Q, team, [&](unsigned e) {
 		const uint2 t = targets[e];
 		const int r = radius[e]; // (a new target's is not set yet)
 		if (!replaces(state[t.x], par))
@@ -600,7 +741,10 @@ __device__ __forceinline__ void late_replace(const FrameDesc *__restrict__ frame
 			return true;
 		const FrameDesc &fd = frames[t.x];
 		return fresh_in_window(fd, (int)(t.y % (unsigned)fd.w), (int)(t.y / (unsigned)fd.w), r);
-	}, [&](long long e) {
+	}, [&](int k) {
+		if (Q.n >= LATE_BY_THREADS) // block-uniform
+			late_replace_threads(frames, targets, radius, chg, n_chg, Q, k);
+	}, [&](unsigned e) {
 		const uint2 t = targets[e];
 		const FrameDesc &fd = frames[t.x];
 		bool changed = false;
@@ -608,7 +752,7 @@ __device__ __forceinline__ void late_replace(const FrameDesc *__restrict__ frame
 		if ((threadIdx.x & 31) == 0) {
 			radius[e] = (uint8_t)(r < 255 ? r : 255);
 			if (changed)
-				chg[atomicAdd(n_chg, 1ull)] = (unsigned)e;
+				chg[atomicAdd(n_chg, 1ull)] = e;
 		}
 	}, [] {});
 }
@@ -619,9 +763,9 @@ __device__ __forceinline__ void late_replace(const FrameDesc *__restrict__ frame
 constexpr int LN_THREADS = 512;
 
 __global__ void __launch_bounds__(LN_THREADS, 3)
-late_neighbours_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, Control *ctl,
-	uint2 *cands, uint2 *low, uint2 *eval, const uint2 *targets, const unsigned *chg,
-	const FloorJob *__restrict__ jobs, int njobs)
+late_neighbours_kernel(const FrameDesc *__restrict__ frames, const FrameState *state, DetectParams prm,
+	Control *ctl, uint2 *cands, uint2 *low, uint2 *eval, const uint2 *targets, const unsigned *chg,
+	const int2 *__restrict__ rows, int nrows, const FloorJob *__restrict__ jobs, int njobs)
 {
 	__shared__ ListSlots slots;
 	// The noise-model blocks' thresholds, for the long lists' LATE_TESTS (a
@@ -633,6 +777,10 @@ late_neighbours_kernel(const FrameDesc *__restrict__ frames, DetectParams prm, C
 		if (!fd.error)
 			fd.floors[(jb.y0 >> 5) * ((fd.w + 31) >> 5) + (jb.x0 >> 5)].thr =
 				block_threshold(fd, jb.x0 >> 5, jb.y0 >> 5, prm.mode, tmin2);
+	}
+	if (late_by_rows(ctl, ctl->pass[1])) {
+		late_rows(frames, state, rows, nrows, ctl->pass[1], prm.mode, cands, low, eval, whole_grid());
+		return;
 	}
 	late_neighbours<LN_THREADS / 32>(frames, targets, chg, ctl->pass[1], prm.mode, cands, low, eval, slots,
 		whole_grid());
@@ -665,7 +813,7 @@ struct LateShared {
 __global__ void __launch_bounds__(LATE_THREADS, 1)
 late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int nf, DetectParams prm,
 	Control *ctl, int maxiter, uint2 *cands, uint2 *low, uint2 *eval, uint2 *targets, uint8_t *radius,
-	unsigned *chg, BarrierWait bw)
+	unsigned *chg, const int2 *__restrict__ rows, int nrows, BarrierWait bw)
 {
 	extern __shared__ __align__(16) unsigned char late_smem[];
 	LateShared &S = *reinterpret_cast<LateShared *>(late_smem);
@@ -703,7 +851,10 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 		const int par = it & 1;
 		PassLists &L = ctl->pass[par], &next = ctl->pass[par ^ 1];
 		if (it > 1) {
-			late_neighbours<LATE_WARPS>(frames, targets, chg, L, prm.mode, cands, low, eval, S.slots, team);
+			if (late_by_rows(ctl, L))
+				late_rows(frames, state, rows, nrows, L, prm.mode, cands, low, eval, team);
+			else
+				late_neighbours<LATE_WARPS>(frames, targets, chg, L, prm.mode, cands, low, eval, S.slots, team);
 			// The last growth's FRESH bits: its replacement is done.
 			for (long long i = (long long)ctl->fresh0 + team.block * (long long)blockDim.x + threadIdx.x;
 			     i < (long long)ctl->n_targets; i += (long long)team.blocks * blockDim.x) {
