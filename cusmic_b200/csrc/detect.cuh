@@ -930,6 +930,87 @@ __device__ __forceinline__ void grow_group(const FrameDesc &fd, int f, int x, in
 		targets[slot++] = make_uint2((unsigned)f, base + __ffs(now) - 1);
 }
 
+// The same for every pixel of the frames, a warp per row of 32 words: two dilations
+// on bit words, for a pass whose high list holds over a 16th of the pixels (eight
+// lanes for each of 0.9 million listed pixels of a 2048 x 2048 frame took about 250 us,
+// the rows 20; at a 64th the two are even).
+// late: HIGH pixels only, the new pixels' FRESH bits, and the high list's LISTED bits
+// cleared.  A function of its own: its registers are not its callers'.
+__device__ __forceinline__ bool grows_by_rows(const Control *ctl, int par)
+{
+	return 16 * ctl->pass[par].n_cand > ctl->cand_cap;
+}
+
+// Columns 32 k - 2 .. 32 k + 33 of row y of a plane (bit 0: the first), zero outside.
+__device__ __forceinline__ unsigned long long window2(const uint32_t *plane, int words, int h, int y, int k)
+{
+	if (y < 0 || y >= h)
+		return 0ull;
+	const uint32_t *row = plane + (long long)y * words;
+	const unsigned long long l = k > 0 ? row[k - 1] >> 30 : 0u, r = k + 1 < words ? row[k + 1] & 3u : 0u;
+	return l | (unsigned long long)row[k] << 2 | r << 34;
+}
+
+__device__ __noinline__ void grow_rows(const FrameDesc *__restrict__ frames, FrameState *state,
+	const int2 *__restrict__ rows, int nrows, bool late, Control *ctl, int par, uint2 *targets, Team team)
+{
+	const int lane = threadIdx.x & 31;
+	const int gw = (team.block * blockDim.x + threadIdx.x) >> 5, nw = (team.blocks * blockDim.x) >> 5;
+	for (int i = gw; i < nrows; i += nw) {
+		const int2 item = rows[i];
+		const int f = item.x, y = item.y;
+		if (!state[f].active)
+			continue; // warp-uniform
+		const FrameDesc &fd = frames[f];
+		const int words = fd.words, h = fd.h;
+		for (int k0 = 0; k0 < words; k0 += 32) {
+			const int k = k0 + lane;
+			const long long o = (long long)y * words + k;
+			uint32_t now = 0;
+			int lost = 0;
+			if (k < words) {
+				if (late)
+					plane_ptr(fd, P_LISTED)[o] = 0u;
+				unsigned long long c[5], v = 0; // CAND; S1 cells that touch one
+#pragma unroll
+				for (int r = 0; r < 5; ++r)
+					c[r] = window2(plane_ptr(fd, P_CAND), words, h, y - 2 + r, k);
+#pragma unroll
+				for (int r = 0; r < 3; ++r) {
+					const unsigned long long m = c[r] | c[r + 1] | c[r + 2];
+					if (m)
+						v |= (m | m << 1 | m >> 1) & window2(plane_ptr(fd, P_S1), words, h, y - 1 + r, k);
+				}
+				uint32_t g = (uint32_t)((v | v << 1 | v >> 1) >> 2);
+				if (g) {
+					g &= plane_ptr(fd, P_S2)[o];
+					if (late)
+						g &= plane_ptr(fd, P_HIGH)[o];
+				}
+				if (g) // (low pixels join the mask beside this)
+					now = g & ~atomicOr(plane_ptr(fd, P_CRMASK) + o, g);
+				if (now) {
+					lost = __popc(now & plane_ptr(fd, P_DONOR)[o]);
+					if (late)
+						atomicOr(plane_ptr(fd, P_FRESH) + o, now);
+				}
+			}
+			if (!__any_sync(0xffffffffu, now != 0))
+				continue;
+			unsigned long long slot = warp_append(&ctl->n_targets, __popc(now));
+			lost = __reduce_add_sync(0xffffffffu, lost);
+			if (lane == 0) {
+				atomicOr(&state[f].todo[par], 1u);
+				if (lost)
+					atomicAdd(&state[f].masked, (unsigned long long)lost);
+			}
+			const unsigned pix = (unsigned)((long long)y * fd.w + 32 * k);
+			for (; now; now &= now - 1)
+				targets[slot++] = make_uint2((unsigned)f, pix + __ffs((int)now) - 1);
+		}
+	}
+}
+
 // Any CAND pixel within two pixels of (x, y) (S2 is read only by the second
 // growth step, within that distance of a CAND pixel), and no hole there.
 __device__ __forceinline__ bool low_near(const FrameDesc &fd, int x, int y)
@@ -963,13 +1044,17 @@ __device__ __forceinline__ void low_eval(const FrameDesc *__restrict__ frames, F
 template <int PATH>
 __global__ void __launch_bounds__(256, PATH == PATH_ERROR ? 4 : 3)
 low_grow_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const uint2 *__restrict__ cands,
-	DetectParams prm, Control *ctl, int par, uint2 *targets, int grow)
+	DetectParams prm, Control *ctl, int par, uint2 *targets, int grow, const int2 *__restrict__ rows, int nrows)
 {
 	__shared__ double patches[8][81];
 	__shared__ double scratch[8][PATH == PATH_ERROR ? 25 : CS_RUNS];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const long long stride = (long long)gridDim.x * blockDim.x;
-	const long long nc = grow ? (long long)ctl->pass[par].n_cand : 0, nl = (long long)ctl->pass[par].n_low;
+	const bool by_rows = grow && grows_by_rows(ctl, par);
+	if (by_rows)
+		grow_rows(frames, state, rows, nrows, false, ctl, par, targets, whole_grid());
+	const long long nc = grow && !by_rows ? (long long)ctl->pass[par].n_cand : 0;
+	const long long nl = (long long)ctl->pass[par].n_low;
 	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, nw = stride >> 5;
 	// Entries per warp and sweep: 32 for a long list, fewer for a short one,
 	// whose survivors then land on different warps.  (Dealing the entries to the

@@ -885,10 +885,10 @@ static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	}
 	if (L.error_frames)
 		low_grow_kernel<PATH_ERROR><<<sparse, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.cands.p, L.prm,
-			ws.ctl.p, 0, ws.targets.p, 1);
+			ws.ctl.p, 0, ws.targets.p, 1, ws.rows.p, (int)L.rows.size());
 	if (model)
 		low_grow_kernel<PATH_MODEL><<<sparse, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.cands.p, L.prm,
-			ws.ctl.p, 0, ws.targets.p, L.error_frames == 0);
+			ws.ctl.p, 0, ws.targets.p, L.error_frames == 0, ws.rows.p, (int)L.rows.size());
 	mark(rec, K_GROW);
 	replace_kernel<<<di.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(ws.frames.p, ws.state.p, nf, ws.targets.p,
 		ws.ctl.p, 0, ws.radius.p, ws.chg.p);
@@ -2262,7 +2262,7 @@ extern "C" int remove_cosmics_device_noalloc(const cusmic_image *im, const cusmi
 					par, seeds);
 				seed_kernel<<<nd.sms * 8, 256, 0, s>>>(frames, seeds, prm, ctl, par);
 				low_grow_kernel<PATH_ANY><<<nd.sms * 3, 256, 0, s>>>(frames, state, cands, prm, ctl, par,
-					targets, 1);
+					targets, 1, rows, h);
 				replace_kernel<<<nd.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(frames, state, 1, targets,
 					ctl, par, nullptr, nullptr);
 			}

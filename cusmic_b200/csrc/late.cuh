@@ -659,7 +659,7 @@ __device__ __forceinline__ void late_grow(const FrameDesc *__restrict__ frames, 
 // Stage 4: the growth, and the low list's pixels near a CAND pixel, a warp each.
 __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, FrameState *state,
 	const uint2 *cands, const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par,
-	uint2 *targets, LateQueue &Q, Team team, double *P, double *S)
+	uint2 *targets, const int2 *rows, int nrows, LateQueue &Q, Team team, double *P, double *S)
 {
 	block_sweep([&] { return (long long)L.n_low; }, Q, team, [&](unsigned e) {
 		const uint2 t = low[e];
@@ -669,7 +669,12 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 		return low_near(fd, x, y);
 	}, [](int) {}, [&](unsigned e) {
 		low_eval<PATH_ANY>(frames, state, low[e], prm, ctl, par, targets, P, S, false);
-	}, [&] { late_grow(frames, state, cands, L, ctl, par, targets, team); });
+	}, [&] {
+		if (grows_by_rows(ctl, par))
+			grow_rows(frames, state, rows, nrows, true, ctl, par, targets, team);
+		else
+			late_grow(frames, state, cands, L, ctl, par, targets, team);
+	});
 }
 
 // Stage 5: the replacement, by warps (few targets are left to do).  A target
@@ -885,7 +890,8 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 			if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 				return;
 		} while (it == 1 && barrier.calls * team.blocks < gridDim.x);
-		late_low(frames, state, cands, low, prm, L, ctl, par, targets, S.Q, team, S.patches[warp], S.scratch[warp]);
+		late_low(frames, state, cands, low, prm, L, ctl, par, targets, rows, nrows, S.Q, team, S.patches[warp],
+			S.scratch[warp]);
 		if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 			return;
 		pass_control(state, nf, ctl, par, team);
