@@ -936,9 +936,16 @@ __device__ __forceinline__ void grow_group(const FrameDesc &fd, int f, int x, in
 // the rows 20; at a 64th the two are even).
 // late: HIGH pixels only, the new pixels' FRESH bits, and the high list's LISTED bits
 // cleared.  A function of its own: its registers are not its callers'.
-__device__ __forceinline__ bool grows_by_rows(const Control *ctl, int par)
+// (The rows come with the batch's pixels: a load of those would delay the rule.)
+struct RowItems {
+	const int2 *rows;
+	int n;
+	unsigned long long px;
+};
+
+__device__ __forceinline__ bool grows_by_rows(unsigned long long n_cand, const RowItems &rows)
 {
-	return 16 * ctl->pass[par].n_cand > ctl->cand_cap;
+	return 16 * n_cand > rows.px;
 }
 
 // Columns 32 k - 2 .. 32 k + 33 of row y of a plane (bit 0: the first), zero outside.
@@ -952,12 +959,12 @@ __device__ __forceinline__ unsigned long long window2(const uint32_t *plane, int
 }
 
 __device__ __noinline__ void grow_rows(const FrameDesc *__restrict__ frames, FrameState *state,
-	const int2 *__restrict__ rows, int nrows, bool late, Control *ctl, int par, uint2 *targets, Team team)
+	const RowItems &rows, bool late, Control *ctl, int par, uint2 *targets, Team team)
 {
 	const int lane = threadIdx.x & 31;
 	const int gw = (team.block * blockDim.x + threadIdx.x) >> 5, nw = (team.blocks * blockDim.x) >> 5;
-	for (int i = gw; i < nrows; i += nw) {
-		const int2 item = rows[i];
+	for (int i = gw; i < rows.n; i += nw) {
+		const int2 item = rows.rows[i];
 		const int f = item.x, y = item.y;
 		if (!state[f].active)
 			continue; // warp-uniform
@@ -1044,17 +1051,18 @@ __device__ __forceinline__ void low_eval(const FrameDesc *__restrict__ frames, F
 template <int PATH>
 __global__ void __launch_bounds__(256, PATH == PATH_ERROR ? 4 : 3)
 low_grow_kernel(const FrameDesc *__restrict__ frames, FrameState *state, const uint2 *__restrict__ cands,
-	DetectParams prm, Control *ctl, int par, uint2 *targets, int grow, const int2 *__restrict__ rows, int nrows)
+	DetectParams prm, Control *ctl, int par, uint2 *targets, int grow, RowItems rows)
 {
 	__shared__ double patches[8][81];
 	__shared__ double scratch[8][PATH == PATH_ERROR ? 25 : CS_RUNS];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const long long stride = (long long)gridDim.x * blockDim.x;
-	const bool by_rows = grow && grows_by_rows(ctl, par);
-	if (by_rows)
-		grow_rows(frames, state, rows, nrows, false, ctl, par, targets, whole_grid());
-	const long long nc = grow && !by_rows ? (long long)ctl->pass[par].n_cand : 0;
+	long long nc = grow ? (long long)ctl->pass[par].n_cand : 0;
 	const long long nl = (long long)ctl->pass[par].n_low;
+	if (grows_by_rows((unsigned long long)nc, rows)) {
+		grow_rows(frames, state, rows, false, ctl, par, targets, whole_grid());
+		nc = 0;
+	}
 	const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5, nw = stride >> 5;
 	// Entries per warp and sweep: 32 for a long list, fewer for a short one,
 	// whose survivors then land on different warps.  (Dealing the entries to the

@@ -839,6 +839,11 @@ static inline void mark(Recorder *r, int kind)
 // no waves of idle blocks.
 constexpr int WINDOW_BLOCKS_PER_SM = 3, MAP_BLOCKS_PER_SM = 2;
 
+static RowItems row_items(const Workspace &ws, const Layout &L)
+{
+	return RowItems{ws.rows.p, (int)L.rows.size(), (unsigned long long)L.total_px};
+}
+
 // The first detection pass of a call is full: the dense kernel lists every
 // candidate and the classification fills the HIGH / LOW planes.  It ends with
 // the replacement; the later passes start from the pixels that changed and
@@ -883,12 +888,13 @@ static void launch_pass(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 		seed_kernel<<<sparse, 256, 0, s>>>(ws.frames.p, ws.seeds.p, L.prm, ws.ctl.p, 0);
 		mark(rec, K_SEED);
 	}
+	const RowItems rows = row_items(ws, L);
 	if (L.error_frames)
 		low_grow_kernel<PATH_ERROR><<<sparse, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.cands.p, L.prm,
-			ws.ctl.p, 0, ws.targets.p, 1, ws.rows.p, (int)L.rows.size());
+			ws.ctl.p, 0, ws.targets.p, 1, rows);
 	if (model)
 		low_grow_kernel<PATH_MODEL><<<sparse, 256, 0, s>>>(ws.frames.p, ws.state.p, ws.cands.p, L.prm,
-			ws.ctl.p, 0, ws.targets.p, L.error_frames == 0, ws.rows.p, (int)L.rows.size());
+			ws.ctl.p, 0, ws.targets.p, L.error_frames == 0, rows);
 	mark(rec, K_GROW);
 	replace_kernel<<<di.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(ws.frames.p, ws.state.p, nf, ws.targets.p,
 		ws.ctl.p, 0, ws.radius.p, ws.chg.p);
@@ -921,6 +927,7 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	static_assert(sizeof(PreCand) == 2 * sizeof(uint2), "the pre list holds both lists");
 	uint8_t *radius = ws.radius.p;
 	unsigned *chg = ws.chg.p;
+	const RowItems rows = row_items(ws, L);
 	// The class of the noise-model frames' pixels near the first pass's
 	// targets: in parts with a thread per median above 8 Mpixel, a warp per median
 	// below.  All passes after the first with the parts and with warps, in us, by the
@@ -929,7 +936,7 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	// 524, 647.  Between 8 and 16 Mpixel the two are within 5%.
 	const bool model = L.error_frames < nf, thresholds = model && L.total_px > 8u << 20;
 	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, state, prm, ctl, cands, low,
-		eval, targets, chg, ws.rows.p, (int)L.rows.size(), ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
+		eval, targets, chg, rows, ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
 	mark(rec, K_RECLASS);
 	if (!model)
 		late_classes_kernel<LATE_TESTS, false><<<wide, 256, 0, s>>>(frames, prm, ctl, cands, low, eval);
@@ -946,7 +953,7 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	if (L.poison_wait[2])
 		bw = BarrierWait{L.poison_wait[2], 1};
 	late_passes_kernel<<<grid, LATE_THREADS, sizeof(LateShared), s>>>(frames, state, nf, prm, ctl, maxiter, cands,
-		low, eval, targets, radius, chg, ws.rows.p, (int)L.rows.size(), bw);
+		low, eval, targets, radius, chg, rows, bw);
 	mark(rec, K_RECLASS);
 }
 
@@ -2262,7 +2269,7 @@ extern "C" int remove_cosmics_device_noalloc(const cusmic_image *im, const cusmi
 					par, seeds);
 				seed_kernel<<<nd.sms * 8, 256, 0, s>>>(frames, seeds, prm, ctl, par);
 				low_grow_kernel<PATH_ANY><<<nd.sms * 3, 256, 0, s>>>(frames, state, cands, prm, ctl, par,
-					targets, 1, rows, h);
+					targets, 1, RowItems{rows, h, (unsigned long long)im->width * im->height});
 				replace_kernel<<<nd.sms * WINDOW_BLOCKS_PER_SM, 256, 0, s>>>(frames, state, 1, targets,
 					ctl, par, nullptr, nullptr);
 			}

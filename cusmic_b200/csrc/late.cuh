@@ -59,11 +59,15 @@
 
 namespace cb {
 
-// One block of 32 warps per SM: the fewest arrivals at a grid barrier for the
-// warps that 64 registers a thread allow.  (The candidate evaluation and the
-// replacement want more: a 176-byte stack frame, 176 bytes of spill stores and 348
-// of loads a thread.)
-constexpr int LATE_THREADS = 1024;
+// One block of 24 warps per SM: the fewest arrivals at a grid barrier, with 80
+// registers a thread.  (The candidate evaluation and the replacement want more: 124
+// bytes of spill stores and 224 of loads a thread; with 32 warps of 64 registers 192
+// and 364.)  Whole calls with 1024, 768, 640 and 512 threads, in us: 256 cutouts of 40
+// to 200 pixels a side 316, 305, 296, 297; one 2048 x 2048 frame 377, 370, 363, 365;
+// five of 1018 x 1001 550, 540, 537, 535; 64 ragged frames of 256 to 4096 pixels a side
+// 2710, 2713, 2723, 2763; a 2048 x 2048 frame at thresholds of 1 and 0.5 3013, 3197, not
+// timed, 3819.
+constexpr int LATE_THREADS = 768;
 constexpr int LATE_WARPS = LATE_THREADS / 32;
 
 __device__ __forceinline__ int wrap_index(int i, int n)
@@ -289,9 +293,10 @@ __device__ __forceinline__ void late_neighbours(const FrameDesc *__restrict__ fr
 // words take 30 us whatever changed, and then four million pixels are classified.
 // Hence the rule: when the changed targets are over a 64th of the pixels and a
 // quarter of the mask.
-__device__ __forceinline__ bool late_by_rows(const Control *ctl, const PassLists &L)
+__device__ __forceinline__ bool late_by_rows(const Control *ctl, const PassLists &L, const RowItems &rows)
 {
-	return 64 * L.n_chg > ctl->cand_cap && 4 * L.n_chg > ctl->n_targets;
+	const unsigned long long n = L.n_chg;
+	return 64 * n > rows.px && 4 * n > ctl->n_targets;
 }
 
 // Columns 32 k - 6 .. 32 k + 37 of row y of a plane (bit 0: the first); zero
@@ -318,14 +323,13 @@ __device__ __forceinline__ unsigned long long window6(const uint32_t *plane, int
 }
 
 __device__ __forceinline__ void late_rows(const FrameDesc *__restrict__ frames, const FrameState *state,
-	const int2 *__restrict__ rows, int nrows, PassLists &L, int mode, uint2 *cands, uint2 *low, uint2 *eval,
-	Team team)
+	const RowItems &rows, PassLists &L, int mode, uint2 *cands, uint2 *low, uint2 *eval, Team team)
 {
 	const int lane = threadIdx.x & 31;
 	const int gw = (team.block * blockDim.x + threadIdx.x) >> 5, nw = (team.blocks * blockDim.x) >> 5;
 	auto wide2 = [](unsigned long long m) { return m | m << 1 | m >> 1 | m << 2 | m >> 2; };
-	for (int i = gw; i < nrows; i += nw) {
-		const int2 item = rows[i];
+	for (int i = gw; i < rows.n; i += nw) {
+		const int2 item = rows.rows[i];
 		if (!state[item.x].active)
 			continue; // warp-uniform
 		const FrameDesc &fd = frames[item.x];
@@ -561,7 +565,7 @@ __device__ __forceinline__ void late_classes(const FrameDesc *__restrict__ frame
 // the survivors of chunk k queued; it may take some.
 //
 // What is the same for the whole block stays in shared memory: the work holds
-// every register of a thread (64 at this block size), and what lives across it
+// every register of a thread (80 at this block size), and what lives across it
 // spills.
 struct LateQueue {
 	uint16_t e[LATE_THREADS];
@@ -659,7 +663,7 @@ __device__ __forceinline__ void late_grow(const FrameDesc *__restrict__ frames, 
 // Stage 4: the growth, and the low list's pixels near a CAND pixel, a warp each.
 __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, FrameState *state,
 	const uint2 *cands, const uint2 *low, const DetectParams &prm, const PassLists &L, Control *ctl, int par,
-	uint2 *targets, const int2 *rows, int nrows, LateQueue &Q, Team team, double *P, double *S)
+	uint2 *targets, const RowItems &rows, LateQueue &Q, Team team, double *P, double *S)
 {
 	block_sweep([&] { return (long long)L.n_low; }, Q, team, [&](unsigned e) {
 		const uint2 t = low[e];
@@ -670,8 +674,8 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 	}, [](int) {}, [&](unsigned e) {
 		low_eval<PATH_ANY>(frames, state, low[e], prm, ctl, par, targets, P, S, false);
 	}, [&] {
-		if (grows_by_rows(ctl, par))
-			grow_rows(frames, state, rows, nrows, true, ctl, par, targets, team);
+		if (grows_by_rows(L.n_cand, rows))
+			grow_rows(frames, state, rows, true, ctl, par, targets, team);
 		else
 			late_grow(frames, state, cands, L, ctl, par, targets, team);
 	});
@@ -684,9 +688,9 @@ __device__ __forceinline__ void late_low(const FrameDesc *__restrict__ frames, F
 // windows still hold none, the same window holds the same donors, and the same
 // median would come out.  A new target is itself a FRESH pixel.
 //
-// A block with LATE_BY_THREADS or more of a chunk's 1024 targets left gives them a
-// thread each first, as replace_targets does (at 64 registers a thread the 25 values
-// spill, and are still faster than a warp per target).
+// A block with LATE_BY_THREADS or more of a chunk's targets left (LATE_THREADS at
+// most) gives them a thread each first, as replace_targets does (the 25 values spill,
+// and are still faster than a warp per target).
 constexpr int LATE_BY_THREADS = 256;
 
 // (Called by the whole block; a function of its own, so that its registers are not
@@ -770,7 +774,7 @@ constexpr int LN_THREADS = 512;
 __global__ void __launch_bounds__(LN_THREADS, 3)
 late_neighbours_kernel(const FrameDesc *__restrict__ frames, const FrameState *state, DetectParams prm,
 	Control *ctl, uint2 *cands, uint2 *low, uint2 *eval, const uint2 *targets, const unsigned *chg,
-	const int2 *__restrict__ rows, int nrows, const FloorJob *__restrict__ jobs, int njobs)
+	RowItems rows, const FloorJob *__restrict__ jobs, int njobs)
 {
 	__shared__ ListSlots slots;
 	// The noise-model blocks' thresholds, for the long lists' LATE_TESTS (a
@@ -783,8 +787,8 @@ late_neighbours_kernel(const FrameDesc *__restrict__ frames, const FrameState *s
 			fd.floors[(jb.y0 >> 5) * ((fd.w + 31) >> 5) + (jb.x0 >> 5)].thr =
 				block_threshold(fd, jb.x0 >> 5, jb.y0 >> 5, prm.mode, tmin2);
 	}
-	if (late_by_rows(ctl, ctl->pass[1])) {
-		late_rows(frames, state, rows, nrows, ctl->pass[1], prm.mode, cands, low, eval, whole_grid());
+	if (late_by_rows(ctl, ctl->pass[1], rows)) {
+		late_rows(frames, state, rows, ctl->pass[1], prm.mode, cands, low, eval, whole_grid());
 		return;
 	}
 	late_neighbours<LN_THREADS / 32>(frames, targets, chg, ctl->pass[1], prm.mode, cands, low, eval, slots,
@@ -818,7 +822,7 @@ struct LateShared {
 __global__ void __launch_bounds__(LATE_THREADS, 1)
 late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int nf, DetectParams prm,
 	Control *ctl, int maxiter, uint2 *cands, uint2 *low, uint2 *eval, uint2 *targets, uint8_t *radius,
-	unsigned *chg, const int2 *__restrict__ rows, int nrows, BarrierWait bw)
+	unsigned *chg, RowItems rows, BarrierWait bw)
 {
 	extern __shared__ __align__(16) unsigned char late_smem[];
 	LateShared &S = *reinterpret_cast<LateShared *>(late_smem);
@@ -856,8 +860,8 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 		const int par = it & 1;
 		PassLists &L = ctl->pass[par], &next = ctl->pass[par ^ 1];
 		if (it > 1) {
-			if (late_by_rows(ctl, L))
-				late_rows(frames, state, rows, nrows, L, prm.mode, cands, low, eval, team);
+			if (late_by_rows(ctl, L, rows))
+				late_rows(frames, state, rows, L, prm.mode, cands, low, eval, team);
 			else
 				late_neighbours<LATE_WARPS>(frames, targets, chg, L, prm.mode, cands, low, eval, S.slots, team);
 			// The last growth's FRESH bits: its replacement is done.
@@ -890,7 +894,7 @@ late_passes_kernel(const FrameDesc *__restrict__ frames, FrameState *state, int 
 			if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 				return;
 		} while (it == 1 && barrier.calls * team.blocks < gridDim.x);
-		late_low(frames, state, cands, low, prm, L, ctl, par, targets, rows, nrows, S.Q, team, S.patches[warp],
+		late_low(frames, state, cands, low, prm, L, ctl, par, targets, rows, S.Q, team, S.patches[warp],
 			S.scratch[warp]);
 		if (!grid_barrier(ctl, barrier, state, nf, bw, team))
 			return;
