@@ -931,9 +931,9 @@ static void launch_late(Workspace &ws, const Layout &L, const DeviceInfo &di, cu
 	// The class of the noise-model frames' pixels near the first pass's
 	// targets: in parts with a thread per median above 8 Mpixel, a warp per median
 	// below.  All passes after the first with the parts and with warps, in us, by the
-	// batch's size: 2.3 Mpixel (256 frames of 40 to 200 a side) 188, 176; 4 177, 174; 8
-	// 195, 186; 12 207, 199; 16 214, 215; 24 227, 238; 32 249, 264; 64 336, 389; 128
-	// 524, 647.  Between 8 and 16 Mpixel the two are within 5%.
+	// batch's size: 2.3 Mpixel (256 frames of 40 to 200 a side) 180, 168; 4 173, 171; 8
+	// 191, 182; 12 201, 195; 16 209, 211; 24 223, 230; 32 244, 258; 64 355, 408; 128
+	// 531, 657.  Between 8 and 16 Mpixel the two are within 5%.
 	const bool model = L.error_frames < nf, thresholds = model && L.total_px > 8u << 20;
 	late_neighbours_kernel<<<std::min(wide, di.sms * 3), LN_THREADS, 0, s>>>(frames, state, prm, ctl, cands, low,
 		eval, targets, chg, rows, ws.jobs.p, thresholds ? (int)L.jobs.size() : 0);
